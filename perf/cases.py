@@ -2,7 +2,8 @@
 
 ``listed()`` holds the cases, ``draw(rng)`` gives another of the same ranges, ``prepare`` makes what a program has in
 hand before the call, ``run`` is one pass through the public operators, ``work`` the bytes and operations that the pass
-cannot do without and ``tolerance`` the error that another correct evaluation at the same precision shows.
+cannot do without, ``tolerance`` the error that another correct evaluation at the same precision shows and ``exact`` the
+outputs in 64 bits.
 """
 import math
 
@@ -167,3 +168,63 @@ def tolerance(case):
         return "exact"
     # neighbours: 1e-4 of the indices trade places with a neighbour whose distance agrees to float32 rounding
     return {"rel": _REL[kind], "differ": 5e-4} if kind == "neighbours" else {"rel": _REL[kind]}
+
+
+def _differences(x1, x2, grad, p, w):
+    """A batch's distances by direct differences, (sum w |x - y|^p)^(1/p), and their gradients; x1 a block of rows at a time."""
+    out, g1, g2 = x1.new_empty(x1.size(0), x2.size(0)), torch.empty_like(x1), torch.zeros_like(x2)
+    rows = max(1, (1 << 26) // (x2.size(0) * x2.size(1)))
+    for i in range(0, x1.size(0), rows):
+        at = slice(i, i + rows)
+        d = x1[at, None] - x2
+        if p == math.inf:
+            # a coordinate attains the maximum where its float32 difference does: that is what the inputs' type resolves
+            d = d.float().double()
+            out[at] = d.abs().amax(2)
+            t = torch.where(d.abs() == out[at, :, None], d.sign(), 0.0)
+            c = grad[at]
+        else:
+            t = d.sign() if p == 1 else d * d.abs() ** (p - 2) if p > 2 else d
+            t = t if w is None else t * w
+            out[at] = (t * d).sum(2) ** (1 / p)
+            c = grad[at] if p == 1 else grad[at] / out[at] ** (p - 1)
+        t = t * c[..., None]
+        g1[at] = t.sum(1)
+        g2 -= t.sum(0)
+    return out, g1, g2
+
+
+def exact(case, seed):
+    s = prepare(case, seed)
+    kind = case["kind"]
+    if kind == "boolean":
+        return None
+    x1, x2 = s["x1"].detach().double(), s["x2"].detach().double()
+    if kind == "sqeuclidean_dense":
+        out = torch.addmm(x1.square().sum(1)[:, None], x1, x2.T, alpha=-2)
+        return out.add_(x2.square().sum(1)).clamp_(min=0)
+    if kind == "neighbours":
+        best = []
+        for a in x1.split(8192):
+            d = torch.addmm(a.square().sum(1)[:, None], a, x2.T, alpha=-2).add_(x2.square().sum(1)).clamp_(min=0).sqrt_()
+            best.append(d.topk(case["k"], largest=False).values)
+        return None, torch.cat(best)
+    grad = s["grad"].double()
+    if kind == "hausdorff":
+        out, g1, g2 = torch.empty_like(grad), torch.zeros_like(x1), torch.zeros_like(x2)
+        for b in range(x1.size(0)):
+            nearest, at = sum((x1[b, 0, :, None, c] - x2[b, 0, None, :, c]).square() for c in range(x1.size(3))).min(1)
+            m = nearest.argmax()
+            out[b] = nearest[m].sqrt()
+            g = grad[b, 0, 0] * (x1[b, 0, m] - x2[b, 0, at[m]]) / out[b, 0, 0]
+            g1[b, 0, m], g2[b, 0, at[m]] = g, -g
+        return out, None, None, g1, g2
+    if kind == "cosine_bf16":
+        x1.requires_grad_(), x2.requires_grad_()
+        out = 1 - (x1 / x1.norm(dim=1, keepdim=True)) @ (x2 / x2.norm(dim=1, keepdim=True)).T
+        return out.detach(), *torch.autograd.grad(out, (x1, x2), grad)
+    p = {"manhattan": 1, "minkowski3": 3, "chebyshev": math.inf}.get(kind, 2)
+    w = 1 / s["V"] if kind == "seuclidean_f64" else None
+    if "b" not in case:
+        return _differences(x1, x2, grad, p, w)
+    return [torch.stack(v) for v in zip(*(_differences(x1[b], x2[b], grad[b], p, w) for b in range(case["b"])))]
