@@ -413,6 +413,20 @@ TPW_API int tpw_bool_metric_forward_tc(int metric, const uint8_t *x1, const uint
                                const int32_t *x1_popcount, const int32_t *x2_popcount, float *out,
                                int64_t B, int64_t N1, int64_t N2, int64_t D, tpw_stream_t stream);
 
+/*
+ * The same kernel for rows of any length.  tpw_bool_rows_pitch returns the bytes per row it reads (D rounded up to a
+ * multiple of 16), or 0 when tpw_bool_metric_forward is to be used; the sizes it serves are those of
+ * tpw_bool_metric_tc_eligible without the condition on D's divisibility.  tpw_bool_rows counts the rows of one-byte
+ * booleans src [rows,D] and, unless dst is NULL, writes them as 0 / 1 bytes padded with zeros to dst [rows,pitch] (16-byte
+ * aligned); dst may be NULL where D is a multiple of 16 and src is 16-byte aligned, and the rows are then used in place.
+ */
+TPW_API int64_t tpw_bool_rows_pitch(int64_t B, int64_t N1, int64_t N2, int64_t D);
+TPW_API int tpw_bool_rows(const uint8_t *src, uint8_t *dst, int32_t *row_popcount, int64_t rows, int64_t D, int64_t pitch,
+                  tpw_stream_t stream);
+TPW_API int tpw_bool_metric_forward_rows(int metric, const uint8_t *x1, const uint8_t *x2,
+                                 const int32_t *x1_popcount, const int32_t *x2_popcount, float *out,
+                                 int64_t B, int64_t N1, int64_t N2, int64_t D, int64_t pitch, tpw_stream_t stream);
+
 enum tpw_cmp_op { TPW_CMP_EQ = 0, TPW_CMP_NE = 1 };
 enum tpw_cmp_reduction { TPW_RED_SUM = 0, TPW_RED_MEAN = 1 };
 

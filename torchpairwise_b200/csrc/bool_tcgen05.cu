@@ -12,13 +12,15 @@
 // (warp - 2) / 4).  Output tile 128 x 256; a k-step is 128 features = one 128-byte swizzled row per operand row,
 // consumed by four MMAs of K = 32; three stages of 16 KB (x1) + 32 KB (x2); two 256-column accumulators in tensor
 // memory, so the epilogue of tile t overlaps the MMAs of tile t + 1.  The operands are the caller's boolean
-// matrices as they lie in memory (row pitch D bytes): no packed or padded copy is made, the TMA unit zero-fills
-// rows and features past the edge, and zeros add nothing to a count.  Every CTA loads its own tiles with plain
-// per-CTA TMA loads from this GPU's memory.
+// matrices as they lie in memory when their rows start on 16-byte boundaries, else copies with the rows padded by zeros
+// to a multiple of 16 bytes (bool_rows_kernel, which also counts the rows); the TMA unit zero-fills rows and features
+// past the edge, and zeros add nothing to a count.  Every CTA loads its own tiles with plain per-CTA TMA loads from
+// this GPU's memory.
 //
 // An epilogue warp stages its 32 x 32 block of results in shared memory (128-byte swizzle) and writes it out either
 // with its own 128-bit stores or, for the metrics whose arithmetic is long enough to hide it, by handing the block to
-// the copy engine (a TMA store on the output's tensor map, which also clips the rows past N1).
+// the copy engine (a TMA store on the output's tensor map, which also clips the rows past N1).  Where N2 is no multiple
+// of 4 the staged block is written one 128-byte row segment per instruction, lane l its word l.
 //
 // Every mbarrier wait is bounded; a role that gives up raises a CTA-wide abort flag, everybody falls through to the
 // final barrier, tensor memory is released and the device status word reports the site.  The one wait without a
@@ -80,6 +82,40 @@ __device__ __forceinline__ void tc_mma_i8(uint32_t tmem_d, uint64_t adesc, uint6
 // [10,13) = 0), both K-major (bits 15 and 16 = 0), N >> 3 in bits [17,23), M >> 4 in bits [24,29); dense, no saturation.
 __device__ __forceinline__ uint32_t make_idesc_i8(int M, int N) {
     return (2u << 4) | ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
+}
+
+// Row counts of one-byte booleans and, when dst is given, the rows as 0 / 1 bytes padded with zeros to `pitch` bytes.  One
+// warp per row; reads the rows once, which is the bound (the bit-packing pass it replaces in front of this kernel read
+// one byte per lane: 81920 x 1024 bytes 73 -> 30 us).  VEC: rows start on 16-byte boundaries and D is a multiple of 16.
+template <bool VEC>
+__global__ void __launch_bounds__(256)
+bool_rows_kernel(const uint8_t *__restrict__ src, uint8_t *__restrict__ dst, int32_t *__restrict__ row_pop, long long rows,
+                 long long D, long long pitch) {
+    const int lane = threadIdx.x & 31;
+    const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+    for (long long row = warp; row < rows; row += nwarps) {
+        const uint8_t *s = src + row * D;
+        int pop = 0;
+        if (VEC) {
+            for (long long k = lane * 16; k < D; k += 512) {
+                const uint4 v = __ldg(reinterpret_cast<const uint4 *>(s + k));
+                pop += __popc(__vcmpne4(v.x, 0u) & 0x01010101u) + __popc(__vcmpne4(v.y, 0u) & 0x01010101u) +
+                       __popc(__vcmpne4(v.z, 0u) & 0x01010101u) + __popc(__vcmpne4(v.w, 0u) & 0x01010101u);
+            }
+        } else {
+            for (long long k = lane * 4; k < pitch; k += 128) {
+                uint32_t w = 0;
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (k + e < D && s[k + e] != 0) w |= 1u << (8 * e);
+                pop += __popc(w);
+                *reinterpret_cast<uint32_t *>(dst + row * pitch + k) = w;
+            }
+        }
+        pop = __reduce_add_sync(0xffffffffu, pop);
+        if (lane == 0) row_pop[row] = pop;
+    }
 }
 
 // One instantiation per metric: with the metric a compile-time constant the epilogue's switch folds to the one case,
@@ -171,9 +207,12 @@ bool_count_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
                     tc_fence_after();
                     const uint32_t sb = smem_u32(smem + s * STAGE_BYTES);
                     const uint64_t dx = make_smem_desc(sb), dy = make_smem_desc(sb + A_BYTES);
-                    // one MMA consumes 32 bytes of the swizzled row: the start address advances by 2 units of 16 bytes
+                    // one MMA consumes 32 bytes of the swizzled row: the start address advances by 2 units of 16 bytes; the
+                    // last k-step leaves out the MMAs that would only see zero fill
+                    const int kmma = kb + 1 < nkb ? BKB / 32 : (int)((P.D - (long long)kb * BKB + 31) / 32);
 #pragma unroll
-                    for (int k = 0; k < BKB / 32; ++k) tc_mma_i8(d_tmem, dx + 2 * k, dy + 2 * k, idesc, (kb | k) != 0);
+                    for (int k = 0; k < BKB / 32; ++k)
+                        if (k < kmma) tc_mma_i8(d_tmem, dx + 2 * k, dy + 2 * k, idesc, (kb | k) != 0);
                     tc_commit(&empty[s]);   // the stage may be refilled once these MMAs have read it
                 }
                 if (ok) tc_commit(&tmem_full[a]);
@@ -220,7 +259,6 @@ bool_count_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
                 break;
             }
             tc_fence_after();
-            float *orow = P.out + (b * P.N1 + (row_ok ? i : 0)) * P.N2;
             const long long row_base = tm * BM + q * 32;
             // the mean metrics multiply by 1 / D where D is a power of two and divide otherwise: decided here, once per
             // tile, so that the per-element code holds one of the two
@@ -233,8 +271,9 @@ bool_count_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
                 tmem_ld_wait();
                 const long long j0 = tn * BN + c * 32;
                 if (j0 >= P.N2) continue;
-                if (P.vec_store && j0 + 32 <= P.N2) {
-                    // this thread's row ...
+                const bool whole = P.vec_store && j0 + 32 <= P.N2;
+                {
+                    // this thread's row (past N2 the counts are zero and nothing is stored) ...
                     float4 o[8];
 #pragma unroll
                     for (int v = 0; v < 8; ++v) {
@@ -252,7 +291,7 @@ bool_count_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
                     // ... staged with a 16-byte-chunk XOR swizzle ...
 #pragma unroll
                     for (int v = 0; v < 8; ++v) *reinterpret_cast<float4 *>(stg + lane * 128 + ((v ^ (lane & 7)) << 4)) = o[v];
-                    if (P.tma_store) {
+                    if (whole && P.tma_store) {
                         // ... which is the layout of a 128-byte swizzled 32 x 32 box: one lane hands the block to the copy
                         // engine (rows past N1 are clipped by the tensor map) and the warp goes on to its next block
                         fence_proxy_async_smem();
@@ -261,7 +300,7 @@ bool_count_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
                             tma_store_3d(&map_out, stg, (int)j0, (int)row_base, (int)b);
                             tma_store_commit();
                         }
-                    } else {
+                    } else if (whole) {
                         __syncwarp();
                         // ... and written out four full 128-byte row segments per instruction
 #pragma unroll
@@ -272,12 +311,17 @@ bool_count_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
                                 __stcs(reinterpret_cast<float4 *>(P.out + (b * P.N1 + row_base + rr) * P.N2 + j0) + cc, o);
                         }
                         __syncwarp();
-                    }
-                } else if (row_ok) {
-#pragma unroll
-                    for (int v = 0; v < 32; ++v) {
-                        const long long j = j0 + v;
-                        if (j < P.N2) orow[j] = bool_epilogue<true, INV>(METRIC, (int)r[v], pa, popw[(c - cpart * NCB) * 32 + v], D, P.inv_d);
+                    } else {
+                        __syncwarp();
+                        // ... and written out one row segment of up to 32 words per instruction
+                        const int rows = P.N1 - row_base < 32 ? (int)(P.N1 - row_base) : 32;
+                        float *op = P.out + (b * P.N1 + row_base) * P.N2 + j0 + lane;
+                        if (j0 + lane < P.N2) {
+#pragma unroll 8
+                            for (int rr = 0; rr < rows; ++rr)
+                                op[rr * P.N2] = *reinterpret_cast<const float *>(stg + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) + (lane & 3) * 4);
+                        }
+                        __syncwarp();
                     }
                 }
             }
@@ -309,26 +353,62 @@ bool_count_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
 
 using namespace tpw;
 
+static bool tc_serves(int64_t B, int64_t N1, int64_t N2, int64_t D) {
+    if (getenv("TPW_DISABLE_BOOL_TC")) return false;
+    // up to 128 features the few-words popcount kernel is faster; the epilogue converts counts below 2^23 exactly with
+    // one logic operation and one addition instead of the quarter-rate conversion instruction
+    if (B <= 0 || N1 < BM || N2 < BN || D <= 128 || D >= (1 << 23)) return false;
+    if (N1 >= (1ll << 31) || N2 >= (1ll << 31) || B >= (1ll << 31)) return false;
+    return (double)B * (double)N1 * (double)N2 * (double)D >= 268435456.0;
+}
+
 // 1 when tpw_bool_metric_forward_tc serves this problem: rows of at least 128 bytes whose pitch keeps every row
 // 16-byte aligned (a TMA requirement), counts that stay exact, and enough pairs to fill the persistent grid.
 extern "C" int tpw_bool_metric_tc_eligible(int64_t B, int64_t N1, int64_t N2, int64_t D) {
-    if (getenv("TPW_DISABLE_BOOL_TC")) return 0;
-    // up to 128 features the few-words popcount kernel is faster; the epilogue converts counts below 2^23 exactly with
-    // one logic operation and one addition instead of the quarter-rate conversion instruction
-    if (B <= 0 || N1 < BM || N2 < BN || D <= 128 || D % 16 != 0 || D >= (1 << 23)) return 0;
-    if (N1 >= (1ll << 31) || N2 >= (1ll << 31) || B >= (1ll << 31)) return 0;
-    return (double)B * (double)N1 * (double)N2 * (double)D >= 268435456.0 ? 1 : 0;
+    return D % 16 == 0 && tc_serves(B, N1, N2, D) ? 1 : 0;
+}
+
+// Any other row length of those problems goes the same way on padded rows.  The padded copy costs two passes over the
+// operands, (N1 + N2) D bytes, against B N1 N2 outputs of at least 4 bytes each; the popcount tile, the other route, is
+// several times slower wherever this one applies: hamming [30011, 10007, 167] 2.01 -> 0.55 ms.
+extern "C" int64_t tpw_bool_rows_pitch(int64_t B, int64_t N1, int64_t N2, int64_t D) {
+    return tc_serves(B, N1, N2, D) ? (D + 15) / 16 * 16 : 0;
+}
+
+extern "C" int tpw_bool_rows(const uint8_t *src, uint8_t *dst, int32_t *row_popcount, int64_t rows, int64_t D, int64_t pitch,
+                             tpw_stream_t stream) {
+    clear_error();
+    TPW_CHECK_ARG(rows >= 0 && D > 0, "tpw_bool_rows: negative size");
+    if (rows == 0) return TPW_OK;
+    TPW_CHECK_ARG(src && row_popcount, "tpw_bool_rows: NULL pointer");
+    TPW_CHECK_ARG(dst ? pitch >= D && pitch % 16 == 0 && aligned16(dst) : D % 16 == 0 && aligned16(src),
+                  "tpw_bool_rows: padded rows need a 16-byte aligned copy and a pitch that is a multiple of 16, rows used in place "
+                  "have to be 16-byte aligned themselves");
+    long long blocks = (rows + 7) / 8;
+    const long long cap = (long long)sm_count() * 16;
+    if (blocks > cap) blocks = cap;
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    if (dst) bool_rows_kernel<false><<<(unsigned)blocks, 256, 0, s>>>(src, dst, row_popcount, rows, D, pitch);
+    else bool_rows_kernel<true><<<(unsigned)blocks, 256, 0, s>>>(src, nullptr, row_popcount, rows, D, D);
+    TPW_LAUNCH_OK("bool_rows_kernel");
+    return TPW_OK;
 }
 
 extern "C" int tpw_bool_metric_forward_tc(int metric, const uint8_t *x1, const uint8_t *x2,
                                           const int32_t *x1_popcount, const int32_t *x2_popcount, float *out,
                                           int64_t B, int64_t N1, int64_t N2, int64_t D, tpw_stream_t stream) {
+    return tpw_bool_metric_forward_rows(metric, x1, x2, x1_popcount, x2_popcount, out, B, N1, N2, D, D, stream);
+}
+
+extern "C" int tpw_bool_metric_forward_rows(int metric, const uint8_t *x1, const uint8_t *x2,
+                                            const int32_t *x1_popcount, const int32_t *x2_popcount, float *out,
+                                            int64_t B, int64_t N1, int64_t N2, int64_t D, int64_t pitch, tpw_stream_t stream) {
     clear_error();
     TPW_CHECK_ARG(metric >= 0 && metric < TPW_BOOL_METRIC_COUNT, "tpw_bool_metric_forward_tc: unknown metric %d", metric);
     TPW_CHECK_ARG(B >= 0 && N1 >= 0 && N2 >= 0 && D >= 0, "tpw_bool_metric_forward_tc: negative size");
     if (B == 0 || N1 == 0 || N2 == 0) return TPW_OK;
     TPW_CHECK_ARG(D > 0 && D < (1 << 23), "tpw_bool_metric_forward_tc: D must be in [1, 2^23) (exact float32 counts)");
-    TPW_CHECK_ARG(D % 16 == 0, "tpw_bool_metric_forward_tc: D must be a multiple of 16 (row pitch in bytes); use tpw_bool_metric_forward");
+    TPW_CHECK_ARG(pitch >= D && pitch % 16 == 0, "tpw_bool_metric_forward_tc: D (the row pitch in bytes) must be a multiple of 16; use tpw_bool_metric_forward or padded rows");
     TPW_CHECK_ARG(x1 && x2 && x1_popcount && x2_popcount && out, "tpw_bool_metric_forward_tc: NULL pointer");
     TPW_CHECK_ARG(aligned16(x1) && aligned16(x2), "tpw_bool_metric_forward_tc: the boolean matrices must be 16-byte aligned");
     TPW_CHECK_ARG(N1 < (1ll << 31) && N2 < (1ll << 31) && B < (1ll << 31), "tpw_bool_metric_forward_tc: a dimension exceeds 2^31-1");
@@ -344,9 +424,9 @@ extern "C" int tpw_bool_metric_forward_tc(int metric, const uint8_t *x1, const u
     P.tiles = B * P.tiles_m * P.tiles_n;
     P.status = device_status_ptr();
     CUtensorMap mx, my;
-    int st = make_tensor_map_3d(&mx, x1, 1, D, N1, B, BKB, BM, true);
+    int st = make_tensor_map_3d(&mx, x1, 1, pitch, N1, B, BKB, BM, true);
     if (st != TPW_OK) return st;
-    st = make_tensor_map_3d(&my, x2, 1, D, N2, B, BKB, BN, true);
+    st = make_tensor_map_3d(&my, x2, 1, pitch, N2, B, BKB, BN, true);
     if (st != TPW_OK) return st;
     CUtensorMap mo;
     memset(&mo, 0, sizeof(mo));

@@ -641,6 +641,17 @@ std::tuple<Tensor, Tensor, int64_t> pack_bool(const Tensor &xb) {
     return {words, pops, W};
 }
 
+// rows for the tensor-core counts: in place where they start on 16-byte boundaries, else padded; and their counts
+std::pair<Tensor, Tensor> bool_rows(const Tensor &xb, int64_t pitch) {
+    const int64_t B = xb.size(0), N = xb.size(1), D = xb.size(2);
+    Tensor src = xb.contiguous(), pops = at::empty({B, N}, xb.options().dtype(at::kInt)), rows = src;
+    const bool in_place = pitch == D && reinterpret_cast<uintptr_t>(src.data_ptr()) % 16 == 0;
+    if (!in_place) rows = at::empty({B, N, pitch}, xb.options());
+    TPW_CALL(tpw_bool_rows(static_cast<const uint8_t *>(src.data_ptr()), in_place ? nullptr : static_cast<uint8_t *>(rows.data_ptr()),
+                           static_cast<int32_t *>(pops.data_ptr()), B * N, D, pitch, stream_of(xb)));
+    return {rows, pops};
+}
+
 Tensor bool_metric(const Tensor &x1, const Tensor &x2, int metric) {
     require_cuda(x1);
     require_cuda(x2);
@@ -657,22 +668,24 @@ Tensor bool_metric(const Tensor &x1, const Tensor &x2, int metric) {
         out.fill_(metric <= TPW_BOOL_NE_SUM || metric == TPW_BOOL_JACCARD || metric == TPW_BOOL_YULE
                       ? 0.0 : std::numeric_limits<double>::quiet_NaN());
     } else if (out.numel() > 0) {
-        auto pa = pack_bool(a);
-        auto pb = x2.is_same(x1) ? pa : pack_bool(b);
-        Tensor ab = a.contiguous(), bb = x2.is_same(x1) ? ab : b.contiguous();
-        if (tpw_bool_metric_tc_eligible(B, N1, N2, D) && reinterpret_cast<uintptr_t>(ab.data_ptr()) % 16 == 0 &&
-            reinterpret_cast<uintptr_t>(bb.data_ptr()) % 16 == 0) {
+        const bool same = x2.is_same(x1);
+        if (const int64_t pitch = tpw_bool_rows_pitch(B, N1, N2, D)) {
             // large problem: the counts come from the tensor cores (8-bit integer contraction of the 0 / 1 bytes)
-            TPW_CALL(tpw_bool_metric_forward_tc(metric, static_cast<const uint8_t *>(ab.data_ptr()), static_cast<const uint8_t *>(bb.data_ptr()),
-                                                static_cast<const int32_t *>(std::get<1>(pa).data_ptr()),
-                                                static_cast<const int32_t *>(std::get<1>(pb).data_ptr()), out.data_ptr<float>(),
-                                                B, N1, N2, D, stream_of(a)));
-        } else
-        TPW_CALL(tpw_bool_metric_forward(metric, static_cast<const uint32_t *>(std::get<0>(pa).data_ptr()),
-                                         static_cast<const uint32_t *>(std::get<0>(pb).data_ptr()),
-                                         static_cast<const int32_t *>(std::get<1>(pa).data_ptr()),
-                                         static_cast<const int32_t *>(std::get<1>(pb).data_ptr()), out.data_ptr<float>(),
-                                         B, N1, N2, D, std::get<2>(pa), stream_of(a)));
+            auto ra = bool_rows(a, pitch), rb = same ? ra : bool_rows(b, pitch);
+            TPW_CALL(tpw_bool_metric_forward_rows(metric, static_cast<const uint8_t *>(ra.first.data_ptr()),
+                                                  static_cast<const uint8_t *>(rb.first.data_ptr()),
+                                                  static_cast<const int32_t *>(ra.second.data_ptr()),
+                                                  static_cast<const int32_t *>(rb.second.data_ptr()), out.data_ptr<float>(),
+                                                  B, N1, N2, D, pitch, stream_of(a)));
+        } else {
+            auto pa = pack_bool(a);
+            auto pb = same ? pa : pack_bool(b);
+            TPW_CALL(tpw_bool_metric_forward(metric, static_cast<const uint32_t *>(std::get<0>(pa).data_ptr()),
+                                             static_cast<const uint32_t *>(std::get<0>(pb).data_ptr()),
+                                             static_cast<const int32_t *>(std::get<1>(pa).data_ptr()),
+                                             static_cast<const int32_t *>(std::get<1>(pb).data_ptr()), out.data_ptr<float>(),
+                                             B, N1, N2, D, std::get<2>(pa), stream_of(a)));
+        }
     }
     return ub ? out.squeeze(0) : out;
 }

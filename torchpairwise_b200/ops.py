@@ -641,6 +641,18 @@ def _pack_bool(xb: Tensor):
     return words, pops, W
 
 
+def _bool_rows(xb: Tensor, pitch: int):
+    """Rows for the tensor-core counts, in place where they start on 16-byte boundaries, else padded; and their counts."""
+    B, N, D = xb.shape
+    src = xb.contiguous().view(torch.uint8)
+    pops = torch.empty((B, N), dtype=torch.int32, device=xb.device)
+    in_place = pitch == D and src.data_ptr() % 16 == 0
+    rows = src if in_place else torch.empty((B, N, pitch), dtype=torch.uint8, device=xb.device)
+    with torch.cuda.device(xb.device):
+        check(lib.tpw_bool_rows(_ptr(src), None if in_place else _ptr(rows), _ptr(pops), B * N, D, pitch, _stream(xb)), "tpw_bool_rows")
+    return rows, pops
+
+
 def _bool_metric_raw(x1: Tensor, x2: Tensor, metric: str) -> Tensor:
     """x1, x2 boolean, 2-D or 3-D; float32 result."""
     _require_cuda(x1, x2)
@@ -663,19 +675,19 @@ def _bool_metric_raw(x1: Tensor, x2: Tensor, metric: str) -> Tensor:
                       "rogerstanimoto", "sokalmichener", "sokalsneath"):
             out.fill_(float("nan"))
     elif out.numel() > 0:
-        w1, p1, W = _pack_bool(x1c)
-        if x2c is x1c or (x2c.data_ptr() == x1c.data_ptr() and x2c.shape == x1c.shape):
-            w2, p2 = w1, p1
+        same = x2c is x1c or (x2c.data_ptr() == x1c.data_ptr() and x2c.shape == x1c.shape)
+        pitch = lib.tpw_bool_rows_pitch(B, N1, N2, D)
+        if pitch > 0:
+            # large problem: the counts come from the tensor cores (8-bit integer contraction of the 0 / 1 bytes)
+            b1, p1 = _bool_rows(x1c, pitch)
+            b2, p2 = (b1, p1) if same else _bool_rows(x2c, pitch)
+            with torch.cuda.device(x1.device):
+                check(lib.tpw_bool_metric_forward_rows(_abi.BOOL_METRICS[metric], _ptr(b1), _ptr(b2), _ptr(p1), _ptr(p2),
+                                                       _ptr(out), B, N1, N2, D, pitch, _stream(x1)), "tpw_bool_metric_forward_rows")
         else:
-            w2, p2, _ = _pack_bool(x2c)
-        with torch.cuda.device(x1.device):
-            b1 = x1c.contiguous().view(torch.uint8)
-            b2 = b1 if w2 is w1 else x2c.contiguous().view(torch.uint8)
-            if lib.tpw_bool_metric_tc_eligible(B, N1, N2, D) and b1.data_ptr() % 16 == 0 and b2.data_ptr() % 16 == 0:
-                # large problem: the counts come from the tensor cores (8-bit integer contraction of the 0 / 1 bytes)
-                check(lib.tpw_bool_metric_forward_tc(_abi.BOOL_METRICS[metric], _ptr(b1), _ptr(b2), _ptr(p1), _ptr(p2),
-                                                     _ptr(out), B, N1, N2, D, _stream(x1)), "tpw_bool_metric_forward_tc")
-            else:
+            w1, p1, W = _pack_bool(x1c)
+            w2, p2, _ = (w1, p1, W) if same else _pack_bool(x2c)
+            with torch.cuda.device(x1.device):
                 check(lib.tpw_bool_metric_forward(_abi.BOOL_METRICS[metric], _ptr(w1), _ptr(w2), _ptr(p1), _ptr(p2),
                                                   _ptr(out), B, N1, N2, D, W, _stream(x1)), "tpw_bool_metric_forward")
     return out.squeeze(0) if unbatched else out
