@@ -186,10 +186,11 @@ TPW_API int tpw_lp_backward(int dtype, int mode, const void *grad, const void *a
  * second kernel: no atomics, fixed summation order, bit-reproducible; the order differs from
  * tpw_lp_backward's, so the two agree to rounding, not bit for bit.
  * tpw_lp_backward_scratch_bytes() returns 0 where the kernel does not apply (float64, p = +inf, the
- * plain contraction, fewer than 256 rows of x1, N2 or D not a multiple of 4, small problems,
- * TPW_DISABLE_ONEPASS_BWD=1), else the scratch it wants: B * ceil(N1/256) * N2 * D * 4 bytes up to
+ * plain contraction, fewer than 256 rows of x1, D not a multiple of 4, small problems,
+ * TPW_DISABLE_ONEPASS_BWD=1), else the scratch it wants: B * (N1 + ceil(N1/256) * D) * N2 * 4 bytes (the
+ * coefficients of all pairs, transposed, and the block sums; N1 rounded up to a multiple of 4) up to
  * 2 GiB (larger problems run as several launches over batch or row-block ranges).  With scratch ==
- * NULL, less than N2 * D * 4 bytes, a NULL gradient pointer or a pointer that is not 16-byte aligned the
+ * NULL, less than one row block needs, (256 + D) * N2 * 4 bytes, a NULL gradient pointer or a pointer that is not 16-byte aligned the
  * call is tpw_lp_backward.  Replaces the same reference kernels as tpw_lp_backward
  * (OPS/cuda/ppminkowski_kernel.cu:133-218, OPS/cuda/wminkowski_kernel.cu:146-196, ATen's cdist backward).
  */

@@ -1,0 +1,89 @@
+"""Edges of the kernels' tiles and of the rules that choose between them, each against the other route."""
+import math
+
+import pytest
+import torch
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def tpw():
+    if not torch.cuda.is_available():
+        pytest.skip("needs a CUDA device")
+    import torchpairwise_b200
+    return torchpairwise_b200
+
+
+@pytest.mark.parametrize("shape", [(1, 1030, 2051, 167), (1, 2048, 1025, 129), (2, 900, 1111, 255), (1, 1200, 1604, 1000), (1, 5000, 260, 257)])
+def test_boolean_rows_of_any_length_equal_popcount(tpw, monkeypatch, shape):
+    """Rows that fill no whole 16 bytes go to the tensor-core counts as padded copies, results of ragged rows leave word by
+    word: every metric's float32 bits are those of the popcount kernels."""
+    from torchpairwise_b200 import _abi
+    b, n1, n2, d = shape
+    g = torch.Generator().manual_seed(d)
+    x1, x2 = (torch.rand(b, n1, d, generator=g) < 0.3).cuda(), (torch.rand(b, n2, d, generator=g) < 0.3).cuda()
+    x1[0, 3], x2[0, 5] = False, False            # empty rows: 0 / 0 in the metrics that divide
+    assert _abi.lib.tpw_bool_rows_pitch(b, n1, n2, d) == (d + 15) // 16 * 16
+    for metric in ("hamming", "jaccard", "yule", "russellrao"):
+        fn = getattr(tpw, metric + "_distances")
+        got = fn(x1, x2)
+        monkeypatch.setenv("TPW_DISABLE_BOOL_TC", "1")
+        want = fn(x1, x2)
+        monkeypatch.delenv("TPW_DISABLE_BOOL_TC")
+        assert torch.equal(got.view(torch.int32), want.view(torch.int32)), (metric, shape)
+    # any non-zero byte counts as true in a padded copy, as it does when the rows are packed to bits
+    y = (torch.randint(0, 3, (n1, d), generator=g, dtype=torch.uint8)).cuda()
+    torch.testing.assert_close(tpw.hamming_distances(y.view(torch.bool), x2[0]), tpw.hamming_distances(y != 0, x2[0]), rtol=0, atol=0)
+
+
+@pytest.mark.parametrize("m1,m2,d", [(700, 1031, 3), (513, 2, 3), (1, 4097, 2), (1025, 1, 5), (600, 777, 8), (257, 1500, 16)])
+def test_hausdorff_point_pairs_and_split_walks(tpw, monkeypatch, m1, m2, d):
+    """Odd clouds (a lone last point), clouds shared by several CTAs, one to sixteen coordinates, NaN and infinite
+    coordinates: values and indices of the exact loop."""
+    g = torch.Generator().manual_seed(m1 + m2 + d)
+    x1, x2 = torch.randn(2, 1, m1, d, generator=g), torch.randn(2, 1, m2, d, generator=g)
+    x1[1, 0, m1 // 2, 0] = math.inf
+    x2[1, 0, m2 // 2, d - 1] = math.nan
+    got = tpw.directed_hausdorff_distances(x1.cuda(), x2.cuda())
+    monkeypatch.setenv("TPW_HAUSDORFF_EXACT_LOOP", "1")
+    want = tpw.directed_hausdorff_distances(x1.cuda(), x2.cuda())
+    for a, w in zip(got, want):
+        assert torch.equal(a, w)
+
+
+@pytest.mark.parametrize("n2,d", [(1029, 320), (2047, 130), (258, 1030)])
+@pytest.mark.parametrize("fn", ["sqeuclidean_distances", "cosine_distances"])
+def test_tensor_core_matrix_with_ragged_rows(tpw, n2, d, fn):
+    """Rows of the result that start on no 16-byte boundary leave the staged block word by word; an element does not depend on
+    the other columns, so the bits are those of the same columns of a wider matrix."""
+    g = torch.Generator().manual_seed(n2)
+    x1, x2 = torch.randn(1100, d, generator=g).cuda(), torch.randn((n2 + 3) // 4 * 4, d, generator=g).cuda()
+    wide = getattr(tpw, fn)(x1, x2)
+    assert torch.equal(getattr(tpw, fn)(x1, x2[:n2]), wide[:, :n2])
+
+
+@pytest.mark.parametrize("shape,p", [((8, 700, 301, 192), 3.0), ((3, 1000, 1035, 128), 1.0), ((20, 500, 45, 256), 2.5)])
+def test_one_pass_backward_with_ragged_columns(tpw, shape, p):
+    """x2 row counts that are no multiple of 4 take the one-pass backward as well; against the two-launch form, whose terms are
+    the same in another order of addition (sums of up to 1035 float32 terms), and bit-reproducible."""
+    from torchpairwise_b200 import _abi
+    b, n1, n2, d = shape
+    g = torch.Generator().manual_seed(n2)
+    x1, x2 = torch.randn(b, n1, d, generator=g).cuda(), torch.randn(b, n2, d, generator=g).cuda()
+    gr = torch.randn(b, n1, n2, generator=g).cuda()
+    out = tpw.minkowski_distances(x1, x2, p)
+    lib, stream = _abi.lib, torch.cuda.current_stream().cuda_stream
+    want = lib.tpw_lp_backward_scratch_bytes(_abi.F32, _abi.LP_BWD_CDIST, b, n1, n2, d, p)
+    assert want > 0
+    res = []
+    for scratch in (torch.empty(want, dtype=torch.uint8, device="cuda"), torch.empty(want, dtype=torch.uint8, device="cuda"), None):
+        g1, g2 = torch.full_like(x1, math.nan), torch.full_like(x2, math.nan)
+        _abi.check(lib.tpw_lp_backward_ws(_abi.F32, _abi.LP_BWD_CDIST, gr.data_ptr(), out.data_ptr(), x1.data_ptr(), x2.data_ptr(), None,
+                                          g1.data_ptr(), g2.data_ptr(), b, n1, n2, d, p, None if scratch is None else scratch.data_ptr(),
+                                          0 if scratch is None else want, stream))
+        assert _abi.device_status(stream) == 0
+        res.append((g1, g2))
+    for one, again, two in zip(*res):
+        assert torch.equal(one, again)
+        assert float((one - two).abs().max()) <= 2e-5 * float(two.abs().max())   # sqrt(1035) * 2^-24 per sum, ten times over

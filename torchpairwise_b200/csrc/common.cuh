@@ -75,6 +75,7 @@ int lp_small_d_rowmin(const void *x1, const void *x2, unsigned long long *keys, 
 // lp_backward_onepass.cu: both gradients of an L_p reduction from one walk over the pairs (float32).  The query
 // returns 0 where that kernel does not apply.
 long long lp_backward_onepass_scratch_bytes(int mode, long long B, long long N1, long long N2, long long D, double p);
+long long lp_backward_onepass_min_bytes(long long N1, long long N2, long long D);
 int lp_backward_onepass(int mode, const void *grad, const void *aux, const void *x1, const void *x2, const void *w,
                         void *grad_x1, void *grad_x2, long long B, long long N1, long long N2, long long D, double p,
                         void *scratch, long long scratch_bytes, cudaStream_t stream);

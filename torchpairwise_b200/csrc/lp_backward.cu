@@ -579,7 +579,7 @@ extern "C" int tpw_lp_backward_ws(int dtype, int mode, const void *grad, const v
     const int64_t want = dtype == TPW_F32 && B >= 0 && N1 >= 0 && N2 >= 0 && D >= 0 && !isnan(p)
                              ? lp_backward_onepass_scratch_bytes(mode, B, N1, N2, D, p) : 0;
     const bool needs_aux = (mode == TPW_LP_BWD_WMINKOWSKI) || (mode == TPW_LP_BWD_CDIST && p != 1.0);
-    const bool usable = want > 0 && scratch != nullptr && scratch_bytes >= N2 * D * 4 && grad_x1 && grad_x2 && grad && x1 && x2 &&
+    const bool usable = want > 0 && scratch != nullptr && scratch_bytes >= lp_backward_onepass_min_bytes(N1, N2, D) && grad_x1 && grad_x2 && grad && x1 && x2 &&
                         (!needs_aux || aux) && (mode != TPW_LP_BWD_WMINKOWSKI || w) &&
                         aligned16(grad) && aligned16(x1) && aligned16(x2) && aligned16(grad_x1) && aligned16(grad_x2) &&
                         aligned16(scratch) && (!needs_aux || aligned16(aux)) && (!w || aligned16(w));
