@@ -449,24 +449,31 @@ struct WMinkowskiFn : torch::autograd::Function<WMinkowskiFn> {
         ctx->saved_data["dt"] = static_cast<int64_t>(in_dt);
         return finish(out, q.unbatched, in_dt);
     }
+    // need_w = false: the weights' gradient, a pass over all pairs of its own, is left out (undefined)
     static std::tuple<Tensor, Tensor, Tensor> raw_backward(const Tensor &grad, const Tensor &a, const Tensor &b, const Tensor &w,
-                                                           double p, bool ub) {
+                                                           double p, bool ub, bool need_w = true) {
         c10::cuda::CUDAGuard dg(a.device());
         Tensor g = grad.to(a.scalar_type()).contiguous();
         if (ub) g = g.unsqueeze(0);
-        Tensor g1 = at::zeros_like(a), g2 = at::zeros_like(b), gw = at::zeros_like(w);
         const int64_t B = a.size(0), N1 = a.size(1), N2 = b.size(1), D = a.size(2);
-        if (p != 0 && B * N1 * N2 * D > 0) {
+        // the finite-p kernels write every element, the p = inf kernel adds into zeros
+        const bool work = p != 0 && B * N1 * N2 * D > 0;
+        auto make = [&](const Tensor &t) { return work && !std::isinf(p) ? at::empty_like(t) : at::zeros_like(t); };
+        Tensor g1 = make(a), g2 = make(b), gw;
+        if (need_w) gw = make(w);
+        if (work) {
             if (std::isinf(p)) {
                 TPW_CALL(tpw_lp_inf_backward(code_of(a), g.data_ptr(), a.data_ptr(), b.data_ptr(), w.data_ptr(), g1.data_ptr(),
-                                             g2.data_ptr(), gw.data_ptr(), B, N1, N2, D, p < 0, stream_of(a)));
+                                             g2.data_ptr(), need_w ? gw.data_ptr() : nullptr, B, N1, N2, D, p < 0, stream_of(a)));
             } else {
                 Prepared q{a, b, false, B, N1, N2, D};
                 Tensor coef = lp_forward(q, &w, p, 1.0 / p - 1.0); // S^(1/p-1), OPS/cuda/wminkowski_kernel.cu:16-37
                 lp_backward_call(code_of(a), TPW_LP_BWD_WMINKOWSKI, g, coef.data_ptr(), a, b, w.data_ptr(), g1, g2, B, N1, N2, D, p);
-                Tensor scratch = at::empty({B, N1, D}, a.options());
-                TPW_CALL(tpw_wminkowski_backward_w(code_of(a), g.data_ptr(), coef.data_ptr(), a.data_ptr(), b.data_ptr(), gw.data_ptr(),
-                                                   scratch.data_ptr(), B, N1, N2, D, p, stream_of(a)));
+                if (need_w) {
+                    Tensor scratch = at::empty({B, N1, D}, a.options());
+                    TPW_CALL(tpw_wminkowski_backward_w(code_of(a), g.data_ptr(), coef.data_ptr(), a.data_ptr(), b.data_ptr(), gw.data_ptr(),
+                                                       scratch.data_ptr(), B, N1, N2, D, p, stream_of(a)));
+                }
             }
         }
         return {g1, g2, gw};
@@ -475,8 +482,9 @@ struct WMinkowskiFn : torch::autograd::Function<WMinkowskiFn> {
         auto s = ctx->get_saved_variables();
         const bool ub = ctx->saved_data["unbatched"].toBool();
         const auto dt = static_cast<at::ScalarType>(ctx->saved_data["dt"].toInt());
-        auto g = raw_backward(go[0], s[0], s[1], s[2], ctx->saved_data["p"].toDouble(), ub);
-        return {finish(std::get<0>(g), ub, dt), finish(std::get<1>(g), ub, dt), finish(std::get<2>(g), ub, dt), Tensor()};
+        auto g = raw_backward(go[0], s[0], s[1], s[2], ctx->saved_data["p"].toDouble(), ub, ctx->needs_input_grad(2));
+        const Tensor &gw = std::get<2>(g);
+        return {finish(std::get<0>(g), ub, dt), finish(std::get<1>(g), ub, dt), gw.defined() ? finish(gw, ub, dt) : Tensor(), Tensor()};
     }
 };
 

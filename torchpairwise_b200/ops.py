@@ -422,18 +422,22 @@ class _WMinkowskiFunction(torch.autograd.Function):
     @staticmethod
     def backward(ctx, grad):
         x1c, x2c, wc = ctx.saved_tensors
-        g1, g2, gw = _wminkowski_backward_raw(grad, x1c, x2c, wc, ctx.p, ctx.unbatched)
-        return g1.to(ctx.in_dtype), g2.to(ctx.in_dtype), gw.to(ctx.in_dtype), None
+        g1, g2, gw = _wminkowski_backward_raw(grad, x1c, x2c, wc, ctx.p, ctx.unbatched, ctx.needs_input_grad[2])
+        return g1.to(ctx.in_dtype), g2.to(ctx.in_dtype), None if gw is None else gw.to(ctx.in_dtype), None
 
 
-def _wminkowski_backward_raw(grad, x1c, x2c, wc, p, unbatched):
+def _wminkowski_backward_raw(grad, x1c, x2c, wc, p, unbatched, need_w=True):
+    """``need_w=False``: the weights' gradient, a pass over all pairs of its own, is left out (None)."""
     g = grad.to(x1c.dtype).contiguous()
     if unbatched:
         g = g.unsqueeze(0)
     B, N1, N2, D = _sizes(x1c, x2c)
     code = _FLOAT_CODES[x1c.dtype]
-    g1, g2, gw = torch.zeros_like(x1c), torch.zeros_like(x2c), torch.zeros_like(wc)
-    if p != 0 and B * N1 * N2 * D > 0:
+    # the finite-p kernels write every element, the p = inf kernel adds into zeros
+    work = p != 0 and B * N1 * N2 * D > 0
+    new = torch.empty_like if work and not math.isinf(p) else torch.zeros_like
+    g1, g2, gw = new(x1c), new(x2c), new(wc) if need_w else None
+    if work:
         with torch.cuda.device(x1c.device):
             if math.isinf(p):
                 check(lib.tpw_lp_inf_backward(code, _ptr(g), _ptr(x1c), _ptr(x2c), _ptr(wc), _ptr(g1), _ptr(g2),
@@ -444,12 +448,13 @@ def _wminkowski_backward_raw(grad, x1c, x2c, wc, p, unbatched):
                 # (OPS/cuda/wminkowski_kernel.cu:16-37 called at :300-320)
                 coef = _lp_forward_raw(x1c, x2c, wc, p, 1.0 / p - 1.0)
                 _lp_backward_call(_abi.LP_BWD_WMINKOWSKI, g, coef, x1c, x2c, wc, g1, g2, p)
-                scratch = torch.empty((B, N1, D), dtype=x1c.dtype, device=x1c.device)
-                check(lib.tpw_wminkowski_backward_w(code, _ptr(g), _ptr(coef), _ptr(x1c), _ptr(x2c), _ptr(gw),
-                                                    _ptr(scratch), B, N1, N2, D, float(p), _stream(x1c)),
-                      "tpw_wminkowski_backward_w")
+                if need_w:
+                    scratch = torch.empty((B, N1, D), dtype=x1c.dtype, device=x1c.device)
+                    check(lib.tpw_wminkowski_backward_w(code, _ptr(g), _ptr(coef), _ptr(x1c), _ptr(x2c), _ptr(gw),
+                                                        _ptr(scratch), B, N1, N2, D, float(p), _stream(x1c)),
+                          "tpw_wminkowski_backward_w")
     if unbatched:
-        g1, g2, gw = g1.squeeze(0), g2.squeeze(0), gw.squeeze(0)
+        g1, g2, gw = g1.squeeze(0), g2.squeeze(0), None if gw is None else gw.squeeze(0)
     return g1, g2, gw
 
 
