@@ -12,12 +12,16 @@
 // add (no FMA contraction), i.e. bit-for-bit what the reference's CPU loop computes, so the
 // selected indices agree with it whenever they are determined at all.
 //
-// With caller-provided scratch the hot loop (hausdorff_rowmin_fused_kernel) does not pay for that: it forms
-// the squared distance with fused multiply-adds, which is within a few units in the last place of the
-// separately rounded value, and stores every row's approximate minimum.  The refining kernel then
-// re-evaluates, with the exact arithmetic, only the rows whose approximate minimum lies within that
-// error of the largest one (usually one or two per set pair) and applies the tie rules to them, so
-// values and indices are still bit-identical to the exact path.
+// With caller-provided scratch the hot loop (hausdorff_rowmin_fused_kernel) does not pay for that: it stores
+// every row's approximate minimum, and the refining kernel then re-evaluates, with the exact arithmetic, only
+// the rows whose approximate minimum lies within the approximation's error of the largest one (usually one
+// to three per set pair) and applies the tie rules to them, so values and indices are still bit-identical to
+// the exact path.  Two approximations:
+//   expanded   |y|^2 - 2 x.y + |x|^2 about a point of the x2 cloud: D fused multiply-adds per point pair.  Its error is
+//              bounded by the clouds' extent, not by the distance, so where many rows lie that close together (equal
+//              clouds, a far outlier, coordinates that are not finite) a set pair is handed over to the other one;
+//   direct     sum of squared differences with fused multiply-adds, 2 D per point pair, within a few units in the last
+//              place of the separately rounded value.
 //
 // Any other dtype / feature count runs a plain one-CTA-per-set-pair kernel with the same rules.
 #include "common.cuh"
@@ -62,6 +66,7 @@ struct HdParams {
     long long B, N1, N2, M1, M2, D;
     long long mtiles;
     int splits;       // CTAs that share the x2 points of one row block (fused path)
+    int handed_over;  // direct form: only the set pairs that the expanded form has handed over
 };
 
 // An upper bound on the relative difference between the fused and the separately rounded sum of up to 8 squares
@@ -155,26 +160,35 @@ hausdorff_rowmin_kernel(const HdParams P) {
 }
 
 // The fused loop.  Bound: FP32 issue.  Two x2 points lie side by side in shared memory, coordinate by coordinate, so that
-// one packed subtract and one packed fused multiply-add serve two point pairs, and one three-operand minimum folds both
-// distances in: at D = 3 a point pair costs 6 lane-operations of the FMA pipe in 3 instructions and half a minimum
-// instead of 7 instructions.  A lone last point is paired with a point of NaNs, whose distance no minimum takes.
+// one packed instruction serves two point pairs, and one three-operand minimum folds both distances in: at D = 3 a
+// point pair costs 3 lane-operations of the FMA pipe (direct: 6) in 1.5 (3) instructions and half a minimum, where it
+// took 7 instructions.  A lone last point is paired with a point of NaNs, whose distance no minimum takes.
 // CTAs of 128 threads (512 rows) leave a smaller last wave than 256 threads would; where a small batch has fewer row
 // blocks than fill the GPU, `splits` CTAs share the x2 points of a row block and merge by an integer minimum
 // (order-independent: the result does not depend on the split).
-// Measured at 64 pairs of 8192-point clouds, D = 3: 1.17 -> 0.92 ms.
+// Measured at 64 pairs of 8192-point clouds, D = 3: 1.17 ms scalar, 0.92 ms direct, 0.56 ms expanded.
 constexpr int kFThreads = 128;
 constexpr int FCHUNK_BYTES = 16384;
 template <int D> struct Fused {
     static constexpr int PM = D <= 8 ? 4 : 2;            // x1 points per thread, both lanes of a packed register
-    static constexpr int DP = (D + 1) / 2 * 2;           // packed words per pair of x2 points (16-byte loads)
-    static constexpr int CHUNK = FCHUNK_BYTES / (DP * 8);   // pairs of x2 points staged per pass
     static constexpr int ROWS = kFThreads * PM;
 };
 
-template <int D>
+// What the two kernels agree on per set pair, in the eight bytes the exact path uses for its key: the largest squared
+// norm about the centre (infinite: not bounded) and whether the pair has been handed over to the direct form.
+struct PairState {
+    unsigned int extent, direct;
+};
+constexpr float kExtentMax = 1e36f;   // beyond it the products could overflow
+constexpr int kMaxCandidates = 32;    // more rows within the error of the largest: hand the pair over
+
+template <int D, bool EXPAND>
 __global__ void __launch_bounds__(kFThreads)
 hausdorff_rowmin_fused_kernel(const HdParams P) {
     typedef Fused<D> F;
+    // packed words per pair of x2 points, an even number for 16-byte loads: the coordinates (EXPAND: times -2, and the squared norm)
+    constexpr int W = EXPAND ? D + 1 : D, DP = (W + 1) / 2 * 2;
+    constexpr int CHUNK = FCHUNK_BYTES / (DP * 8);   // pairs of x2 points staged per pass
     __shared__ ulonglong2 pts[FCHUNK_BYTES / 16];
     const int tid = threadIdx.x;
     long long blk = blockIdx.x;
@@ -182,55 +196,87 @@ hausdorff_rowmin_fused_kernel(const HdParams P) {
     blk /= P.splits;
     const long long mt = blk % P.mtiles;
     const long long pair = blk / P.mtiles; // (b*N1 + i)*N2 + j
+    PairState *state = reinterpret_cast<PairState *>(P.keys) + pair;
+    if (!EXPAND && P.handed_over && state->direct == 0) return;
     const long long j = pair % P.N2;
     const long long bi = pair / P.N2;
     const long long b = bi / P.N1;
     const float *x1 = reinterpret_cast<const float *>(P.x1) + bi * P.M1 * D;
     const float *x2 = reinterpret_cast<const float *>(P.x2) + (b * P.N2 + j) * P.M2 * D;
+    float centre[D];
+#pragma unroll
+    for (int k = 0; k < D; ++k) centre[k] = EXPAND ? x2[k] : 0.f;
+    float extent = 0.f;          // largest squared norm this thread has seen
+    bool unbounded = false;
     // this CTA's range of x2 points, cut at even positions
     const long long per = ((P.M2 + 1) / 2 + P.splits - 1) / P.splits * 2;
     const long long n_end = (sp + 1) * per < P.M2 ? (sp + 1) * per : P.M2;
 
     f32x2 px[F::PM][D];
-    float rowmin[F::PM];
+    float rowmin[F::PM], xsq[F::PM];
 #pragma unroll
     for (int q = 0; q < F::PM; ++q) {
         const long long m = mt * F::ROWS + q * kFThreads + tid;
         rowmin[q] = INFINITY;
+        xsq[q] = 0.f;
 #pragma unroll
         for (int k = 0; k < D; ++k) {
-            const float v = m < P.M1 ? x1[m * D + k] : 0.f;
+            const float v = m < P.M1 ? x1[m * D + k] - centre[k] : 0.f;
             px[q][k] = pack2(v, v);
+            xsq[q] = fmaf(v, v, xsq[q]);
         }
+        extent = fmaxf(extent, xsq[q]);
+        unbounded |= !(xsq[q] < kExtentMax);
     }
 
-    for (long long n0 = sp * per; n0 < n_end; n0 += 2 * F::CHUNK) {
-        const int cnt = (int)((n_end - n0 + 1) / 2 < F::CHUNK ? (n_end - n0 + 1) / 2 : F::CHUNK);
+    for (long long n0 = sp * per; n0 < n_end; n0 += 2 * CHUNK) {
+        const int cnt = (int)((n_end - n0 + 1) / 2 < CHUNK ? (n_end - n0 + 1) / 2 : CHUNK);
         __syncthreads();
         for (int e = tid; e < cnt; e += kFThreads) {
             const float *s = x2 + (n0 + 2 * e) * D;
             const bool two = n0 + 2 * e + 1 < n_end;
-            f32x2 *dst = reinterpret_cast<f32x2 *>(pts) + e * F::DP;
+            f32x2 *dst = reinterpret_cast<f32x2 *>(pts) + e * DP;
+            if (EXPAND) {
+                float lo = 0.f, hi = 0.f;
 #pragma unroll
-            for (int k = 0; k < D; ++k) dst[k] = pack2(s[k], two ? s[D + k] : NAN);
+                for (int k = 0; k < D; ++k) {
+                    const float u = s[k] - centre[k], v = two ? s[D + k] - centre[k] : 0.f;
+                    lo = fmaf(u, u, lo);
+                    hi = fmaf(v, v, hi);
+                    dst[k] = pack2(-2.f * u, -2.f * v);
+                }
+                extent = fmaxf(extent, fmaxf(lo, hi));
+                unbounded |= !(lo < kExtentMax) || !(hi < kExtentMax);
+                dst[D] = pack2(lo, two ? hi : NAN);
+            } else {
+#pragma unroll
+                for (int k = 0; k < D; ++k) dst[k] = pack2(s[k], two ? s[D + k] : NAN);
+            }
         }
         __syncthreads();
 #pragma unroll 4
         for (int e = 0; e < cnt; ++e) {
-            f32x2 c[F::DP];
+            f32x2 c[DP];
 #pragma unroll
-            for (int v = 0; v < F::DP / 2; ++v) {
-                const ulonglong2 t = pts[e * (F::DP / 2) + v];
+            for (int v = 0; v < DP / 2; ++v) {
+                const ulonglong2 t = pts[e * (DP / 2) + v];
                 c[2 * v] = t.x; c[2 * v + 1] = t.y;
             }
 #pragma unroll
             for (int q = 0; q < F::PM; ++q) {
-                f32x2 diff = sub2(px[q][0], c[0]);
-                f32x2 d = mul2(diff, diff);
+                f32x2 d;
+                if (EXPAND) {
+                    d = fma2(px[q][0], c[0], c[D]);
 #pragma unroll
-                for (int k = 1; k < D; ++k) {
-                    diff = sub2(px[q][k], c[k]);
-                    d = fma2(diff, diff, d);
+                    for (int k = 1; k < D; ++k) d = fma2(px[q][k], c[k], d);
+                } else {
+                    f32x2 diff = sub2(px[q][0], c[0]);
+                    d = mul2(diff, diff);
+#pragma unroll
+                    for (int k = 1; k < D; ++k) {
+                        diff = sub2(px[q][k], c[k]);
+                        d = fma2(diff, diff, d);
+                    }
                 }
                 float lo, hi;
                 unpack2(d, lo, hi);
@@ -238,13 +284,18 @@ hausdorff_rowmin_fused_kernel(const HdParams P) {
             }
         }
     }
+    if (EXPAND) {
+        const unsigned int bits = __reduce_max_sync(0xffffffffu, unbounded ? 0x7f800000u : __float_as_uint(extent));
+        if ((tid & 31) == 0) atomicMax(&state->extent, bits);
+    }
 #pragma unroll
     for (int q = 0; q < F::PM; ++q) {
         const long long m = mt * F::ROWS + q * kFThreads + tid;
         if (m >= P.M1) continue;
+        const float v = EXPAND ? fmaxf(rowmin[q] + xsq[q], 0.f) : rowmin[q];
         float *dst = P.rowmins + pair * P.M1 + m;
-        if (P.splits == 1) *dst = rowmin[q];
-        else atomicMin(reinterpret_cast<unsigned int *>(dst), __float_as_uint(rowmin[q]));   // non-negative: bits order like values
+        if (P.splits == 1) *dst = v;
+        else atomicMin(reinterpret_cast<unsigned int *>(dst), __float_as_uint(v));   // non-negative: bits order like values
     }
 }
 
@@ -309,9 +360,10 @@ hausdorff_finish_kernel(const HdParams P) {
 }
 
 // Fused path: one CTA per set pair.  Every row whose approximate minimum could be the exact maximum is re-evaluated with
-// the separately rounded arithmetic by one warp (lanes over n, first visited n on ties); the largest exact minimum wins,
-// the last visited m on ties.
-template <int D>
+// the separately rounded arithmetic (first visited n on ties); the largest exact minimum wins, the last visited m on ties.
+// Up to kMaxCandidates rows are evaluated one after another by the whole CTA (one warp to a row had seven warps waiting for
+// it: 56 -> 10 us at 64 pairs of 8192-point clouds), more of them a warp to a row.
+template <int D, bool EXPAND>
 __global__ void __launch_bounds__(kThreads)
 hausdorff_refine_kernel(const HdParams P) {
     constexpr int kWarps = kThreads / 32;
@@ -325,7 +377,9 @@ hausdorff_refine_kernel(const HdParams P) {
     const long long b = bi / P.N1;
     const float *x1 = reinterpret_cast<const float *>(P.x1) + bi * P.M1 * D;
     const float *x2 = reinterpret_cast<const float *>(P.x2) + (b * P.N2 + j) * P.M2 * D;
-    const float *rm = P.rowmins + pair * P.M1;
+    float *rm = P.rowmins + pair * P.M1;
+    PairState *state = reinterpret_cast<PairState *>(P.keys) + pair;
+    if (!EXPAND && P.handed_over && state->direct == 0) return;
     // the largest approximate minimum, the last visited row on ties
     unsigned long long key = 0ull;
     for (long long m = tid; m < P.M1; m += kThreads) {
@@ -348,8 +402,83 @@ hausdorff_refine_kernel(const HdParams P) {
     // An approximate minimum of exactly 0 means every difference squared to 0, in either arithmetic: all rows then
     // tie at 0 and the last visited one, which the key already names, wins.  Otherwise a row can hold the exact
     // maximum only if its approximate minimum is within the rounding slack of the largest approximate minimum.
-    const bool all_zero = amax == 0.f;
-    const float lower = amax * (1.f - fused_slack<D>()) - kTiny;
+    // EXPAND: with R^2 the largest squared norm about the centre, the centred coordinates' roundings change a squared distance
+    // by at most 8 u R^2 (u = 2^-24), the two norms' by 2 D u R^2, the D multiply-adds' by 3 D u R^2 and the last addition's by
+    // 4 u R^2: E = (5 D + 12) u R^2.  A row of the largest distance lies within 2 E of the largest minimum; 16 D + 64 leaves room.
+    const bool all_zero = !EXPAND && amax == 0.f;
+    float lower = amax * (1.f - fused_slack<D>()) - kTiny;
+    if (EXPAND) lower -= 2.f * (float)(8 * (D + 1) + 24) * 5.9604645e-8f * __uint_as_float(state->extent);
+
+    // the rows to look at; their order does not matter
+    __shared__ int s_count;
+    __shared__ unsigned int s_cand[kMaxCandidates];
+    if (tid == 0) s_count = 0;
+    __syncthreads();
+    for (long long m = tid; m < P.M1; m += kThreads) {
+        const bool cand = all_zero ? (unsigned int)(P.order1 ? P.order1[b * P.M1 + m] : m) == pos_max : rm[m] >= lower;
+        if (cand) {
+            const int at = atomicAdd(&s_count, 1);
+            if (at < kMaxCandidates) s_cand[at] = (unsigned int)m;
+        }
+    }
+    __syncthreads();
+    const int count = s_count;
+    if (EXPAND && (count > kMaxCandidates || !(__uint_as_float(state->extent) < kExtentMax))) {
+        // too close together for the expanded form: the direct one starts from untouched minima
+        for (long long m = tid; m < P.M1; m += kThreads) rm[m] = __uint_as_float(0xffffffffu);
+        if (tid == 0) state->direct = 1;
+        return;
+    }
+    if (count <= kMaxCandidates) {
+        unsigned long long row_key = 0ull, n_key = ~0ull;    // best (bits(min) << 32 | position(m)) and its n key, the same in all threads
+        long long row = -1;
+        for (int c = 0; c < count; ++c) {
+            const long long m = s_cand[c];
+            const unsigned int pos = (unsigned int)(P.order1 ? P.order1[b * P.M1 + m] : m);
+            float a[D];
+#pragma unroll
+            for (int k = 0; k < D; ++k) a[k] = x1[m * D + k];
+            unsigned long long mine = ~0ull;
+#pragma unroll 4
+            for (long long n = tid; n < P.M2; n += kThreads) {
+                float v[D];
+#pragma unroll
+                for (int k = 0; k < D; ++k) v[k] = x2[n * D + k];
+                const float d = sqdist_exact(a, v, D);
+                const unsigned long long p2 = (unsigned long long)(P.order2 ? P.order2[b * P.M2 + n] : n);
+                const unsigned long long kq = ((unsigned long long)__float_as_uint(d) << 32) | (p2 & 0xffffffffull);
+                if (d == d && kq < mine) mine = kq;   // a NaN distance never lowers a minimum
+            }
+#pragma unroll
+            for (int off = 16; off > 0; off >>= 1) {
+                const unsigned long long other = __shfl_xor_sync(0xffffffffu, mine, off);
+                mine = other < mine ? other : mine;
+            }
+            if (lane == 0) s_n[warp] = mine;
+            __syncthreads();
+#pragma unroll
+            for (int w = 0; w < kWarps; ++w) mine = s_n[w] < mine ? s_n[w] : mine;
+            __syncthreads();
+            // a row without any comparable distance has the minimum +inf, as in the streaming kernel
+            const unsigned int vbits = mine == ~0ull ? 0x7f800000u : (unsigned int)(mine >> 32);
+            const unsigned long long rkey = ((unsigned long long)vbits << 32) | pos;
+            if (row < 0 || rkey > row_key) { row_key = rkey; n_key = mine; row = m; }
+        }
+        const unsigned int npos = (unsigned int)(n_key & 0xffffffffull);
+        if (tid == 0) s_nstar = (P.order2 || n_key == ~0ull) ? 0 : (long long)npos;
+        __syncthreads();
+        if (P.order2 && n_key != ~0ull) {
+            for (long long n = tid; n < P.M2; n += kThreads)
+                if ((unsigned int)P.order2[b * P.M2 + n] == npos) s_nstar = n;
+            __syncthreads();
+        }
+        if (tid == 0) {
+            reinterpret_cast<float *>(P.out)[pair] = sqrtf(__uint_as_float((unsigned int)(row_key >> 32)));
+            P.idx1[pair] = row < 0 ? 0 : row;
+            P.idx2[pair] = s_nstar;
+        }
+        return;
+    }
 
     unsigned long long wrow = 0ull, wn = ~0ull;   // best (bits(min) << 32 | position(m)) of this warp, its n key
     long long wm = -1;
@@ -628,9 +757,18 @@ int launch_fast(HdParams P, cudaStream_t s) {
         const long long blocks = pairs * P.mtiles * P.splits;
         TPW_CHECK_ARG(blocks < (1ll << 31), "hausdorff: too many blocks");
         if (P.splits > 1) TPW_CUDA_OK(cudaMemsetAsync(P.rowmins, 0xff, (size_t)(pairs * P.M1) * sizeof(float), s));
-        hausdorff_rowmin_fused_kernel<D><<<(unsigned)blocks, kFThreads, 0, s>>>(P);
+        // the expanded form pays for the two launches that serve handed-over pairs from about 2^26 point pairs on
+        if ((double)pairs * (double)P.M1 * (double)P.M2 >= 67108864.0) {
+            TPW_CUDA_OK(cudaMemsetAsync(P.keys, 0, (size_t)pairs * sizeof(PairState), s));
+            hausdorff_rowmin_fused_kernel<D, true><<<(unsigned)blocks, kFThreads, 0, s>>>(P);
+            TPW_LAUNCH_OK("hausdorff_rowmin_fused_kernel");
+            hausdorff_refine_kernel<D, true><<<(unsigned)pairs, kThreads, 0, s>>>(P);
+            TPW_LAUNCH_OK("hausdorff_refine_kernel");
+            P.handed_over = 1;
+        }
+        hausdorff_rowmin_fused_kernel<D, false><<<(unsigned)blocks, kFThreads, 0, s>>>(P);
         TPW_LAUNCH_OK("hausdorff_rowmin_fused_kernel");
-        hausdorff_refine_kernel<D><<<(unsigned)pairs, kThreads, 0, s>>>(P);
+        hausdorff_refine_kernel<D, false><<<(unsigned)pairs, kThreads, 0, s>>>(P);
         TPW_LAUNCH_OK("hausdorff_refine_kernel");
         return TPW_OK;
     }
