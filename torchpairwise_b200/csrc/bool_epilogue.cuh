@@ -16,7 +16,25 @@ __device__ __forceinline__ float count_to_float(int v) {
     return FAST ? __int_as_float(0x4B000000 | v) - 8388608.f : (float)v;
 }
 
-// INV: -1 = decide per call from inv_d, 1 = D is a power of two and inv_d its reciprocal, 0 = divide.  A caller that
+// x / y rounded to nearest for integers 0 <= x, 0 < y < 2^18 with the quotient at most 1, given an approximate reciprocal r of
+// y (2 ulp): one Newton step on the quotient with an exact residual (P. Markstein, "Computation of elementary functions on the
+// IBM RISC System/6000 processor", 1990).  q = x r is within a few ulp of x / y, x - q y is exact in a fused multiply-add, and the sum
+// q + (x - q y) r is, before its one rounding, within 2^-20 ulp of x / y.  A quotient of integers below 2^18 that is not
+// itself a float lies at least 2^-19 ulp from every rounding boundary, so the rounding is that of x / y.  Four instructions
+// without a branch: jaccard [65536, 16384, 1024] 1.62 -> 1.41 ms.
+__device__ __forceinline__ float quotient_of_counts(float x, float y, float r) {
+    const float q = __fmul_rn(x, r);
+    return __fmaf_rn(__fmaf_rn(-q, y, x), r, q);
+}
+constexpr int kQuotientMax = 1 << 18;
+__device__ __forceinline__ float approximate_reciprocal(float y) {
+    float r;
+    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(y));
+    return r;
+}
+
+// INV: -1 = decide per call from inv_d, 1 = D is a power of two and inv_d its reciprocal, 0 = divide, 2 = D is below kQuotientMax
+// and inv_d an approximate reciprocal of it (the means), or any value (jaccard): quotients as above.  A caller that
 // knows which holds for a whole tile passes it as a constant: decided per element, the division sequence is
 // if-converted and executed next to the multiplication for every element.
 template <bool FAST = false, int INV = -1>
@@ -35,12 +53,16 @@ __device__ __forceinline__ float bool_epilogue(int metric, int n11, int a, int b
         case TPW_BOOL_EQ_MEAN:
             if (INV == 1) return __fmul_rn(feq, inv_d);
             if (INV == 0) return __fdiv_rn(feq, fD);
+            if (INV == 2) return quotient_of_counts(feq, fD, inv_d);
             return inv_d != 0.f ? __fmul_rn(feq, inv_d) : __fdiv_rn(feq, fD);
         case TPW_BOOL_NE_MEAN:
             if (INV == 1) return __fmul_rn(fxor, inv_d);
             if (INV == 0) return __fdiv_rn(fxor, fD);
+            if (INV == 2) return quotient_of_counts(fxor, fD, inv_d);
             return inv_d != 0.f ? __fmul_rn(fxor, inv_d) : __fdiv_rn(fxor, fD);
-        case TPW_BOOL_JACCARD: return f_or != 0.f ? __fdiv_rn(fxor, f_or) : 0.f;
+        case TPW_BOOL_JACCARD:
+            if (INV == 2) return f_or != 0.f ? quotient_of_counts(fxor, f_or, approximate_reciprocal(f_or)) : 0.f;
+            return f_or != 0.f ? __fdiv_rn(fxor, f_or) : 0.f;
         case TPW_BOOL_KULSINSKI: return __fdiv_rn(__fadd_rn(__fsub_rn(fxor, fand), fD), __fadd_rn(fxor, fD));
         case TPW_BOOL_KULCZYNSKI1: return __fdiv_rn(fand, fxor);
         case TPW_BOOL_YULE: {

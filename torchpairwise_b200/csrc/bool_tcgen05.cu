@@ -262,7 +262,7 @@ bool_count_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
             const long long row_base = tm * BM + q * 32;
             // the mean metrics multiply by 1 / D where D is a power of two and divide otherwise: decided here, once per
             // tile, so that the per-element code holds one of the two
-            auto drain = [&](auto inv_tag) {
+            auto drain = [&](auto inv_tag, float inv_d) {
                 constexpr int INV = decltype(inv_tag)::value;
 #pragma unroll 1
             for (int c = cpart * NCB; c < (cpart + 1) * NCB; ++c) {
@@ -278,10 +278,10 @@ bool_count_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
 #pragma unroll
                     for (int v = 0; v < 8; ++v) {
                         const int4 nb = *reinterpret_cast<const int4 *>(popw + (c - cpart * NCB) * 32 + 4 * v);
-                        o[v].x = bool_epilogue<true, INV>(METRIC, (int)r[4 * v + 0], pa, nb.x, D, P.inv_d);
-                        o[v].y = bool_epilogue<true, INV>(METRIC, (int)r[4 * v + 1], pa, nb.y, D, P.inv_d);
-                        o[v].z = bool_epilogue<true, INV>(METRIC, (int)r[4 * v + 2], pa, nb.z, D, P.inv_d);
-                        o[v].w = bool_epilogue<true, INV>(METRIC, (int)r[4 * v + 3], pa, nb.w, D, P.inv_d);
+                        o[v].x = bool_epilogue<true, INV>(METRIC, (int)r[4 * v + 0], pa, nb.x, D, inv_d);
+                        o[v].y = bool_epilogue<true, INV>(METRIC, (int)r[4 * v + 1], pa, nb.y, D, inv_d);
+                        o[v].z = bool_epilogue<true, INV>(METRIC, (int)r[4 * v + 2], pa, nb.z, D, inv_d);
+                        o[v].w = bool_epilogue<true, INV>(METRIC, (int)r[4 * v + 3], pa, nb.w, D, inv_d);
                     }
                     if (P.tma_store) {
                         // by now the copy engine has read the previous block out of the staging area
@@ -327,10 +327,13 @@ bool_count_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
             }
             };
             if (METRIC == TPW_BOOL_EQ_MEAN || METRIC == TPW_BOOL_NE_MEAN) {
-                if (P.inv_d != 0.f) drain(std::integral_constant<int, 1>{});
-                else drain(std::integral_constant<int, 0>{});
+                if (P.inv_d != 0.f) drain(std::integral_constant<int, 1>{}, P.inv_d);
+                else if (P.D < kQuotientMax) drain(std::integral_constant<int, 2>{}, approximate_reciprocal((float)P.D));
+                else drain(std::integral_constant<int, 0>{}, 0.f);
+            } else if (METRIC == TPW_BOOL_JACCARD && P.D < kQuotientMax) {
+                drain(std::integral_constant<int, 2>{}, 0.f);
             } else {
-                drain(std::integral_constant<int, -1>{});
+                drain(std::integral_constant<int, -1>{}, P.inv_d);
             }
             // this warp has drained its part of accumulator `a`
             tc_fence_before();
