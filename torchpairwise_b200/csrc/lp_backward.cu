@@ -361,6 +361,114 @@ __global__ void __launch_bounds__(256) lp_backward_small_kernel(const BwdParams 
     reinterpret_cast<T *>(P.out)[idx] = v;
 }
 
+// The same problems on rows of more than 8 features.  One thread per element loads a streamed value, the gradient and the
+// auxiliary value for every term; here a thread has R rows of one feature, so a streamed value serves R terms, and the CTA
+// forms the coefficients of its rows and of 32 streamed rows once, in shared memory, from where a warp reads R of them with one or two
+// broadcast loads.  KL lanes span the features (16 where that leaves fewer lanes idle), 256 / KL groups of R rows make a
+// CTA.  The terms of an element are added in the same order, so the results are still those of the tile kernel bit for bit.
+// Bound: arithmetic and the broadcast loads.  Weighted p = 2 in float64 [1500, 1301, 75], both gradients: 351 -> 256 us.
+constexpr int SB_THREADS = 256;
+constexpr int SB_S = 32;       // streamed rows per stage
+
+template <typename T, int PHI, bool NEED_AUX, bool TRANS, int KL, int R>
+__global__ void __launch_bounds__(SB_THREADS) lp_backward_rows_kernel(const BwdParams P) {
+    if (P.only_if && *P.only_if <= P.only_if_above) return;
+    constexpr int GROUPS = SB_THREADS / KL, RB = GROUPS * R, PER = RB * SB_S / SB_THREADS;
+    constexpr int PITCH = RB + 16 / (int)sizeof(T);      // rows of 16-byte multiples, shifted by a bank group from row to row
+    constexpr bool NEED_O = PHI == PHI_SGN_EQ;            // the term looks at the auxiliary value itself
+    __shared__ __align__(16) T cs[2][SB_S * PITCH];
+    __shared__ __align__(16) T os[NEED_O ? 2 : 1][NEED_O ? SB_S * PITCH : 1];
+    const int tid = threadIdx.x, lane = tid % KL, group = tid / KL;
+    long long tile = blockIdx.x;
+    const long long tk = tile % P.tiles_k;
+    tile /= P.tiles_k;
+    const long long tr = tile % P.tiles_r, b = tile / P.tiles_r;
+    const long long k = tk * KL + lane, r0 = tr * RB, row = r0 + group * R;
+    const bool k_ok = k < P.D;
+    const T *stream = reinterpret_cast<const T *>(P.stream) + b * P.NS * P.D + (k_ok ? k : 0);
+    const T *grad = reinterpret_cast<const T *>(P.grad) + b * P.N1 * P.N2;
+    const T *aux = NEED_AUX ? reinterpret_cast<const T *>(P.aux) + b * P.N1 * P.N2 : nullptr;
+    T x[R], acc[R];
+#pragma unroll
+    for (int a = 0; a < R; ++a) {
+        x[a] = PHI != PHI_Y && k_ok && row + a < P.NR ? reinterpret_cast<const T *>(P.rowop)[(b * P.NR + row + a) * P.D + k] : T(0);
+        acc[a] = T(0);
+    }
+    // this thread's pairs of a stage: consecutive threads along the dimension that is contiguous in memory
+    T g[PER], o[PER];
+    auto fetch = [&](long long s0) {
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            const int e = tid + u * SB_THREADS;
+            const long long r = r0 + (TRANS ? e % RB : e / SB_S), s = s0 + (TRANS ? e / RB : e % SB_S);
+            const bool ok = r < P.NR && s < P.NS;
+            const long long at = TRANS ? s * P.N2 + r : r * P.N2 + s;
+            g[u] = ok ? grad[at] : T(0);
+            o[u] = NEED_AUX && ok ? aux[at] : T(0);
+        }
+    };
+    const T q = (T)P.q;
+    fetch(0);
+    int buf = 0;
+    for (long long s0 = 0; s0 < P.NS; s0 += SB_S, buf ^= 1) {
+        // a warp may still be reading the other buffer; this one was last read before the previous barrier
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
+            const int e = tid + u * SB_THREADS;
+            const int at = (TRANS ? e / RB : e % SB_S) * PITCH + (TRANS ? e % RB : e / SB_S);
+            cs[buf][at] = NEED_AUX ? bwd_coefficient<T>(P.coef_mode, g[u], o[u], P.q) : g[u];
+            if (NEED_O) os[NEED_O ? buf : 0][NEED_O ? at : 0] = o[u];
+        }
+        __syncthreads();
+        if (s0 + SB_S < P.NS) fetch(s0 + SB_S);
+        const int cnt = (int)(P.NS - s0 < SB_S ? P.NS - s0 : SB_S);
+        const T *sp = stream + s0 * P.D;
+        auto term = [&](int s, T y) {
+            T c[R], ov[R];
+#pragma unroll
+            for (int a = 0; a < R; ++a) {
+                c[a] = cs[buf][s * PITCH + group * R + a];
+                ov[a] = NEED_O ? os[NEED_O ? buf : 0][NEED_O ? s * PITCH + group * R + a : 0] : T(0);
+            }
+#pragma unroll
+            for (int a = 0; a < R; ++a) bwd_accumulate<PHI, T>(acc[a], x[a], y, c[a], ov[a], q, P.pow_spec);
+        };
+        int s = 0;
+        for (; s + 8 <= cnt; s += 8) {
+            T y[8];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) y[u] = sp[(s + u) * P.D];
+#pragma unroll
+            for (int u = 0; u < 8; ++u) term(s + u, y[u]);
+        }
+        for (; s < cnt; ++s) term(s, sp[s * P.D]);
+    }
+    if (!k_ok) return;
+#pragma unroll
+    for (int a = 0; a < R; ++a) {
+        if (row + a >= P.NR) continue;
+        T v = acc[a] * (T)P.post;
+        if (P.w) v *= reinterpret_cast<const T *>(P.w)[b * P.D + k];
+        reinterpret_cast<T *>(P.out)[(b * P.NR + row + a) * P.D + k] = v;
+    }
+}
+
+template <typename T, int PHI, bool NEED_AUX, bool TRANS, int KL>
+int launch_backward_rows(BwdParams P, cudaStream_t stream) {
+    P.tiles_k = (P.D + KL - 1) / KL;
+    // four rows to a thread where that still gives every SM a CTA, else two
+    const long long four = P.B * P.tiles_k * ((P.NR + SB_THREADS / KL * 4 - 1) / (SB_THREADS / KL * 4));
+    constexpr bool FOUR = !(sizeof(T) == 8 && PHI == PHI_SGN_EQ && KL == 16);   // two float64 tiles of 64 rows exceed 48 KB
+    const int R = FOUR && four >= sm_count() ? 4 : 2;
+    P.tiles_r = (P.NR + SB_THREADS / KL * R - 1) / (SB_THREADS / KL * R);
+    const long long tiles = P.B * P.tiles_r * P.tiles_k;
+    TPW_CHECK_ARG(tiles < (1ll << 31), "lp backward: too many tiles (%lld)", tiles);
+    if (FOUR && R == 4) lp_backward_rows_kernel<T, PHI, NEED_AUX, TRANS, KL, FOUR ? 4 : 2><<<(unsigned)tiles, SB_THREADS, 0, stream>>>(P);
+    else lp_backward_rows_kernel<T, PHI, NEED_AUX, TRANS, KL, 2><<<(unsigned)tiles, SB_THREADS, 0, stream>>>(P);
+    TPW_LAUNCH_OK("lp_backward_rows_kernel");
+    return TPW_OK;
+}
+
 template <typename T, int PHI, bool NEED_AUX, bool TRANS>
 int launch_backward(BwdParams P, cudaStream_t stream) {
     constexpr int RR = 4;
@@ -379,6 +487,9 @@ int launch_backward(BwdParams P, cudaStream_t stream) {
     // fewer gradient blocks than a third of the SMs: one thread per gradient element instead (TPW_DISABLE_SMALL_BWD=1
     // keeps the tile kernel); the walk per thread is bounded so that a launch stays in the millisecond range
     if (tiles * 3 < sm_count() && P.NS <= 65536 && P.B * P.NR * P.D < (1ll << 31) * 256 && !getenv("TPW_DISABLE_SMALL_BWD")) {
+        if (P.D > 8)
+            return (P.D + 15) / 16 * 16 < (P.D + 31) / 32 * 32 ? launch_backward_rows<T, PHI, NEED_AUX, TRANS, 16>(P, stream)
+                                                               : launch_backward_rows<T, PHI, NEED_AUX, TRANS, 32>(P, stream);
         const long long n = P.B * P.NR * P.D;
         lp_backward_small_kernel<T, PHI, NEED_AUX, TRANS><<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(P);
         TPW_LAUNCH_OK("lp_backward_small_kernel");
