@@ -14,7 +14,7 @@
 //      are formed once more, and one attaining coordinate makes the pair's code k | sign << 31.  None (out == 0, NaN,
 //      padding): the pair is skipped.  Several (a tied maximum): the pair is marked and counted in a device counter.
 //      Bound: issue and both arithmetic pipes; six instructions per four features (packed subtract, three-operand
-//      maximum) where a compare and two multiply-adds for every feature took sixteen.  [16, 4096, 4096, 256]: 12.0 -> 7.05 ms.
+//      maximum) where a compare and two multiply-adds for every feature took sixteen.  [16, 4096, 4096, 256]: 12.0 -> 6.9 ms.
 //   2. chebyshev_scatter_kernel (once per gradient): one thread per x1 row (x2 row) walks over the row's pairs in
 //      order and adds +-g into its row of a shared-memory gradient block at the coded coordinate; for a marked pair
 //      it walks over the features itself.  Every gradient element has one owner and a fixed order of additions:
@@ -28,10 +28,11 @@
 namespace tpw {
 namespace {
 
-constexpr int kThreads = 256;
+constexpr int kThreads = 128;                // four CTAs per SM: while one resolves its groups the others compute
 constexpr int kStages = 3;
 constexpr int RI = 8, RJ = 4;               // pairs per thread: 8 x1 rows by 4 x2 rows (two registers per pair)
-constexpr int TI = 16 * RI, TJ = 16 * RJ;   // 128 x 64 pairs per CTA
+constexpr int TS = kThreads / 16;           // x1 rows between a thread's rows
+constexpr int TI = TS * RI, TJ = 16 * RJ;   // 64 x 64 pairs per CTA
 constexpr int KC = 32;                      // features per staged chunk (128 bytes per row)
 constexpr int XB = TI * 128, YB = TJ * 128; // bytes of one stage's x1 and x2 tiles
 constexpr int STAGE = XB + YB;
@@ -69,7 +70,7 @@ __device__ __forceinline__ void stage_rows_plain(unsigned char *tile, const floa
 }
 
 template <bool USE_TMA>
-__global__ void __launch_bounds__(kThreads, 2)
+__global__ void __launch_bounds__(kThreads, 4)
 chebyshev_match_kernel(const __grid_constant__ CUtensorMap map1, const __grid_constant__ CUtensorMap map2, const MatchParams P) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -113,7 +114,7 @@ chebyshev_match_kernel(const __grid_constant__ CUtensorMap map1, const __grid_co
     float acc[RI][RJ];   // sum of (65536 + group) over the attaining groups: exact in float32 up to 255 of them
 #pragma unroll
     for (int ri = 0; ri < RI; ++ri) {
-        const long long i = i0 + ti + 16 * ri;
+        const long long i = i0 + ti + TS * ri;
 #pragma unroll
         for (int rj = 0; rj < RJ; ++rj) {
             const long long j = j0 + tj + 16 * rj;
@@ -157,7 +158,7 @@ chebyshev_match_kernel(const __grid_constant__ CUtensorMap map1, const __grid_co
         }
         const unsigned char *xs = smem + stage * STAGE;
         const unsigned char *ys = xs + XB;
-        const uint32_t xrow = ti, yrow = tj;      // (row + 16 r) & 7 == row & 7
+        const uint32_t xrow = ti, yrow = tj;      // rows 8 or 16 apart share row & 7
         const long long kleft = P.D - (long long)t * KC;
         const int cmax = kleft < KC ? (int)((kleft + 3) / 4) : 8;
 #pragma unroll 1
@@ -169,7 +170,7 @@ chebyshev_match_kernel(const __grid_constant__ CUtensorMap map1, const __grid_co
                 yb[r] = *reinterpret_cast<const float4 *>(ys + (yrow + 16 * r) * 128u + ((c ^ (yrow & 7u)) << 4));
 #pragma unroll
             for (int ri = 0; ri < RI; ++ri) {
-                const float4 xa = *reinterpret_cast<const float4 *>(xs + (xrow + 16 * ri) * 128u + ((c ^ (xrow & 7u)) << 4));
+                const float4 xa = *reinterpret_cast<const float4 *>(xs + (xrow + TS * ri) * 128u + ((c ^ (xrow & 7u)) << 4));
 #pragma unroll
                 for (int rj = 0; rj < RJ; ++rj) {
                     // six instructions per four features: two packed subtracts, the largest |difference| of the group in
@@ -205,7 +206,7 @@ chebyshev_match_kernel(const __grid_constant__ CUtensorMap map1, const __grid_co
     int tied = 0;
 #pragma unroll 4
     for (int e = 0; e < RI * RJ; ++e) {
-        const long long i = i0 + ti + 16 * (e / RJ), j = j0 + tj + 16 * (e % RJ);
+        const long long i = i0 + ti + TS * (e / RJ), j = j0 + tj + 16 * (e % RJ);
         const float2 v = park[e * kThreads];
         const uint32_t a = (uint32_t)v.x;
         uint32_t cd = kSkip;
@@ -241,8 +242,8 @@ chebyshev_match_kernel(const __grid_constant__ CUtensorMap map1, const __grid_co
 }
 
 // ---- scatter ---------------------------------------------------------------------------------------------------------
-constexpr int SR = 128;          // gradient rows per CTA, each walked by one thread of the first four warps
-constexpr int STHR = 512;        // all sixteen warps stage the pairs
+constexpr int SR = 64;           // gradient rows per CTA, each walked by one thread of the first two warps; two CTAs per SM
+constexpr int STHR = 256;        // all eight warps stage the pairs
 constexpr int SD = 256;          // most features per CTA
 constexpr int SP = 32;           // pairs per gradient row staged at a time
 constexpr int SB = 4;            // pairs a walker applies together
@@ -271,19 +272,19 @@ __device__ __noinline__ void scatter_tied(float *row, const float *a, const floa
     }
 }
 
-// COLS = false: grad_x1.  Thread r of the first 128 walks over the pairs of x1 row r0 + r, j ascending, and adds +-g into
+// COLS = false: grad_x1.  Thread r of the first 64 walks over the pairs of x1 row r0 + r, j ascending, and adds +-g into
 // its row of a shared-memory gradient block.  COLS = true: grad_x2, the same with x2 row r0 + r, i ascending and the sign
-// flipped.  The pairs are staged 32 per gradient row at a time by all 512 threads (whole 128-byte segments of g and of
+// flipped.  The pairs are staged 32 per gradient row at a time by all 256 threads (whole 128-byte segments of g and of
 // the codes from global memory, held in registers while the walkers apply the tile before) into one of two buffers.
 //
 // The bound is the latency of the chain load accumulator -> add -> store.  A walker takes four pairs into registers,
 // loads their four accumulators together, adds in order (a pair whose coordinate occurred earlier in the four continues
 // from that sum) and stores in order: the additions and their order are those of one pair at a time.  Pairs that do
 // not concern the CTA's features go to a spare word beside the row, so that no lane of the warp branches.
-// Measured on [16, 4096, 4096] pairs, 256 features: 1.50 -> 0.90 ms per gradient against one pair at a time by four
+// Measured on [16, 4096, 4096] pairs, 256 features: 1.50 -> 0.77 ms per gradient against one pair at a time by four
 // walkers a row, each looking at all pairs for those in its quarter of the features; 0.33 ms to read g and the codes.
 template <bool COLS>
-__global__ void __launch_bounds__(STHR, 1) chebyshev_scatter_kernel(const ScatterParams P) {
+__global__ void __launch_bounds__(STHR, 2) chebyshev_scatter_kernel(const ScatterParams P) {
     if (*P.ties > tie_limit(P.B * P.N1 * P.N2)) return;   // tied maxima everywhere: the dense kernel that follows writes this gradient
     extern __shared__ float sm[];
     const int tid = threadIdx.x;
