@@ -87,3 +87,49 @@ def test_one_pass_backward_with_ragged_columns(tpw, shape, p):
     for one, again, two in zip(*res):
         assert torch.equal(one, again)
         assert float((one - two).abs().max()) <= 2e-5 * float(two.abs().max())   # sqrt(1035) * 2^-24 per sum, ten times over
+
+
+@pytest.mark.parametrize("case", ["plain", "equal", "offset", "outlier", "infinite", "few coordinates"])
+def test_hausdorff_expanded_form_and_hand_over(tpw, monkeypatch, case):
+    """Large set pairs run the expanded form, and go over to the direct one where its error leaves too many rows undecided:
+    values and indices of the exact loop either way, with and without a shuffled visiting order."""
+    d = 2 if case == "few coordinates" else 3
+    g = torch.Generator().manual_seed(len(case))
+    x1 = torch.rand(2, 1, 6007, d, generator=g) * 2 - 1
+    x2 = x1[:, :, torch.randperm(6007, generator=g)] + 0.05 * torch.randn(2, 1, 6007, d, generator=g)
+    if case == "equal":
+        x2 = x1.clone()
+    elif case == "offset":
+        x1, x2 = x1 + 3e3, x2 + 3e3
+    elif case == "outlier":
+        x2[1, 0, 17] = 1e19
+    elif case == "infinite":
+        x1[0, 0, 4000, 1], x2[1, 0, 0, 0] = math.inf, math.nan
+    for shuffle in (False, True):
+        res = []
+        for exact in (False, True):
+            if exact:
+                monkeypatch.setenv("TPW_HAUSDORFF_EXACT_LOOP", "1")
+            gen = torch.Generator(device="cuda").manual_seed(5) if shuffle else None
+            res.append(tpw.directed_hausdorff_distances(x1.cuda(), x2.cuda(), shuffle=shuffle, generator=gen))
+            monkeypatch.delenv("TPW_HAUSDORFF_EXACT_LOOP", raising=False)
+        for a, w in zip(*res):
+            assert torch.equal(a, w), (case, shuffle)
+
+
+def test_quotients_of_counts_round_as_the_division(tpw):
+    """Every quotient of counts with a denominator up to 300, through the metrics themselves: row i of x1 has its first i
+    features set, row j of x2 its first j, so jaccard is |i - j| / max(i, j) and hamming |i - j| / D for every i, j, D."""
+    for d in (129, 160, 257, 300):
+        n = d + 1
+        x = (torch.arange(d)[None, :] < torch.arange(n)[:, None]).cuda()
+        x2 = x.repeat(40, 1)                      # enough pairs for the tensor-core counts
+        from torchpairwise_b200 import _abi
+        if _abi.lib.tpw_bool_rows_pitch(1, n, 40 * n, d) == 0:
+            x, x2 = x.repeat(2, 1), x.repeat(200, 1)
+        assert _abi.lib.tpw_bool_rows_pitch(1, x.size(0), x2.size(0), d) > 0
+        i, j = x.sum(1).float(), x2.sum(1).float()
+        diff, most = (i[:, None] - j[None, :]).abs(), torch.maximum(i[:, None], j[None, :])
+        # float64 division of integers this small, rounded once more to float32, is the correctly rounded quotient
+        assert torch.equal(tpw.jaccard_distances(x, x2), torch.where(most > 0, diff.double() / most.double(), 0.0).float())
+        assert torch.equal(tpw.hamming_distances(x, x2), (diff.double() / d).float())

@@ -82,6 +82,8 @@ def load_torch_ops() -> str:
     if not TORCH_OPS_LIBRARY.exists():
         raise ImportError(f"{TORCH_OPS_LIBRARY} is missing; run `python torchpairwise_b200/build.py`")
     torch.ops.load_library(str(TORCH_OPS_LIBRARY))
+    from . import ops
+    ops._native_ops = torch.ops.torchpairwise
     return str(TORCH_OPS_LIBRARY)
 
 

@@ -155,17 +155,21 @@ bool tensor_engine_selected(const Prepared &p) {
 // With `cosine` set (epilogue >= 0, the two norm vectors) the call is the whole cosine-family backward,
 // tpw_cosine_backward_ws, with g the upstream gradient and aux the saved forward result; it returns
 // false without doing anything when the engine rule keeps the problem on the CUDA cores.
-// tpw_lp_backward, through the one-pass kernel (both gradients from one walk over the pairs) where the library offers it
+// NULL for a gradient nobody asked for
+void *data_or_null(const Tensor &t) { return t.defined() ? t.data_ptr() : nullptr; }
+
+// tpw_lp_backward, through the one-pass kernel (both gradients from one walk over the pairs) where the library offers it;
+// an undefined g1 or g2 is left out
 void lp_backward_call(int code, int mode, const Tensor &g, const void *aux, const Tensor &a, const Tensor &b, const void *w,
                       Tensor &g1, Tensor &g2, int64_t B, int64_t N1, int64_t N2, int64_t D, double p) {
-    const int64_t bytes = tpw_lp_backward_scratch_bytes(code, mode, B, N1, N2, D, p);
+    const int64_t bytes = g1.defined() && g2.defined() ? tpw_lp_backward_scratch_bytes(code, mode, B, N1, N2, D, p) : 0;
     if (bytes <= 0) {
-        TPW_CALL(tpw_lp_backward(code, mode, g.data_ptr(), aux, a.data_ptr(), b.data_ptr(), w, g1.data_ptr(), g2.data_ptr(),
+        TPW_CALL(tpw_lp_backward(code, mode, g.data_ptr(), aux, a.data_ptr(), b.data_ptr(), w, data_or_null(g1), data_or_null(g2),
                                  B, N1, N2, D, p, stream_of(a)));
         return;
     }
     Tensor scratch = at::empty({bytes}, a.options().dtype(at::kByte));
-    TPW_CALL(tpw_lp_backward_ws(code, mode, g.data_ptr(), aux, a.data_ptr(), b.data_ptr(), w, g1.data_ptr(), g2.data_ptr(),
+    TPW_CALL(tpw_lp_backward_ws(code, mode, g.data_ptr(), aux, a.data_ptr(), b.data_ptr(), w, data_or_null(g1), data_or_null(g2),
                                 B, N1, N2, D, p, scratch.data_ptr(), bytes, stream_of(a)));
 }
 
@@ -203,8 +207,10 @@ bool dense_backward(int mode, const Tensor &g, const Tensor *aux, const Tensor &
         for (int64_t r0 = 0; r0 < N1; r0 += rows) {
             const int64_t rn = std::min(rows, N1 - r0);
             Tensor gv = g.narrow(0, b0, bn).narrow(1, r0, rn), av = a.narrow(0, b0, bn).narrow(1, r0, rn);
-            Tensor g1v = g1.narrow(0, b0, bn).narrow(1, r0, rn), g2v = g2.narrow(0, b0, bn);
-            if (r0 > 0) {
+            Tensor g1v, g2v;
+            if (g1.defined()) g1v = g1.narrow(0, b0, bn).narrow(1, r0, rn);
+            if (g2.defined()) g2v = g2.narrow(0, b0, bn);
+            if (r0 > 0 && g2.defined()) {
                 if (!part.defined()) part = at::empty_like(g2v);
                 g2v = part;
             }
@@ -212,11 +218,11 @@ bool dense_backward(int mode, const Tensor &g, const Tensor *aux, const Tensor &
             if (cosine.epilogue >= 0)
                 TPW_CALL(tpw_cosine_backward_ws(cosine.epilogue, gv.data_ptr(), auxp, cosine.n1->narrow(0, b0, bn).narrow(1, r0, rn).data_ptr(),
                                                 cosine.n2->narrow(0, b0, bn).data_ptr(), av.data_ptr(), b.narrow(0, b0, bn).data_ptr(),
-                                                g1v.data_ptr(), g2v.data_ptr(), scratch.data_ptr(), bytes, bn, rn, N2, D, st));
+                                                data_or_null(g1v), data_or_null(g2v), scratch.data_ptr(), bytes, bn, rn, N2, D, st));
             else
                 TPW_CALL(tpw_dot_backward_ws(code, mode, eng, gv.data_ptr(), auxp, av.data_ptr(), b.narrow(0, b0, bn).data_ptr(),
-                                             g1v.data_ptr(), g2v.data_ptr(), scratch.data_ptr(), bytes, bn, rn, N2, D, st));
-            if (r0 > 0) g2.narrow(0, b0, bn).add_(part);
+                                             data_or_null(g1v), data_or_null(g2v), scratch.data_ptr(), bytes, bn, rn, N2, D, st));
+            if (r0 > 0 && g2.defined()) g2.narrow(0, b0, bn).add_(part);
         }
     }
     return true;
@@ -253,18 +259,20 @@ struct CdistFn : torch::autograd::Function<CdistFn> {
         c10::cuda::CUDAGuard dg(a.device());
         Tensor g = go[0].to(a.scalar_type()).contiguous();
         if (ub) g = g.unsqueeze(0);
-        Tensor g1 = at::empty_like(a), g2 = at::empty_like(b);
-        if (p == 0) { g1.zero_(); g2.zero_(); }
+        Tensor g1, g2;
+        if (ctx->needs_input_grad(0)) g1 = p == 0 ? at::zeros_like(a) : at::empty_like(a);
+        if (ctx->needs_input_grad(1)) g2 = p == 0 ? at::zeros_like(b) : at::empty_like(b);
+        if (p == 0 || (!g1.defined() && !g2.defined())) {}
         else if (p == 2 && a.numel() > 0 && b.numel() > 0) dense_backward(TPW_LP_BWD_CDIST, g, &out, a, b, g1, g2);
         else if (std::isinf(p) && tpw_chebyshev_backward_scratch_bytes(code_of(a), a.size(0), a.size(1), b.size(1), a.size(2)) > 0) {
             // Chebyshev: find the attaining coordinate of every pair once, then scatter both gradients
             const int64_t bytes = tpw_chebyshev_backward_scratch_bytes(code_of(a), a.size(0), a.size(1), b.size(1), a.size(2));
             Tensor scratch = at::empty({bytes}, a.options().dtype(at::kByte));
-            TPW_CALL(tpw_chebyshev_backward_ws(g.data_ptr(), out.data_ptr(), a.data_ptr(), b.data_ptr(), g1.data_ptr(), g2.data_ptr(),
+            TPW_CALL(tpw_chebyshev_backward_ws(g.data_ptr(), out.data_ptr(), a.data_ptr(), b.data_ptr(), data_or_null(g1), data_or_null(g2),
                                                scratch.data_ptr(), bytes, a.size(0), a.size(1), b.size(1), a.size(2), stream_of(a)));
         }
         else lp_backward_call(code_of(a), TPW_LP_BWD_CDIST, g, out.data_ptr(), a, b, nullptr, g1, g2, a.size(0), a.size(1), b.size(1), a.size(2), p);
-        return {finish(g1, ub, dt), finish(g2, ub, dt), Tensor()};
+        return {g1.defined() ? finish(g1, ub, dt) : g1, g2.defined() ? finish(g2, ub, dt) : g2, Tensor()};
     }
 };
 

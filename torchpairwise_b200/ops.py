@@ -26,6 +26,9 @@ _ENGINE_NAMES = {"auto": _abi.ENGINE_AUTO, "simt": _abi.ENGINE_SIMT_FP32, "tcgen
 _dot_engine = _ENGINE_NAMES.get(os.environ.get("TPW_DOT_ENGINE", "auto").lower(), _abi.ENGINE_AUTO)
 
 
+_native_ops = None  # torch.ops.torchpairwise after load_torch_ops()
+
+
 def set_dot_engine(name: str) -> None:
     """Engine of the dense-contraction metrics (sqeuclidean, euclidean, cosine, correlation,
     linear kernel) for float32 inputs: "auto" (tensor cores for large problems, CUDA cores
@@ -802,6 +805,12 @@ def _cdist_p(x1: Tensor, x2: Tensor, p: float) -> Tensor:
         raise RuntimeError("cdist only supports non-negative p values")
     if x1.dim() == 3 and x2.dim() == 3 and x1.size(0) != x2.size(0):
         raise RuntimeError("batch_size of x1 and x2 do not match.")
+    if _native_ops is not None and _dot_engine == _abi.ENGINE_AUTO and x1.dtype == x2.dtype and x1.is_floating_point() \
+            and x1.dim() == x2.dim() and x1.size(-1) == x2.size(-1):
+        # The same launches and the same gradient formulas from the C++ host layer, once it is loaded: an autograd node that
+        # the engine's device thread runs without the interpreter.  euclidean [75, 5, 64] forward and backward, bound by
+        # the host: 146 -> 77 us.  Anything the checks above would refuse, and a chosen engine, stays below.
+        return _native_ops.minkowski_distances(x1, x2, float(p))
     return _CdistFunction.apply(x1, x2, float(p))
 
 
