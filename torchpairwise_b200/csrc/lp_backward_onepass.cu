@@ -473,7 +473,10 @@ long long lp_backward_onepass_scratch_bytes(int mode, long long B, long long N1,
     if (B <= 0 || N1 < OP_ROWS || N2 < OP_JT || D < 16 || D % 4 != 0) return 0;
     if (B >= (1ll << 31) || N1 >= kMaxRows || N2 >= (1ll << 31) || D >= (1ll << 31)) return 0;
     const long long nblk = (N1 + OP_ROWS - 1) / OP_ROWS, tiles_k = (D + OP_FEAT - 1) / OP_FEAT;
-    if (nblk * OP_ROWS * 4 > N1 * 5 || tiles_k * OP_FEAT * 4 > D * 5) return 0;   // more than a quarter of a tile idle
+    // The two-launch tile has 128 rows and 128 features, so features idle in this tile's 64 idle there too; rows may be idle up
+    // to the half of them by which the second launch costs more.  minkowski p = 3, forward and backward: [5, 2910, 1602, 100]
+    // 2860 -> 998 us, [6, 384, 663, 192] 318 -> 146 us.
+    if (nblk * OP_ROWS * 2 > N1 * 3) return 0;
     // four launches instead of two, and one CTA per SM: from 2^26 terms on, on at least half of the SMs
     if ((double)B * (double)N1 * (double)N2 * (double)D < 67108864.0) return 0;
     const long long splits = walk_splits(B * nblk * tiles_k, N2);

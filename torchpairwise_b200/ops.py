@@ -138,7 +138,20 @@ def _sizes(x1c: Tensor, x2c: Tensor):
 # --------------------------------------------------------------------------------------------
 # raw launches (no autograd)
 # --------------------------------------------------------------------------------------------
+def _worth_padding(x1c: Tensor, x2c: Tensor, p: float) -> bool:
+    """float32 rows that start on no 16-byte boundary, from 2^26 terms on: zero features cost less than kernels without TMA
+    (the reasons and figures stand at ``worth_padding`` in csrc/torch/tpw_torch.cpp)."""
+    B, N1, N2, D = _sizes(x1c, x2c)
+    return x1c.dtype == torch.float32 and D % 4 != 0 and D > 32 and p > 0 and B * N1 * N2 * D >= 1 << 26
+
+
+def _pad_features(xc: Tensor) -> Tensor:
+    return torch.nn.functional.pad(xc, (0, -xc.size(2) % 4))
+
+
 def _lp_forward_raw(x1c: Tensor, x2c: Tensor, w: Optional[Tensor], p: float, out_exponent: float) -> Tensor:
+    if w is None and _worth_padding(x1c, x2c, p):
+        return _lp_forward_raw(_pad_features(x1c), _pad_features(x2c), w, p, out_exponent)
     B, N1, N2, D = _sizes(x1c, x2c)
     out = torch.empty((B, N1, N2), dtype=x1c.dtype, device=x1c.device)
     if D == 0:
@@ -152,6 +165,9 @@ def _lp_forward_raw(x1c: Tensor, x2c: Tensor, w: Optional[Tensor], p: float, out
 def _lp_backward_raw(mode: int, grad: Tensor, aux: Optional[Tensor], x1c: Tensor, x2c: Tensor,
                      w: Optional[Tensor], p: float, need1: bool = True, need2: bool = True):
     B, N1, N2, D = _sizes(x1c, x2c)
+    if mode == _abi.LP_BWD_CDIST and w is None and p != 2 and _worth_padding(x1c, x2c, p):
+        res = _lp_backward_raw(mode, grad, aux, _pad_features(x1c), _pad_features(x2c), w, p, need1, need2)
+        return tuple(None if r is None else r[..., :D].contiguous() for r in res)
     if mode == _abi.LP_BWD_CDIST and w is None and math.isinf(p) and p > 0 and (need1 or need2):
         # Chebyshev: find the attaining coordinate of every pair once, then scatter both gradients
         code = _FLOAT_CODES[x1c.dtype]
