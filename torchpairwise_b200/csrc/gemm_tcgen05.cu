@@ -27,10 +27,13 @@
 // roles poll, everybody falls through to the final barrier, tensor memory is released, and the
 // device status word reports the site.
 #include "common.cuh"
+#include "packed_f32x2.cuh"
 #include "tcgen05.cuh"
 
 #include <cuda_bf16.h>
 #include <math.h>
+
+#include <type_traits>
 
 namespace tpw {
 namespace {
@@ -66,11 +69,14 @@ struct GemmParams {
     int vec_store;            // N2 % 4 == 0 and out 16-byte aligned
     int kchunk;               // k-steps accumulated in tensor memory before the sum moves to registers (0: all)
     unsigned long long *rowmin_keys; // ROWMIN instantiation: [B*N1] keys (float bits << 32 | x2 row), nothing is stored to out
-    // TOPK instantiations: per row and per (column tile, half) a sorted list of the k smallest keys,
-    // [B*N1][topk_L][topk_k], and [B*N1] published upper bounds of the row's k-th smallest key
+    // TOPK > 0: [B*N1] upper bounds of the row's k-th smallest key, [B*N1] numbers of keys written so far, and per row
+    // room for k keys from every (column tile, half), [B*N1][topk_L * topk_k], filled from the front
     unsigned long long *topk_lists, *topk_thr;
+    int *topk_count;
     int topk_k, topk_L;
-    long long tn0;            // first column tile of this launch (tiles_n counts from it); top-k runs in column ranges
+    float *gmin;              // TOPK < 0: [B*N1][8 * tiles_n] minima of the groups of 32 columns
+    const int *lo_any;        // [2] whether any low part of the x (y) operand is non-zero; NULL: treat both as non-zero
+    int lo_always;            // bit 0 / 1: the x / y operand's low parts are used whatever lo_any says
     int *status;
 };
 
@@ -129,6 +135,17 @@ __device__ __forceinline__ float dot_epilogue(float dot, float n1, float n2, boo
     return dist;
 }
 
+// dot_epilogue without the cosine distance's upper clamp, for the top-k epilogue: columns are ordered the same way as long as
+// the limit they are compared with lies below 2, so only the few that pass are clamped.
+template <int EPI>
+__device__ __forceinline__ float raw_distance(float dot, float n1, float n2) {
+    return EPI == TPW_DOT_SQEUCLIDEAN ? dot_epilogue<EPI>(dot, n1, n2, false) : fmaxf(1.f - dot * (n1 * n2), 0.f);
+}
+template <int EPI>
+__device__ __forceinline__ float clamp_distance(float raw) {
+    return EPI == TPW_DOT_SQEUCLIDEAN ? raw : fminf(raw, 2.f);
+}
+
 // TF32 = false: operands are bf16 high/low parts, 64 per k-step; true: tf32 high/low parts in fp32
 // containers, 32 per k-step.  Either way a k-step is one 128-byte swizzled row per operand row and
 // four MMAs per operand pair, so the pipeline below is the same.
@@ -140,7 +157,7 @@ template <bool ROW_TILES_FASTEST>
 __device__ __forceinline__ void decode_tile(long long tile, const GemmParams &P, long long &tn, long long &tm, long long &b) {
     if (ROW_TILES_FASTEST) {
         tm = tile % P.tiles_m; tile /= P.tiles_m;
-        tn = tile % P.tiles_n + P.tn0;
+        tn = tile % P.tiles_n;
         b = tile / P.tiles_n;
     } else {
         tn = tile % P.tiles_n; tile /= P.tiles_n;
@@ -215,6 +232,12 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
     __syncthreads();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr;
+    // Operands that the high parts hold exactly (16-bit inputs, small integers) have no low parts: their tiles are neither
+    // loaded nor multiplied.  The products left out are zeros added to a finished sum; an infinite or NaN input has a NaN low part.
+    // cosine of bfloat16 [5000, 768] x [4111, 768], forward and backward: 707 -> 652 us.
+    const bool need_xl = !P.lo_any || (P.lo_always & 1) || P.lo_any[0] != 0;
+    const bool need_yl = !P.lo_any || (P.lo_always & 2) || P.lo_any[1] != 0;
+    const uint32_t lo_bytes = (need_xl ? A_BYTES : 0) + (need_yl ? B_BYTES : 0);
 
     if (warp == 0) {
         // ---------------- TMA producer ----------------
@@ -250,15 +273,18 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                     } else {
                         tma_load_3d(st + 2 * A_BYTES, &map_yh, &full[s], kb * BKE, (int)(tn * BN), (int)b);
                     }
-                    mbar_expect_tx(&full_lo[s], A_BYTES + B_BYTES);
-                    if constexpr (AMN) {
+                    if (lo_bytes == 0) continue;
+                    mbar_expect_tx(&full_lo[s], lo_bytes);
+                    if (!need_xl) {
+                    } else if constexpr (AMN) {
 #pragma unroll
                         for (int m = 0; m < BM / 32; ++m)
                             tma_load_3d(st + A_BYTES + m * 4096, &map_xl, &full_lo[s], (int)(tm * BM) + 32 * m, kb * BKE, (int)b);
                     } else {
                         tma_load_3d(st + A_BYTES, &map_xl, &full_lo[s], kb * BKE, (int)(tm * BM), (int)b);
                     }
-                    if constexpr (BMN) {
+                    if (!need_yl) {
+                    } else if constexpr (BMN) {
 #pragma unroll
                         for (int m = 0; m < BN / 32; ++m)
                             tma_load_3d(st + 2 * A_BYTES + B_BYTES + m * 4096, &map_yl, &full_lo[s], (int)(tn * BN) + 32 * m, kb * BKE, (int)b);
@@ -309,6 +335,10 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
 #pragma unroll
                         for (int k = 0; k < kMmasPerStep; ++k)
                             tc_mma<TF32>(d_tmem, dxh + ka * k, dyh + kbn * k, idesc, ((kb - kb0) | k) != 0);
+                        if (lo_bytes == 0) {
+                            tc_commit(&empty[s]);
+                            continue;
+                        }
                         if (!wait_or_abort(&full_lo[s], (it / kStages) & 1, abort_flag)) {
                             *abort_flag = 1;
                             if (P.status) atomicCAS(P.status, 0, (4 << 16) | 5);
@@ -316,10 +346,16 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                             break;
                         }
                         tc_fence_after();
+                        if (need_xl && need_yl) {
 #pragma unroll
-                        for (int k = 0; k < kMmasPerStep; ++k) {
-                            tc_mma<TF32>(d_tmem, dxh + ka * k, dyl + kbn * k, idesc, 1);
-                            tc_mma<TF32>(d_tmem, dxl + ka * k, dyh + kbn * k, idesc, 1);
+                            for (int k = 0; k < kMmasPerStep; ++k) {
+                                tc_mma<TF32>(d_tmem, dxh + ka * k, dyl + kbn * k, idesc, 1);
+                                tc_mma<TF32>(d_tmem, dxl + ka * k, dyh + kbn * k, idesc, 1);
+                            }
+                        } else {
+                            const uint64_t da = need_xl ? dxl : dxh, db = need_xl ? dyh : dyl;
+#pragma unroll
+                            for (int k = 0; k < kMmasPerStep; ++k) tc_mma<TF32>(d_tmem, da + ka * k, db + kbn * k, idesc, 1);
                         }
                         tc_commit(&empty[s]); // the stage may be refilled once these MMAs have read it
                     }
@@ -412,36 +448,102 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
             const float n1 = (EPI != TPW_DOT_LINEAR && row_ok) ? P.n1sq[b * P.N1 + i] : 0.f;
             const float *n2p = P.n2sq + b * P.N2;
             unsigned long long best = ~0ull;
-            // TOPK: a fresh list per tile half; candidates at or above an already published bound of the
-            // row's k-th smallest key cannot be among its k smallest and are dropped before the insertion
-            unsigned long long lst[TOPK > 0 ? TOPK : 1];
+            // TOPK > 0: keys at or above the bound of the row's k-th smallest key cannot be among its k smallest
             unsigned long long bound = 0;
             if constexpr (TOPK > 0) {
-#pragma unroll
-                for (int t = 0; t < TOPK; ++t) lst[t] = ~0ull;
-                if (row_ok) bound = *reinterpret_cast<volatile unsigned long long *>(P.topk_thr + b * P.N1 + i);
+                if (row_ok) bound = __ldg(P.topk_thr + b * P.N1 + i);   // rows past N1: nothing passes
             }
-            if constexpr (TOPK > 0) {
-                // eight columns at a time, so that the unrolled body (and its insertion code) stays small;
-                // the insertion is entered only when some lane of the warp has a candidate below its bounds
+            if constexpr (TOPK != 0) {
+                // Columns past N2 count as NaN, which no minimum takes and no comparison passes.  TOPK < 0 keeps the minimum of
+                // every 32 columns.  TOPK > 0: the minimum of eight distances decides for all of them whether any lane of the
+                // warp has one within its limit; then every lane puts its next passing column into its own words of the
+                // staging area, until none has one left (most tile halves have none or one a lane), and once a lane
+                // holds k keys the largest gives way to a smaller one.
+                const int k = P.topk_k;
+                unsigned long long *buf = reinterpret_cast<unsigned long long *>(smem + OFF_STAGE + (warp - 2) * 4096) + lane;   // [k][32 lanes]
+                int cnt = 0, worst = 0;                       // keys held, slot of the largest once there are k
+                unsigned long long limit = bound;             // keys have to stay below it
+                auto limit_value = [&]() {                    // every distance whose key is below the limit is at most this
+                    const uint32_t hi = (uint32_t)(limit >> 32);
+                    // a limit at or above the upper clamp lets every raw value through
+                    return hi >= 0x7f800000u || (EPI == TPW_DOT_COSINE_DIST && hi >= 0x40000000u) ? INFINITY : __uint_as_float(hi);
+                };
+                float lim = limit_value();
 #pragma unroll 1
-                for (int g = 0; g < BN / 16; ++g) {
-                    const long long j0 = tn * BN + chalf * (BN / 2) + g * 8;
-                    if (j0 >= P.N2) break;
-                    uint32_t r8[8];
-                    tmem_ld8(tmem_base + ((uint32_t)(q * 32) << 16) + a * BN + chalf * (BN / 2) + g * 8, r8);
-                    tmem_ld_wait();
+                for (int c = chalf * (BN / 64); c < (chalf + 1) * (BN / 64); ++c) {
+                    const long long j0 = tn * BN + c * 32;
+                    float gm = INFINITY;
+                    if (j0 < P.N2) {
+                        uint32_t r[32];
+                        tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + a * BN + c * 32, r);
+                        tmem_ld_wait();
+                        const bool whole = P.vec_store && j0 + 32 <= P.N2;
 #pragma unroll
-                    for (int v = 0; v < 8; ++v) {
-                        const long long j = j0 + v;
-                        const float nn = j < P.N2 ? __ldg(n2p + j) : 0.f;
-                        const float o = dot_epilogue<EPI>(__uint_as_float(r8[v]), n1, nn, false);
-                        const unsigned long long key = ((unsigned long long)__float_as_uint(o) << 32) | (unsigned long long)(uint32_t)j;
-                        const bool cand = j < P.N2 && key < bound && key < lst[TOPK - 1];
-                        if (__any_sync(0xffffffffu, cand)) {
-                            if (cand) sorted_insert<TOPK>(lst, key);
+                        for (int g = 0; g < 4; ++g) {
+                            float nn[8], o[8];
+                            if (whole) {
+#pragma unroll
+                                for (int u = 0; u < 2; ++u) {
+                                    const float4 v4 = __ldg(reinterpret_cast<const float4 *>(n2p + j0 + 8 * g) + u);
+                                    nn[4 * u] = v4.x; nn[4 * u + 1] = v4.y; nn[4 * u + 2] = v4.z; nn[4 * u + 3] = v4.w;
+                                }
+                            } else {
+#pragma unroll
+                                for (int v = 0; v < 8; ++v) nn[v] = j0 + 8 * g + v < P.N2 ? __ldg(n2p + j0 + 8 * g + v) : 0.f;
+                            }
+#pragma unroll
+                            for (int v = 0; v < 8; ++v) {
+                                o[v] = raw_distance<EPI>(__uint_as_float(r[8 * g + v]), n1, nn[v]);
+                                if (!whole && j0 + 8 * g + v >= P.N2) o[v] = NAN;
+                            }
+                            const float m = min3(min3(o[0], o[1], o[2]), min3(o[3], o[4], o[5]), fminf(o[6], o[7]));
+                            if constexpr (TOPK < 0) {
+                                gm = fminf(gm, m);
+                            } else if (__any_sync(0xffffffffu, m <= lim)) {
+                                uint32_t mask = 0;
+#pragma unroll
+                                for (int v = 0; v < 8; ++v)
+                                    if (o[v] <= lim) mask |= 1u << v;
+#pragma unroll 1
+                                while (__any_sync(0xffffffffu, mask != 0)) {
+                                    const int v = __ffs(mask) - 1;       // -1: nothing left in this lane
+                                    mask &= mask - 1;
+                                    float ov = o[0];
+#pragma unroll
+                                    for (int u = 1; u < 8; ++u)
+                                        if (v == u) ov = o[u];
+                                    const unsigned long long key = ((unsigned long long)__float_as_uint(clamp_distance<EPI>(ov)) << 32) |
+                                                                   (unsigned long long)(uint32_t)(j0 + 8 * g + v);
+                                    const bool take = v >= 0 && key < limit;
+                                    if (take) buf[(cnt < k ? cnt : worst) * 32] = key;
+                                    if (take && ++cnt >= k) {
+                                        cnt = k;
+                                        limit = 0;
+#pragma unroll 1
+                                        for (int t = 0; t < k; ++t) {
+                                            const unsigned long long held = buf[t * 32];
+                                            if (held >= limit) { limit = held; worst = t; }
+                                        }
+                                        lim = limit_value();
+                                    }
+                                }
+                            }
                         }
                     }
+                    if constexpr (TOPK < 0) {
+                        if (row_ok) P.gmin[((b * P.N1 + i) * P.tiles_n + tn) * 8 + c] = clamp_distance<EPI>(gm);
+                    }
+                }
+                if constexpr (TOPK > 0) {
+                    // behind the keys that other tile halves have written (their order does not matter: the keys are unique
+                    // and the merge looks at all of them)
+                    if (cnt > 0) {
+                        const int at = atomicAdd(P.topk_count + b * P.N1 + i, cnt);
+                        unsigned long long *dst = P.topk_lists + (b * P.N1 + i) * P.topk_L * k + at;
+#pragma unroll 1
+                        for (int t = 0; t < cnt; ++t) dst[t] = buf[t * 32];
+                    }
+                    __syncwarp();
                 }
             } else
 #pragma unroll 1
@@ -469,26 +571,30 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                 unsigned char *stg = smem + OFF_STAGE + (warp - 2) * 4096;
                 const long long row_base = tm * BM + q * 32;
                 const bool whole = P.vec_store && j0 + 32 <= P.N2;
+                auto stage = [&](auto whole_tag) {
+                    constexpr bool WHOLE = decltype(whole_tag)::value;
 #pragma unroll
-                for (int v = 0; v < 8; ++v) {
-                    float4 nn = make_float4(0.f, 0.f, 0.f, 0.f);
-                    if (EPI != TPW_DOT_LINEAR) {
-                        if (whole) {
-                            nn = __ldg(reinterpret_cast<const float4 *>(n2p + j0) + v);
-                        } else {
-                            if (j0 + 4 * v + 0 < P.N2) nn.x = __ldg(n2p + j0 + 4 * v + 0);
-                            if (j0 + 4 * v + 1 < P.N2) nn.y = __ldg(n2p + j0 + 4 * v + 1);
-                            if (j0 + 4 * v + 2 < P.N2) nn.z = __ldg(n2p + j0 + 4 * v + 2);
-                            if (j0 + 4 * v + 3 < P.N2) nn.w = __ldg(n2p + j0 + 4 * v + 3);
+                    for (int v = 0; v < 8; ++v) {
+                        float4 nn = make_float4(0.f, 0.f, 0.f, 0.f);
+                        if (EPI != TPW_DOT_LINEAR) {
+                            if (WHOLE) {
+                                nn = __ldg(reinterpret_cast<const float4 *>(n2p + j0) + v);
+                            } else {
+                                if (j0 + 4 * v + 0 < P.N2) nn.x = __ldg(n2p + j0 + 4 * v + 0);
+                                if (j0 + 4 * v + 1 < P.N2) nn.y = __ldg(n2p + j0 + 4 * v + 1);
+                                if (j0 + 4 * v + 2 < P.N2) nn.z = __ldg(n2p + j0 + 4 * v + 2);
+                                if (j0 + 4 * v + 3 < P.N2) nn.w = __ldg(n2p + j0 + 4 * v + 3);
+                            }
                         }
+                        float4 o;
+                        o.x = dot_epilogue<EPI>(__uint_as_float(r[4 * v + 0]), n1, nn.x, SELF && i == j0 + 4 * v + 0);
+                        o.y = dot_epilogue<EPI>(__uint_as_float(r[4 * v + 1]), n1, nn.y, SELF && i == j0 + 4 * v + 1);
+                        o.z = dot_epilogue<EPI>(__uint_as_float(r[4 * v + 2]), n1, nn.z, SELF && i == j0 + 4 * v + 2);
+                        o.w = dot_epilogue<EPI>(__uint_as_float(r[4 * v + 3]), n1, nn.w, SELF && i == j0 + 4 * v + 3);
+                        *reinterpret_cast<float4 *>(stg + lane * 128 + ((v ^ (lane & 7)) << 4)) = o;
                     }
-                    float4 o;
-                    o.x = dot_epilogue<EPI>(__uint_as_float(r[4 * v + 0]), n1, nn.x, SELF && i == j0 + 4 * v + 0);
-                    o.y = dot_epilogue<EPI>(__uint_as_float(r[4 * v + 1]), n1, nn.y, SELF && i == j0 + 4 * v + 1);
-                    o.z = dot_epilogue<EPI>(__uint_as_float(r[4 * v + 2]), n1, nn.z, SELF && i == j0 + 4 * v + 2);
-                    o.w = dot_epilogue<EPI>(__uint_as_float(r[4 * v + 3]), n1, nn.w, SELF && i == j0 + 4 * v + 3);
-                    *reinterpret_cast<float4 *>(stg + lane * 128 + ((v ^ (lane & 7)) << 4)) = o;
-                }
+                };
+                if (whole) stage(std::true_type{}); else stage(std::false_type{});
                 __syncwarp();
                 if (whole) {
                     // ... and written out four full 128-byte row segments per instruction
@@ -506,18 +612,6 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
             }
             if constexpr (ROWMIN) {
                 if (row_ok && best != ~0ull) atomicMin(P.rowmin_keys + b * P.N1 + i, best);
-            }
-            if constexpr (TOPK > 0) {
-                if (row_ok) {
-                    unsigned long long *dst = P.topk_lists + ((b * P.N1 + i) * P.topk_L + tn * 2 + chalf) * P.topk_k;
-                    unsigned long long kth = ~0ull;
-#pragma unroll
-                    for (int t = 0; t < TOPK; ++t) {
-                        if (t < P.topk_k && lst[t] != ~0ull) dst[t] = lst[t];
-                        if (t == P.topk_k - 1) kth = lst[t];
-                    }
-                    if (kth != ~0ull) atomicMin(P.topk_thr + b * P.N1 + i, kth); // k entries in this list: a valid bound
-                }
             }
             // this warp has drained its quarter of accumulator `a`
             tc_fence_before();
@@ -537,20 +631,41 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
 // fp32 rows -> bf16 high/low parts (row pitch Dp, zero padded) and a per-row fp32 scalar: the
 // squared norm, or (recip != 0) the reciprocal norm with 0 for an all-zero row; one warp per row
 __global__ void split_rows_kernel(const float *__restrict__ x, __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo,
-                                  float *__restrict__ nsq, long long rows, long long D, long long Dp, int recip) {
+                                  float *__restrict__ nsq, int *__restrict__ lo_any, long long rows, long long D, long long Dp, int recip) {
     const int lane = threadIdx.x & 31;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
+    uint32_t any = 0;                     // bits of all low parts but their signs: zero where they are all zero
+    const bool vec = D == Dp && (reinterpret_cast<uintptr_t>(x) & 15u) == 0;   // D a multiple of 8: 16 bytes in, 8 and 8 out
     for (long long r = warp; r < rows; r += nwarps) {
         const float *row = x + r * D;
         float s = 0.f;
-        for (long long k = lane; k < Dp; k += 32) {
-            const float v = k < D ? row[k] : 0.f;
-            const __nv_bfloat16 h = __float2bfloat16_rn(v);
-            const __nv_bfloat16 l = __float2bfloat16_rn(v - __bfloat162float(h));
-            hi[r * Dp + k] = h;
-            lo[r * Dp + k] = l;
-            s = fmaf(v, v, s);
+        auto split = [&](float v, uint32_t &hb, uint32_t &lb) {
+            const __nv_bfloat16 h = __float2bfloat16_rn(v), l = __float2bfloat16_rn(v - __bfloat162float(h));
+            hb = __bfloat16_as_ushort(h);
+            lb = __bfloat16_as_ushort(l);
+        };
+        if (vec) {
+            for (long long k = lane * 4; k < D; k += 128) {
+                const float4 v = __ldg(reinterpret_cast<const float4 *>(row + k));
+                uint32_t h[4], l[4];
+                split(v.x, h[0], l[0]); split(v.y, h[1], l[1]); split(v.z, h[2], l[2]); split(v.w, h[3], l[3]);
+                const uint2 hv = make_uint2(h[0] | (h[1] << 16), h[2] | (h[3] << 16)), lv = make_uint2(l[0] | (l[1] << 16), l[2] | (l[3] << 16));
+                *reinterpret_cast<uint2 *>(hi + r * Dp + k) = hv;
+                *reinterpret_cast<uint2 *>(lo + r * Dp + k) = lv;
+                any |= (lv.x | lv.y) & 0x7fff7fffu;
+                s = fmaf(v.x, v.x, s); s = fmaf(v.y, v.y, s); s = fmaf(v.z, v.z, s); s = fmaf(v.w, v.w, s);
+            }
+        } else {
+            for (long long k = lane; k < Dp; k += 32) {
+                const float v = k < D ? row[k] : 0.f;
+                uint32_t h, l;
+                split(v, h, l);
+                hi[r * Dp + k] = __ushort_as_bfloat16((unsigned short)h);
+                lo[r * Dp + k] = __ushort_as_bfloat16((unsigned short)l);
+                any |= l & 0x7fffu;
+                s = fmaf(v, v, s);
+            }
         }
 #pragma unroll
         for (int off = 16; off > 0; off >>= 1) s += __shfl_xor_sync(0xffffffffu, s, off);
@@ -563,6 +678,8 @@ __global__ void split_rows_kernel(const float *__restrict__ x, __nv_bfloat16 *__
             }
         }
     }
+    // one store per CTA: one per warp, 19 thousand to one address, queued up for 50 us
+    if (__syncthreads_or(any != 0) && threadIdx.x == 0) *lo_any = 1;
 }
 
 inline long long align_up(long long v, long long a) { return (v + a - 1) / a * a; }
@@ -574,7 +691,7 @@ inline bool auto_picks_tensor_cores(int dtype, long long B, long long N1, long l
 }
 
 struct ScratchLayout {
-    long long Dp, off_xh, off_xl, off_yh, off_yl, off_n1, off_n2, total;
+    long long Dp, off_xh, off_xl, off_yh, off_yl, off_n1, off_n2, off_lo, total;
 };
 
 inline ScratchLayout scratch_layout(long long B, long long N1, long long N2, long long D, bool self) {
@@ -587,7 +704,8 @@ inline ScratchLayout scratch_layout(long long B, long long N1, long long N2, lon
     L.off_yl = self ? L.off_xl : 2 * xa + ya;
     L.off_n1 = 2 * xa + 2 * ya;
     L.off_n2 = self ? L.off_n1 : L.off_n1 + align_up(B * N1 * 4, 1024);
-    L.total = L.off_n2 + align_up(B * N2 * 4, 1024);
+    L.off_lo = L.off_n2 + align_up(B * N2 * 4, 1024);
+    L.total = L.off_lo + 1024;
     return L;
 }
 
@@ -613,6 +731,7 @@ struct SplitParams {
     const float *a, *aux;       // [B,R,C]
     const float *n1, *n2;       // COEF_COSINE: row norms [B,R], [B,C]
     float *hi, *lo;             // [B,R,Cp]   (STRAIGHT)
+    int *lo_any;                // set to 1 where some low part is not zero; may be NULL
     float *rowpart, *colpart;   // [B,TC,R], [B,TR,C]   (SUMS)
     long long R, C, Cp, TR, TC;
     int vec_in;                 // C % 4 == 0 and 16-byte aligned inputs
@@ -668,6 +787,7 @@ split_tile_kernel(const SplitParams P) {
             if (col + e < P.C) nb[e] = P.n2[b * P.C + col + e];
     }
     float colp[4] = {0.f, 0.f, 0.f, 0.f};
+    uint32_t any = 0;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const long long row = r0 + ty + 16 * r;
@@ -707,6 +827,7 @@ split_tile_kernel(const SplitParams P) {
             h.w = rn_tf32(v[3]); l.w = rn_tf32(v[3] - h.w);
             *reinterpret_cast<float4 *>(P.hi + (b * P.R + row) * P.Cp + col) = h;
             *reinterpret_cast<float4 *>(P.lo + (b * P.R + row) * P.Cp + col) = l;
+            if (!SUMS) any |= (__float_as_uint(l.x) | __float_as_uint(l.y) | __float_as_uint(l.z) | __float_as_uint(l.w)) & 0x7fffffffu;
         }
         if (SUMS) {
             float s = (rs[0] + rs[1]) + (rs[2] + rs[3]);
@@ -715,15 +836,18 @@ split_tile_kernel(const SplitParams P) {
             if (tx == 0 && row < P.R) P.rowpart[(b * P.TC + blockIdx.x) * P.R + row] = s;
         }
     }
-    if (!SUMS) return;
+    if constexpr (!SUMS) {
+        if (P.lo_any && __syncthreads_or(any != 0) && tid == 0) *P.lo_any = 1;
+    } else {
 #pragma unroll
-    for (int e = 0; e < 4; ++e) colacc[ty * PT + 4 * tx + e] = colp[e];
-    __syncthreads();
-    if (tid < PT && c0 + tid < P.C) {
-        float s = 0.f;
+        for (int e = 0; e < 4; ++e) colacc[ty * PT + 4 * tx + e] = colp[e];
+        __syncthreads();
+        if (tid < PT && c0 + tid < P.C) {
+            float s = 0.f;
 #pragma unroll
-        for (int y = 0; y < 16; ++y) s += colacc[y * PT + tid];
-        P.colpart[(b * P.TR + blockIdx.y) * P.C + c0 + tid] = s;
+            for (int y = 0; y < 16; ++y) s += colacc[y * PT + tid];
+            P.colpart[(b * P.TR + blockIdx.y) * P.C + c0 + tid] = s;
+        }
     }
 }
 
@@ -750,7 +874,7 @@ __global__ void grad_finish_kernel(float *__restrict__ g, const float *__restric
 struct BwdScratch {
     long long N2p, Dp, TR, TC;
     long long off_chi, off_clo, off_x1hi, off_x1lo, off_x2hi, off_x2lo;
-    long long off_rowpart, off_colpart, off_rowsum, off_colsum, total;
+    long long off_rowpart, off_colpart, off_rowsum, off_colsum, off_lo, total;
 };
 
 inline BwdScratch bwd_scratch_layout(long long B, long long N1, long long N2, long long D) {
@@ -771,6 +895,7 @@ inline BwdScratch bwd_scratch_layout(long long B, long long N1, long long N2, lo
     L.off_colpart = take(B * L.TR * N2 * 4);
     L.off_rowsum = take(B * N1 * 4);
     L.off_colsum = take(B * N2 * 4);
+    L.off_lo = take(4 * sizeof(int));
     L.total = off;
     return L;
 }
@@ -800,7 +925,8 @@ struct Tf32Operand {
 
 // out[b,m,n] = sum_k A[b](m,k) * Bm[b](n,k); K = length of the reduction.  A K-major operand holds
 // `pitch` >= K elements per row (zero beyond K), an MN-major operand has exactly K rows per batch.
-int launch_tf32_product(const Tf32Operand &A, const Tf32Operand &Bm, float *out,
+// lo_any (may be NULL): lo_any[1] says whether Bm has any low part; A's are always used.
+int launch_tf32_product(const Tf32Operand &A, const Tf32Operand &Bm, float *out, const int *lo_any,
                         long long B, long long M, long long N, long long K, cudaStream_t s) {
     CUtensorMap mah, mal, mbh, mbl;
     int st;
@@ -820,6 +946,8 @@ int launch_tf32_product(const Tf32Operand &A, const Tf32Operand &Bm, float *out,
     P.tiles_n = (N + BN - 1) / BN;
     P.tiles = B * P.tiles_m * P.tiles_n;
     P.epilogue = TPW_DOT_LINEAR;
+    P.lo_any = lo_any;
+    P.lo_always = 1;
     // 64 elements per chunk: measured against float64, the products are then as accurate as the fp32
     // FMA chain of the CUDA-core kernel (the error grows in proportion to the chunk length) at no cost in time
     P.kchunk = 2;
@@ -875,52 +1003,89 @@ __global__ void dot_rowmin_finish_kernel(const unsigned long long *__restrict__ 
 
 namespace tpw {
 namespace {
-// One warp per row: the k smallest of the row's n candidate keys (lists written by the top-k epilogue;
-// unused slots hold ~0), ascending.  Every lane keeps the TOPK smallest of its share, then the warp
-// extracts the global minimum k times (keys are unique: the x2 row is part of the key).
-// bound_out (optional): the k-th smallest key itself, left untouched when fewer than k candidates exist.
-template <int TOPK>
-__global__ void topk_merge_kernel(const unsigned long long *__restrict__ lists, float *__restrict__ val_out,
-                                  long long *__restrict__ idx_out, unsigned long long *__restrict__ bound_out,
-                                  long long rows, long long row_stride, long long n, int k, int take_sqrt) {
+// A warp takes the k smallest of the n keys that key_of(e) returns, ascending: take(r, key), key the same in all lanes, ~0 where
+// there are fewer.  Keys are unique (the x2 row, or the group, is part of the key).  Up to 128 keys, the usual case, lie
+// four to a lane as they come, and each round costs two warp-wide minimum reductions; of more keys every lane first
+// keeps the TOPK smallest of its share.  (Sorted insertion and 64-bit shuffles for every row, as it was: 104 keys a row,
+// 50000 rows, 127 -> 40 us.)
+__device__ __forceinline__ unsigned long long warp_min(unsigned long long v) {
+    const uint32_t hi = __reduce_min_sync(0xffffffffu, (uint32_t)(v >> 32));
+    const uint32_t lo = __reduce_min_sync(0xffffffffu, (uint32_t)(v >> 32) == hi ? (uint32_t)v : 0xffffffffu);
+    return ((unsigned long long)hi << 32) | lo;
+}
+template <int TOPK, typename K, typename F>
+__device__ __forceinline__ void warp_smallest(long long n, int k, K key_of, F take) {
     const int lane = threadIdx.x & 31;
-    const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-    if (row >= rows) return;
+    if (n <= 128) {
+        unsigned long long mine[4];
+#pragma unroll
+        for (int t = 0; t < 4; ++t) mine[t] = t * 32 + lane < n ? key_of(t * 32 + lane) : ~0ull;
+        for (int r = 0; r < k; ++r) {
+            const unsigned long long a = mine[0] < mine[1] ? mine[0] : mine[1], b = mine[2] < mine[3] ? mine[2] : mine[3];
+            const unsigned long long m = warp_min(a < b ? a : b);
+#pragma unroll
+            for (int t = 0; t < 4; ++t)
+                if (mine[t] == m) mine[t] = ~0ull;
+            take(r, m);
+        }
+        return;
+    }
     unsigned long long mine[TOPK];
 #pragma unroll
     for (int t = 0; t < TOPK; ++t) mine[t] = ~0ull;
-    const unsigned long long *src = lists + row * row_stride;
     for (long long e = lane; e < n; e += 32) {
-        const unsigned long long key = src[e];
+        const unsigned long long key = key_of(e);
         if (key < mine[TOPK - 1]) sorted_insert<TOPK>(mine, key);
     }
     for (int r = 0; r < k; ++r) {
-        unsigned long long m = mine[0];
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            const unsigned long long other = __shfl_xor_sync(0xffffffffu, m, off);
-            m = other < m ? other : m;
-        }
+        const unsigned long long m = warp_min(mine[0]);
         if (m != ~0ull && mine[0] == m) { // the owner pops its head
 #pragma unroll
             for (int t = 0; t < TOPK - 1; ++t) mine[t] = mine[t + 1];
             mine[TOPK - 1] = ~0ull;
         }
-        if (lane == 0) {
-            const bool none = m == ~0ull;
-            float v = none ? __int_as_float(0x7f800000) : __uint_as_float((uint32_t)(m >> 32));
-            if (take_sqrt) v = sqrtf(v);
-            if (val_out) val_out[row * k + r] = v;
-            if (idx_out) idx_out[row * k + r] = none ? -1ll : (long long)(uint32_t)m;
-            if (bound_out && r == k - 1 && !none) bound_out[row] = m;
-        }
+        take(r, m);
     }
 }
 
-constexpr int kTopkMax = 16;
+// One warp per row: the row's k smallest keys out of those the top-k epilogue wrote, ascending.
+template <int TOPK>
+__global__ void topk_merge_kernel(const unsigned long long *__restrict__ lists, const int *__restrict__ counts,
+                                  float *__restrict__ val_out, long long *__restrict__ idx_out,
+                                  long long rows, long long row_stride, int k, int take_sqrt) {
+    const int lane = threadIdx.x & 31;
+    const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (row >= rows) return;
+    const unsigned long long *src = lists + row * row_stride;
+    unsigned long long out = ~0ull;      // lane r: the r-th key
+    warp_smallest<TOPK>(counts[row], k, [&](long long e) { return src[e]; }, [&](int r, unsigned long long m) { if (lane == r) out = m; });
+    if (lane >= k) return;
+    const bool none = out == ~0ull;
+    float v = none ? __int_as_float(0x7f800000) : __uint_as_float((uint32_t)(out >> 32));
+    if (take_sqrt) v = sqrtf(v);
+    if (val_out) val_out[row * k + lane] = v;
+    if (idx_out) idx_out[row * k + lane] = none ? -1ll : (long long)(uint32_t)out;
+}
+
+// One warp per row: an upper bound of the row's k-th smallest key from the minima of n groups of columns.  Each minimum is
+// the distance of a column of its own, so k columns are no farther than the k-th smallest minimum; the bound is the
+// first key above all keys of that distance (~0: fewer than k groups hold a finite distance).
+template <int TOPK>
+__global__ void topk_bound_kernel(const float *__restrict__ gmin, unsigned long long *__restrict__ bound, long long rows, long long n, int k) {
+    const int lane = threadIdx.x & 31;
+    const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    if (row >= rows) return;
+    const float *src = gmin + row * n;
+    warp_smallest<TOPK>(n, k, [&](long long e) { return ((unsigned long long)__float_as_uint(src[e]) << 32) | (unsigned long long)(uint32_t)e; },
+                        [&](int r, unsigned long long m) {
+                            if (lane == 0 && r == k - 1) bound[row] = (uint32_t)(m >> 32) < 0x7f800000u ? ((m >> 32) + 1) << 32 : ~0ull;
+                        });
+}
+
+constexpr int kTopkMax = 16;      // a tile half's keys fit the warp's 4 KB of staging
 
 struct TopkScratch {
-    long long L, off_lists, off_thr, total;
+    long long L, off_lists, off_thr, off_count, total;
 };
 inline TopkScratch topk_scratch_layout(long long B, long long N1, long long N2, long long D, long long k) {
     TopkScratch T;
@@ -928,7 +1093,8 @@ inline TopkScratch topk_scratch_layout(long long B, long long N1, long long N2, 
     const long long gemm = scratch_layout(B, N1, N2, D, false).total;
     T.off_lists = gemm;
     T.off_thr = gemm + align_up(B * N1 * T.L * k * 8, 1024);
-    T.total = T.off_thr + align_up(B * N1 * 8, 1024);
+    T.off_count = T.off_thr + align_up(B * N1 * 8, 1024);
+    T.total = T.off_count + align_up(B * N1 * 4, 1024);
     return T;
 }
 } // namespace
@@ -950,12 +1116,14 @@ int prepare_bf16_operands(const void *x1, const void *x2, void *scratch, bool re
     __nv_bfloat16 *xh = reinterpret_cast<__nv_bfloat16 *>(base + L.off_xh), *xl = reinterpret_cast<__nv_bfloat16 *>(base + L.off_xl);
     __nv_bfloat16 *yh = reinterpret_cast<__nv_bfloat16 *>(base + L.off_yh), *yl = reinterpret_cast<__nv_bfloat16 *>(base + L.off_yl);
     float *n1 = reinterpret_cast<float *>(base + L.off_n1), *n2 = reinterpret_cast<float *>(base + L.off_n2);
+    int *lo_any = reinterpret_cast<int *>(base + L.off_lo);
+    TPW_CUDA_OK(cudaMemsetAsync(lo_any, 0, 2 * sizeof(int), s));
     const int threads = 256;
     const long long cap = (long long)sm_count() * 16;
     long long blocks = (B * N1 * 32 + threads - 1) / threads;
-    split_rows_kernel<<<(unsigned)(blocks < cap ? blocks : cap), threads, 0, s>>>((const float *)x1, xh, xl, n1, B * N1, D, L.Dp, reciprocal_norms ? 1 : 0);
+    split_rows_kernel<<<(unsigned)(blocks < cap ? blocks : cap), threads, 0, s>>>((const float *)x1, xh, xl, n1, lo_any, B * N1, D, L.Dp, reciprocal_norms ? 1 : 0);
     blocks = (B * N2 * 32 + threads - 1) / threads;
-    split_rows_kernel<<<(unsigned)(blocks < cap ? blocks : cap), threads, 0, s>>>((const float *)x2, yh, yl, n2, B * N2, D, L.Dp, reciprocal_norms ? 1 : 0);
+    split_rows_kernel<<<(unsigned)(blocks < cap ? blocks : cap), threads, 0, s>>>((const float *)x2, yh, yl, n2, lo_any + 1, B * N2, D, L.Dp, reciprocal_norms ? 1 : 0);
     TPW_LAUNCH_OK("split_rows_kernel");
     int st;
     if ((st = make_tensor_map_3d(&M.mxh, xh, 2, L.Dp, N1, B, BK, BM, true)) != TPW_OK) return st;
@@ -964,6 +1132,7 @@ int prepare_bf16_operands(const void *x1, const void *x2, void *scratch, bool re
     if ((st = make_tensor_map_3d(&M.myl, yl, 2, L.Dp, N2, B, BK, BN, true)) != TPW_OK) return st;
     memset(&P, 0, sizeof(P));
     P.n1sq = n1; P.n2sq = n2;
+    P.lo_any = lo_any;
     P.B = B; P.N1 = N1; P.N2 = N2; P.D = L.Dp;
     P.tiles_m = (N1 + BM - 1) / BM;
     P.tiles_n = (N2 + BN - 1) / BN;
@@ -1000,13 +1169,15 @@ extern "C" int tpw_dot_topk_forward_ws(int epilogue, int k, const void *x1, cons
     unsigned char *base = static_cast<unsigned char *>(scratch);
     unsigned long long *lists = reinterpret_cast<unsigned long long *>(base + T.off_lists);
     unsigned long long *thr = reinterpret_cast<unsigned long long *>(base + T.off_thr);
-    TPW_CUDA_OK(cudaMemsetAsync(lists, 0xFF, (size_t)(T.total - T.off_lists), s)); // lists and bounds: "nothing yet"
+    int *counts = reinterpret_cast<int *>(base + T.off_count);
+    TPW_CUDA_OK(cudaMemsetAsync(counts, 0, (size_t)(B * N1) * 4, s));
     Bf16Operands M;
     GemmParams P;
     int st;
     if ((st = prepare_bf16_operands(x1, x2, scratch, cosine, B, N1, N2, D, s, M, P)) != TPW_OK) return st;
     P.epilogue = cosine ? TPW_DOT_COSINE_DIST : TPW_DOT_SQEUCLIDEAN;
-    P.topk_lists = lists; P.topk_thr = thr; P.topk_k = k; P.topk_L = (int)T.L;
+    P.topk_lists = lists; P.topk_thr = thr; P.topk_count = counts; P.topk_k = k; P.topk_L = (int)T.L;
+    P.vec_store = N2 % 4 == 0 ? 1 : 0;   // the squared x2 norms of a batch start on 16-byte boundaries
     const long long nsm = sm_count();
     const long long tiles_n_all = (N2 + BN - 1) / BN;
     const long long rows = B * N1;
@@ -1018,27 +1189,33 @@ extern "C" int tpw_dot_topk_forward_ws(int epilogue, int k, const void *x1, cons
         auto kern = gemm_metric_kernel<EPI, false, false, false, false, false, CAP>;                                      \
         TPW_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_ALLOC));                 \
         kern<<<grid, kThreads, SMEM_ALLOC, s>>>(M.mxh, M.mxl, M.myh, M.myl, P);                                           \
+        TPW_LAUNCH_OK("gemm_metric_kernel (top-k)");                                                                      \
     } while (0)
-    // Column ranges [0, 1/16), [1/16, 1/4), [1/4, 1) of the column tiles: after each range the lists so far
-    // are merged into an exact bound of every row's k-th smallest key, which prunes the next range down to
-    // the few candidates that can still matter (an insertion costs the whole warp as soon as one lane has one).
-    const long long cut[4] = {0, tiles_n_all >= 16 ? tiles_n_all / 16 : 0, tiles_n_all >= 16 ? tiles_n_all / 4 : 0, tiles_n_all};
-    for (int ph = 0; ph < 3; ++ph) {
-        if (cut[ph + 1] <= cut[ph]) continue;
-        P.tn0 = cut[ph];
-        P.tiles_n = cut[ph + 1] - cut[ph];
+    // An insertion costs the whole warp as soon as one lane has one, so first a bound: the contraction over a sixth of the
+    // column tiles keeps only the minimum of every 32 columns, and the k-th smallest of a row's minima bounds its k-th
+    // smallest distance almost as closely as the distances themselves would.  With that bound the pass over all columns
+    // inserts about 6 k keys a row, and the sixth that is computed twice costs less than the insertions it saves.
+    // (Lists over a sixteenth, a quarter and the rest, each bounding the next, as it was: k = 10 of [50000, 20000, 128]
+    // 4.00 -> 1.49 ms.)  Fewer than 8 column tiles are not worth a second pass.
+    const long long sample = tiles_n_all / 6;
+    if (tiles_n_all >= 8 && (sample > 1 ? sample : 2) * 8 >= k) {
+        P.tiles_n = sample > 1 ? sample : 2;
         P.tiles = B * P.tiles_m * P.tiles_n;
+        P.gmin = reinterpret_cast<float *>(lists);   // 32 bytes per row and tile, where the pass below keeps 16 k
         const unsigned grid = (unsigned)(P.tiles < nsm ? P.tiles : nsm);
-        if (cosine) { if (k <= 8) TPW_TOPK_LAUNCH(TPW_DOT_COSINE_DIST, 8); else TPW_TOPK_LAUNCH(TPW_DOT_COSINE_DIST, 16); }
-        else { if (k <= 8) TPW_TOPK_LAUNCH(TPW_DOT_SQEUCLIDEAN, 8); else TPW_TOPK_LAUNCH(TPW_DOT_SQEUCLIDEAN, 16); }
-        TPW_LAUNCH_OK("gemm_metric_kernel (top-k)");
-        const bool last = cut[ph + 1] == tiles_n_all;
-        const long long n = 2 * cut[ph + 1] * k; // the lists of all column tiles processed so far
-        if (k <= 8) topk_merge_kernel<8><<<mblocks, 256, 0, s>>>(lists, last ? val_out : nullptr, last ? idx64 : nullptr, last ? nullptr : thr,
-                                                                  rows, T.L * k, n, k, take_sqrt);
-        else topk_merge_kernel<16><<<mblocks, 256, 0, s>>>(lists, last ? val_out : nullptr, last ? idx64 : nullptr, last ? nullptr : thr,
-                                                                   rows, T.L * k, n, k, take_sqrt);
+        if (cosine) TPW_TOPK_LAUNCH(TPW_DOT_COSINE_DIST, -1); else TPW_TOPK_LAUNCH(TPW_DOT_SQEUCLIDEAN, -1);
+        if (k <= 8) topk_bound_kernel<8><<<mblocks, 256, 0, s>>>(P.gmin, thr, rows, 8 * P.tiles_n, k);
+        else topk_bound_kernel<16><<<mblocks, 256, 0, s>>>(P.gmin, thr, rows, 8 * P.tiles_n, k);
+        TPW_LAUNCH_OK("topk_bound_kernel");
+    } else {
+        TPW_CUDA_OK(cudaMemsetAsync(thr, 0xFF, (size_t)rows * 8, s));
     }
+    P.tiles_n = tiles_n_all;
+    P.tiles = B * P.tiles_m * P.tiles_n;
+    const unsigned grid = (unsigned)(P.tiles < nsm ? P.tiles : nsm);
+    if (cosine) TPW_TOPK_LAUNCH(TPW_DOT_COSINE_DIST, 1); else TPW_TOPK_LAUNCH(TPW_DOT_SQEUCLIDEAN, 1);
+    if (k <= 8) topk_merge_kernel<8><<<mblocks, 256, 0, s>>>(lists, counts, val_out, idx64, rows, T.L * k, k, take_sqrt);
+    else topk_merge_kernel<16><<<mblocks, 256, 0, s>>>(lists, counts, val_out, idx64, rows, T.L * k, k, take_sqrt);
 #undef TPW_TOPK_LAUNCH
     TPW_LAUNCH_OK("topk_merge_kernel");
     return TPW_OK;
@@ -1131,7 +1308,7 @@ extern "C" int tpw_dot_metric_forward_ws(int dtype, int epilogue, int engine,
             X.vec_in = (D % 4 == 0 && aligned16(X.a)) ? 1 : 0;
             if ((st = launch_split<COEF_ID, false>(X, B, s)) != TPW_OK) return st;
         }
-        return launch_tf32_product(Tf32Operand{xhi, xlo, Dp, false}, Tf32Operand{yhi, ylo, Dp, false}, static_cast<float *>(out), B, N1, N2, Dp, s);
+        return launch_tf32_product(Tf32Operand{xhi, xlo, Dp, false}, Tf32Operand{yhi, ylo, Dp, false}, static_cast<float *>(out), nullptr, B, N1, N2, Dp, s);
     }
     if (engine == TPW_ENGINE_AUTO && auto_picks_tensor_cores(dtype, B, N1, N2, D) && scratch != nullptr &&
         scratch_bytes >= scratch_layout(B, N1, N2, D, false).total)
@@ -1239,6 +1416,8 @@ static int dense_backward_tensor(int coef, int epilogue, bool sums, float s_mm, 
         TPW_LAUNCH_OK("reduce_partials_kernel");
     }
     const long long cap = (long long)sm_count() * 8;
+    int *lo_any = reinterpret_cast<int *>(base + L.off_lo);   // [side][coefficients (not used), x]
+    TPW_CUDA_OK(cudaMemsetAsync(lo_any, 0, 4 * sizeof(int), s));
     const Tf32Operand Ck{F(L.off_chi), F(L.off_clo), L.N2p, false}, Cmn{F(L.off_chi), F(L.off_clo), L.N2p, true};
     for (int side = 0; side < 2; ++side) {
         void *gout = side == 0 ? grad_x1 : grad_x2;
@@ -1254,10 +1433,11 @@ static int dense_backward_tensor(int coef, int epilogue, bool sums, float s_mm, 
         X.hi = xhi; X.lo = xlo;
         X.R = Nk; X.C = D; X.Cp = L.Dp;
         X.vec_in = (D % 4 == 0 && aligned16(xk)) ? 1 : 0;
+        X.lo_any = lo_any + 2 * side + 1;
         if ((st = launch_split<COEF_ID, false>(X, B, s)) != TPW_OK) return st;
         const Tf32Operand Xmn{xhi, xlo, L.Dp, true};
-        if (side == 0) st = launch_tf32_product(Ck, Xmn, static_cast<float *>(gout), B, N1, D, N2, s);
-        else st = launch_tf32_product(Cmn, Xmn, static_cast<float *>(gout), B, N2, D, N1, s);
+        if (side == 0) st = launch_tf32_product(Ck, Xmn, static_cast<float *>(gout), lo_any, B, N1, D, N2, s);
+        else st = launch_tf32_product(Cmn, Xmn, static_cast<float *>(gout), lo_any + 2, B, N2, D, N1, s);
         if (st != TPW_OK) return st;
         const float *sumv = F(side == 0 ? L.off_rowsum : L.off_colsum);
         if (coef == COEF_COSINE) {
