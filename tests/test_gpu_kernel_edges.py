@@ -133,3 +133,45 @@ def test_quotients_of_counts_round_as_the_division(tpw):
         # float64 division of integers this small, rounded once more to float32, is the correctly rounded quotient
         assert torch.equal(tpw.jaccard_distances(x, x2), torch.where(most > 0, diff.double() / most.double(), 0.0).float())
         assert torch.equal(tpw.hamming_distances(x, x2), (diff.double() / d).float())
+
+
+@pytest.mark.parametrize("p", [1.0, 3.0, math.inf])
+def test_rows_padded_to_whole_vectors(tpw, p):
+    """Large problems whose feature count is no multiple of 4 run on zero-padded copies; the same batches one at a time are too
+    small for that.  The forward and the Chebyshev gradients add the same terms in the same order (bit-equal), the others in
+    another order (sums of up to 600 float32 terms)."""
+    g = torch.Generator().manual_seed(7)
+    x1, x2 = torch.randn(4, 600, 201, generator=g).cuda(), torch.randn(4, 500, 201, generator=g).cuda()
+    gr = torch.randn(4, 600, 500, generator=g).cuda()
+
+    def grads(a, c, up):
+        a, c = a.clone().requires_grad_(), c.clone().requires_grad_()
+        out = tpw.chebyshev_distances(a, c) if math.isinf(p) else tpw.minkowski_distances(a, c, p)
+        return (out.detach(), *torch.autograd.grad(out, (a, c), up))
+
+    whole = grads(x1, x2, gr)
+    parts = [torch.stack(t) for t in zip(*(grads(x1[b], x2[b], gr[b]) for b in range(4)))]
+    assert whole[1].shape == x1.shape and whole[2].shape == x2.shape and whole[1].is_contiguous()
+    assert torch.equal(whole[0], parts[0])
+    for w, q in zip(whole[1:], parts[1:]):
+        if math.isinf(p):
+            assert torch.equal(w, q)
+        else:
+            assert float((w - q).abs().max()) <= 2e-5 * float(q.abs().max())
+
+
+@pytest.mark.parametrize("shape", [(1, 300, 1100, 192), (2, 1030, 1500, 256), (1, 20000, 1025, 72), (3, 1024, 2048, 260)])
+def test_gradient_products_with_dealt_out_chunks(tpw, shape):
+    """Products whose tiles do not fill the last wave share them chunk by chunk between CTAs: against float64, and bit-reproducible.
+    The products keep 22 bits of each factor and add up to 20000 terms in float32: 1e-5 of the largest element, as for whole tiles."""
+    b, n1, n2, d = shape
+    g = torch.Generator().manual_seed(n1)
+    x1, x2 = torch.randn(b, n1, d, generator=g).cuda().requires_grad_(), torch.randn(b, n2, d, generator=g).cuda().requires_grad_()
+    up = torch.randn(b, n1, n2, generator=g).cuda()
+    one = torch.autograd.grad(tpw.sqeuclidean_distances(x1, x2), (x1, x2), up)
+    two = torch.autograd.grad(tpw.sqeuclidean_distances(x1, x2), (x1, x2), up)
+    assert all(torch.equal(a, c) for a, c in zip(one, two))
+    u, a, c = up.double(), x1.detach().double(), x2.detach().double()
+    want = (2 * (u.sum(2, keepdim=True) * a - u @ c), 2 * (u.sum(1)[..., None] * c - u.transpose(1, 2) @ a))
+    for got, ref in zip(one, want):
+        assert float((got - ref).abs().max()) <= 1e-5 * float(ref.abs().max())

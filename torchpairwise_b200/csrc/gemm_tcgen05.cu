@@ -77,6 +77,7 @@ struct GemmParams {
     float *gmin;              // TOPK < 0: [B*N1][8 * tiles_n] minima of the groups of 32 columns
     const int *lo_any;        // [2] whether any low part of the x (y) operand is non-zero; NULL: treat both as non-zero
     int lo_always;            // bit 0 / 1: the x / y operand's low parts are used whatever lo_any says
+    float *partial;           // tf32: [grid][2][BM][BN] sums of the tiles that a CTA has only a part of (NULL: whole tiles only)
     int *status;
 };
 
@@ -190,6 +191,42 @@ __device__ __forceinline__ void store_block_ragged(const unsigned char *stg, flo
         dst[rr * pitch + lane] = *reinterpret_cast<const float *>(stg + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) + (lane & 3) * 4);
 }
 
+// The share of a product that falls to one CTA: whole tiles, every gridDim.x-th.  With a scratch for partial tiles (tf32) only
+// the full waves go that way; the chunks of the tiles that are left over are dealt out evenly, and a tile cut by the end of
+// a share is finished by product_fixup_kernel.
+template <typename I>
+struct ProductShare {
+    I tile_at, tile_last, base;   // whole tiles; first tile of those dealt out
+    int stride, nch;
+    int at, last;                 // this CTA's chunks of the tiles dealt out
+    __device__ __forceinline__ ProductShare(const GemmParams &P, int nch_) {
+        nch = nch_;
+        stride = (int)gridDim.x;
+        const long long left = P.partial ? P.tiles % stride : 0, all = left * nch;
+        base = (I)(P.tiles - left);
+        tile_at = (I)blockIdx.x;
+        tile_last = base;
+        at = (int)(all * blockIdx.x / stride);
+        last = (int)(all * (blockIdx.x + 1) / stride);
+    }
+    // the next piece: chunks [c0, c1) of a tile
+    __device__ __forceinline__ bool next(I &tile, int &c0, int &c1) {
+        if (tile_at < tile_last) {
+            tile = tile_at;
+            c0 = 0;
+            c1 = nch;
+            tile_at += stride;
+            return true;
+        }
+        if (at >= last) return false;
+        tile = base + at / nch;
+        c0 = at % nch;
+        c1 = last - at < nch - c0 ? c0 + (last - at) : nch;
+        at += c1 - c0;
+        return true;
+    }
+};
+
 // AMN / BMN (tf32 only): the operand is MN-major, i.e. its global rows run along k and each row holds
 // the tile's M (or N) values contiguously, so a matrix can be contracted over its row index without a
 // transposed copy.  Such a tile is staged as blocks of {32 values, 32 k-rows} (one TMA box each, 4 KB,
@@ -212,6 +249,7 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     constexpr int BKE = TF32 ? BK / 2 : BK; // operand elements per k-step
+    typedef std::conditional_t<TF32, int, long long> Index;   // a stored product has fewer than 2^31 tiles
     const int nkb = (int)((P.D + BKE - 1) / BKE);
 
     if (threadIdx.x == 0) {
@@ -244,10 +282,14 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
         if (lane == 0) {
             uint32_t it = 0;
             bool ok = true;
-            for (long long tile = blockIdx.x; tile < P.tiles && ok; tile += gridDim.x) {
+            const int kchunk = (P.kchunk > 0 && P.kchunk < nkb) ? P.kchunk : nkb;
+            ProductShare<Index> share(P, (nkb + kchunk - 1) / kchunk);
+            Index tile;
+            for (int c0, c1; ok && share.next(tile, c0, c1);) {
                 long long tn, tm, b;
                 decode_tile<TOPK != 0>(tile, P, tn, tm, b);
-                for (int kb = 0; kb < nkb; ++kb, ++it) {
+                const int kend = c1 * kchunk < nkb ? c1 * kchunk : nkb;
+                for (int kb = c0 * kchunk; kb < kend; ++kb, ++it) {
                     const int s = it % kStages;
                     const uint32_t use = it / kStages;
                     if (use > 0 && !wait_or_abort(&empty[s], (use - 1) & 1, abort_flag)) {
@@ -301,10 +343,13 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
             uint32_t it = 0, acount = 0;
             bool ok = true;
             const int kchunk = (P.kchunk > 0 && P.kchunk < nkb) ? P.kchunk : nkb;
-            for (long long tile = blockIdx.x; tile < P.tiles && ok; tile += gridDim.x) {
+            ProductShare<Index> share(P, (nkb + kchunk - 1) / kchunk);
+            Index tile;
+            for (int c0, c1; ok && share.next(tile, c0, c1);) {
                 // one accumulator per chunk of k-steps: the tensor cores add into tensor memory with
                 // truncation, so long reductions are cut into chunks that the epilogue sums in registers
-                for (int kb0 = 0; kb0 < nkb && ok; kb0 += kchunk, ++acount) {
+                const int kend = c1 * kchunk < nkb ? c1 * kchunk : nkb;
+                for (int kb0 = c0 * kchunk; kb0 < kend && ok; kb0 += kchunk, ++acount) {
                     const uint32_t a = acount & 1, ause = acount >> 1;
                     if (ause > 0 && !wait_or_abort(&tmem_empty[a], (ause - 1) & 1, abort_flag)) {
                         *abort_flag = 1;
@@ -376,7 +421,10 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
             const int kchunk = (P.kchunk > 0 && P.kchunk < nkb) ? P.kchunk : nkb;
             const int nchunks = (nkb + kchunk - 1) / kchunk;
             uint32_t acount = 0;
-            for (long long tile = blockIdx.x; tile < P.tiles && ok; tile += gridDim.x) {
+            ProductShare<Index> share(P, nchunks);
+            const int start = share.at;
+            Index tile;
+            for (int c0, c1; ok && share.next(tile, c0, c1);) {
                 long long t = tile;
                 const long long tn = t % P.tiles_n; t /= P.tiles_n;
                 const long long tm = t % P.tiles_m;
@@ -384,7 +432,7 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                 float sums[BN / 2];
 #pragma unroll
                 for (int v = 0; v < BN / 2; ++v) sums[v] = 0.f;
-                for (int ch = 0; ch < nchunks && ok; ++ch, ++acount) {
+                for (int ch = c0; ch < c1 && ok; ++ch, ++acount) {
                     const uint32_t a = acount & 1;
                     if (!wait_or_abort(&tmem_full[a], (acount >> 1) & 1, abort_flag)) {
                         *abort_flag = 1;
@@ -394,12 +442,12 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                     }
                     tc_fence_after();
 #pragma unroll
-                    for (int c = 0; c < BN / 64; ++c) {
-                        uint32_t r[32];
-                        tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + a * BN + (chalf * (BN / 64) + c) * 32, r);
+                    for (int c = 0; c < BN / 32; ++c) {   // sixteen columns at a time: 128 sums leave few registers
+                        uint32_t r[16];
+                        tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + a * BN + chalf * (BN / 2) + c * 16, r);
                         tmem_ld_wait();
 #pragma unroll
-                        for (int v = 0; v < 32; ++v) sums[c * 32 + v] += __uint_as_float(r[v]);
+                        for (int v = 0; v < 16; ++v) sums[c * 16 + v] += __uint_as_float(r[v]);
                     }
                     tc_fence_before();
                     __syncwarp();
@@ -408,22 +456,27 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                 if (!ok) break;
                 unsigned char *stg = smem + OFF_STAGE + (warp - 2) * 4096;
                 const long long row_base = tm * BM + q * 32;
+                const bool part = c1 - c0 < nchunks;
+                // a share holds at most two parts of tiles, one at its start and one at its end
+                float *pdst = P.partial + ((long long)blockIdx.x * 2 + ((tile - share.base) * nchunks + c0 == start ? 0 : 1)) * (BM * BN);
 #pragma unroll
                 for (int c = 0; c < BN / 64; ++c) {
-                    const long long j0 = tn * BN + (chalf * (BN / 64) + c) * 32;
+                    const int col = (chalf * (BN / 64) + c) * 32;
+                    const long long j0 = tn * BN + col;
                     if (j0 >= P.N2) continue;
 #pragma unroll
                     for (int v = 0; v < 8; ++v)
                         *reinterpret_cast<float4 *>(stg + lane * 128 + ((v ^ (lane & 7)) << 4)) =
                             make_float4(sums[c * 32 + 4 * v], sums[c * 32 + 4 * v + 1], sums[c * 32 + 4 * v + 2], sums[c * 32 + 4 * v + 3]);
                     __syncwarp();
-                    if (P.vec_store && j0 + 32 <= P.N2) {
+                    if (part || (P.vec_store && j0 + 32 <= P.N2)) {
+                        float *dst = part ? pdst + q * 32 * BN + col : P.out + (b * P.N1 + row_base) * P.N2 + j0;
+                        const long long pitch = part ? BN : P.N2;
 #pragma unroll
                         for (int it = 0; it < 8; ++it) {
                             const int rr = it * 4 + (lane >> 3), cc = lane & 7;
                             const float4 o = *reinterpret_cast<const float4 *>(stg + rr * 128 + ((cc ^ (rr & 7)) << 4));
-                            if (row_base + rr < P.N1)
-                                reinterpret_cast<float4 *>(P.out + (b * P.N1 + row_base + rr) * P.N2 + j0)[cc] = o;
+                            if (row_base + rr < P.N1) reinterpret_cast<float4 *>(dst + rr * pitch)[cc] = o;
                         }
                     } else {
                         store_block_ragged(stg, P.out + (b * P.N1 + row_base) * P.N2 + j0, P.N2, P.N1 - row_base, P.N2 - j0, lane);
@@ -625,6 +678,40 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc(tmem_base, kTmemCols);
+    }
+}
+
+// Tiles whose chunks several CTAs share: the parts' sums, added in the order of the chunks.  One CTA per 16 rows of a tile.
+__global__ void __launch_bounds__(BN)
+product_fixup_kernel(const GemmParams P, int nch, long long ctas) {
+    const long long left = P.tiles % ctas, base = P.tiles - left, local = blockIdx.x / (BM / 16), tile = base + local;
+    const int row0 = (int)(blockIdx.x % (BM / 16)) * 16, col = threadIdx.x;
+    const long long all = left * nch, u0 = local * nch, u1 = u0 + nch;
+    auto start_of = [&](long long c) { return all * c / ctas; };
+    long long c = u0 * ctas / all;                  // the share that holds chunk u0, up to rounding
+    while (c > 0 && start_of(c) > u0) --c;
+    while (start_of(c + 1) <= u0) ++c;
+    if (start_of(c + 1) >= u1) return;              // one CTA had the whole tile
+    long long t = tile;
+    const long long tn = t % P.tiles_n; t /= P.tiles_n;
+    const long long tm = t % P.tiles_m;
+    const long long b = t / P.tiles_m;
+    const long long j = tn * BN + col;
+    if (j >= P.N2) return;
+    float s[16];
+#pragma unroll
+    for (int r = 0; r < 16; ++r) s[r] = 0.f;
+    for (; c < ctas && start_of(c) < u1; ++c) {
+        if (start_of(c + 1) == start_of(c)) continue;   // fewer chunks than CTAs: an empty share
+        const float *src = P.partial + (c * 2 + (start_of(c) >= u0 ? 0 : 1)) * (BM * BN) + row0 * BN + col;
+#pragma unroll
+        for (int r = 0; r < 16; ++r)
+            if (tm * BM + row0 + r < P.N1) s[r] += src[r * BN];
+    }
+#pragma unroll
+    for (int r = 0; r < 16; ++r) {
+        const long long i = tm * BM + row0 + r;
+        if (i < P.N1) P.out[(b * P.N1 + i) * P.N2 + j] = s[r];
     }
 }
 
@@ -871,10 +958,32 @@ __global__ void grad_finish_kernel(float *__restrict__ g, const float *__restric
     }
 }
 
+// How a tf32 product of M x N outputs over K is cut.  Whole tiles, one wave of persistent CTAs after another, leave the last
+// wave as empty as it happens to be.  Where it is less than 0.92 full, its tiles' chunks of 64 are dealt out evenly instead, at least four to
+// a CTA, and the parts of split tiles (two at most per CTA) are added by a kernel of their own, 5 to 15 us.  (Dealing out all
+// tiles scatters the CTAs over batches whose operands do not fit L2 together: 660 -> 880 us a product of euclidean
+// [16, 4096, 4096, 256].)  cosine bfloat16 [5000, 4111, 768], both products: 302 -> 277 us; euclidean [2, 1500, 1100, 192]: 100 -> 50 us.
+constexpr int kProductChunk = 2;               // k-steps of 32
+constexpr long long kPartialBytes = 2ll * BM * BN * 4;
+inline long long product_chunks(long long K) { return ((K + BK / 2 - 1) / (BK / 2) + kProductChunk - 1) / kProductChunk; }
+inline long long product_tiles(long long B, long long M, long long N) { return B * ((M + BM - 1) / BM) * ((N + BN - 1) / BN); }
+inline bool deals_chunks(long long B, long long M, long long N, long long K) {
+    const long long tiles = product_tiles(B, M, N), nsm = sm_count(), left = tiles % nsm;
+    // one wave more or less in a long queue, or a tile of a few chunks, is not worth the second kernel
+    return tiles <= 8 * nsm && product_chunks(K) >= 16 && product_chunks(K) < (1 << 20) && left > 0 && left * 100 < nsm * 92;
+}
+inline long long product_ctas(long long B, long long M, long long N, long long K, bool room) {
+    const long long tiles = product_tiles(B, M, N), nsm = sm_count();
+    if (tiles >= nsm) return nsm;
+    const long long most = room && deals_chunks(B, M, N, K) ? tiles * product_chunks(K) / 4 : tiles;
+    return most < nsm ? (most > tiles ? most : tiles) : nsm;
+}
+
 struct BwdScratch {
     long long N2p, Dp, TR, TC;
     long long off_chi, off_clo, off_x1hi, off_x1lo, off_x2hi, off_x2lo;
     long long off_rowpart, off_colpart, off_rowsum, off_colsum, off_lo, total;
+    long long off_part, with_part;   // partial tiles of the products, where they are worth it (with_part == total: not)
 };
 
 inline BwdScratch bwd_scratch_layout(long long B, long long N1, long long N2, long long D) {
@@ -897,6 +1006,8 @@ inline BwdScratch bwd_scratch_layout(long long B, long long N1, long long N2, lo
     L.off_colsum = take(B * N2 * 4);
     L.off_lo = take(4 * sizeof(int));
     L.total = off;
+    L.off_part = off;
+    L.with_part = deals_chunks(B, N1, D, N2) || deals_chunks(B, N2, D, N1) ? off + sm_count() * kPartialBytes : off;
     return L;
 }
 
@@ -926,7 +1037,8 @@ struct Tf32Operand {
 // out[b,m,n] = sum_k A[b](m,k) * Bm[b](n,k); K = length of the reduction.  A K-major operand holds
 // `pitch` >= K elements per row (zero beyond K), an MN-major operand has exactly K rows per batch.
 // lo_any (may be NULL): lo_any[1] says whether Bm has any low part; A's are always used.
-int launch_tf32_product(const Tf32Operand &A, const Tf32Operand &Bm, float *out, const int *lo_any,
+// partial (may be NULL): kPartialBytes per SM, for products that deal out chunks instead of whole tiles.
+int launch_tf32_product(const Tf32Operand &A, const Tf32Operand &Bm, float *out, const int *lo_any, float *partial,
                         long long B, long long M, long long N, long long K, cudaStream_t s) {
     CUtensorMap mah, mal, mbh, mbl;
     int st;
@@ -950,11 +1062,12 @@ int launch_tf32_product(const Tf32Operand &A, const Tf32Operand &Bm, float *out,
     P.lo_always = 1;
     // 64 elements per chunk: measured against float64, the products are then as accurate as the fp32
     // FMA chain of the CUDA-core kernel (the error grows in proportion to the chunk length) at no cost in time
-    P.kchunk = 2;
+    P.kchunk = kProductChunk;
     P.vec_store = (N % 4 == 0 && aligned16(out)) ? 1 : 0;
     P.status = device_status_ptr();
-    const long long nsm = sm_count();
-    const unsigned grid = (unsigned)(P.tiles < nsm ? P.tiles : nsm);
+    const long long ctas = product_ctas(B, M, N, K, partial != nullptr);
+    P.partial = partial != nullptr && deals_chunks(B, M, N, K) ? partial : nullptr;
+    const unsigned grid = (unsigned)ctas;
 #define TPW_TF32_LAUNCH(AMN, BMN)                                                                                         \
     do {                                                                                                                  \
         auto kern = gemm_metric_kernel<TPW_DOT_LINEAR, false, true, false, AMN, BMN>;                                     \
@@ -967,6 +1080,10 @@ int launch_tf32_product(const Tf32Operand &A, const Tf32Operand &Bm, float *out,
     else return fail(TPW_ERR_UNSUPPORTED, "tf32 product: MN-major A with K-major B is not instantiated");
 #undef TPW_TF32_LAUNCH
     TPW_LAUNCH_OK("gemm_metric_kernel (tf32)");
+    if (P.partial && P.tiles % ctas != 0) {
+        product_fixup_kernel<<<(unsigned)(P.tiles % ctas * (BM / 16)), BN, 0, s>>>(P, (int)product_chunks(K), ctas);
+        TPW_LAUNCH_OK("product_fixup_kernel");
+    }
     return TPW_OK;
 }
 
@@ -1196,7 +1313,7 @@ extern "C" int tpw_dot_topk_forward_ws(int epilogue, int k, const void *x1, cons
     // smallest distance almost as closely as the distances themselves would.  With that bound the pass over all columns
     // inserts about 6 k keys a row, and the sixth that is computed twice costs less than the insertions it saves.
     // (Lists over a sixteenth, a quarter and the rest, each bounding the next, as it was: k = 10 of [50000, 20000, 128]
-    // 4.00 -> 1.49 ms.)  Fewer than 8 column tiles are not worth a second pass.
+    // 4.00 -> 1.45 ms.)  Fewer than 8 column tiles are not worth a second pass.
     const long long sample = tiles_n_all / 6;
     if (tiles_n_all >= 8 && (sample > 1 ? sample : 2) * 8 >= k) {
         P.tiles_n = sample > 1 ? sample : 2;
@@ -1308,7 +1425,7 @@ extern "C" int tpw_dot_metric_forward_ws(int dtype, int epilogue, int engine,
             X.vec_in = (D % 4 == 0 && aligned16(X.a)) ? 1 : 0;
             if ((st = launch_split<COEF_ID, false>(X, B, s)) != TPW_OK) return st;
         }
-        return launch_tf32_product(Tf32Operand{xhi, xlo, Dp, false}, Tf32Operand{yhi, ylo, Dp, false}, static_cast<float *>(out), nullptr, B, N1, N2, Dp, s);
+        return launch_tf32_product(Tf32Operand{xhi, xlo, Dp, false}, Tf32Operand{yhi, ylo, Dp, false}, static_cast<float *>(out), nullptr, nullptr, B, N1, N2, Dp, s);
     }
     if (engine == TPW_ENGINE_AUTO && auto_picks_tensor_cores(dtype, B, N1, N2, D) && scratch != nullptr &&
         scratch_bytes >= scratch_layout(B, N1, N2, D, false).total)
@@ -1376,7 +1493,7 @@ static bool backward_uses_tensor_cores(int dtype, int mode, int engine, int64_t 
 
 extern "C" int64_t tpw_dot_backward_scratch_bytes(int dtype, int mode, int engine, int64_t B, int64_t N1, int64_t N2, int64_t D) {
     if (!backward_uses_tensor_cores(dtype, mode, engine, B, N1, N2, D)) return 0;
-    return bwd_scratch_layout(B, N1, N2, D).total;
+    return bwd_scratch_layout(B, N1, N2, D).with_part;
 }
 
 extern "C" int tpw_cosine_backward_finish(int dtype, void *grad_x, const void *x, const void *norm, const void *term,
@@ -1385,11 +1502,12 @@ extern "C" int tpw_cosine_backward_finish(int dtype, void *grad_x, const void *x
 // Shared body of the two entry points below.  coef: COEF_ID / COEF_DIV_AUX / COEF_COSINE.
 static int dense_backward_tensor(int coef, int epilogue, bool sums, float s_mm, float s_row,
                                  const void *grad, const void *aux, const void *norm1, const void *norm2,
-                                 const void *x1, const void *x2, void *grad_x1, void *grad_x2, void *scratch,
+                                 const void *x1, const void *x2, void *grad_x1, void *grad_x2, void *scratch, int64_t scratch_bytes,
                                  int64_t B, int64_t N1, int64_t N2, int64_t D, cudaStream_t s) {
     const BwdScratch L = bwd_scratch_layout(B, N1, N2, D);
     unsigned char *base = static_cast<unsigned char *>(scratch);
     auto F = [&](long long off) { return reinterpret_cast<float *>(base + off); };
+    float *partial = L.with_part > L.total && scratch_bytes >= L.with_part ? F(L.off_part) : nullptr;
     int st;
 
     // coefficient matrix C [N1,N2] as tf32 high/low parts, written once: grad_x1 = C . X2 reads it K-major
@@ -1436,8 +1554,8 @@ static int dense_backward_tensor(int coef, int epilogue, bool sums, float s_mm, 
         X.lo_any = lo_any + 2 * side + 1;
         if ((st = launch_split<COEF_ID, false>(X, B, s)) != TPW_OK) return st;
         const Tf32Operand Xmn{xhi, xlo, L.Dp, true};
-        if (side == 0) st = launch_tf32_product(Ck, Xmn, static_cast<float *>(gout), lo_any, B, N1, D, N2, s);
-        else st = launch_tf32_product(Cmn, Xmn, static_cast<float *>(gout), lo_any + 2, B, N2, D, N1, s);
+        if (side == 0) st = launch_tf32_product(Ck, Xmn, static_cast<float *>(gout), lo_any, partial, B, N1, D, N2, s);
+        else st = launch_tf32_product(Cmn, Xmn, static_cast<float *>(gout), lo_any + 2, partial, B, N2, D, N1, s);
         if (st != TPW_OK) return st;
         const float *sumv = F(side == 0 ? L.off_rowsum : L.off_colsum);
         if (coef == COEF_COSINE) {
@@ -1480,7 +1598,7 @@ extern "C" int tpw_dot_backward_ws(int dtype, int mode, int engine, const void *
     const float s_mm = mode == TPW_LP_BWD_MATMUL ? 1.f : (mode == TPW_LP_BWD_PPMINKOWSKI ? -2.f : -1.f);
     const float s_row = mode == TPW_LP_BWD_PPMINKOWSKI ? 2.f : 1.f;
     return dense_backward_tensor(mode == TPW_LP_BWD_CDIST ? COEF_DIV_AUX : COEF_ID, 0, mode != TPW_LP_BWD_MATMUL, s_mm, s_row,
-                                 grad, aux, nullptr, nullptr, x1, x2, grad_x1, grad_x2, scratch, B, N1, N2, D,
+                                 grad, aux, nullptr, nullptr, x1, x2, grad_x1, grad_x2, scratch, scratch_bytes, B, N1, N2, D,
                                  static_cast<cudaStream_t>(stream));
 }
 
@@ -1498,6 +1616,6 @@ extern "C" int tpw_cosine_backward_ws(int epilogue, const void *grad, const void
     TPW_CHECK_ARG(scratch != nullptr && scratch_bytes >= need,
                   "tpw_cosine_backward_ws: needs %lld bytes of scratch (got %lld)", need, (long long)scratch_bytes);
     TPW_CHECK_ARG(aligned16(scratch), "tpw_cosine_backward_ws: scratch must be 16-byte aligned");
-    return dense_backward_tensor(COEF_COSINE, epilogue, true, 1.f, 0.f, grad, out, norm1, norm2, x1, x2, grad_x1, grad_x2, scratch,
+    return dense_backward_tensor(COEF_COSINE, epilogue, true, 1.f, 0.f, grad, out, norm1, norm2, x1, x2, grad_x1, grad_x2, scratch, scratch_bytes,
                                  B, N1, N2, D, static_cast<cudaStream_t>(stream));
 }
