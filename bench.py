@@ -56,16 +56,16 @@ PAIRS_PER_STEP = B * N1 * N2
 # lane-operations of the dominant kernel per pair and feature: subtract, d*|d| and one fused multiply-add into each of
 # the two gradient sums -- the algorithmic count for both gradients, and what the one-pass kernel executes
 BWD_OPS_PER_ELEMENT = 4
-# lane-operations per point pair of the Hausdorff row-minimum loop as executed
-HAUSDORFF_EXECUTED_OPS = 7
+# lane-operations per point pair of the Hausdorff row-minimum loop as executed (expanded form: three multiply-adds, and
+# half a minimum at half rate)
+HAUSDORFF_EXECUTED_OPS = 4
 # algorithmic HBM bytes of the backward: upstream gradient + forward output read once, both operands read once,
 # both gradients written
 BWD_BYTES_PER_LAUNCH = 4 * (2 * B * N1 * N2 + 2 * B * N1 * D + 2 * B * N2 * D)
-# dram__bytes_read.sum + dram__bytes_write.sum of the backward call measured by ncu at batch 4
-# (profiles/lp_kernels_c2_minkowski_p3.md): 831.9 MB in the one-pass kernel (gradient and forward output streamed
-# once, 256 MB of row-block sums written) + 281.3 MB in the finishing kernel that reads them back; both grow in
-# proportion to the batch
-BWD_DRAM_TRAFFIC_BYTES_PER_BATCH = (831.9e6 + 281.3e6) / 4
+# dram__bytes_read.sum + dram__bytes_write.sum of the backward call: the walk measured by ncu at batch 2 (303.5 MB: the
+# coefficients streamed once, 128 MB of row-block sums written), the finishing kernel that reads those back at batch 4
+# (281.3 MB); the coefficient pass by its 12 bytes per pair.  All grow in proportion to the batch.
+BWD_DRAM_TRAFFIC_BYTES_PER_BATCH = 303.5e6 / 2 + 281.3e6 / 4 + 12 * N1 * N2
 
 REF_SO = ROOT / "oracle" / "_ref" / "torchpairwise_ref.so"
 
@@ -760,7 +760,7 @@ def run_ours(args, rank: int, world: int, local_rank: int):
                     "unit": "Tlane-op/s", "frac": algorithmic / (k_ms * 1e-3) / fp32_peak,
                     "frac_executed": algorithmic / (k_ms * 1e-3) / fp32_peak,
                     "traffic": BWD_DRAM_TRAFFIC_BYTES_PER_BATCH * B,
-                    "kernel": "lp_backward_onepass_kernel (both gradients, p=3) with its finishing lp_backward_onepass_sum_kernel"
+                    "kernel": "lp_backward_onepass_kernel (both gradients, p=3) between its onepass_coef_kernel and lp_backward_onepass_sum_kernel"
                               if nbytes > 0 else "lp_backward_kernel, two launches",
                     "ms_per_launch": k_ms, "two_launch_ms": two_ms,
                     "algorithmic_work": "4 lane-ops per pair and feature for both gradients (subtract, d*|d|, one fused multiply-add "
@@ -808,7 +808,7 @@ def run_ours(args, rank: int, world: int, local_rank: int):
             "e2e": {"value": e2e, "unit": "Gpairs/s", "ms_per_step": ms_e2e / args.steps,
                     "h2d_bytes_per_step": h2d_bytes, "d2h_bytes_per_step": 4 * (B * N1 * D + B * N2 * D),
                     "host_h2d_gbs_ceiling": h2d_ceiling, "host_placement": affinity},
-            "gpu_launches": 3 * args.steps,
+            "gpu_launches": 4 * args.steps,
             "roofline": roofline, "roofline_hbm": roofline_hbm, "cpu_baseline": cpu_baseline,
             "drop_in": {"ms_per_step": ms / args.steps, "python_mirror_ms_per_step": mirror_ms,
                         "same_bits_as_mirror": drop_in_same_bits},
