@@ -717,8 +717,21 @@ product_fixup_kernel(const GemmParams P, int nch, long long ctas) {
 
 // fp32 rows -> bf16 high/low parts (row pitch Dp, zero padded) and a per-row fp32 scalar: the
 // squared norm, or (recip != 0) the reciprocal norm with 0 for an all-zero row; one warp per row
-__global__ void split_rows_kernel(const float *__restrict__ x, __nv_bfloat16 *__restrict__ hi, __nv_bfloat16 *__restrict__ lo,
-                                  float *__restrict__ nsq, int *__restrict__ lo_any, long long rows, long long D, long long Dp, int recip) {
+struct SplitRows {
+    const float *x;
+    __nv_bfloat16 *hi, *lo;
+    float *nsq;
+    int *lo_any;
+    long long rows;
+};
+__global__ void split_rows_kernel(const SplitRows first, const SplitRows second, long long D, long long Dp, int recip) {
+    // both operands in one launch: the clearing of lo_any in front of it then costs no launch more than two splits did
+    const SplitRows &P = blockIdx.y == 0 ? first : second;
+    const float *__restrict__ x = P.x;
+    __nv_bfloat16 *__restrict__ hi = P.hi, *__restrict__ lo = P.lo;
+    float *__restrict__ nsq = P.nsq;
+    int *lo_any = P.lo_any;
+    const long long rows = P.rows;
     const int lane = threadIdx.x & 31;
     const long long warp = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const long long nwarps = ((long long)gridDim.x * blockDim.x) >> 5;
@@ -819,6 +832,7 @@ struct SplitParams {
     const float *n1, *n2;       // COEF_COSINE: row norms [B,R], [B,C]
     float *hi, *lo;             // [B,R,Cp]   (STRAIGHT)
     int *lo_any;                // set to 1 where some low part is not zero; may be NULL
+    int *clear;                 // four words to set to 0 for the launches that follow; may be NULL
     float *rowpart, *colpart;   // [B,TC,R], [B,TR,C]   (SUMS)
     long long R, C, Cp, TR, TC;
     int vec_in;                 // C % 4 == 0 and 16-byte aligned inputs
@@ -864,6 +878,7 @@ split_tile_kernel(const SplitParams P) {
     const int tid = threadIdx.x, ty = tid >> 4, tx = tid & 15;
     const long long b = blockIdx.z;
     const long long r0 = (long long)blockIdx.y * PT, c0 = (long long)blockIdx.x * PT;
+    if (P.clear && tid < 4 && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) P.clear[tid] = 0;
     const float *a = P.a + b * P.R * P.C;
     const float *aux = MODE != COEF_ID ? P.aux + b * P.R * P.C : nullptr;
     const long long col = c0 + 4 * tx;
@@ -1237,10 +1252,9 @@ int prepare_bf16_operands(const void *x1, const void *x2, void *scratch, bool re
     TPW_CUDA_OK(cudaMemsetAsync(lo_any, 0, 2 * sizeof(int), s));
     const int threads = 256;
     const long long cap = (long long)sm_count() * 16;
-    long long blocks = (B * N1 * 32 + threads - 1) / threads;
-    split_rows_kernel<<<(unsigned)(blocks < cap ? blocks : cap), threads, 0, s>>>((const float *)x1, xh, xl, n1, lo_any, B * N1, D, L.Dp, reciprocal_norms ? 1 : 0);
-    blocks = (B * N2 * 32 + threads - 1) / threads;
-    split_rows_kernel<<<(unsigned)(blocks < cap ? blocks : cap), threads, 0, s>>>((const float *)x2, yh, yl, n2, lo_any + 1, B * N2, D, L.Dp, reciprocal_norms ? 1 : 0);
+    const long long blocks = (B * (N1 > N2 ? N1 : N2) * 32 + threads - 1) / threads;
+    const SplitRows first{(const float *)x1, xh, xl, n1, lo_any, B * N1}, second{(const float *)x2, yh, yl, n2, lo_any + 1, B * N2};
+    split_rows_kernel<<<dim3((unsigned)(blocks < cap ? blocks : cap), 2), threads, 0, s>>>(first, second, D, L.Dp, reciprocal_norms ? 1 : 0);
     TPW_LAUNCH_OK("split_rows_kernel");
     int st;
     if ((st = make_tensor_map_3d(&M.mxh, xh, 2, L.Dp, N1, B, BK, BM, true)) != TPW_OK) return st;
@@ -1519,7 +1533,9 @@ static int dense_backward_tensor(int coef, int epilogue, bool sums, float s_mm, 
     C.n1 = static_cast<const float *>(norm1);
     C.n2 = static_cast<const float *>(norm2);
     C.epilogue = epilogue;
+    int *lo_any = reinterpret_cast<int *>(base + L.off_lo);   // [side][coefficients (not used), x]
     C.hi = F(L.off_chi); C.lo = F(L.off_clo);
+    C.clear = lo_any;
     C.rowpart = F(L.off_rowpart); C.colpart = F(L.off_colpart);
     C.R = N1; C.C = N2; C.Cp = L.N2p; C.TR = L.TR; C.TC = L.TC;
     C.vec_in = (N2 % 4 == 0 && aligned16(grad) && (coef == COEF_ID || aligned16(aux))) ? 1 : 0;
@@ -1534,8 +1550,6 @@ static int dense_backward_tensor(int coef, int epilogue, bool sums, float s_mm, 
         TPW_LAUNCH_OK("reduce_partials_kernel");
     }
     const long long cap = (long long)sm_count() * 8;
-    int *lo_any = reinterpret_cast<int *>(base + L.off_lo);   // [side][coefficients (not used), x]
-    TPW_CUDA_OK(cudaMemsetAsync(lo_any, 0, 4 * sizeof(int), s));
     const Tf32Operand Ck{F(L.off_chi), F(L.off_clo), L.N2p, false}, Cmn{F(L.off_chi), F(L.off_clo), L.N2p, true};
     for (int side = 0; side < 2; ++side) {
         void *gout = side == 0 ? grad_x1 : grad_x2;

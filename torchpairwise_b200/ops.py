@@ -815,14 +815,18 @@ def prf_div(x: Tensor, y: Tensor, mode: str = "zero") -> Tensor:
     return _PRFDivFunction.apply(x, y, _abi.PRF_IDENTITY if mode == "identity" else _abi.PRF_ZERO)
 
 
+def _takes_native_node(x1: Tensor, x2: Tensor) -> bool:
+    return (_native_ops is not None and _dot_engine == _abi.ENGINE_AUTO and x1.dtype == x2.dtype and x1.is_floating_point()
+            and x1.dim() == x2.dim() and x1.size(-1) == x2.size(-1) and (x1.dim() == 2 or x1.size(0) == x2.size(0)))
+
+
 def _cdist_p(x1: Tensor, x2: Tensor, p: float) -> Tensor:
     _require_cuda(x1, x2)
     if p < 0:
         raise RuntimeError("cdist only supports non-negative p values")
     if x1.dim() == 3 and x2.dim() == 3 and x1.size(0) != x2.size(0):
         raise RuntimeError("batch_size of x1 and x2 do not match.")
-    if _native_ops is not None and _dot_engine == _abi.ENGINE_AUTO and x1.dtype == x2.dtype and x1.is_floating_point() \
-            and x1.dim() == x2.dim() and x1.size(-1) == x2.size(-1):
+    if _takes_native_node(x1, x2):
         # The same launches and the same gradient formulas from the C++ host layer, once it is loaded: an autograd node that
         # the engine's device thread runs without the interpreter.  euclidean [75, 5, 64] forward and backward, bound by
         # the host: 146 -> 77 us.  Anything the checks above would refuse, and a chosen engine, stays below.
@@ -868,12 +872,16 @@ def sqeuclidean_distances(x1: Tensor, x2: Optional[Tensor] = None) -> Tensor:
 def cosine_similarity(x1: Tensor, x2: Optional[Tensor] = None) -> Tensor:
     x1_, x2_ = check_pairwise_inputs("cosine_similarity", x1, x2)
     _require_cuda(x1_, x2_)
+    if _takes_native_node(x1_, x2_):   # as in _cdist_p
+        return _native_ops.cosine_similarity(x1_, x2_)
     return _CosineSimilarityFunction.apply(x1_, x2_, _abi.DOT_COSINE_SIM)
 
 
 def cosine_distances(x1: Tensor, x2: Optional[Tensor] = None) -> Tensor:
     x1_, x2_ = check_pairwise_inputs("cosine_similarity", x1, x2)
     _require_cuda(x1_, x2_)
+    if _takes_native_node(x1_, x2_):   # as in _cdist_p
+        return _native_ops.cosine_distances(x1_, x2_)
     return _CosineSimilarityFunction.apply(x1_, x2_, _abi.DOT_COSINE_DIST)
 
 
