@@ -1556,9 +1556,10 @@ TORCH_LIBRARY_FRAGMENT(torchpairwise, m) {
     if (!defined("_cuda_arch_flags")) m.def("_cuda_arch_flags", &cuda_arch_flags_op);
 }
 
-// CUDA tensors of every op above.  AutogradCUDA sits in front of both the reference's
-// CompositeImplicitAutograd bodies and its `Autograd` alias kernels, for CUDA tensors only.
-TORCH_LIBRARY_IMPL(torchpairwise, AutogradCUDA, m) {
+// The ops above, for CUDA tensors.  AutogradCUDA sits in front of both the reference's CompositeImplicitAutograd bodies and its
+// `Autograd` alias kernels.  Calls below autograd, which inference mode and the body of a custom operator make, skip that
+// key and arrive at CUDA: the same bodies serve them, and record no node there.
+void register_ops(torch::Library &m) {
     m.impl("euclidean_distances", euclidean_distances);
     m.impl("l2_distances", l2_distances);
     m.impl("manhattan_distances", manhattan_distances);
@@ -1575,7 +1576,6 @@ TORCH_LIBRARY_IMPL(torchpairwise, AutogradCUDA, m) {
     m.impl("laplacian_kernel", laplacian_kernel);
     m.impl("mahalanobis_distances", mahalanobis_distances);
     m.impl("_sqmahalanobis", sqmahalanobis_raw);
-    m.impl("__sqmahalanobis_backward", sqmahalanobis_backward_op);  // runs a differentiable composition: needs the autograd key
     m.impl("pdist", pdist);
     m.impl("k_neighbors_mask", k_neighbors_mask);
     m.impl("radius_neighbors_mask", radius_neighbors_mask);
@@ -1622,9 +1622,14 @@ TORCH_LIBRARY_IMPL(torchpairwise, AutogradCUDA, m) {
     m.impl("prf_div_.Scalar", prf_div_inplace_scalar<false>);
     m.impl("prf_ldiv_.Scalar", prf_div_inplace_scalar<true>);
 }
+TORCH_LIBRARY_IMPL(torchpairwise, AutogradCUDA, m) {
+    register_ops(m);
+    m.impl("__sqmahalanobis_backward", sqmahalanobis_backward_op);  // runs a differentiable composition: needs the autograd key
+}
 
 // Ops without a gradient, and the stand-alone backward ops the reference's own Autograd kernels call.
 TORCH_LIBRARY_IMPL(torchpairwise, CUDA, m) {
+    register_ops(m);
     m.impl("pwand_sum", [](const Tensor &a, const Tensor &b) { return pw_logic(a, b, TPW_BOOL_AND_SUM); });
     m.impl("pwor_sum", [](const Tensor &a, const Tensor &b) { return pw_logic(a, b, TPW_BOOL_OR_SUM); });
     m.impl("pwxor_sum", [](const Tensor &a, const Tensor &b) { return pw_logic(a, b, TPW_BOOL_XOR_SUM); });
