@@ -57,3 +57,65 @@ def test_compositions_below_autograd(tpw):
             want = call()
         with torch.inference_mode():
             assert torch.equal(call(), want)
+
+
+SAVES_RESULT = ["euclidean_distances", "chebyshev_distances", "minkowski_distances", "cosine_distances", "cosine_similarity", "jensenshannon_distances"]
+
+
+@pytest.mark.parametrize("layer", ["python", "dispatcher"])
+@pytest.mark.parametrize("lead", [(), (2,)])
+@pytest.mark.parametrize("name", SAVES_RESULT + ["manhattan_distances", "sqeuclidean_distances", "linear_kernel", "canberra_distances", "wminkowski_distances",
+                                                 "haversine_distances", "directed_hausdorff_distances"])
+def test_changes_in_place_before_backward_are_noticed(tpw, layer, lead, name):
+    """A saved operand or result that the caller changes between forward and backward is an error, not a wrong gradient; changing
+    something that was not saved stays allowed."""
+    fn = getattr(tpw if layer == "python" else torch.ops.torchpairwise, name)
+
+    def forward():
+        x1, x2 = (t.abs().requires_grad_() for t in _inputs(lead))
+        if name == "wminkowski_distances":
+            w = torch.ones(*lead, 12, device="cuda", requires_grad=True)
+            return (x1, x2, w), fn(x1, x2, 3.0, w)
+        if name == "haversine_distances":
+            x1, x2 = (t.detach()[..., :2].contiguous().requires_grad_() for t in (x1, x2))
+        if name == "directed_hausdorff_distances":
+            x1, x2 = (t.detach().unsqueeze(len(lead)).requires_grad_() for t in (x1, x2))
+        return (x1, x2), fn(x1, x2, 3.0) if name == "minkowski_distances" else fn(x1, x2)
+
+    def total(out):
+        return (out[0] if isinstance(out, tuple) else out).sum()
+
+    inputs, out = forward()
+    total(out).backward()                                # unchanged: works
+    for i in range(len(inputs)):
+        inputs, out = forward()
+        with torch.no_grad():
+            inputs[i].mul_(1.5)
+        with pytest.raises(RuntimeError, match="inplace"):
+            total(out).backward()
+    if name in SAVES_RESULT or name == "directed_hausdorff_distances":
+        inputs, out = forward()
+        with pytest.raises(RuntimeError, match="inplace"):
+            out = out[0] if isinstance(out, tuple) else out
+            loss = out.sum()
+            with torch.no_grad():
+                out.mul_(1.5)
+            loss.backward()
+
+
+@pytest.mark.parametrize("layer", ["python", "dispatcher"])
+def test_converted_operands_may_change(tpw, layer):
+    """Operands that were converted or made contiguous are saved as copies: changing the originals afterwards changes no gradient."""
+    fn = getattr(tpw if layer == "python" else torch.ops.torchpairwise, "minkowski_distances")
+    x1, x2 = _inputs()
+    for make in (lambda t: t.bfloat16(), lambda t: t.t().contiguous().t()):
+        grads = []
+        for change in (False, True):
+            a, b = make(x1).requires_grad_(), make(x2).requires_grad_()
+            out = fn(a, b, 3.0)
+            if change:
+                with torch.no_grad():
+                    a.mul_(2), b.mul_(2)
+            out.sum().backward()
+            grads.append((a.grad, b.grad))
+        assert all(torch.equal(u, v) for u, v in zip(*grads))

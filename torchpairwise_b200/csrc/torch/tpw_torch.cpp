@@ -94,6 +94,7 @@ struct Prepared {
     Tensor a, b;
     bool unbatched;
     int64_t B, N1, N2, D;
+    Tensor s1, s2;   // a and b without the leading dimension that an unbatched call lacks
 };
 
 // contiguous() + leading batch dimension (e.g. OPS/cuda/ppminkowski_kernel.cu:70-90)
@@ -110,6 +111,8 @@ Prepared prepare(const Tensor &x1, const Tensor &x2, at::ScalarType dt) {
     p.a = x1.to(dt).contiguous();
     p.b = x2.is_same(x1) ? p.a : x2.to(dt).contiguous();
     p.unbatched = unbatched;
+    p.s1 = p.a;
+    p.s2 = p.b;
     if (unbatched) {
         p.a = p.a.unsqueeze(0);
         p.b = p.b.unsqueeze(0);
@@ -122,6 +125,12 @@ Tensor finish(Tensor out, bool unbatched, at::ScalarType dt) {
     if (unbatched) out = out.squeeze(0);
     return out.scalar_type() == dt ? out : out.to(dt);
 }
+
+// What a node saves are tensors of the caller's rank: x1 and x2 themselves where nothing converted or copied them (Prepared::s1,
+// s2), and the result as it is returned.  They share the version counter that a SavedVariable checks, so a change in place between
+// forward and backward is an error; an unsqueezed or squeezed alias made below ADInplaceOrView has a counter of its own.
+Tensor saved_result(const Tensor &out, const Tensor &returned) { return returned.scalar_type() == out.scalar_type() ? returned : out; }
+Tensor batched(const Tensor &t, bool unbatched, int64_t rank = 3) { return unbatched && t.dim() == rank - 1 ? t.unsqueeze(0) : t; }
 
 // Rows of a float32 matrix that start on no 16-byte boundary keep the L_p kernels off TMA, and the forward and the backward then
 // take several times as long; a zero feature changes no distance (0 < p) and receives no gradient that is kept.  From 2^26
@@ -264,18 +273,19 @@ struct CdistFn : torch::autograd::Function<CdistFn> {
         else if (std::isinf(p)) out = lp_forward(q, nullptr, p, 1.0);
         else if (p == 2 && tensor_engine_selected(q)) out = dot_forward(q, TPW_DOT_EUCLIDEAN, TPW_ENGINE_AUTO);
         else out = lp_forward(q, nullptr, p, 1.0 / p);
-        ctx->save_for_backward({q.a, q.b, out});
+        Tensor res = finish(out, q.unbatched, in_dt);
+        ctx->save_for_backward({q.s1, q.s2, saved_result(out, res)});
         ctx->saved_data["p"] = p;
         ctx->saved_data["unbatched"] = q.unbatched;
         ctx->saved_data["dt"] = static_cast<int64_t>(in_dt);
-        return finish(out, q.unbatched, in_dt);
+        return res;
     }
     static variable_list backward(AutogradContext *ctx, variable_list go) {
         auto s = ctx->get_saved_variables();
-        Tensor a = s[0], b = s[1];
-        const Tensor &out = s[2];
         const double p = ctx->saved_data["p"].toDouble();
         const bool ub = ctx->saved_data["unbatched"].toBool();
+        Tensor a = batched(s[0], ub), b = batched(s[1], ub);
+        const Tensor out = batched(s[2], ub);
         const auto dt = static_cast<at::ScalarType>(ctx->saved_data["dt"].toInt());
         c10::cuda::CUDAGuard dg(a.device());
         const int64_t D = a.size(2);
@@ -318,7 +328,7 @@ struct PPMinkowskiFn : torch::autograd::Function<PPMinkowskiFn> {
         if (p == 0) out = at::full({q.B, q.N1, q.N2}, static_cast<double>(q.D), q.a.options());
         else if (p == 2 && tensor_engine_selected(q)) out = dot_forward(q, TPW_DOT_SQEUCLIDEAN, TPW_ENGINE_AUTO);
         else out = lp_forward(q, nullptr, p, 1.0);
-        ctx->save_for_backward({q.a, q.b});
+        ctx->save_for_backward({q.s1, q.s2});
         ctx->saved_data["p"] = p;
         ctx->saved_data["unbatched"] = q.unbatched;
         ctx->saved_data["dt"] = static_cast<int64_t>(in_dt);
@@ -345,7 +355,7 @@ struct PPMinkowskiFn : torch::autograd::Function<PPMinkowskiFn> {
         auto s = ctx->get_saved_variables();
         const bool ub = ctx->saved_data["unbatched"].toBool();
         const auto dt = static_cast<at::ScalarType>(ctx->saved_data["dt"].toInt());
-        auto g = raw_backward(go[0], s[0], s[1], ctx->saved_data["p"].toDouble(), ub);
+        auto g = raw_backward(go[0], batched(s[0], ub), batched(s[1], ub), ctx->saved_data["p"].toDouble(), ub);
         return {finish(g.first, ub, dt), finish(g.second, ub, dt), Tensor()};
     }
 };
@@ -366,11 +376,12 @@ struct JensenShannonFn : torch::autograd::Function<JensenShannonFn> {
         else
             TPW_CALL(tpw_jensenshannon_forward(code_of(q.a), q.a.data_ptr(), q.b.data_ptr(), out.data_ptr(), q.B, q.N1, q.N2, q.D,
                                                scale, rooted ? 1 : 0, stream_of(q.a)));
-        ctx->save_for_backward({q.a, q.b, rooted ? out : Tensor()});
+        Tensor res = finish(out, q.unbatched, in_dt);
+        ctx->save_for_backward({q.s1, q.s2, rooted ? saved_result(out, res) : Tensor()});
         ctx->saved_data["scale"] = scale;
         ctx->saved_data["unbatched"] = q.unbatched;
         ctx->saved_data["dt"] = static_cast<int64_t>(in_dt);
-        return finish(out, q.unbatched, in_dt);
+        return res;
     }
     static std::pair<Tensor, Tensor> raw_backward(const Tensor &grad, const Tensor &a, const Tensor &b, const Tensor &out,
                                                   double scale, bool ub) {
@@ -386,7 +397,8 @@ struct JensenShannonFn : torch::autograd::Function<JensenShannonFn> {
         auto s = ctx->get_saved_variables();
         const bool ub = ctx->saved_data["unbatched"].toBool();
         const auto dt = static_cast<at::ScalarType>(ctx->saved_data["dt"].toInt());
-        auto g = raw_backward(go[0], s[0], s[1], s[2], ctx->saved_data["scale"].toDouble(), ub);
+        auto g = raw_backward(go[0], batched(s[0], ub), batched(s[1], ub), s[2].defined() ? batched(s[2], ub) : s[2],
+                              ctx->saved_data["scale"].toDouble(), ub);
         return {finish(g.first, ub, dt), finish(g.second, ub, dt), Tensor(), Tensor()};
     }
 };
@@ -404,7 +416,7 @@ struct PairSumFn : torch::autograd::Function<PairSumFn> {
         else
             TPW_CALL(tpw_pair_sum_forward(code_of(q.a), static_cast<int>(metric), q.a.data_ptr(), q.b.data_ptr(), out.data_ptr(),
                                           q.B, q.N1, q.N2, q.D, stream_of(q.a)));
-        ctx->save_for_backward({q.a, q.b});
+        ctx->save_for_backward({q.s1, q.s2});
         ctx->saved_data["metric"] = metric;
         ctx->saved_data["unbatched"] = q.unbatched;
         ctx->saved_data["dt"] = static_cast<int64_t>(in_dt);
@@ -423,7 +435,7 @@ struct PairSumFn : torch::autograd::Function<PairSumFn> {
         auto s = ctx->get_saved_variables();
         const bool ub = ctx->saved_data["unbatched"].toBool();
         const auto dt = static_cast<at::ScalarType>(ctx->saved_data["dt"].toInt());
-        auto g = raw_backward(go[0], s[0], s[1], static_cast<int>(ctx->saved_data["metric"].toInt()), ub);
+        auto g = raw_backward(go[0], batched(s[0], ub), batched(s[1], ub), static_cast<int>(ctx->saved_data["metric"].toInt()), ub);
         return {finish(g.first, ub, dt), finish(g.second, ub, dt), Tensor()};
     }
 };
@@ -439,7 +451,7 @@ struct HaversineFn : torch::autograd::Function<HaversineFn> {
         c10::cuda::CUDAGuard dg(q.a.device());
         Tensor out = at::empty({q.B, q.N1, q.N2}, q.a.options());
         TPW_CALL(tpw_haversine_forward(code_of(q.a), q.a.data_ptr(), q.b.data_ptr(), out.data_ptr(), q.B, q.N1, q.N2, stream_of(q.a)));
-        ctx->save_for_backward({q.a, q.b});
+        ctx->save_for_backward({q.s1, q.s2});
         ctx->saved_data["unbatched"] = q.unbatched;
         ctx->saved_data["dt"] = static_cast<int64_t>(in_dt);
         return finish(out, q.unbatched, in_dt);
@@ -457,7 +469,7 @@ struct HaversineFn : torch::autograd::Function<HaversineFn> {
         auto s = ctx->get_saved_variables();
         const bool ub = ctx->saved_data["unbatched"].toBool();
         const auto dt = static_cast<at::ScalarType>(ctx->saved_data["dt"].toInt());
-        auto g = raw_backward(go[0], s[0], s[1], ub);
+        auto g = raw_backward(go[0], batched(s[0], ub), batched(s[1], ub), ub);
         return {finish(g.first, ub, dt), finish(g.second, ub, dt)};
     }
 };
@@ -472,8 +484,8 @@ struct WMinkowskiFn : torch::autograd::Function<WMinkowskiFn> {
         require_cuda(w);
         Prepared q = prepare(x1, x2, compute_type(in_dt));
         TORCH_CHECK(q.unbatched ? w.dim() == 1 : w.dim() == 2, "w must be 1-D (unbatched) or 2-D (batched) tensor.");
-        Tensor wc = w.to(q.a.scalar_type()).contiguous();
-        if (q.unbatched) wc = wc.unsqueeze(0);
+        const Tensor ws = w.to(q.a.scalar_type()).contiguous();
+        const Tensor wc = batched(ws, q.unbatched, 2);
         TORCH_CHECK(wc.size(0) == q.B, "batch_size of x1, x2, and w do not match.");
         // the reference compares w.size(1) with N1 here (OPS/cuda/wminkowski_kernel.cu:91); the feature count is meant
         TORCH_CHECK(wc.size(1) == q.D, "feature dimension of x1, x2, and w do not match.");
@@ -481,7 +493,7 @@ struct WMinkowskiFn : torch::autograd::Function<WMinkowskiFn> {
         Tensor out;
         if (p == 0) out = at::full({q.B, q.N1, q.N2}, static_cast<double>(q.D), q.a.options());
         else out = lp_forward(q, &wc, p, std::isinf(p) ? 1.0 : 1.0 / p);
-        ctx->save_for_backward({q.a, q.b, wc});
+        ctx->save_for_backward({q.s1, q.s2, ws});
         ctx->saved_data["p"] = p;
         ctx->saved_data["unbatched"] = q.unbatched;
         ctx->saved_data["dt"] = static_cast<int64_t>(in_dt);
@@ -520,7 +532,8 @@ struct WMinkowskiFn : torch::autograd::Function<WMinkowskiFn> {
         auto s = ctx->get_saved_variables();
         const bool ub = ctx->saved_data["unbatched"].toBool();
         const auto dt = static_cast<at::ScalarType>(ctx->saved_data["dt"].toInt());
-        auto g = raw_backward(go[0], s[0], s[1], s[2], ctx->saved_data["p"].toDouble(), ub, ctx->needs_input_grad(2));
+        auto g = raw_backward(go[0], batched(s[0], ub), batched(s[1], ub), batched(s[2], ub, 2), ctx->saved_data["p"].toDouble(), ub,
+                              ctx->needs_input_grad(2));
         const Tensor &gw = std::get<2>(g);
         return {finish(std::get<0>(g), ub, dt), finish(std::get<1>(g), ub, dt), gw.defined() ? finish(gw, ub, dt) : Tensor(), Tensor()};
     }
@@ -535,16 +548,17 @@ struct CosineFn : torch::autograd::Function<CosineFn> {
         Prepared q = prepare(x1, x2, compute_type(in_dt));
         c10::cuda::CUDAGuard dg(q.a.device());
         Tensor out = dot_forward(q, static_cast<int>(epilogue), TPW_ENGINE_AUTO);
-        ctx->save_for_backward({q.a, q.b, out});
+        Tensor res = finish(out, q.unbatched, in_dt);
+        ctx->save_for_backward({q.s1, q.s2, saved_result(out, res)});
         ctx->saved_data["epilogue"] = epilogue;
         ctx->saved_data["unbatched"] = q.unbatched;
         ctx->saved_data["dt"] = static_cast<int64_t>(in_dt);
-        return finish(out, q.unbatched, in_dt);
+        return res;
     }
     static variable_list backward(AutogradContext *ctx, variable_list go) {
         auto s = ctx->get_saved_variables();
-        const Tensor &a = s[0], &b = s[1], &out = s[2];
         const bool ub = ctx->saved_data["unbatched"].toBool();
+        const Tensor a = batched(s[0], ub), b = batched(s[1], ub), out = batched(s[2], ub);
         const auto dt = static_cast<at::ScalarType>(ctx->saved_data["dt"].toInt());
         const int epilogue = static_cast<int>(ctx->saved_data["epilogue"].toInt());
         c10::cuda::CUDAGuard dg(a.device());
@@ -596,6 +610,7 @@ struct HausdorffRun {
     Tensor a, b, out, i1, i2;
     bool unbatched;
     at::ScalarType in_dt;
+    Tensor s1, s2;   // as in Prepared
 };
 
 // Checks, contiguous float32/float64 operands with a leading batch dimension, the visiting orders when
@@ -612,6 +627,7 @@ HausdorffRun hausdorff_run(const Tensor &x1, const Tensor &x2, bool shuffle, c10
     TORCH_CHECK(x1.size(-1) == x2.size(-1), "feature dimension of x1 and x2 do not match.");
     const auto dt = compute_type(in_dt);
     Tensor a = x1.to(dt).contiguous(), b = x2.is_same(x1) ? a : x2.to(dt).contiguous();
+    const Tensor s1 = a, s2 = b;
     if (ub) { a = a.unsqueeze(0); b = b.unsqueeze(0); }
     const int64_t B = a.size(0), N1 = a.size(1), M1 = a.size(2), D = a.size(3), N2 = b.size(1), M2 = b.size(2);
     c10::cuda::CUDAGuard dg(a.device());
@@ -633,7 +649,7 @@ HausdorffRun hausdorff_run(const Tensor &x1, const Tensor &x2, bool shuffle, c10
     TPW_CALL(tpw_hausdorff_forward(code_of(a), a.data_ptr(), b.data_ptr(), o1.defined() ? o1.data_ptr<int64_t>() : nullptr,
                                    o2.defined() ? o2.data_ptr<int64_t>() : nullptr, out.data_ptr(), i1.data_ptr<int64_t>(),
                                    i2.data_ptr<int64_t>(), scratch.data_ptr(), B, N1, N2, M1, M2, D, stream_of(a)));
-    return {a, b, out, i1, i2, ub, in_dt};
+    return {a, b, out, i1, i2, ub, in_dt, s1, s2};
 }
 
 // grad [B,N1,N2] (batched layout) -> one point per set and pair (OPS/cuda/hausdorff_kernel.cu:198-246)
@@ -652,20 +668,20 @@ struct HausdorffFn : torch::autograd::Function<HausdorffFn> {
                                  c10::optional<at::Generator> generator) {
         at::AutoDispatchBelowADInplaceOrView guard;
         HausdorffRun r0 = hausdorff_run(x1, x2, shuffle, generator);
-        const Tensor &a = r0.a, &b = r0.b, &out = r0.out, &i1 = r0.i1, &i2 = r0.i2;
+        const Tensor &out = r0.out, &i1 = r0.i1, &i2 = r0.i2;
         const bool ub = r0.unbatched;
         const auto in_dt = r0.in_dt;
-        ctx->save_for_backward({a, b, out, i1, i2});
+        Tensor r = finish(out, ub, in_dt), r1 = ub ? i1.squeeze(0) : i1, r2 = ub ? i2.squeeze(0) : i2;
+        ctx->save_for_backward({r0.s1, r0.s2, saved_result(out, r), r1, r2});
         ctx->saved_data["unbatched"] = ub;
         ctx->saved_data["dt"] = static_cast<int64_t>(in_dt);
-        Tensor r = finish(out, ub, in_dt), r1 = ub ? i1.squeeze(0) : i1, r2 = ub ? i2.squeeze(0) : i2;
         ctx->mark_non_differentiable({r1, r2});
         return {r, r1, r2};
     }
     static variable_list backward(AutogradContext *ctx, variable_list go) {
         auto s = ctx->get_saved_variables();
-        const Tensor &a = s[0], &b = s[1], &out = s[2], &i1 = s[3], &i2 = s[4];
         const bool ub = ctx->saved_data["unbatched"].toBool();
+        const Tensor a = batched(s[0], ub, 4), b = batched(s[1], ub, 4), out = batched(s[2], ub), i1 = batched(s[3], ub), i2 = batched(s[4], ub);
         const auto dt = static_cast<at::ScalarType>(ctx->saved_data["dt"].toInt());
         Tensor g = go[0].to(a.scalar_type()).contiguous();
         if (ub) g = g.unsqueeze(0);
@@ -1119,15 +1135,15 @@ struct LinearKernelFn : torch::autograd::Function<LinearKernelFn> {
         Prepared q = prepare(x1, x2, compute_type(in_dt));
         c10::cuda::CUDAGuard dg(q.a.device());
         Tensor out = dot_forward(q, TPW_DOT_LINEAR, tensor_engine_selected(q) ? TPW_ENGINE_TCGEN05_TF32X3 : TPW_ENGINE_SIMT_FP32);
-        ctx->save_for_backward({q.a, q.b});
+        ctx->save_for_backward({q.s1, q.s2});
         ctx->saved_data["unbatched"] = q.unbatched;
         ctx->saved_data["dt"] = static_cast<int64_t>(in_dt);
         return finish(out, q.unbatched, in_dt);
     }
     static variable_list backward(AutogradContext *ctx, variable_list go) {
         auto s = ctx->get_saved_variables();
-        const Tensor &a = s[0], &b = s[1];
         const bool ub = ctx->saved_data["unbatched"].toBool();
+        const Tensor a = batched(s[0], ub), b = batched(s[1], ub);
         const auto dt = static_cast<at::ScalarType>(ctx->saved_data["dt"].toInt());
         c10::cuda::CUDAGuard dg(a.device());
         Tensor g = go[0].to(a.scalar_type()).contiguous();
