@@ -119,3 +119,35 @@ def test_converted_operands_may_change(tpw, layer):
             out.sum().backward()
             grads.append((a.grad, b.grad))
         assert all(torch.equal(u, v) for u, v in zip(*grads))
+
+
+@pytest.mark.parametrize("name", ["euclidean_distances", "minkowski_distances", "cosine_distances", "cosine_similarity"])
+def test_refusals_and_result_types_do_not_depend_on_the_library_being_loaded(tpw, monkeypatch, name):
+    """Transforms without a rule, subclasses and arguments out of range: with the dispatcher's library loaded, what happens without."""
+    from torchpairwise_b200 import ops
+    fn = getattr(tpw, name)
+    x1, x2 = _inputs()
+
+    class Sub(torch.Tensor):
+        pass
+
+    def dual():
+        with torch.autograd.forward_ad.dual_level():
+            return fn(torch.autograd.forward_ad.make_dual(x1, x1.clone()), x2)
+
+    calls = [lambda: torch.func.vmap(fn)(torch.stack([x1, x1]), torch.stack([x2, x2])), lambda: torch.func.grad(lambda a: fn(a, x2).sum())(x1),
+             lambda: torch.func.jvp(lambda a: fn(a, x2), (x1,), (x1,)), dual, lambda: fn(x1.as_subclass(Sub), x2), lambda: fn(x1, x2.as_subclass(Sub))]
+    if name == "minkowski_distances":
+        calls += [lambda p=p: fn(x1, x2, p) for p in (float("nan"), -1.0, float("-inf"))]
+    seen = []
+    for native in (True, False):
+        if not native:
+            monkeypatch.setattr(ops, "_native_ops", None)
+        seen.append([])
+        for call in calls:
+            try:
+                seen[-1].append(type(call()))
+            except Exception as e:
+                seen[-1].append(type(e))
+    assert seen[0] == seen[1]
+    assert all(issubclass(t, Exception) for t in seen[0][:4] + seen[0][6:]) and seen[0][4:6] == [torch.Tensor] * 2

@@ -16,6 +16,8 @@ from typing import Optional, Tuple
 
 import torch
 from torch import Tensor
+from torch.autograd import forward_ad
+from torch.overrides import has_torch_function_variadic
 
 from . import _abi
 from ._abi import check, lib
@@ -816,8 +818,13 @@ def prf_div(x: Tensor, y: Tensor, mode: str = "zero") -> Tensor:
 
 
 def _takes_native_node(x1: Tensor, x2: Tensor) -> bool:
+    """Calls that the C++ node of an operator answers as the Python autograd function here does.  The function is what refuses
+    transforms it has no rule for (the dispatcher would batch the operator under vmap), and it returns a plain tensor for a
+    subclass."""
     return (_native_ops is not None and _dot_engine == _abi.ENGINE_AUTO and x1.dtype == x2.dtype and x1.is_floating_point()
-            and x1.dim() == x2.dim() and x1.size(-1) == x2.size(-1) and (x1.dim() == 2 or x1.size(0) == x2.size(0)))
+            and x1.dim() == x2.dim() and x1.size(-1) == x2.size(-1) and (x1.dim() == 2 or x1.size(0) == x2.size(0))
+            and not has_torch_function_variadic(x1, x2) and not torch._C._are_functorch_transforms_active()
+            and forward_ad._current_level < 0)
 
 
 def _cdist_p(x1: Tensor, x2: Tensor, p: float) -> Tensor:
@@ -826,7 +833,7 @@ def _cdist_p(x1: Tensor, x2: Tensor, p: float) -> Tensor:
         raise RuntimeError("cdist only supports non-negative p values")
     if x1.dim() == 3 and x2.dim() == 3 and x1.size(0) != x2.size(0):
         raise RuntimeError("batch_size of x1 and x2 do not match.")
-    if _takes_native_node(x1, x2):
+    if p == p and _takes_native_node(x1, x2):
         # The same launches and the same gradient formulas from the C++ host layer, once it is loaded: an autograd node that
         # the engine's device thread runs without the interpreter.  euclidean [75, 5, 64] forward and backward, bound by
         # the host: 146 -> 77 us.  Anything the checks above would refuse, and a chosen engine, stays below.
