@@ -175,3 +175,49 @@ def test_gradient_products_with_dealt_out_chunks(tpw, shape):
     want = (2 * (u.sum(2, keepdim=True) * a - u @ c), 2 * (u.sum(1)[..., None] * c - u.transpose(1, 2) @ a))
     for got, ref in zip(one, want):
         assert float((got - ref).abs().max()) <= 1e-5 * float(ref.abs().max())
+
+
+def test_chebyshev_backward_from_several_threads(tpw):
+    """Threads that run the Chebyshev backward with different feature counts, each on its own stream: every launch is accepted and
+    every gradient is that of a call alone.  (The kernels' shared-memory size depends on the feature count.)"""
+    import threading
+    from torchpairwise_b200 import _abi
+    lib, n = _abi.lib, 64
+
+    def problem(d):
+        g = torch.Generator().manual_seed(d)
+        x1, x2, up = torch.randn(1, n, d, generator=g).cuda(), torch.randn(1, n, d, generator=g).cuda(), torch.randn(1, n, n, generator=g).cuda()
+        out = tpw.chebyshev_distances(x1, x2)
+        scratch = torch.empty(lib.tpw_chebyshev_backward_scratch_bytes(_abi.F32, 1, n, n, d), dtype=torch.uint8, device="cuda")
+        return x1, x2, up, out, scratch, torch.empty_like(x1), torch.empty_like(x2)
+
+    def call(pr, d, stream):
+        x1, x2, up, out, scratch, g1, g2 = pr
+        return lib.tpw_chebyshev_backward_ws(up.data_ptr(), out.data_ptr(), x1.data_ptr(), x2.data_ptr(), g1.data_ptr(), g2.data_ptr(),
+                                             scratch.data_ptr(), scratch.numel(), 1, n, n, d, stream)
+
+    dims = [16, 256, 64, 252]
+    problems = [problem(d) for d in dims]
+    torch.cuda.synchronize()
+    want = []
+    for pr, d in zip(problems, dims):
+        assert call(pr, d, torch.cuda.current_stream().cuda_stream) == 0
+        torch.cuda.synchronize()
+        want.append((pr[5].clone(), pr[6].clone()))
+    status = [0] * len(dims)
+    streams = [torch.cuda.Stream() for _ in dims]
+
+    def work(t):
+        torch.cuda.set_device(0)
+        for _ in range(1000):
+            status[t] |= call(problems[t], dims[t], streams[t].cuda_stream)
+
+    threads = [threading.Thread(target=work, args=(t,)) for t in range(len(dims))]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    torch.cuda.synchronize()
+    assert status == [0] * len(dims)
+    for pr, (w1, w2) in zip(problems, want):
+        assert torch.equal(pr[5], w1) and torch.equal(pr[6], w2)

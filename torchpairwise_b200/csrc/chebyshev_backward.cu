@@ -478,12 +478,13 @@ extern "C" int tpw_chebyshev_backward_ws(const void *grad, const void *out, cons
     S.x1 = M.x1; S.x2 = M.x2; S.fwd = M.out;
     S.B = B; S.N1 = N1; S.N2 = N2; S.D = D;
     S.tiles_k = (D + SD - 1) / SD;
+    // the limit belongs to the kernel, not to the call: always the largest, so that threads with other feature counts may launch
     const int smem = scatter_smem(D < SD ? (int)D : SD);
     if (grad_x1) {
         S.out = static_cast<float *>(grad_x1); S.NR = N1; S.tiles_r = (N1 + SR - 1) / SR;
         const long long n = B * S.tiles_r * S.tiles_k;
         TPW_CHECK_ARG(n < (1ll << 31), "tpw_chebyshev_backward_ws: too many row blocks");
-        TPW_CUDA_OK(cudaFuncSetAttribute(chebyshev_scatter_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        TPW_CUDA_OK(cudaFuncSetAttribute(chebyshev_scatter_kernel<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, scatter_smem(SD)));
         chebyshev_scatter_kernel<false><<<(unsigned)n, STHR, smem, s>>>(S);
         TPW_LAUNCH_OK("chebyshev_scatter_kernel (grad_x1)");
     }
@@ -491,7 +492,7 @@ extern "C" int tpw_chebyshev_backward_ws(const void *grad, const void *out, cons
         S.out = static_cast<float *>(grad_x2); S.NR = N2; S.tiles_r = (N2 + SR - 1) / SR;
         const long long n = B * S.tiles_r * S.tiles_k;
         TPW_CHECK_ARG(n < (1ll << 31), "tpw_chebyshev_backward_ws: too many row blocks");
-        TPW_CUDA_OK(cudaFuncSetAttribute(chebyshev_scatter_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        TPW_CUDA_OK(cudaFuncSetAttribute(chebyshev_scatter_kernel<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, scatter_smem(SD)));
         chebyshev_scatter_kernel<true><<<(unsigned)n, STHR, smem, s>>>(S);
         TPW_LAUNCH_OK("chebyshev_scatter_kernel (grad_x2)");
     }
