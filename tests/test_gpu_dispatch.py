@@ -151,3 +151,12 @@ def test_refusals_and_result_types_do_not_depend_on_the_library_being_loaded(tpw
                 seen[-1].append(type(e))
     assert seen[0] == seen[1]
     assert all(issubclass(t, Exception) for t in seen[0][:4] + seen[0][6:]) and seen[0][4:6] == [torch.Tensor] * 2
+
+
+@pytest.mark.parametrize("n", [96, 520])
+def test_boolean_rows_of_a_matrix_against_its_columns(tpw, n):
+    """x and x.t() share pointer and shape, and are not the same rows (96: packed words, 520: tensor-core counts)."""
+    x = (torch.rand(n, n, generator=torch.Generator().manual_seed(n)) < 0.3).cuda()
+    for fn in (tpw.jaccard_distances, tpw.hamming_distances, torch.ops.torchpairwise.jaccard_distances):
+        assert torch.equal(fn(x, x.t()), fn(x, x.t().contiguous()))
+        assert torch.equal(fn(x, x[:]), fn(x, x.clone()))

@@ -701,7 +701,7 @@ def _bool_metric_raw(x1: Tensor, x2: Tensor, metric: str) -> Tensor:
                       "rogerstanimoto", "sokalmichener", "sokalsneath"):
             out.fill_(float("nan"))
     elif out.numel() > 0:
-        same = x2c is x1c or (x2c.data_ptr() == x1c.data_ptr() and x2c.shape == x1c.shape)
+        same = x2c is x1c or (x2c.data_ptr() == x1c.data_ptr() and x2c.shape == x1c.shape and x2c.stride() == x1c.stride())
         pitch = lib.tpw_bool_rows_pitch(B, N1, N2, D)
         if pitch > 0:
             # large problem: the counts come from the tensor cores (8-bit integer contraction of the 0 / 1 bytes)
