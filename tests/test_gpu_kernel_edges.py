@@ -221,3 +221,32 @@ def test_chebyshev_backward_from_several_threads(tpw):
     assert status == [0] * len(dims)
     for pr, (w1, w2) in zip(problems, want):
         assert torch.equal(pr[5], w1) and torch.equal(pr[6], w2)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("shape", [(1, 15, 33, 9), (2, 17, 31, 33), (1, 300, 65, 32), (1, 64, 300, 40), (1, 1400, 40, 64), (1, 1420, 33, 64), (1, 45, 2100, 64),
+                                   (3, 700, 31, 64)])
+def test_small_backward_kernels_equal_the_tile_kernel(tpw, monkeypatch, dtype, shape):
+    """Few gradient blocks run with one or two elements to a thread, by a rule on type, metric, side and number of elements; either
+    way every metric's gradients are the tile kernel's bit for bit."""
+    from torchpairwise_b200 import _abi
+    lib, (b, n1, n2, d) = _abi.lib, shape
+    g = torch.Generator().manual_seed(n1 + n2)
+    x1, x2 = torch.randn(b, n1, d, generator=g).to(dtype).cuda(), torch.randn(b, n2, d, generator=g).to(dtype).cuda()
+    up, aux, w = torch.randn(b, n1, n2, generator=g).to(dtype).cuda(), (torch.rand(b, n1, n2, generator=g) + 0.5).to(dtype).cuda(), torch.rand(b, d, generator=g).to(dtype).cuda()
+    largest = (x1[:, :, None] - x2[:, None]).abs().amax(3)
+    code = _abi.F32 if dtype == torch.float32 else _abi.F64
+    modes = [(_abi.LP_BWD_CDIST, p) for p in (1.0, 2.0, 3.0, 2.5, math.inf)] + [(m, p) for m in (_abi.LP_BWD_PPMINKOWSKI, _abi.LP_BWD_WMINKOWSKI) for p in (1.0, 2.0, 3.0, 1.5)]
+    for mode, p in modes + [(_abi.LP_BWD_MATMUL, 2.0)]:
+        res = []
+        for tile in (False, True):
+            if tile:
+                monkeypatch.setenv("TPW_DISABLE_SMALL_BWD", "1")
+            g1, g2 = torch.full_like(x1, math.nan), torch.full_like(x2, math.nan)
+            _abi.check(lib.tpw_lp_backward(code, mode, up.data_ptr(), (largest if math.isinf(p) else aux).data_ptr(), x1.data_ptr(), x2.data_ptr(),
+                                           w.data_ptr() if mode == _abi.LP_BWD_WMINKOWSKI else None, g1.data_ptr(), g2.data_ptr(), b, n1, n2, d, p,
+                                           torch.cuda.current_stream().cuda_stream))
+            monkeypatch.delenv("TPW_DISABLE_SMALL_BWD", raising=False)
+            res.append((g1, g2))
+        assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1]), (mode, p)
+        assert not torch.isnan(res[0][0]).any() and not torch.isnan(res[0][1]).any()

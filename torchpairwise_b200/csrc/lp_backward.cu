@@ -361,46 +361,46 @@ __global__ void __launch_bounds__(256) lp_backward_small_kernel(const BwdParams 
     reinterpret_cast<T *>(P.out)[idx] = v;
 }
 
-// The same problems on rows of more than 8 features.  One thread per element loads a streamed value, the gradient and the
-// auxiliary value for every term; here a thread has R rows of one feature, so a streamed value serves R terms, and the CTA
-// forms the coefficients of its rows and of 32 streamed rows once, in shared memory, from where a warp reads R of them with one or two
-// broadcast loads.  KL lanes span the features (16 where that leaves fewer lanes idle), 256 / KL groups of R rows make a
-// CTA.  The terms of an element are added in the same order, so the results are still those of the tile kernel bit for bit.
-// Bound: arithmetic and the broadcast loads.  Weighted p = 2 in float64 [1500, 1301, 75], both gradients: 351 -> 256 us.
+// The same problems on rows of more than 8 features, where rows_pay() below says so.  One thread per element loads a streamed
+// value, the gradient and the auxiliary value for every term; here a thread has two rows of one feature, so a streamed value serves
+// two terms, and the CTA forms the coefficients of its 16 rows and of 32 streamed rows once, in shared memory, from where a warp
+// reads them with one broadcast load.  The terms of an element are added in the same order, so the results are still those of the
+// tile kernel bit for bit.  Bound: latency of that load and of the terms' chain; eight warps, each over 32 features.  (Four rows to
+// a thread, or 16 features to a group, were slower or within 5 % in all but a few of 24 combinations of metric, type and side.)
+// Weighted p = 2 in float64 [1500, 1301, 75], both gradients: 351 -> 237 us.
 constexpr int SB_THREADS = 256;
 constexpr int SB_S = 32;       // streamed rows per stage
+constexpr int SB_R = 2;        // rows per thread
+constexpr int SB_ROWS = SB_THREADS / 32 * SB_R;
+constexpr int SB_PER = SB_ROWS * SB_S / SB_THREADS;   // pairs of a stage that a thread forms the coefficients of
 
-template <typename T, int PHI, bool NEED_AUX, bool TRANS, int KL, int R>
+template <typename T, int PHI, bool NEED_AUX, bool TRANS>
 __global__ void __launch_bounds__(SB_THREADS) lp_backward_rows_kernel(const BwdParams P) {
-    if (P.only_if && *P.only_if <= P.only_if_above) return;
-    constexpr int GROUPS = SB_THREADS / KL, RB = GROUPS * R, PER = RB * SB_S / SB_THREADS;
-    constexpr int PITCH = RB + 16 / (int)sizeof(T);      // rows of 16-byte multiples, shifted by a bank group from row to row
-    constexpr bool NEED_O = PHI == PHI_SGN_EQ;            // the term looks at the auxiliary value itself
+    constexpr int PITCH = SB_ROWS + 16 / (int)sizeof(T);      // rows of 16-byte multiples, shifted by a bank group from row to row
     __shared__ __align__(16) T cs[2][SB_S * PITCH];
-    __shared__ __align__(16) T os[NEED_O ? 2 : 1][NEED_O ? SB_S * PITCH : 1];
-    const int tid = threadIdx.x, lane = tid % KL, group = tid / KL;
+    const int tid = threadIdx.x, lane = tid & 31, group = tid >> 5;
     long long tile = blockIdx.x;
     const long long tk = tile % P.tiles_k;
     tile /= P.tiles_k;
     const long long tr = tile % P.tiles_r, b = tile / P.tiles_r;
-    const long long k = tk * KL + lane, r0 = tr * RB, row = r0 + group * R;
+    const long long k = tk * 32 + lane, r0 = tr * SB_ROWS, row = r0 + group * SB_R;
     const bool k_ok = k < P.D;
     const T *stream = reinterpret_cast<const T *>(P.stream) + b * P.NS * P.D + (k_ok ? k : 0);
     const T *grad = reinterpret_cast<const T *>(P.grad) + b * P.N1 * P.N2;
     const T *aux = NEED_AUX ? reinterpret_cast<const T *>(P.aux) + b * P.N1 * P.N2 : nullptr;
-    T x[R], acc[R];
+    T x[SB_R], acc[SB_R];
 #pragma unroll
-    for (int a = 0; a < R; ++a) {
+    for (int a = 0; a < SB_R; ++a) {
         x[a] = PHI != PHI_Y && k_ok && row + a < P.NR ? reinterpret_cast<const T *>(P.rowop)[(b * P.NR + row + a) * P.D + k] : T(0);
         acc[a] = T(0);
     }
     // this thread's pairs of a stage: consecutive threads along the dimension that is contiguous in memory
-    T g[PER], o[PER];
+    T g[SB_PER], o[SB_PER];
     auto fetch = [&](long long s0) {
 #pragma unroll
-        for (int u = 0; u < PER; ++u) {
+        for (int u = 0; u < SB_PER; ++u) {
             const int e = tid + u * SB_THREADS;
-            const long long r = r0 + (TRANS ? e % RB : e / SB_S), s = s0 + (TRANS ? e / RB : e % SB_S);
+            const long long r = r0 + (TRANS ? e % SB_ROWS : e / SB_S), s = s0 + (TRANS ? e / SB_ROWS : e % SB_S);
             const bool ok = r < P.NR && s < P.NS;
             const long long at = TRANS ? s * P.N2 + r : r * P.N2 + s;
             g[u] = ok ? grad[at] : T(0);
@@ -413,25 +413,21 @@ __global__ void __launch_bounds__(SB_THREADS) lp_backward_rows_kernel(const BwdP
     for (long long s0 = 0; s0 < P.NS; s0 += SB_S, buf ^= 1) {
         // a warp may still be reading the other buffer; this one was last read before the previous barrier
 #pragma unroll
-        for (int u = 0; u < PER; ++u) {
+        for (int u = 0; u < SB_PER; ++u) {
             const int e = tid + u * SB_THREADS;
-            const int at = (TRANS ? e / RB : e % SB_S) * PITCH + (TRANS ? e % RB : e / SB_S);
+            const int at = (TRANS ? e / SB_ROWS : e % SB_S) * PITCH + (TRANS ? e % SB_ROWS : e / SB_S);
             cs[buf][at] = NEED_AUX ? bwd_coefficient<T>(P.coef_mode, g[u], o[u], P.q) : g[u];
-            if (NEED_O) os[NEED_O ? buf : 0][NEED_O ? at : 0] = o[u];
         }
         __syncthreads();
         if (s0 + SB_S < P.NS) fetch(s0 + SB_S);
         const int cnt = (int)(P.NS - s0 < SB_S ? P.NS - s0 : SB_S);
         const T *sp = stream + s0 * P.D;
         auto term = [&](int s, T y) {
-            T c[R], ov[R];
+            T c[SB_R];
 #pragma unroll
-            for (int a = 0; a < R; ++a) {
-                c[a] = cs[buf][s * PITCH + group * R + a];
-                ov[a] = NEED_O ? os[NEED_O ? buf : 0][NEED_O ? s * PITCH + group * R + a : 0] : T(0);
-            }
+            for (int a = 0; a < SB_R; ++a) c[a] = cs[buf][s * PITCH + group * SB_R + a];
 #pragma unroll
-            for (int a = 0; a < R; ++a) bwd_accumulate<PHI, T>(acc[a], x[a], y, c[a], ov[a], q, P.pow_spec);
+            for (int a = 0; a < SB_R; ++a) bwd_accumulate<PHI, T>(acc[a], x[a], y, c[a], T(0), q, P.pow_spec);
         };
         int s = 0;
         for (; s + 8 <= cnt; s += 8) {
@@ -445,7 +441,7 @@ __global__ void __launch_bounds__(SB_THREADS) lp_backward_rows_kernel(const BwdP
     }
     if (!k_ok) return;
 #pragma unroll
-    for (int a = 0; a < R; ++a) {
+    for (int a = 0; a < SB_R; ++a) {
         if (row + a >= P.NR) continue;
         T v = acc[a] * (T)P.post;
         if (P.w) v *= reinterpret_cast<const T *>(P.w)[b * P.D + k];
@@ -453,20 +449,36 @@ __global__ void __launch_bounds__(SB_THREADS) lp_backward_rows_kernel(const BwdP
     }
 }
 
-template <typename T, int PHI, bool NEED_AUX, bool TRANS, int KL>
-int launch_backward_rows(BwdParams P, cudaStream_t stream) {
-    P.tiles_k = (P.D + KL - 1) / KL;
-    // four rows to a thread where that still gives every SM a CTA, else two
-    const long long four = P.B * P.tiles_k * ((P.NR + SB_THREADS / KL * 4 - 1) / (SB_THREADS / KL * 4));
-    constexpr bool FOUR = !(sizeof(T) == 8 && PHI == PHI_SGN_EQ && KL == 16);   // two float64 tiles of 64 rows exceed 48 KB
-    const int R = FOUR && four >= sm_count() ? 4 : 2;
-    P.tiles_r = (P.NR + SB_THREADS / KL * R - 1) / (SB_THREADS / KL * R);
-    const long long tiles = P.B * P.tiles_r * P.tiles_k;
-    TPW_CHECK_ARG(tiles < (1ll << 31), "lp backward: too many tiles (%lld)", tiles);
-    if (FOUR && R == 4) lp_backward_rows_kernel<T, PHI, NEED_AUX, TRANS, KL, FOUR ? 4 : 2><<<(unsigned)tiles, SB_THREADS, 0, stream>>>(P);
-    else lp_backward_rows_kernel<T, PHI, NEED_AUX, TRANS, KL, 2><<<(unsigned)tiles, SB_THREADS, 0, stream>>>(P);
-    TPW_LAUNCH_OK("lp_backward_rows_kernel");
-    return TPW_OK;
+// Where the rows kernel is faster than one thread per element.  Each of its walks is a chain of shared loads with a barrier every
+// 32 rows, at twice the elements per thread; it pays where forming a coefficient costs more than that (a division in float64, a power),
+// where the other kernel reads the gradient across its rows (some grad_x2 walks), or where one thread per element runs in more waves
+// than the GPU holds.  Times over one thread per element at 20 to 3000 rows, 9 to 500 features, 1000 streamed rows, for n = rows x
+// features (grad_x1 / grad_x2):
+//   float32  no coefficient  sign 1.3 / 0.4, d 1.5 / 0.7, d|d| 0.85 / 0.85 (n > 2^17.5: 1.0 / 0.8), power 2.1 / 1.4, product 1.1 / 1.2
+//            g / out         0.95 to 1.05 / 0.65, from n = 2^16.5 0.75 / 0.5;   g / out^2  1.3 / 1.4, from 2^17 0.75 / 0.65;
+//            power of out    0.2 to 0.4;   weights  1.2 to 3, d from 2^17 0.85 / 0.7
+//   float64  no coefficient  sign 1.0, d 0.5 / 0.9, d|d| 1.25, power 1.4 to 1.9, product 0.4 / 1.05
+//            any of out      0.3 to 0.95;   weights  1.1 to 1.9, from 2^16.5 0.6 to 0.8 (power never below 1.1)
+//   the maximum's gradient (it compares with the auxiliary value in every term) 1.5 to 3 in both types
+template <typename T, int PHI, bool NEED_AUX, bool TRANS>
+constexpr bool rows_may_pay() {
+    if (PHI == PHI_SGN_EQ) return false;
+    if (NEED_AUX) return true;
+    if (sizeof(T) == 4) return PHI == PHI_DABS || (TRANS && (PHI == PHI_SGN || PHI == PHI_D));
+    return PHI == PHI_D || (PHI == PHI_Y && !TRANS);
+}
+template <typename T, int PHI, bool NEED_AUX, bool TRANS>
+bool rows_pay(const BwdParams &P) {
+    if (!rows_may_pay<T, PHI, NEED_AUX, TRANS>() || P.D <= 8) return false;
+    const long long n = P.B * P.NR * P.D, more = 90000, many = 131072;
+    if (!NEED_AUX) return sizeof(T) == 8 || TRANS || n < many;
+    switch (P.coef_mode) {
+        case COEF_DIV_POW: return true;
+        case COEF_DIV_O: return sizeof(T) == 8 || TRANS || n >= more;
+        case COEF_DIV_O2: return sizeof(T) == 8 || n >= many;
+        case COEF_MUL: return sizeof(T) == 8 ? PHI != PHI_SGNPOW && n >= more : PHI == PHI_D && n >= many;
+        default: return false;
+    }
 }
 
 template <typename T, int PHI, bool NEED_AUX, bool TRANS>
@@ -484,12 +496,20 @@ int launch_backward(BwdParams P, cudaStream_t stream) {
                   "lp backward: a dimension exceeds 2^31-1");
     P.status = device_status_ptr();
 
-    // fewer gradient blocks than a third of the SMs: one thread per gradient element instead (TPW_DISABLE_SMALL_BWD=1
-    // keeps the tile kernel); the walk per thread is bounded so that a launch stays in the millisecond range
+    // fewer gradient blocks than a third of the SMs: one thread per gradient element, or two rows of a feature to a thread, instead
+    // (TPW_DISABLE_SMALL_BWD=1 keeps the tile kernel); the walk per thread is bounded so that a launch stays in the millisecond range
     if (tiles * 3 < sm_count() && P.NS <= 65536 && P.B * P.NR * P.D < (1ll << 31) * 256 && !getenv("TPW_DISABLE_SMALL_BWD")) {
-        if (P.D > 8)
-            return (P.D + 15) / 16 * 16 < (P.D + 31) / 32 * 32 ? launch_backward_rows<T, PHI, NEED_AUX, TRANS, 16>(P, stream)
-                                                               : launch_backward_rows<T, PHI, NEED_AUX, TRANS, 32>(P, stream);
+        if constexpr (rows_may_pay<T, PHI, NEED_AUX, TRANS>()) {
+            if (rows_pay<T, PHI, NEED_AUX, TRANS>(P)) {
+                P.tiles_k = (P.D + 31) / 32;
+                P.tiles_r = (P.NR + SB_ROWS - 1) / SB_ROWS;
+                const long long ctas = P.B * P.tiles_r * P.tiles_k;
+                TPW_CHECK_ARG(ctas < (1ll << 31), "lp backward: too many tiles (%lld)", ctas);
+                lp_backward_rows_kernel<T, PHI, NEED_AUX, TRANS><<<(unsigned)ctas, SB_THREADS, 0, stream>>>(P);
+                TPW_LAUNCH_OK("lp_backward_rows_kernel");
+                return TPW_OK;
+            }
+        }
         const long long n = P.B * P.NR * P.D;
         lp_backward_small_kernel<T, PHI, NEED_AUX, TRANS><<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(P);
         TPW_LAUNCH_OK("lp_backward_small_kernel");
