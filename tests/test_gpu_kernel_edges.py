@@ -135,14 +135,19 @@ def test_quotients_of_counts_round_as_the_division(tpw):
         assert torch.equal(tpw.hamming_distances(x, x2), (diff.double() / d).float())
 
 
+@pytest.mark.parametrize("layer", ["python", "dispatcher"])
 @pytest.mark.parametrize("p", [1.0, 3.0, math.inf])
-def test_rows_padded_to_whole_vectors(tpw, p):
+def test_rows_padded_to_whole_vectors(tpw, monkeypatch, p, layer):
     """Large problems whose feature count is no multiple of 4 run on zero-padded copies; the same batches one at a time are too
     small for that.  The forward and the Chebyshev gradients add the same terms in the same order (bit-equal), the others in
     another order (sums of up to 600 float32 terms)."""
+    from torchpairwise_b200 import ops
+    tpw.load_torch_ops()
+    monkeypatch.setattr(ops, "_native_ops", None if layer == "python" else torch.ops.torchpairwise)
     g = torch.Generator().manual_seed(7)
-    x1, x2 = torch.randn(4, 600, 201, generator=g).cuda(), torch.randn(4, 500, 201, generator=g).cuda()
-    gr = torch.randn(4, 600, 500, generator=g).cuda()
+    n = 7   # 4e8 terms: forward, one-pass backward and Chebyshev backward are all padded
+    x1, x2 = torch.randn(n, 600, 201, generator=g).cuda(), torch.randn(n, 500, 201, generator=g).cuda()
+    gr = torch.randn(n, 600, 500, generator=g).cuda()
 
     def grads(a, c, up):
         a, c = a.clone().requires_grad_(), c.clone().requires_grad_()
@@ -150,7 +155,7 @@ def test_rows_padded_to_whole_vectors(tpw, p):
         return (out.detach(), *torch.autograd.grad(out, (a, c), up))
 
     whole = grads(x1, x2, gr)
-    parts = [torch.stack(t) for t in zip(*(grads(x1[b], x2[b], gr[b]) for b in range(4)))]
+    parts = [torch.stack(t) for t in zip(*(grads(x1[b], x2[b], gr[b]) for b in range(n)))]
     assert whole[1].shape == x1.shape and whole[2].shape == x2.shape and whole[1].is_contiguous()
     assert torch.equal(whole[0], parts[0])
     for w, q in zip(whole[1:], parts[1:]):

@@ -15,6 +15,7 @@
 // CPU; a CPU tensor reaching one of these kernels is an error.
 #include <ATen/ATen.h>
 #include <ATen/core/dispatch/Dispatcher.h>
+#include <ATen/cuda/CUDAContext.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <c10/cuda/CUDAStream.h>
 #include <c10/util/Logging.h>
@@ -132,13 +133,27 @@ Tensor finish(Tensor out, bool unbatched, at::ScalarType dt) {
 Tensor saved_result(const Tensor &out, const Tensor &returned) { return returned.scalar_type() == out.scalar_type() ? returned : out; }
 Tensor batched(const Tensor &t, bool unbatched, int64_t rank = 3) { return unbatched && t.dim() == rank - 1 ? t.unsqueeze(0) : t; }
 
-// Rows of a float32 matrix that start on no 16-byte boundary keep the L_p kernels off TMA, and the forward and the backward then
-// take several times as long; a zero feature changes no distance (0 < p) and receives no gradient that is kept.  From 2^26
-// terms on, the copies cost a few hundredths of that.  minkowski p = 3 [9, 462, 1648, 201], forward and backward:
-// 1619 -> 649 us.  (Up to 32 features the forward has kernels that read any row.)
-bool worth_padding(const Tensor &a, const Tensor &b, double p) {
-    return a.scalar_type() == at::kFloat && a.size(2) % 4 != 0 && a.size(2) > 32 && p > 0 &&
-           static_cast<double>(a.size(0)) * a.size(1) * b.size(1) * a.size(2) >= 67108864.0;
+// Rows of a float32 matrix that start on no 16-byte boundary keep the L_p kernels off TMA; a zero feature changes no distance
+// (0 < p) and receives no gradient that is kept, so large problems run on padded copies.  (Up to 32 features the forward has
+// kernels that read any row.)  The copies are two to six short launches, 5 to 15 us.
+// Forward: that is more than TMA gives below 4e8 terms: p = 1 [2000, 1100, 33] 21 -> 28 us, [1500, 1301, 75] 33 -> 37 us, from there
+// on 0.95 to 0.65 of the time; other powers are bound by arithmetic and gain only from 2^30 terms on.
+bool may_pad(const Tensor &a, double p) { return a.scalar_type() == at::kFloat && a.size(2) % 4 != 0 && a.size(2) > 32 && p > 0; }
+double terms(const Tensor &a, const Tensor &b) { return static_cast<double>(a.size(0)) * a.size(1) * b.size(1) * a.size(2); }
+bool pads_forward(const Tensor &a, const Tensor &b, double p) {
+    return may_pad(a, p) && terms(a, b) >= (p == 1 || p == 2 || p == 3 || std::isinf(p) ? 4e8 : 1073741824.0);
+}
+// Backward: the one-pass kernel, where it serves the padded problem, is worth the copies at any size (p = 3 [1000, 1000, 129] 296 -> 99 us),
+// the tile kernels from 2^29 terms on (0.5 to 0.9) unless one side has so few rows that the other's copy counts ([60000, 60, 350], grad_x1
+// of p = 1, 364 -> 440 us), the kernels that few gradient blocks run with never ([16, 150, 857, 75] 171 -> 214 us).  Chebyshev: from 2^28 terms on ([1500, 1301, 75] 178 -> 189 us, beyond 0.6 to 1.0).
+bool pads_backward(const Tensor &a, const Tensor &b, double p, bool one, bool two) {
+    if (!may_pad(a, p)) return false;
+    if (std::isinf(p)) return terms(a, b) >= 268435456.0;
+    const int64_t B = a.size(0), N1 = a.size(1), N2 = b.size(1), D = (a.size(2) + 3) / 4 * 4;
+    if (one && two && tpw_lp_backward_scratch_bytes(TPW_F32, TPW_LP_BWD_CDIST, B, N1, N2, D, p) > 0) return true;
+    const int64_t sms = at::cuda::getCurrentDeviceProperties()->multiProcessorCount;
+    auto tiles = [&](int64_t rows) { return B * ((rows + 127) / 128) * ((D + 127) / 128) * 3 >= sms; };   // of lp_backward.cu
+    return terms(a, b) >= 536870912.0 && std::min(N1, N2) >= 256 && (!one || tiles(N1)) && (!two || tiles(N2));
 }
 Tensor pad_features(const Tensor &x) {
     const int64_t D = x.size(2);
@@ -146,7 +161,7 @@ Tensor pad_features(const Tensor &x) {
 }
 
 Tensor lp_forward(const Prepared &p, const Tensor *w, double pw, double exponent) {
-    if (!w && worth_padding(p.a, p.b, pw)) {
+    if (!w && pads_forward(p.a, p.b, pw)) {
         Prepared r = p;
         r.a = pad_features(p.a);
         r.b = p.b.is_same(p.a) ? r.a : pad_features(p.b);
@@ -289,7 +304,7 @@ struct CdistFn : torch::autograd::Function<CdistFn> {
         const auto dt = static_cast<at::ScalarType>(ctx->saved_data["dt"].toInt());
         c10::cuda::CUDAGuard dg(a.device());
         const int64_t D = a.size(2);
-        if (p != 2 && worth_padding(a, b, p)) {
+        if (p != 2 && pads_backward(a, b, p, ctx->needs_input_grad(0), ctx->needs_input_grad(1))) {
             a = pad_features(a);
             b = pad_features(b);
         }

@@ -140,11 +140,33 @@ def _sizes(x1c: Tensor, x2c: Tensor):
 # --------------------------------------------------------------------------------------------
 # raw launches (no autograd)
 # --------------------------------------------------------------------------------------------
-def _worth_padding(x1c: Tensor, x2c: Tensor, p: float) -> bool:
-    """float32 rows that start on no 16-byte boundary, from 2^26 terms on: zero features cost less than kernels without TMA
-    (the reasons and figures stand at ``worth_padding`` in csrc/torch/tpw_torch.cpp)."""
+# Zero features for float32 rows that start on no 16-byte boundary, by the rules of ``pads_forward`` and ``pads_backward`` in
+# csrc/torch/tpw_torch.cpp (the reasons and figures stand there).
+def _may_pad(x1c: Tensor, p: float) -> bool:
+    return x1c.dtype == torch.float32 and x1c.size(2) % 4 != 0 and x1c.size(2) > 32 and p > 0
+
+
+def _pads_forward(x1c: Tensor, x2c: Tensor, p: float) -> bool:
+    return _may_pad(x1c, p) and math.prod(_sizes(x1c, x2c)) >= (4e8 if p in (1, 2, 3, math.inf) else 1 << 30)
+
+
+def _pads_backward(x1c: Tensor, x2c: Tensor, p: float, one: bool, two: bool) -> bool:
+    if not _may_pad(x1c, p):
+        return False
     B, N1, N2, D = _sizes(x1c, x2c)
-    return x1c.dtype == torch.float32 and D % 4 != 0 and D > 32 and p > 0 and B * N1 * N2 * D >= 1 << 26
+    terms = B * N1 * N2 * D
+    if math.isinf(p):
+        return terms >= 1 << 28
+    D += -D % 4
+    if one and two:
+        with torch.cuda.device(x1c.device):
+            if lib.tpw_lp_backward_scratch_bytes(_abi.F32, _abi.LP_BWD_CDIST, B, N1, N2, D, float(p)) > 0:
+                return True
+    sms = torch.cuda.get_device_properties(x1c.device).multi_processor_count
+
+    def tiles(rows: int) -> bool:
+        return B * -(-rows // 128) * -(-D // 128) * 3 >= sms
+    return terms >= 1 << 29 and min(N1, N2) >= 256 and (not one or tiles(N1)) and (not two or tiles(N2))
 
 
 def _pad_features(xc: Tensor) -> Tensor:
@@ -152,7 +174,7 @@ def _pad_features(xc: Tensor) -> Tensor:
 
 
 def _lp_forward_raw(x1c: Tensor, x2c: Tensor, w: Optional[Tensor], p: float, out_exponent: float) -> Tensor:
-    if w is None and _worth_padding(x1c, x2c, p):
+    if w is None and _pads_forward(x1c, x2c, p):
         return _lp_forward_raw(_pad_features(x1c), _pad_features(x2c), w, p, out_exponent)
     B, N1, N2, D = _sizes(x1c, x2c)
     out = torch.empty((B, N1, N2), dtype=x1c.dtype, device=x1c.device)
@@ -167,7 +189,7 @@ def _lp_forward_raw(x1c: Tensor, x2c: Tensor, w: Optional[Tensor], p: float, out
 def _lp_backward_raw(mode: int, grad: Tensor, aux: Optional[Tensor], x1c: Tensor, x2c: Tensor,
                      w: Optional[Tensor], p: float, need1: bool = True, need2: bool = True):
     B, N1, N2, D = _sizes(x1c, x2c)
-    if mode == _abi.LP_BWD_CDIST and w is None and p != 2 and _worth_padding(x1c, x2c, p):
+    if mode == _abi.LP_BWD_CDIST and w is None and p != 2 and _pads_backward(x1c, x2c, p, need1, need2):
         res = _lp_backward_raw(mode, grad, aux, _pad_features(x1c), _pad_features(x2c), w, p, need1, need2)
         return tuple(None if r is None else r[..., :D].contiguous() for r in res)
     if mode == _abi.LP_BWD_CDIST and w is None and math.isinf(p) and p > 0 and (need1 or need2):
