@@ -255,3 +255,15 @@ def test_small_backward_kernels_equal_the_tile_kernel(tpw, monkeypatch, dtype, s
             res.append((g1, g2))
         assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1]), (mode, p)
         assert not torch.isnan(res[0][0]).any() and not torch.isnan(res[0][1]).any()
+
+
+@pytest.mark.parametrize("n1,n2,d", [(1024, 2048, 128), (1280, 1408, 96), (1500, 1301, 64), (1500, 1301, 100)])
+@pytest.mark.parametrize("p", [1.0, 3.0, math.inf])
+def test_forward_tiles_of_either_size_agree(tpw, n1, n2, d, p):
+    """The forward's tile size follows the number of tiles; an element does not depend on the other rows, so its bits are those of a
+    call on fewer rows (smaller tiles) and of one on more (larger tiles)."""
+    g = torch.Generator().manual_seed(d)
+    x1, x2 = torch.randn(4 * n1, d, generator=g).cuda(), torch.randn(n2, d, generator=g).cuda()
+    out = tpw.minkowski_distances(x1[:n1].clone(), x2, p)
+    assert torch.equal(out, tpw.minkowski_distances(x1, x2, p)[:n1])
+    assert torch.equal(out[:100, :70], tpw.minkowski_distances(x1[:100].clone(), x2[:70].clone(), p))

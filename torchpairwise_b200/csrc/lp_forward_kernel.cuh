@@ -662,13 +662,18 @@ int launch_forward_tile(FwdParams P, cudaStream_t stream) {
 // float32 tiles are 128 x 128 outputs, two CTAs per SM, where they fill the GPU.  Fewer of them than SMs leave one CTA, or none,
 // to an SM, and a small matrix pays for the padding to 128 rows: 64 x 64 tiles, four CTAs per SM, then (each loads twice the
 // operand bytes per output, which is why large problems keep 128).  The terms of an output and their order are the same.
-// [75, 5, 64] L2: 19.2 -> 7.2 us, [1024, 2048, 128] L1: 30.3 -> 29.3 us.
+// [75, 5, 64] L2: 19.2 -> 7.2 us, [1024, 2048, 128] L1: 30.3 -> 29.3 us.  The p = 3 tile on whole chunks is packed at 128 x 128 only:
+// four scalar tiles of 64 on an SM take longer than the one packed tile, three do not ([1024, 2048, 128] 43.2 against 41.6 us,
+// [1280, 1408, 256] 61.6 against 76.6 us).
 template <typename T, typename OutT, int KIND, bool WEIGHTED, int EPI = EPI_STORE>
 int launch_forward(const FwdParams &P, cudaStream_t stream) {
     constexpr int R = sizeof(T) == 4 ? 8 : 4;
     if constexpr (sizeof(T) == 4 && !WEIGHTED && EPI == EPI_STORE && (KIND <= K_DOT && KIND != K_MIN)) {
         const long long t1 = (P.N1 + 127) / 128, t2 = (P.N2 + 127) / 128;
-        if (P.B > 0 && t1 < sm_count() && t2 < sm_count() && P.B < sm_count() && P.B * t1 * t2 < sm_count())
+        const long long s1 = (P.N1 + 63) / 64, s2 = (P.N2 + 63) / 64;
+        const bool packed = KIND == K_P3 && P.D % FwdSmem<T, R>::KC == 0 && !tma_disabled() && aligned16(P.x1) && aligned16(P.x2);
+        if (P.B > 0 && t1 < sm_count() && t2 < sm_count() && P.B < sm_count() && P.B * t1 * t2 < sm_count() &&
+            !(packed && P.B * s1 * s2 > 3ll * sm_count()))
             return launch_forward_tile<T, OutT, KIND, WEIGHTED, EPI, 4>(P, stream);
     }
     return launch_forward_tile<T, OutT, KIND, WEIGHTED, EPI, R>(P, stream);
