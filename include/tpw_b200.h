@@ -293,9 +293,9 @@ TPW_API int tpw_dot_rowmin_forward_ws(int epilogue, const void *x1, const void *
 /*
  * The k nearest x2 rows of every x1 row (k <= tpw_dot_topk_max_k()), same distances and pipeline as
  * tpw_dot_rowmin_forward_ws: val_out [B,N1,k] ascending, idx_out [B,N1,k] (ties towards the smaller
- * row; -1 / +inf when N2 < k).  Each epilogue thread keeps a sorted register list of the k smallest
- * keys of its accumulator row, candidates at or above an already published bound of the row's k-th
- * smallest are dropped first, the per-tile lists are merged by one warp per row.  Deterministic.
+ * row; -1 / +inf when N2 < k).  A pass over every 4th to 8th x2 row bounds each row's k-th
+ * smallest key; the pass over all of them collects the keys below the bound, at most k from every 128
+ * columns, and one warp per row takes the k smallest.  Deterministic.
  * No [B,N1,N2] matrix is written (the reference sorts every row of it: OPS/neighbors.cpp:10-35;
  * its README lists argkmin as future work).
  */

@@ -267,3 +267,37 @@ def test_forward_tiles_of_either_size_agree(tpw, n1, n2, d, p):
     out = tpw.minkowski_distances(x1[:n1].clone(), x2, p)
     assert torch.equal(out, tpw.minkowski_distances(x1, x2, p)[:n1])
     assert torch.equal(out[:100, :70], tpw.minkowski_distances(x1[:100].clone(), x2[:70].clone(), p))
+
+
+@pytest.mark.parametrize("n2", [129, 255, 257, 1000, 1025, 2049, 5000])
+@pytest.mark.parametrize("order", ["random", "clusters", "falling", "equal rows", "not finite"])
+def test_k_nearest_whatever_the_order_of_the_rows(tpw, n2, order):
+    """The top-k bound comes from a sample of the x2 rows and from tiles that found k keys; whatever the order of x2, the values are those
+    of a selection on the matrix the same engine writes, and the columns are distinct and hold them."""
+    g = torch.Generator().manual_seed(n2)
+    x1, x2 = torch.randn(700, 64, generator=g), torch.randn(n2, 64, generator=g)
+    if order == "clusters":
+        c = 5 * torch.randn(20, 64, generator=g)
+        x1, x2 = 0.3 * x1 + c[torch.arange(700) % 20], 0.3 * x2 + c[torch.arange(n2) * 20 // n2]
+    elif order == "falling":
+        x2 = x2 * torch.linspace(3, 0.5, n2)[:, None]
+    elif order == "equal rows":
+        x2 = x2[:3].repeat(n2 // 3 + 1, 1)[:n2]
+    elif order == "not finite":
+        x1[5, 3], x1[6, 0], x2[n2 // 2, 1], x2[7, 2] = math.inf, math.nan, math.inf, math.nan
+    x1, x2 = x1.cuda(), x2.cuda()
+    was = tpw.get_dot_engine()
+    tpw.set_dot_engine("tcgen05")
+    try:
+        for metric, fn in (("sqeuclidean", tpw.sqeuclidean_distances), ("cosine", tpw.cosine_distances)):
+            full = fn(x1, x2)
+            for k in (1, 2, 3, 8, 16):
+                inds, vals = tpw.pairwise_argkmin(x1, x2, k, metric)
+                # the kernels keep no NaN: a distance is clamped from below by 0, which a NaN becomes
+                assert torch.equal(full.topk(k, dim=-1, largest=False, sorted=True).values, vals), (metric, k)
+                assert torch.equal(full.gather(-1, inds), vals), (metric, k)
+                assert all(len(set(r)) == k for r in inds.tolist())
+                if order == "equal rows":                 # ties go to the smaller rows
+                    assert bool((inds[:, 1:][vals[:, 1:] == vals[:, :-1]] > inds[:, :-1][vals[:, 1:] == vals[:, :-1]]).all())
+    finally:
+        tpw.set_dot_engine(was)

@@ -84,7 +84,7 @@ static encode_tiled_fn resolve_encode_tiled() {
 
 static int encode_map_3d(CUtensorMap *map, const void *base, int elem_bytes,
                          uint64_t dim0, uint64_t dim1, uint64_t dim2,
-                         uint32_t box0, uint32_t box1, bool swizzle128, CUtensorMapSwizzle swizzle);
+                         uint32_t box0, uint32_t box1, bool swizzle128, CUtensorMapSwizzle swizzle, uint64_t pitch1 = 0, uint64_t pitch2 = 0);
 
 int make_tensor_map_3d(CUtensorMap *map, const void *base, int elem_bytes,
                        uint64_t dim0, uint64_t dim1, uint64_t dim2,
@@ -98,9 +98,14 @@ int make_tensor_map_3d_atom32(CUtensorMap *map, const void *base, int elem_bytes
     return encode_map_3d(map, base, elem_bytes, dim0, dim1, dim2, box0, box1, true, CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B);
 }
 
+int make_tensor_map_3d_pitched(CUtensorMap *map, const void *base, int elem_bytes, uint64_t dim0, uint64_t dim1, uint64_t dim2,
+                               uint64_t pitch1, uint64_t pitch2, uint32_t box0, uint32_t box1) {
+    return encode_map_3d(map, base, elem_bytes, dim0, dim1, dim2, box0, box1, true, CU_TENSOR_MAP_SWIZZLE_128B, pitch1, pitch2);
+}
+
 static int encode_map_3d(CUtensorMap *map, const void *base, int elem_bytes,
                          uint64_t dim0, uint64_t dim1, uint64_t dim2,
-                         uint32_t box0, uint32_t box1, bool swizzle128, CUtensorMapSwizzle swizzle) {
+                         uint32_t box0, uint32_t box1, bool swizzle128, CUtensorMapSwizzle swizzle, uint64_t pitch1, uint64_t pitch2) {
     encode_tiled_fn encode = resolve_encode_tiled();
     if (!encode) return fail(TPW_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
     // The encoder is a driver call and needs a context bound to the calling thread.  A thread that
@@ -130,6 +135,8 @@ static int encode_map_3d(CUtensorMap *map, const void *base, int elem_bytes,
         return fail(TPW_ERR_INVALID, "tensor map: a 128-byte swizzled box must span 128 bytes");
     cuuint64_t dims[3] = {dim0, dim1 ? dim1 : 1, dim2 ? dim2 : 1};
     cuuint64_t strides[2] = {dim0 * (uint64_t)elem_bytes, dim0 * dims[1] * (uint64_t)elem_bytes};
+    if (pitch1) { strides[0] = pitch1; strides[1] = pitch2; }
+    if (strides[0] % 16 != 0 || strides[1] % 16 != 0) return fail(TPW_ERR_INVALID, "tensor map: pitches are no multiples of 16 bytes");
     cuuint32_t box[3] = {box0, box1, 1};
     cuuint32_t estr[3] = {1, 1, 1};
     CUresult r = encode(map, dt, 3, const_cast<void *>(base), dims, strides, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE,

@@ -57,6 +57,9 @@ int sm_count();
 int make_tensor_map_3d(CUtensorMap *map, const void *base, int elem_bytes,
                        uint64_t dim0, uint64_t dim1, uint64_t dim2,
                        uint32_t box0, uint32_t box1, bool swizzle128);
+// Same, swizzled, over rows and matrices that lie `pitch1` and `pitch2` bytes apart (every s-th row of a matrix).
+int make_tensor_map_3d_pitched(CUtensorMap *map, const void *base, int elem_bytes, uint64_t dim0, uint64_t dim1, uint64_t dim2,
+                               uint64_t pitch1, uint64_t pitch2, uint32_t box0, uint32_t box1);
 // Same with CU_TENSOR_MAP_SWIZZLE_128B_ATOM_32B: 128-byte rows whose 32-byte groups are permuted by
 // the row index modulo 4, the shared-memory layout tcgen05 expects for MN-major 32-bit operands.
 int make_tensor_map_3d_atom32(CUtensorMap *map, const void *base, int elem_bytes,

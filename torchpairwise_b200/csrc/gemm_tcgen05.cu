@@ -69,12 +69,17 @@ struct GemmParams {
     int vec_store;            // N2 % 4 == 0 and out 16-byte aligned
     int kchunk;               // k-steps accumulated in tensor memory before the sum moves to registers (0: all)
     unsigned long long *rowmin_keys; // ROWMIN instantiation: [B*N1] keys (float bits << 32 | x2 row), nothing is stored to out
-    // TOPK > 0: [B*N1] upper bounds of the row's k-th smallest key, [B*N1] numbers of keys written so far, and per row
-    // room for k keys from every (column tile, half), [B*N1][topk_L * topk_k], filled from the front
+    // TOPK > 0: [B*N1] upper bounds of the row's k-th smallest key (lowered by every tile half that finds k keys), [B*N1]
+    // numbers of keys written so far, and per row room for k keys from every (column tile, half), [B*N1][topk_L * topk_k],
+    // filled from the front
     unsigned long long *topk_lists, *topk_thr;
     int *topk_count;
     int topk_k, topk_L;
-    float *gmin;              // TOPK < 0: [B*N1][8 * tiles_n] minima of the groups of 32 columns
+    // TOPK < 0: the columns of this launch are every col_step-th x2 row, cols of them; [B*N1][32 or 8 per column tile] minima of
+    // groups of col_group columns (8: equal modulo 16 in a tile half, 32: modulo 4)
+    float *gmin;
+    int col_step, col_group;
+    long long cols;
     const int *lo_any;        // [2] whether any low part of the x (y) operand is non-zero; NULL: treat both as non-zero
     int lo_always;            // bit 0 / 1: the x / y operand's low parts are used whatever lo_any says
     float *partial;           // tf32: [grid][2][BM][BN] sums of the tiles that a CTA has only a part of (NULL: whole tiles only)
@@ -153,7 +158,7 @@ __device__ __forceinline__ float clamp_distance(float raw) {
 // Tile index -> (column tile, row tile, batch).  Column tiles vary fastest, so that consecutive tiles
 // share the x1 rows and stream the (usually L2-resident) x2 rows -- except for the top-k epilogue, where
 // row tiles vary fastest: a row's column tiles are then visited one after another over the run, and the
-// bound published by its earlier column tiles prunes the later ones.
+// bound that its earlier column tiles have lowered prunes the later ones.
 template <bool ROW_TILES_FASTEST>
 __device__ __forceinline__ void decode_tile(long long tile, const GemmParams &P, long long &tn, long long &tm, long long &b) {
     if (ROW_TILES_FASTEST) {
@@ -189,6 +194,26 @@ __device__ __forceinline__ void store_block_ragged(const unsigned char *stg, flo
 #pragma unroll 8
     for (int rr = 0; rr < n; ++rr)
         dst[rr * pitch + lane] = *reinterpret_cast<const float *>(stg + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) + (lane & 3) * 4);
+}
+
+// The largest of a lane's k keys (32 words apart) and its slot.  Not inlined: the top-k epilogue has four copies of its caller, and
+// few tile halves come here.
+struct KeySlot {
+    unsigned long long key;
+    int slot;
+};
+__device__ __noinline__ KeySlot largest_key(const unsigned long long *buf, int k) {
+    KeySlot m{0, 0};
+#pragma unroll 1
+    for (int t = 0; t < k; t += 8) {   // eight loads under way together
+        unsigned long long held[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) held[u] = t + u < k ? buf[(t + u) * 32] : 0;
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            if (t + u < k && held[u] >= m.key) m = {held[u], t + u};
+    }
+    return m;
 }
 
 // The share of a product that falls to one CTA: whole tiles, every gridDim.x-th.  With a scratch for partial tiles (tf32) only
@@ -504,15 +529,17 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
             // TOPK > 0: keys at or above the bound of the row's k-th smallest key cannot be among its k smallest
             unsigned long long bound = 0;
             if constexpr (TOPK > 0) {
-                if (row_ok) bound = __ldg(P.topk_thr + b * P.N1 + i);   // rows past N1: nothing passes
+                // rows past N1: nothing passes; any value read while other tiles lower it is a bound
+                if (row_ok) bound = *reinterpret_cast<volatile unsigned long long *>(P.topk_thr + b * P.N1 + i);
             }
             if constexpr (TOPK != 0) {
-                // Columns past N2 count as NaN, which no minimum takes and no comparison passes.  TOPK < 0 keeps the minimum of
-                // every 32 columns.  TOPK > 0: the minimum of eight distances decides for all of them whether any lane of the
+                // Columns past the last count as NaN, which no minimum takes and no comparison passes.  TOPK < 0 keeps the minimum
+                // of every group of columns.  TOPK > 0: the minimum of eight distances decides for all of them whether any lane of the
                 // warp has one within its limit; then every lane puts its next passing column into its own words of the
                 // staging area, until none has one left (most tile halves have none or one a lane), and once a lane
                 // holds k keys the largest gives way to a smaller one.
                 const int k = P.topk_k;
+                const long long cols = TOPK < 0 ? P.cols : P.N2;
                 unsigned long long *buf = reinterpret_cast<unsigned long long *>(smem + OFF_STAGE + (warp - 2) * 4096) + lane;   // [k][32 lanes]
                 int cnt = 0, worst = 0;                       // keys held, slot of the largest once there are k
                 unsigned long long limit = bound;             // keys have to stay below it
@@ -522,15 +549,17 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                     return hi >= 0x7f800000u || (EPI == TPW_DOT_COSINE_DIST && hi >= 0x40000000u) ? INFINITY : __uint_as_float(hi);
                 };
                 float lim = limit_value();
+                float gm[16];                                 // TOPK < 0: minima of the half's columns of every residue modulo 16
+#pragma unroll
+                for (int t = 0; t < 16; ++t) gm[t] = INFINITY;
 #pragma unroll 1
                 for (int c = chalf * (BN / 64); c < (chalf + 1) * (BN / 64); ++c) {
                     const long long j0 = tn * BN + c * 32;
-                    float gm = INFINITY;
-                    if (j0 < P.N2) {
+                    if (j0 < cols) {
                         uint32_t r[32];
                         tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + a * BN + c * 32, r);
                         tmem_ld_wait();
-                        const bool whole = P.vec_store && j0 + 32 <= P.N2;
+                        const bool whole = TOPK > 0 && P.vec_store && j0 + 32 <= cols;
 #pragma unroll
                         for (int g = 0; g < 4; ++g) {
                             float nn[8], o[8];
@@ -542,16 +571,18 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                                 }
                             } else {
 #pragma unroll
-                                for (int v = 0; v < 8; ++v) nn[v] = j0 + 8 * g + v < P.N2 ? __ldg(n2p + j0 + 8 * g + v) : 0.f;
+                                for (int v = 0; v < 8; ++v)
+                                    nn[v] = j0 + 8 * g + v < cols ? __ldg(n2p + (j0 + 8 * g + v) * (TOPK < 0 ? P.col_step : 1)) : 0.f;
                             }
 #pragma unroll
                             for (int v = 0; v < 8; ++v) {
                                 o[v] = raw_distance<EPI>(__uint_as_float(r[8 * g + v]), n1, nn[v]);
-                                if (!whole && j0 + 8 * g + v >= P.N2) o[v] = NAN;
+                                if (!whole && j0 + 8 * g + v >= cols) o[v] = NAN;
                             }
                             const float m = min3(min3(o[0], o[1], o[2]), min3(o[3], o[4], o[5]), fminf(o[6], o[7]));
                             if constexpr (TOPK < 0) {
-                                gm = fminf(gm, m);
+#pragma unroll
+                                for (int v = 0; v < 8; ++v) gm[(g & 1) * 8 + v] = fminf(gm[(g & 1) * 8 + v], o[v]);
                             } else if (__any_sync(0xffffffffu, m <= lim)) {
                                 uint32_t mask = 0;
 #pragma unroll
@@ -571,25 +602,34 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                                     if (take) buf[(cnt < k ? cnt : worst) * 32] = key;
                                     if (take && ++cnt >= k) {
                                         cnt = k;
-                                        limit = 0;
-#pragma unroll 1
-                                        for (int t = 0; t < k; ++t) {
-                                            const unsigned long long held = buf[t * 32];
-                                            if (held >= limit) { limit = held; worst = t; }
-                                        }
+                                        const KeySlot last = largest_key(buf, k);
+                                        limit = last.key;
+                                        worst = last.slot;
                                         lim = limit_value();
                                     }
                                 }
                             }
                         }
                     }
-                    if constexpr (TOPK < 0) {
-                        if (row_ok) P.gmin[((b * P.N1 + i) * P.tiles_n + tn) * 8 + c] = clamp_distance<EPI>(gm);
+                }
+                if constexpr (TOPK < 0) {
+#pragma unroll
+                    for (int t = 0; t < 16; ++t) gm[t] = clamp_distance<EPI>(gm[t]);
+                    const long long at = ((b * P.N1 + i) * P.tiles_n + tn) * 2 + chalf;
+                    float4 *dst = reinterpret_cast<float4 *>(P.gmin) + (P.col_group == 8 ? at * 4 : at);
+                    if (!row_ok) {
+                    } else if (P.col_group == 8) {
+#pragma unroll
+                        for (int t = 0; t < 4; ++t) dst[t] = make_float4(gm[4 * t], gm[4 * t + 1], gm[4 * t + 2], gm[4 * t + 3]);
+                    } else {
+                        auto least = [&](int t) { return fminf(min3(gm[t], gm[t + 4], gm[t + 8]), gm[t + 12]); };
+                        dst[0] = make_float4(least(0), least(1), least(2), least(3));
                     }
                 }
                 if constexpr (TOPK > 0) {
                     // behind the keys that other tile halves have written (their order does not matter: the keys are unique
                     // and the merge looks at all of them)
+                    if (cnt == k) atomicMin(P.topk_thr + b * P.N1 + i, limit);   // k keys up to it, which are written here
                     if (cnt > 0) {
                         const int at = atomicAdd(P.topk_count + b * P.N1 + i, cnt);
                         unsigned long long *dst = P.topk_lists + (b * P.N1 + i) * P.topk_L * k + at;
@@ -1199,19 +1239,28 @@ __global__ void topk_merge_kernel(const unsigned long long *__restrict__ lists, 
     if (idx_out) idx_out[row * k + lane] = none ? -1ll : (long long)(uint32_t)out;
 }
 
-// One warp per row: an upper bound of the row's k-th smallest key from the minima of n groups of columns.  Each minimum is
-// the distance of a column of its own, so k columns are no farther than the k-th smallest minimum; the bound is the
-// first key above all keys of that distance (~0: fewer than k groups hold a finite distance).
-template <int TOPK>
-__global__ void topk_bound_kernel(const float *__restrict__ gmin, unsigned long long *__restrict__ bound, long long rows, long long n, int k) {
+// One warp per row: an upper bound of the row's k-th smallest key from the minima of n groups of columns.  Each lane takes the
+// smallest of its groups' minima, 32 distances of different columns, so k columns are no farther than the k-th smallest of them;
+// the bound is the first key above all keys of that distance (~0: fewer than k lanes hold a finite distance).  Neighbouring
+// columns belong to different groups and lanes, so that a row whose neighbours lie side by side in x2 is bounded like any other.
+__global__ void topk_bound_kernel(const float *__restrict__ gmin, unsigned long long *__restrict__ bound, int *__restrict__ counts, long long rows,
+                                  int n, int k) {
     const int lane = threadIdx.x & 31;
     const long long row = ((long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     if (row >= rows) return;
     const float *src = gmin + row * n;
-    warp_smallest<TOPK>(n, k, [&](long long e) { return ((unsigned long long)__float_as_uint(src[e]) << 32) | (unsigned long long)(uint32_t)e; },
-                        [&](int r, unsigned long long m) {
-                            if (lane == 0 && r == k - 1) bound[row] = (uint32_t)(m >> 32) < 0x7f800000u ? ((m >> 32) + 1) << 32 : ~0ull;
-                        });
+    float least = INFINITY;
+#pragma unroll 4
+    for (int e = lane; e < n; e += 32) least = fminf(least, src[e]);
+    uint32_t mine = __float_as_uint(least), kth = 0;     // not negative: bits order like values
+    for (int r = 0; r < k; ++r) {
+        kth = __reduce_min_sync(0xffffffffu, mine);
+        if (lane == __ffs(__ballot_sync(0xffffffffu, mine == kth)) - 1) mine = 0xffffffffu;
+    }
+    if (lane == 0) {
+        bound[row] = kth < 0x7f800000u ? (unsigned long long)(kth + 1) << 32 : ~0ull;
+        counts[row] = 0;
+    }
 }
 
 constexpr int kTopkMax = 16;      // a tile half's keys fit the warp's 4 KB of staging
@@ -1294,6 +1343,7 @@ extern "C" int tpw_dot_topk_forward_ws(int epilogue, int k, const void *x1, cons
                   "tpw_dot_topk_forward_ws: a dimension exceeds 2^31-1");
     const bool cosine = epilogue == TPW_DOT_COSINE_DIST;
     const TopkScratch T = topk_scratch_layout(B, N1, N2, D, k);
+    const ScratchLayout L = scratch_layout(B, N1, N2, D, false);
     TPW_CHECK_ARG(scratch != nullptr && scratch_bytes >= T.total && aligned16(scratch),
                   "tpw_dot_topk_forward_ws: needs %lld bytes of 16-byte aligned scratch (got %lld)", T.total, (long long)scratch_bytes);
     cudaStream_t s = static_cast<cudaStream_t>(stream);
@@ -1301,7 +1351,6 @@ extern "C" int tpw_dot_topk_forward_ws(int epilogue, int k, const void *x1, cons
     unsigned long long *lists = reinterpret_cast<unsigned long long *>(base + T.off_lists);
     unsigned long long *thr = reinterpret_cast<unsigned long long *>(base + T.off_thr);
     int *counts = reinterpret_cast<int *>(base + T.off_count);
-    TPW_CUDA_OK(cudaMemsetAsync(counts, 0, (size_t)(B * N1) * 4, s));
     Bf16Operands M;
     GemmParams P;
     int st;
@@ -1322,24 +1371,39 @@ extern "C" int tpw_dot_topk_forward_ws(int epilogue, int k, const void *x1, cons
         kern<<<grid, kThreads, SMEM_ALLOC, s>>>(M.mxh, M.mxl, M.myh, M.myl, P);                                           \
         TPW_LAUNCH_OK("gemm_metric_kernel (top-k)");                                                                      \
     } while (0)
-    // An insertion costs the whole warp as soon as one lane has one, so first a bound: the contraction over a sixth of the
-    // column tiles keeps only the minimum of every 32 columns, and the k-th smallest of a row's minima bounds its k-th
-    // smallest distance almost as closely as the distances themselves would.  With that bound the pass over all columns
-    // inserts about 6 k keys a row, and the sixth that is computed twice costs less than the insertions it saves.
-    // (Lists over a sixteenth, a quarter and the rest, each bounding the next, as it was: k = 10 of [50000, 20000, 128]
-    // 4.00 -> 1.45 ms.)  Fewer than 8 column tiles are not worth a second pass.
-    const long long sample = tiles_n_all / 6;
-    if (tiles_n_all >= 8 && (sample > 1 ? sample : 2) * 8 >= k) {
-        P.tiles_n = sample > 1 ? sample : 2;
+    // An insertion costs the whole warp as soon as one lane has one, so first a bound: the contraction over a sample of the x2 rows
+    // keeps only the minima of groups of 8, and the k-th smallest of 32 of those bounds a row's k-th smallest distance almost as
+    // closely as the distances themselves would; the pass over all columns then inserts about 5 k keys a row.  The sample is every
+    // step-th row, through a tensor map of that pitch, so that the order of x2 does not matter: of 20 clusters one after another,
+    // the first sixth of the columns bounded 17 of them not at all.  A quarter of the rows (an eighth for k up to 3, which inserts
+    // little) was the fastest or within 3 % over 90 shapes and orders; at least one column tile.  Fewer than 8 column
+    // tiles and k = 1 or 2 need no bound.  Microseconds with lists that bound each other / the first sixth, sampled from 8 tiles on / now:
+    //   [50000, 20000, 128] k = 10 3989 / 1440 / 1469;  [50000, 1536, 128] k = 8 387 / 642 / 253, k = 16 806 / 1262 / 376;
+    //   [20000, 20000, 64] in 20 clusters, k = 16 2338 / 4414 / 802;  [50000, 300, 128] k = 2 122 / 108 / 112
+    const long long per = (k <= 3 ? 8 : 4) * BN;
+    const long long sample_tiles = N2 > per ? N2 / per : 1, even = (N2 + sample_tiles * BN - 1) / (sample_tiles * BN), step = even > 1 ? even : 2;
+    const long long cols = (N2 + step - 1) / step, sample = (cols + BN - 1) / BN;
+    // the minima lie where the keys will, in groups as small as fit there (one column tile and k = 1: none do)
+    const long long room = T.L * k * 8 / 4;
+    const int group = BN / 8 * sample <= room ? 8 : BN / 32 * sample <= room ? 32 : 0;
+    const long long groups = group ? (cols + group - 1) / group : 0;
+    if ((tiles_n_all >= 8 || k > 2) && (groups < 32 ? groups : 32) >= k) {
+        const CUtensorMap all_h = M.myh, all_l = M.myl;
+        const unsigned char *yh = base + L.off_yh, *yl = base + L.off_yl;
+        if ((st = make_tensor_map_3d_pitched(&M.myh, yh, 2, L.Dp, cols, B, step * L.Dp * 2, N2 * L.Dp * 2, BK, BN)) != TPW_OK) return st;
+        if ((st = make_tensor_map_3d_pitched(&M.myl, yl, 2, L.Dp, cols, B, step * L.Dp * 2, N2 * L.Dp * 2, BK, BN)) != TPW_OK) return st;
+        P.tiles_n = sample;
         P.tiles = B * P.tiles_m * P.tiles_n;
-        P.gmin = reinterpret_cast<float *>(lists);   // 32 bytes per row and tile, where the pass below keeps 16 k
+        P.cols = cols; P.col_step = (int)step; P.col_group = group;
+        P.gmin = reinterpret_cast<float *>(lists);
         const unsigned grid = (unsigned)(P.tiles < nsm ? P.tiles : nsm);
         if (cosine) TPW_TOPK_LAUNCH(TPW_DOT_COSINE_DIST, -1); else TPW_TOPK_LAUNCH(TPW_DOT_SQEUCLIDEAN, -1);
-        if (k <= 8) topk_bound_kernel<8><<<mblocks, 256, 0, s>>>(P.gmin, thr, rows, 8 * P.tiles_n, k);
-        else topk_bound_kernel<16><<<mblocks, 256, 0, s>>>(P.gmin, thr, rows, 8 * P.tiles_n, k);
+        topk_bound_kernel<<<mblocks, 256, 0, s>>>(P.gmin, thr, counts, rows, (int)(BN / group * sample), k);
         TPW_LAUNCH_OK("topk_bound_kernel");
+        M.myh = all_h; M.myl = all_l;
     } else {
         TPW_CUDA_OK(cudaMemsetAsync(thr, 0xFF, (size_t)rows * 8, s));
+        TPW_CUDA_OK(cudaMemsetAsync(counts, 0, (size_t)rows * 4, s));
     }
     P.tiles_n = tiles_n_all;
     P.tiles = B * P.tiles_m * P.tiles_n;

@@ -1498,8 +1498,8 @@ def pairwise_argkmin(x1: Tensor, x2: Optional[Tensor] = None, k: int = 1, metric
     ``k_neighbors_mask`` sorts every row of the materialised matrix (OPS/neighbors.cpp:10-35).
 
     Large float32 problems with a Euclidean, squared Euclidean or cosine metric and
-    ``k <= tpw_dot_topk_max_k()`` run the tensor-core kernel whose epilogue keeps the k smallest keys
-    of each accumulator row in registers (``tpw_dot_topk_forward_ws``; no distance matrix is written).
+    ``k <= tpw_dot_topk_max_k()`` run the tensor-core kernel whose epilogue collects the keys below a bound of
+    each row's k-th smallest (``tpw_dot_topk_forward_ws``; no distance matrix is written).
     float32 L_p metrics (p in 1, 2, 3, inf) on at most ``tpw_lp_topk_max_features()`` features and at least 4096
     query rows run the streaming kernel that keeps one query row and its k best keys per thread
     (``tpw_lp_topk_forward``).  Everything else takes this package's distance kernel followed by a partial selection."""
