@@ -95,8 +95,8 @@ def test_hausdorff_expanded_form_and_hand_over(tpw, monkeypatch, case):
     values and indices of the exact loop either way, with and without a shuffled visiting order."""
     d = 2 if case == "few coordinates" else 3
     g = torch.Generator().manual_seed(len(case))
-    x1 = torch.rand(2, 1, 6007, d, generator=g) * 2 - 1
-    x2 = x1[:, :, torch.randperm(6007, generator=g)] + 0.05 * torch.randn(2, 1, 6007, d, generator=g)
+    x1 = torch.rand(2, 1, 8207, d, generator=g) * 2 - 1
+    x2 = x1[:, :, torch.randperm(8207, generator=g)] + 0.05 * torch.randn(2, 1, 8207, d, generator=g)
     if case == "equal":
         x2 = x1.clone()
     elif case == "offset":
@@ -301,3 +301,36 @@ def test_k_nearest_whatever_the_order_of_the_rows(tpw, n2, order):
                     assert bool((inds[:, 1:][vals[:, 1:] == vals[:, :-1]] > inds[:, :-1][vals[:, 1:] == vals[:, :-1]]).all())
     finally:
         tpw.set_dot_engine(was)
+
+
+@pytest.mark.parametrize("d", [2, 3, 7, 12])
+@pytest.mark.parametrize("case", ["sigma 0.01", "sigma 0.003", "sigma 0.001", "sigma 0.0003", "shells", "half equal", "one far point", "repeated points"])
+def test_hausdorff_rows_handed_over(tpw, monkeypatch, case, d):
+    """Set pairs whose largest row minima lie within the expanded form's error of one another hand those rows, from a few to all of them,
+    over to the direct form; values and indices are the exact loop's, with and without a shuffled visiting order."""
+    g, m = torch.Generator().manual_seed(d), 6701
+    x1 = torch.rand(3, 1, m, d, generator=g) * 2 - 1
+    noise = torch.randn(3, 1, m, d, generator=g)
+    if case.startswith("sigma"):
+        x2 = x1 + float(case.split()[1]) * noise
+    elif case == "shells":                       # voxel shells of equal radius one voxel apart
+        x1 = (40 * torch.nn.functional.normalize(x1, dim=-1)).round()
+        x2 = (41 * torch.nn.functional.normalize(x1 + 0.02 * noise, dim=-1)).round()
+    elif case == "half equal":
+        x2 = torch.where(torch.arange(m)[None, None, :, None] % 2 == 0, x1, x1 + 1e-3 * noise)
+    elif case == "one far point":
+        x2 = x1 + 0.05 * noise
+        x1[:, :, 4001] = 30.0
+    else:
+        x1 = x1[:, :, :50].repeat(1, 1, m // 50 + 1, 1)[:, :, :m].contiguous()
+        x2 = x1.roll(7, 2) + 2e-3 * noise.roll(1, 2)
+    for shuffle in (False, True):
+        res = []
+        for exact in (False, True):
+            if exact:
+                monkeypatch.setenv("TPW_HAUSDORFF_EXACT_LOOP", "1")
+            gen = torch.Generator(device="cuda").manual_seed(5) if shuffle else None
+            res.append(tpw.directed_hausdorff_distances(x1.cuda(), x2.cuda(), shuffle=shuffle, generator=gen))
+            monkeypatch.delenv("TPW_HAUSDORFF_EXACT_LOOP", raising=False)
+        for a, w in zip(*res):
+            assert torch.equal(a, w), (case, shuffle)

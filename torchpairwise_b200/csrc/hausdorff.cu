@@ -18,8 +18,10 @@
 // to three per set pair) and applies the tie rules to them, so values and indices are still bit-identical to
 // the exact path.  Two approximations:
 //   expanded   |y|^2 - 2 x.y + |x|^2 about a point of the x2 cloud: D fused multiply-adds per point pair.  Its error is
-//              bounded by the clouds' extent, not by the distance, so where many rows lie that close together (equal
-//              clouds, a far outlier, coordinates that are not finite) a set pair is handed over to the other one;
+//              bounded by the clouds' extent, not by the distance, so where more rows than the refining kernel should
+//              look at lie that close together (well registered clouds, voxel shells), those rows are handed over to the
+//              other one, and where a sample of rows says that most do (equal clouds, a far outlier, coordinates that are
+//              not finite) the set pair skips this one;
 //   direct     sum of squared differences with fused multiply-adds, 2 D per point pair, within a few units in the last
 //              place of the separately rounded value.
 //
@@ -66,7 +68,9 @@ struct HdParams {
     long long B, N1, N2, M1, M2, D;
     long long mtiles;
     int splits;       // CTAs that share the x2 points of one row block (fused path)
-    int handed_over;  // direct form: only the set pairs that the expanded form has handed over
+    int handed_over;  // direct form: only the set pairs, and of those the rows, that the expanded form has handed over
+    unsigned int *list;   // [pairs, M1] those rows; before, per sampling CTA of the pair, what it found (kSampleWords)
+    int samples;      // sampling CTAs per set pair (0: none)
 };
 
 // An upper bound on the relative difference between the fused and the separately rounded sum of up to 8 squares
@@ -174,13 +178,109 @@ template <int D> struct Fused {
     static constexpr int ROWS = kFThreads * PM;
 };
 
-// What the two kernels agree on per set pair, in the eight bytes the exact path uses for its key: the largest squared
-// norm about the centre (infinite: not bounded) and whether the pair has been handed over to the direct form.
+// What the kernels agree on per set pair, in the eight bytes the exact path uses for its key: the largest squared norm
+// about the centre (infinite: not bounded) and how many of its rows are handed over to the direct form (kAllRows: no list).
 struct PairState {
     unsigned int extent, direct;
 };
+constexpr unsigned int kAllRows = 0xffffffffu;
 constexpr float kExtentMax = 1e36f;   // beyond it the products could overflow
-constexpr int kMaxCandidates = 32;    // more rows within the error of the largest: hand the pair over
+constexpr unsigned int kMaxCandidates = 32;    // rows that one CTA evaluates one after another, 4 us each at 8192 points
+constexpr unsigned int kMaxExpanded = 8;       // more rows within the expanded form's error of the largest are handed over
+
+// EXPAND: with R^2 the largest squared norm about the centre, the centred coordinates' roundings change a squared distance by at
+// most 8 u R^2 (u = 2^-24), the two norms' by 2 D u R^2, the D multiply-adds' by 3 D u R^2 and the last addition's by 4 u R^2:
+// E = (5 D + 12) u R^2.  A row of the largest distance lies within 2 E of the largest minimum; 16 D + 64 leaves room.
+template <int D> __device__ __forceinline__ float expanded_slack(float extent) { return 2.f * (float)(8 * (D + 1) + 24) * 5.9604645e-8f * extent; }
+
+// Whether the expanded form is worth trying on a set pair: the direct minima of 16 rows over all x2 points.  Where most of them lie
+// within 0.4 of the expanded form's error of the largest, most of all rows will lie within the error of the largest of all
+// (which is about 2.5 times as far from the low ones as the largest of 16 is, for noise), and the expanded pass would be thrown
+// away.  The answer decides the time alone, not the result.  `samples` CTAs share the x2 points of a set pair, each half of a CTA
+// with eight rows in registers; every CTA of the expanded pass combines what they found.
+// Microseconds at 64 pairs of 8192 points in the unit cube, x2 = x1 plus noise, before any expanded form / with it and whole pairs
+// handed over / with the sample and the listed rows: sigma 0.05 1222 / 569 / 602, 0.003 1222 / 1056 / 666, 0.002 1222 / 1537 / 972,
+// equal clouds 1214 / 1476 / 938, two voxel shells 1289 / 622 / 909.
+constexpr int kSampleRows = 16, kSampleWords = kSampleRows + 1;   // minima, and the largest squared norm about the centre
+template <int D>
+__global__ void __launch_bounds__(kThreads)
+hausdorff_sample_kernel(const HdParams P) {
+    constexpr int kRows = kSampleRows / 2, kHalf = kThreads / 2;
+    __shared__ unsigned int s_found[kSampleWords];
+    const int tid = threadIdx.x, half = tid / kHalf;
+    const int part = (int)(blockIdx.x % P.samples);
+    const long long pair = blockIdx.x / P.samples;
+    const long long j = pair % P.N2;
+    const long long bi = pair / P.N2;
+    const long long b = bi / P.N1;
+    const float *x1 = reinterpret_cast<const float *>(P.x1) + bi * P.M1 * D;
+    const float *x2 = reinterpret_cast<const float *>(P.x2) + (b * P.N2 + j) * P.M2 * D;
+    if (tid < kSampleWords) s_found[tid] = tid < kSampleRows ? 0x7f800000u : 0u;
+    __syncthreads();
+    float x[kRows][D], least[kRows], centre[D], extent = 0.f;
+    bool unbounded = false;
+    auto grow = [&](const float *v) {
+        float n = 0.f;
+#pragma unroll
+        for (int k = 0; k < D; ++k) n = fmaf(v[k] - centre[k], v[k] - centre[k], n);
+        extent = fmaxf(extent, n);
+        unbounded |= !(n < kExtentMax);
+    };
+#pragma unroll
+    for (int k = 0; k < D; ++k) centre[k] = x2[k];
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+        const long long m = ((half * kRows + r) * 2 + 1) * P.M1 / (2 * kSampleRows);     // the middles of 16 equal ranges
+        least[r] = INFINITY;
+#pragma unroll
+        for (int k = 0; k < D; ++k) x[r][k] = x1[m * D + k];
+        grow(x[r]);
+    }
+    const long long per = (P.M2 + P.samples - 1) / P.samples, end = (part + 1) * per < P.M2 ? (part + 1) * per : P.M2;
+#pragma unroll 4
+    for (long long n = part * per + tid % kHalf; n < end; n += kHalf) {
+        float y[D];
+#pragma unroll
+        for (int k = 0; k < D; ++k) y[k] = x2[n * D + k];
+        grow(y);
+#pragma unroll
+        for (int r = 0; r < kRows; ++r) {
+            float d = 0.f;
+#pragma unroll
+            for (int k = 0; k < D; ++k) d = fmaf(x[r][k] - y[k], x[r][k] - y[k], d);
+            least[r] = fminf(least[r], d);
+        }
+    }
+    // not negative: bits order like values
+    const unsigned int bits = __reduce_max_sync(0xffffffffu, unbounded ? 0x7f800000u : __float_as_uint(extent));
+    if ((tid & 31) == 0) atomicMax(&s_found[kSampleRows], bits);
+#pragma unroll
+    for (int r = 0; r < kRows; ++r) {
+        const unsigned int m = __reduce_min_sync(0xffffffffu, __float_as_uint(least[r]));
+        if ((tid & 31) == 0) atomicMin(&s_found[half * kRows + r], m);
+    }
+    __syncthreads();
+    if (tid < kSampleWords) P.list[pair * P.M1 + part * kSampleWords + tid] = s_found[tid];
+    if (part == 0 && tid == 0) reinterpret_cast<PairState *>(P.keys)[pair] = PairState{0, 0};
+}
+
+// One warp: whether the sample says that the set pair should go to the direct form at once (the same in all lanes).
+template <int D>
+__device__ __forceinline__ bool sample_says_direct(const HdParams &P, long long pair) {
+    const int lane = threadIdx.x & 31;
+    const unsigned int *found = P.list + pair * P.M1;
+    unsigned int v = lane < kSampleRows ? 0x7f800000u : 0u;
+    for (int s = 0; s < P.samples && lane < kSampleWords; ++s) {
+        const unsigned int w = found[s * kSampleWords + lane];
+        v = lane < kSampleRows ? min(v, w) : max(v, w);
+    }
+    __syncwarp();
+    const float extent = __uint_as_float(__shfl_sync(0xffffffffu, v, kSampleRows));
+    const float most = __uint_as_float(__reduce_max_sync(0xffffffffu, lane < kSampleRows ? v : 0u));
+    const float lower = most * (1.f - fused_slack<D>()) - kTiny - 0.4f * expanded_slack<D>(extent);
+    const int close = __popc(__ballot_sync(0xffffffffu, lane < kSampleRows && __uint_as_float(v) >= lower));
+    return !(extent < kExtentMax) || close >= 10;
+}
 
 template <int D, bool EXPAND>
 __global__ void __launch_bounds__(kFThreads)
@@ -191,13 +291,39 @@ hausdorff_rowmin_fused_kernel(const HdParams P) {
     constexpr int CHUNK = FCHUNK_BYTES / (DP * 8);   // pairs of x2 points staged per pass
     __shared__ ulonglong2 pts[FCHUNK_BYTES / 16];
     const int tid = threadIdx.x;
-    long long blk = blockIdx.x;
-    const int sp = (int)(blk % P.splits);
-    blk /= P.splits;
-    const long long mt = blk % P.mtiles;
-    const long long pair = blk / P.mtiles; // (b*N1 + i)*N2 + j
+    const long long each = P.mtiles * P.splits, pair = blockIdx.x / each; // (b*N1 + i)*N2 + j
+    const int part = (int)(blockIdx.x % each);
     PairState *state = reinterpret_cast<PairState *>(P.keys) + pair;
-    if (!EXPAND && P.handed_over && state->direct == 0) return;
+    long long mt = part / P.splits, rows = P.M1;
+    int sp = part % P.splits, splits = P.splits;
+    const unsigned int *list = nullptr;
+    if (EXPAND) {
+        __shared__ bool s_direct;
+        if (P.samples > 0) {
+            if (tid < 32) {
+                const bool direct = sample_says_direct<D>(P, pair);
+                if (tid == 0) {
+                    s_direct = direct;
+                    if (direct && part == 0) state->direct = kAllRows;
+                }
+            }
+            __syncthreads();
+            if (s_direct) return;
+        }
+    } else if (P.handed_over) {
+        const unsigned int n = state->direct;
+        if (n == 0) return;
+        if (n != kAllRows) {
+            // the pair's CTAs share the x2 points of the listed rows
+            list = P.list + pair * P.M1;
+            rows = n;
+            const long long tiles = (rows + F::ROWS - 1) / F::ROWS;
+            splits = (int)(each / tiles);
+            mt = part / splits;
+            sp = part % splits;
+            if (mt >= tiles) return;
+        }
+    }
     const long long j = pair % P.N2;
     const long long bi = pair / P.N2;
     const long long b = bi / P.N1;
@@ -209,19 +335,19 @@ hausdorff_rowmin_fused_kernel(const HdParams P) {
     float extent = 0.f;          // largest squared norm this thread has seen
     bool unbounded = false;
     // this CTA's range of x2 points, cut at even positions
-    const long long per = ((P.M2 + 1) / 2 + P.splits - 1) / P.splits * 2;
+    const long long per = ((P.M2 + 1) / 2 + splits - 1) / splits * 2;
     const long long n_end = (sp + 1) * per < P.M2 ? (sp + 1) * per : P.M2;
 
     f32x2 px[F::PM][D];
     float rowmin[F::PM], xsq[F::PM];
 #pragma unroll
     for (int q = 0; q < F::PM; ++q) {
-        const long long m = mt * F::ROWS + q * kFThreads + tid;
+        const long long c = mt * F::ROWS + q * kFThreads + tid, m = !EXPAND && list && c < rows ? list[c] : c;
         rowmin[q] = INFINITY;
         xsq[q] = 0.f;
 #pragma unroll
         for (int k = 0; k < D; ++k) {
-            const float v = m < P.M1 ? x1[m * D + k] - centre[k] : 0.f;
+            const float v = c < rows ? x1[m * D + k] - centre[k] : 0.f;
             px[q][k] = pack2(v, v);
             xsq[q] = fmaf(v, v, xsq[q]);
         }
@@ -290,11 +416,11 @@ hausdorff_rowmin_fused_kernel(const HdParams P) {
     }
 #pragma unroll
     for (int q = 0; q < F::PM; ++q) {
-        const long long m = mt * F::ROWS + q * kFThreads + tid;
-        if (m >= P.M1) continue;
+        const long long c = mt * F::ROWS + q * kFThreads + tid;
+        if (c >= rows) continue;
         const float v = EXPAND ? fmaxf(rowmin[q] + xsq[q], 0.f) : rowmin[q];
-        float *dst = P.rowmins + pair * P.M1 + m;
-        if (P.splits == 1) *dst = v;
+        float *dst = P.rowmins + pair * P.M1 + c;     // a listed row's minimum lies where its number in the list says
+        if (splits == 1) *dst = v;
         else atomicMin(reinterpret_cast<unsigned int *>(dst), __float_as_uint(v));   // non-negative: bits order like values
     }
 }
@@ -379,12 +505,17 @@ hausdorff_refine_kernel(const HdParams P) {
     const float *x2 = reinterpret_cast<const float *>(P.x2) + (b * P.N2 + j) * P.M2 * D;
     float *rm = P.rowmins + pair * P.M1;
     PairState *state = reinterpret_cast<PairState *>(P.keys) + pair;
-    if (!EXPAND && P.handed_over && state->direct == 0) return;
+    const unsigned int handed = EXPAND || P.handed_over ? state->direct : kAllRows;
+    if (EXPAND ? handed != 0 : handed == 0) return;
+    unsigned int *list = P.list + pair * P.M1;
+    const bool listed = !EXPAND && handed != kAllRows;
+    const long long rows = listed ? (long long)handed : P.M1;
+    auto row_of = [&](long long c) -> long long { return listed ? (long long)list[c] : c; };
+    auto position = [&](long long m) -> unsigned int { return (unsigned int)(P.order1 ? P.order1[b * P.M1 + m] : m); };
     // the largest approximate minimum, the last visited row on ties
     unsigned long long key = 0ull;
-    for (long long m = tid; m < P.M1; m += kThreads) {
-        const unsigned int pos = (unsigned int)(P.order1 ? P.order1[b * P.M1 + m] : m);
-        const unsigned long long kq = ((unsigned long long)__float_as_uint(rm[m]) << 32) | pos;
+    for (long long c = tid; c < rows; c += kThreads) {
+        const unsigned long long kq = ((unsigned long long)__float_as_uint(rm[c]) << 32) | position(row_of(c));
         key = kq > key ? kq : key;
     }
 #pragma unroll
@@ -402,39 +533,46 @@ hausdorff_refine_kernel(const HdParams P) {
     // An approximate minimum of exactly 0 means every difference squared to 0, in either arithmetic: all rows then
     // tie at 0 and the last visited one, which the key already names, wins.  Otherwise a row can hold the exact
     // maximum only if its approximate minimum is within the rounding slack of the largest approximate minimum.
-    // EXPAND: with R^2 the largest squared norm about the centre, the centred coordinates' roundings change a squared distance
-    // by at most 8 u R^2 (u = 2^-24), the two norms' by 2 D u R^2, the D multiply-adds' by 3 D u R^2 and the last addition's by
-    // 4 u R^2: E = (5 D + 12) u R^2.  A row of the largest distance lies within 2 E of the largest minimum; 16 D + 64 leaves room.
     const bool all_zero = !EXPAND && amax == 0.f;
     float lower = amax * (1.f - fused_slack<D>()) - kTiny;
-    if (EXPAND) lower -= 2.f * (float)(8 * (D + 1) + 24) * 5.9604645e-8f * __uint_as_float(state->extent);
+    if (EXPAND) lower -= expanded_slack<D>(__uint_as_float(state->extent));
 
     // the rows to look at; their order does not matter
-    __shared__ int s_count;
+    __shared__ unsigned int s_count;
     __shared__ unsigned int s_cand[kMaxCandidates];
     if (tid == 0) s_count = 0;
     __syncthreads();
-    for (long long m = tid; m < P.M1; m += kThreads) {
-        const bool cand = all_zero ? (unsigned int)(P.order1 ? P.order1[b * P.M1 + m] : m) == pos_max : rm[m] >= lower;
+    for (long long c = tid; c < rows; c += kThreads) {
+        const bool cand = all_zero ? position(row_of(c)) == pos_max : rm[c] >= lower;
         if (cand) {
-            const int at = atomicAdd(&s_count, 1);
-            if (at < kMaxCandidates) s_cand[at] = (unsigned int)m;
+            const unsigned int at = atomicAdd(&s_count, 1u);
+            if (at < kMaxCandidates) s_cand[at] = (unsigned int)row_of(c);
         }
     }
     __syncthreads();
-    const int count = s_count;
-    if (EXPAND && (count > kMaxCandidates || !(__uint_as_float(state->extent) < kExtentMax))) {
-        // too close together for the expanded form: the direct one starts from untouched minima
-        for (long long m = tid; m < P.M1; m += kThreads) rm[m] = __uint_as_float(0xffffffffu);
-        if (tid == 0) state->direct = 1;
-        return;
+    const unsigned int count = s_count;
+    if (EXPAND) {
+        const bool bounded = __uint_as_float(state->extent) < kExtentMax;
+        if (!bounded || count > kMaxExpanded) {
+            // hand those rows over, or all of them; the direct form starts from untouched minima
+            __syncthreads();
+            if (tid == 0) s_count = 0;
+            __syncthreads();
+            if (bounded)
+                for (long long m = tid; m < P.M1; m += kThreads)
+                    if (rm[m] >= lower) list[atomicAdd(&s_count, 1u)] = (unsigned int)m;
+            __syncthreads();
+            for (long long c = tid; c < (bounded ? (long long)count : P.M1); c += kThreads) rm[c] = __uint_as_float(0xffffffffu);
+            if (tid == 0) state->direct = bounded ? count : kAllRows;
+            return;
+        }
     }
     if (count <= kMaxCandidates) {
         unsigned long long row_key = 0ull, n_key = ~0ull;    // best (bits(min) << 32 | position(m)) and its n key, the same in all threads
         long long row = -1;
-        for (int c = 0; c < count; ++c) {
+        for (unsigned int c = 0; c < count; ++c) {
             const long long m = s_cand[c];
-            const unsigned int pos = (unsigned int)(P.order1 ? P.order1[b * P.M1 + m] : m);
+            const unsigned int pos = position(m);
             float a[D];
 #pragma unroll
             for (int k = 0; k < D; ++k) a[k] = x1[m * D + k];
@@ -482,19 +620,18 @@ hausdorff_refine_kernel(const HdParams P) {
 
     unsigned long long wrow = 0ull, wn = ~0ull;   // best (bits(min) << 32 | position(m)) of this warp, its n key
     long long wm = -1;
-    for (long long base = (long long)warp * 32; base < P.M1; base += kThreads) {
-        const long long m = base + lane;
+    for (long long base = (long long)warp * 32; base < rows; base += kThreads) {
         unsigned int pos = 0;
         bool cand = false;
-        if (m < P.M1) {
-            pos = (unsigned int)(P.order1 ? P.order1[b * P.M1 + m] : m);
-            cand = all_zero ? (pos == pos_max) : (rm[m] >= lower);
+        if (base + lane < rows) {
+            pos = position(row_of(base + lane));
+            cand = all_zero ? (pos == pos_max) : (rm[base + lane] >= lower);
         }
         unsigned int todo = __ballot_sync(0xffffffffu, cand);
         while (todo) {
             const int src = __ffs(todo) - 1;
             todo &= todo - 1;
-            const long long mc = base + src;
+            const long long mc = row_of(base + src);
             const unsigned int posc = __shfl_sync(0xffffffffu, pos, src);
             float a[D];
 #pragma unroll
@@ -757,9 +894,20 @@ int launch_fast(HdParams P, cudaStream_t s) {
         const long long blocks = pairs * P.mtiles * P.splits;
         TPW_CHECK_ARG(blocks < (1ll << 31), "hausdorff: too many blocks");
         if (P.splits > 1) TPW_CUDA_OK(cudaMemsetAsync(P.rowmins, 0xff, (size_t)(pairs * P.M1) * sizeof(float), s));
-        // the expanded form pays for the two launches that serve handed-over pairs from about 2^26 point pairs on
-        if ((double)pairs * (double)P.M1 * (double)P.M2 >= 67108864.0) {
-            TPW_CUDA_OK(cudaMemsetAsync(P.keys, 0, (size_t)pairs * sizeof(PairState), s));
+        P.list = reinterpret_cast<unsigned int *>(P.rowmins + pairs * P.M1);
+        // From 2^27 point pairs on: below, the sample and the two launches that serve handed-over rows cost what the expanded form
+        // saves, and more where rows are handed over (200 pairs of 700 and 800 points: 51 to 99 us, 74 before any expanded form).
+        if ((double)pairs * (double)P.M1 * (double)P.M2 >= 134217728.0) {
+            // sampling CTAs: 1024 x2 points to one, no more than fill the GPU or than a pair's list has room for
+            const long long fill = 4ll * sm_count() / pairs, samples = P.M2 / 1024 < fill ? P.M2 / 1024 : fill;
+            if (P.M1 > 8 * kSampleWords) P.samples = (int)(samples < 1 ? 1 : samples < P.M1 / kSampleWords ? samples : P.M1 / kSampleWords);
+            if (P.samples > 0) {
+                TPW_CHECK_ARG(pairs * P.samples < (1ll << 31), "hausdorff: too many blocks");
+                hausdorff_sample_kernel<D><<<(unsigned)(pairs * P.samples), kThreads, 0, s>>>(P);
+                TPW_LAUNCH_OK("hausdorff_sample_kernel");
+            } else {
+                TPW_CUDA_OK(cudaMemsetAsync(P.keys, 0, (size_t)pairs * sizeof(PairState), s));
+            }
             hausdorff_rowmin_fused_kernel<D, true><<<(unsigned)blocks, kFThreads, 0, s>>>(P);
             TPW_LAUNCH_OK("hausdorff_rowmin_fused_kernel");
             hausdorff_refine_kernel<D, true><<<(unsigned)pairs, kThreads, 0, s>>>(P);
