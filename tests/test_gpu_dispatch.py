@@ -160,3 +160,47 @@ def test_boolean_rows_of_a_matrix_against_its_columns(tpw, n):
     for fn in (tpw.jaccard_distances, tpw.hamming_distances, torch.ops.torchpairwise.jaccard_distances):
         assert torch.equal(fn(x, x.t()), fn(x, x.t().contiguous()))
         assert torch.equal(fn(x, x[:]), fn(x, x.clone()))
+
+
+@pytest.mark.parametrize("name,kw", [("euclidean_distances", {}), ("manhattan_distances", {}), ("chebyshev_distances", {}), ("minkowski_distances", {"p": 3.0}),
+                                     ("minkowski_distances", {"p": 2.5}), ("minkowski_distances", {"p": 0.0}), ("cosine_distances", {}), ("cosine_similarity", {})])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64, torch.bfloat16])
+@pytest.mark.parametrize("shape", [((40, 12), (33, 12)), ((2, 300, 70), (2, 257, 70)), ((2, 2048, 64), (2, 1100, 64))])
+def test_python_functions_and_cpp_nodes_agree(tpw, monkeypatch, name, kw, dtype, shape):
+    """The Python autograd functions, forced, against the C++ nodes that stand in for them: results and gradients, both or one of them,
+    bit for bit (the launches are the same)."""
+    from torchpairwise_b200 import ops
+    g = torch.Generator().manual_seed(len(name))
+    x1, x2 = (torch.randn(*s, generator=g).to(dtype).cuda() for s in shape)
+    up = torch.randn(*shape[0][:-1], shape[1][-2], generator=g).to(dtype).cuda()
+    seen = []
+    for python in (True, False):
+        monkeypatch.setattr(ops, "_native_ops", None if python else torch.ops.torchpairwise)
+        a, b = x1.clone().requires_grad_(), x2.clone().requires_grad_()
+        out = getattr(tpw, name)(a, b, **kw)
+        if dtype != torch.bfloat16 and len(shape[0]) == 3:      # neither a view nor a conversion on top of the node
+            assert (type(out.grad_fn).__name__ in ("_CdistFunctionBackward", "_CosineSimilarityFunctionBackward")) == python
+        res = [out.detach(), *torch.autograd.grad(out, (a, b), up)]
+        for need in ((True, False), (False, True)):
+            a, b = x1.clone().requires_grad_(need[0]), x2.clone().requires_grad_(need[1])
+            res += torch.autograd.grad(getattr(tpw, name)(a, b, **kw), (a,) if need[0] else (b,), up)
+        with torch.no_grad():
+            res.append(getattr(tpw, name)(x1, x2, **kw))
+        seen.append(res)
+    assert all(torch.equal(p, c) and p.dtype == c.dtype == dtype for p, c in zip(*seen))
+
+
+@pytest.mark.parametrize("name", ["euclidean_distances", "manhattan_distances", "chebyshev_distances", "minkowski_distances", "cosine_distances",
+                                  "seuclidean_distances"])
+def test_one_requested_gradient(tpw, name):
+    """One gradient out of two that could be asked for: that of the call for both, to rounding (it may be added in another order)."""
+    for n1, n2, d in ((40, 33, 12), (700, 600, 192)):
+        g = torch.Generator().manual_seed(n1)
+        x1, x2 = torch.randn(n1, d, generator=g).cuda().requires_grad_(), torch.randn(n2, d, generator=g).cuda().requires_grad_()
+        kw = {"seuclidean_distances": {"V": torch.rand(d, generator=g).cuda() + 0.5}, "minkowski_distances": {"p": 3.0}}.get(name, {})
+        out = getattr(tpw, name)(x1, x2, **kw)
+        up = torch.randn(n1, n2, generator=g).cuda()
+        both = torch.autograd.grad(out, (x1, x2), up, retain_graph=True)
+        for t, want in zip((x1, x2), both):
+            got, = torch.autograd.grad(out, (t,), up, retain_graph=True)
+            assert float((got - want).abs().max()) <= 2e-5 * float(want.abs().max())

@@ -117,9 +117,30 @@ def test_hausdorff_expanded_form_and_hand_over(tpw, monkeypatch, case):
             assert torch.equal(a, w), (case, shuffle)
 
 
+@pytest.mark.parametrize("d", [1023, 5003, 65535, 262139, 262143, 262145])
+def test_quotients_of_large_counts_round_as_the_division(tpw, d):
+    """The same up to and across 2^18, where the kernel goes over to the division: prefixes of lengths near d, near the powers of two
+    below it and spread over the range, against each other."""
+    from torchpairwise_b200 import _abi
+    near = [d - t for t in range(60)] + [2 ** e + t for e in range(6, d.bit_length()) for t in (-1, 0, 1) if 2 ** e + t <= d]
+    g = torch.Generator().manual_seed(d)
+    i = torch.tensor(sorted(set(near)) + torch.randint(1, d + 1, (300,), generator=g).tolist())[:256]
+    j = torch.cat([i, torch.randint(1, d + 1, (256,), generator=g)])[:300]
+    k = torch.arange(d, device="cuda")
+    x1, x2 = k[None] < i.cuda()[:, None], k[None] < j.cuda()[:, None]
+    if d < 5000:                                  # enough pairs for the tensor-core counts
+        x1, x2 = x1.repeat(9, 1), x2.repeat(9, 1)
+    assert _abi.lib.tpw_bool_rows_pitch(1, x1.size(0), x2.size(0), d) > 0
+    a, b = x1.sum(1).double(), x2.sum(1).double()
+    diff, most = (a[:, None] - b[None]).abs(), torch.maximum(a[:, None], b[None])
+    # a float64 quotient of integers this small, rounded once more to float32, is the correctly rounded quotient
+    assert torch.equal(tpw.jaccard_distances(x1, x2), (diff / most).float())
+    assert torch.equal(tpw.hamming_distances(x1, x2), (diff / d).float())
+
+
 def test_quotients_of_counts_round_as_the_division(tpw):
-    """Every quotient of counts with a denominator up to 300, through the metrics themselves: row i of x1 has its first i
-    features set, row j of x2 its first j, so jaccard is |i - j| / max(i, j) and hamming |i - j| / D for every i, j, D."""
+    """Every quotient of counts with a denominator of up to 300 for four feature counts, through the metrics themselves: row i of
+    x1 has its first i features set, row j of x2 its first j, so jaccard is |i - j| / max(i, j) and hamming |i - j| / D."""
     for d in (129, 160, 257, 300):
         n = d + 1
         x = (torch.arange(d)[None, :] < torch.arange(n)[:, None]).cuda()
@@ -334,3 +355,46 @@ def test_hausdorff_rows_handed_over(tpw, monkeypatch, case, d):
             monkeypatch.delenv("TPW_HAUSDORFF_EXACT_LOOP", raising=False)
         for a, w in zip(*res):
             assert torch.equal(a, w), (case, shuffle)
+
+
+@pytest.mark.parametrize("shape", [(1, 70, 50, 16), (2, 129, 67, 36), (1, 64, 64, 70), (1, 300, 130, 257)])
+def test_chebyshev_backward_with_values_that_are_not_finite(tpw, shape):
+    """Infinite and NaN coordinates in the group match: an infinite difference attains an infinite maximum, a NaN attains none and hides
+    nothing; against the dense kernel, which tests every coordinate."""
+    from torchpairwise_b200 import _abi
+    b, n1, n2, d = shape
+    g = torch.Generator().manual_seed(d)
+    x1, x2 = torch.randn(b, n1, d, generator=g), torch.randn(b, n2, d, generator=g)
+    x1[0, 3, 1], x1[0, 5, d - 1], x2[0, 7, 0], x2[0, 9, 2], x1[0, 11, 3], x2[0, 11, 3] = math.inf, math.nan, -math.inf, math.nan, math.inf, math.inf
+    up = torch.randn(b, n1, n2, generator=g).cuda()
+    a, c = x1.cuda().requires_grad_(), x2.cuda().requires_grad_()
+    out = tpw.chebyshev_distances(a, c)
+    g1, g2 = torch.autograd.grad(out, (a, c), up)
+    d1, d2 = torch.empty_like(g1), torch.empty_like(g2)
+    _abi.check(_abi.lib.tpw_lp_backward(_abi.F32, _abi.LP_BWD_CDIST, up.data_ptr(), out.data_ptr(), a.data_ptr(), c.data_ptr(), None, d1.data_ptr(),
+                                        d2.data_ptr(), b, n1, n2, d, math.inf, torch.cuda.current_stream().cuda_stream))
+    for got, want in ((g1, d1), (g2, d2)):
+        torch.testing.assert_close(got, want, rtol=1e-5, atol=1e-5 * float(want.nan_to_num().abs().max()), equal_nan=True)
+
+
+@pytest.mark.parametrize("low", ["x1", "x2", "both", "neither"])
+def test_low_parts_that_are_left_out_next_to_values_that_are_not_finite(tpw, low):
+    """An operand that 16 bits hold exactly has no low part to multiply; an infinity or NaN in either operand still reaches every result it
+    reaches in float64, and no other, forward and backward."""
+    g = torch.Generator().manual_seed(3)
+    x1, x2 = torch.randn(1100, 192, generator=g), torch.randn(1300, 192, generator=g)
+    if low in ("x1", "both"):
+        x1 = x1.bfloat16().float()
+    if low in ("x2", "both"):
+        x2 = x2.bfloat16().float()
+    x1[17, 5], x2[33, 7], x2[40, 0] = math.inf, -math.inf, math.nan
+    up = torch.randn(1100, 1300, generator=g).cuda()
+    a, c = x1.cuda().requires_grad_(), x2.cuda().requires_grad_()
+    out = tpw.linear_kernel(a, c)
+    g1, g2 = torch.autograd.grad(out, (a, c), up)
+    w, w1, w2 = x1.cuda().double() @ x2.cuda().double().T, up.double() @ x2.cuda().double(), up.double().T @ x1.cuda().double()
+    for got, want in ((out.detach(), w), (g1, w1), (g2, w2)):
+        # a split infinity has a NaN low part, so an infinite result may come out as NaN; finite ones are finite and right
+        ok = torch.isfinite(want)
+        assert torch.equal(torch.isfinite(got), ok)
+        assert float((got[ok] - want[ok]).abs().max()) <= 1e-5 * float(want[ok].abs().max())

@@ -370,8 +370,10 @@ def test_one_pass_backward(tpw, mode, p):
         ptr = lambda t: None if t is None else t.data_ptr()
         want = lib.tpw_lp_backward_scratch_bytes(_abi.F32, code, b, n1, n2, d, p)
         assert want > 0, shape
-        slab = n2 * d * 4
+        # scratch of one row block of one batch, and of one batch: transposed coefficients and the block sums of grad_x2
         blocks = (n1 + 255) // 256
+        block, batch = (256 + d) * n2 * 4, ((n1 + 3) // 4 * 4 + blocks * d) * n2 * 4
+        assert want >= b * batch, shape
 
         def run(nbytes):
             g1, g2 = torch.full_like(x1, float("nan")), torch.full_like(x2, float("nan"))
@@ -390,11 +392,17 @@ def test_one_pass_backward(tpw, mode, p):
         again = run(want)
         assert torch.equal(one[0], again[0]) and torch.equal(one[1], again[1]), shape
         scale = float(two[0].abs().max()) + float(two[1].abs().max())
-        for nbytes in (want, slab * blocks * 2, slab * max(1, blocks - 1), slab):
+        # as given, all batches, two batches and a remainder that no third fits into, one batch, all row blocks but one, one row block
+        for nbytes in (want, b * batch, 3 * batch - 16, batch, max(1, blocks - 1) * block, block):
             res = run(nbytes)
             for a, r in zip(res, two):
                 assert not torch.isnan(a).any()
                 assert float((a - r).abs().max()) <= 2e-5 * scale, (shape, nbytes)
+            # all of these reach the one-pass kernel, whose order of addition is another
+            assert not torch.equal(res[1], two[1]), (shape, nbytes)
+        # 16 bytes less than one row block: the two launches
+        res = run(block - 16)
+        assert torch.equal(res[0], two[0]) and torch.equal(res[1], two[1]), shape
         # oracle: float64 autograd of the same composite
         a64, b64 = x1.double().requires_grad_(), x2.double().requires_grad_()
         if mode == "cdist":
