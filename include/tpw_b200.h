@@ -188,9 +188,10 @@ TPW_API int tpw_lp_backward(int dtype, int mode, const void *grad, const void *a
  * tpw_lp_backward_scratch_bytes() returns 0 where the kernel does not apply (float64, p = +inf, the
  * plain contraction, fewer than 256 rows of x1, D not a multiple of 4, small problems,
  * TPW_DISABLE_ONEPASS_BWD=1), else the scratch it wants: B * (N1 + ceil(N1/256) * D) * N2 * 4 bytes (the
- * coefficients of all pairs, transposed, and the block sums; N1 rounded up to a multiple of 4) up to
- * 2 GiB (larger problems run as several launches over batch or row-block ranges).  With scratch ==
- * NULL, less than one row block needs, (256 + D) * N2 * 4 bytes, a NULL gradient pointer or a pointer that is not 16-byte aligned the
+ * coefficients of all pairs, transposed, and the block sums; N1 rounded up to a multiple of 4) and, where
+ * few blocks share each walk over x2 in up to 32 ranges, ranges * B * N1 * D * 4 for the ranges' sums of
+ * grad_x1; at most 2 GiB (larger problems run as several launches over batch or row-block ranges).  Less
+ * scratch than that runs more launches and unshared walks; with scratch == NULL, less than one row block needs, (256 + D) * N2 * 4 bytes, a NULL gradient pointer or a pointer that is not 16-byte aligned the
  * call is tpw_lp_backward.  Replaces the same reference kernels as tpw_lp_backward
  * (OPS/cuda/ppminkowski_kernel.cu:133-218, OPS/cuda/wminkowski_kernel.cu:146-196, ATen's cdist backward).
  */
@@ -505,8 +506,9 @@ TPW_API int tpw_haversine_backward(int dtype, const void *grad, const void *x1, 
  * `scratch` holds tpw_hausdorff_scratch_bytes() bytes (8 per set pair plus 8 per x1 point of every set
  * pair), 8-byte aligned, and needs no initialisation.  float64 clouds of up to 16 coordinates keep every
  * row's exact minimum there and scan them once per set pair (TPW_HAUSDORFF_PLAIN_F64=1, or scratch ==
- * NULL, selects the one-CTA-per-pair kernel instead; same bits).  For float32 the hot loop forms the squared distance with fused multiply-adds
- * (7 operations per point pair) and stores every row's approximate minimum there; the finishing kernel
+ * NULL, selects the one-CTA-per-pair kernel instead; same bits).  For float32 the hot loop stores every row's approximate minimum there:
+ * of the expanded squared distance on large problems, or, for the rows and set pairs that its error leaves
+ * undecided and on small ones, of the direct sum with fused multiply-adds.  The finishing kernel
  * re-evaluates the few rows that can hold the maximum with separately rounded multiply and add, the
  * arithmetic of the reference's CPU loop (OPS/cpu/hausdorff_kernel.cpp:30-33), so values and indices are
  * bit-identical to evaluating every point pair that way (TPW_HAUSDORFF_EXACT_LOOP=1 does exactly that).

@@ -263,10 +263,10 @@ struct ScatterParams {
     long long B, N1, N2, D, NR, tiles_r, tiles_k;
 };
 
-// A pair whose maximum is attained by several coordinates: every one of them in [klo, khi) receives +-g (ascending k).
-__device__ __noinline__ void scatter_tied(float *row, const float *a, const float *c, float o, float g, int k0, int klo, int khi,
+// A pair whose maximum is attained by several coordinates: each of the CTA's kn features among them receives +-g (ascending k).
+__device__ __noinline__ void scatter_tied(float *row, const float *a, const float *c, float o, float g, int k0, int kn,
                                           bool negate) {
-    for (int k = klo; k < khi; ++k) {
+    for (int k = 0; k < kn; ++k) {
         const float d = a[k0 + k] - c[k0 + k];
         if (fabsf(d) == o) row[k] += (d < 0.f) != negate ? -g : g;
     }
@@ -379,7 +379,7 @@ __global__ void __launch_bounds__(STHR, 2) chebyshev_scatter_kernel(const Scatte
                         if (c1 == kTied) {
                             const long long i = COLS ? s0 + ss + u : r0 + tid, j = COLS ? r0 + tid : s0 + ss + u;
                             scatter_tied(mine, P.x1 + (b * P.N1 + i) * P.D, P.x2 + (b * P.N2 + j) * P.D, P.fwd[(b * P.N1 + i) * P.N2 + j],
-                                         g1, k0, 0, kn, COLS);
+                                         g1, k0, kn, COLS);
                         } else if (c1 != kSkip) {
                             const int kk = (int)(c1 & 0xffffu) - k0;
                             if ((unsigned)kk < (unsigned)kn)
