@@ -362,45 +362,55 @@ __global__ void __launch_bounds__(256) lp_backward_small_kernel(const BwdParams 
 }
 
 // The same problems on rows of more than 8 features, where rows_pay() below says so.  One thread per element loads a streamed
-// value, the gradient and the auxiliary value for every term; here a thread has two rows of one feature, so a streamed value serves
-// two terms, and the CTA forms the coefficients of its 16 rows and of 32 streamed rows once, in shared memory, from where a warp
-// reads them with one broadcast load.  The terms of an element are added in the same order, so the results are still those of the
-// tile kernel bit for bit.  Bound: latency of that load and of the terms' chain; eight warps, each over 32 features.  (Four rows to
-// a thread, or 16 features to a group, were slower or within 5 % in all but a few of 24 combinations of metric, type and side.)
-// Weighted p = 2 in float64 [1500, 1301, 75], both gradients: 351 -> 237 us.
+// value, the gradient and the auxiliary value for every term; here a thread has R rows of one feature, so a streamed value serves
+// R terms, and the CTA stages 32 streamed rows and forms the coefficients of its 8 R rows against them once, in shared memory,
+// from where a warp reads them broadcast.  What a stage needs is fetched into registers while the stage before is
+// worked on.  Both gradients go in one launch, grad_x1's CTAs first, so that neither waits for the other's last wave.  The terms
+// of an element are added in the same order, so the results are still those of the tile kernel bit for bit.  Bound: the
+// shared-memory reads, which fill registers at 128 bytes a clock whether the lanes read one word or 32, and, in float64, the
+// arithmetic at half a clock per instruction and warp.  (4 rows by 3 features to a thread halve the reads per term, but leave fewer
+// than five warps to an SM: 161 us where 4 rows by 1 feature take 126.)
+// Weighted p = 2 in float64 [1500, 1301, 75], both gradients: 351 us with one thread per element, 338 with two rows to a thread,
+// the streamed rows read from L2 inside the walk and two launches, 126 now (profiled one by one).
 constexpr int SB_THREADS = 256;
 constexpr int SB_S = 32;       // streamed rows per stage
-constexpr int SB_R = 2;        // rows per thread
-constexpr int SB_ROWS = SB_THREADS / 32 * SB_R;
-constexpr int SB_PER = SB_ROWS * SB_S / SB_THREADS;   // pairs of a stage that a thread forms the coefficients of
 
-template <typename T, int PHI, bool NEED_AUX, bool TRANS>
-__global__ void __launch_bounds__(SB_THREADS) lp_backward_rows_kernel(const BwdParams P) {
-    constexpr int PITCH = SB_ROWS + 16 / (int)sizeof(T);      // rows of 16-byte multiples, shifted by a bank group from row to row
-    __shared__ __align__(16) T cs[2][SB_S * PITCH];
+template <typename T, int R> struct RowsSmem {
+    static constexpr int ROWS = SB_THREADS / 32 * R;
+    static constexpr int PITCH = ROWS + 16 / (int)sizeof(T);      // rows of 16-byte multiples, shifted by a bank group from row to row
+    __align__(16) T cs[2][SB_S * PITCH];
+    T ys[2][SB_S][32];
+};
+
+template <typename T, int PHI, bool NEED_AUX, int R, bool TRANS>
+__device__ __forceinline__ void rows_walk(const BwdParams &P, long long tile, RowsSmem<T, R> &sm) {
+    constexpr int ROWS = RowsSmem<T, R>::ROWS, PITCH = RowsSmem<T, R>::PITCH;
+    constexpr int PER = ROWS * SB_S / SB_THREADS;   // pairs of a stage that a thread forms the coefficients of
+    constexpr int YPER = SB_S * 32 / SB_THREADS;    // streamed values that it stages
     const int tid = threadIdx.x, lane = tid & 31, group = tid >> 5;
-    long long tile = blockIdx.x;
     const long long tk = tile % P.tiles_k;
     tile /= P.tiles_k;
     const long long tr = tile % P.tiles_r, b = tile / P.tiles_r;
-    const long long k = tk * 32 + lane, r0 = tr * SB_ROWS, row = r0 + group * SB_R;
+    const long long k = tk * 32 + lane, r0 = tr * ROWS, row = r0 + group * R;
     const bool k_ok = k < P.D;
     const T *stream = reinterpret_cast<const T *>(P.stream) + b * P.NS * P.D + (k_ok ? k : 0);
     const T *grad = reinterpret_cast<const T *>(P.grad) + b * P.N1 * P.N2;
     const T *aux = NEED_AUX ? reinterpret_cast<const T *>(P.aux) + b * P.N1 * P.N2 : nullptr;
-    T x[SB_R], acc[SB_R];
+    T x[R], acc[R];
 #pragma unroll
-    for (int a = 0; a < SB_R; ++a) {
+    for (int a = 0; a < R; ++a) {
         x[a] = PHI != PHI_Y && k_ok && row + a < P.NR ? reinterpret_cast<const T *>(P.rowop)[(b * P.NR + row + a) * P.D + k] : T(0);
         acc[a] = T(0);
     }
     // this thread's pairs of a stage: consecutive threads along the dimension that is contiguous in memory
-    T g[SB_PER], o[SB_PER];
+    T g[PER], o[PER], yv[YPER];
     auto fetch = [&](long long s0) {
 #pragma unroll
-        for (int u = 0; u < SB_PER; ++u) {
+        for (int u = 0; u < YPER; ++u) yv[u] = s0 + group + 8 * u < P.NS ? stream[(s0 + group + 8 * u) * P.D] : T(0);
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
             const int e = tid + u * SB_THREADS;
-            const long long r = r0 + (TRANS ? e % SB_ROWS : e / SB_S), s = s0 + (TRANS ? e / SB_ROWS : e % SB_S);
+            const long long r = r0 + (TRANS ? e % ROWS : e / SB_S), s = s0 + (TRANS ? e / ROWS : e % SB_S);
             const bool ok = r < P.NR && s < P.NS;
             const long long at = TRANS ? s * P.N2 + r : r * P.N2 + s;
             g[u] = ok ? grad[at] : T(0);
@@ -413,35 +423,40 @@ __global__ void __launch_bounds__(SB_THREADS) lp_backward_rows_kernel(const BwdP
     for (long long s0 = 0; s0 < P.NS; s0 += SB_S, buf ^= 1) {
         // a warp may still be reading the other buffer; this one was last read before the previous barrier
 #pragma unroll
-        for (int u = 0; u < SB_PER; ++u) {
+        for (int u = 0; u < YPER; ++u) sm.ys[buf][group + 8 * u][lane] = yv[u];
+#pragma unroll
+        for (int u = 0; u < PER; ++u) {
             const int e = tid + u * SB_THREADS;
-            const int at = (TRANS ? e / SB_ROWS : e % SB_S) * PITCH + (TRANS ? e % SB_ROWS : e / SB_S);
-            cs[buf][at] = NEED_AUX ? bwd_coefficient<T>(P.coef_mode, g[u], o[u], P.q) : g[u];
+            const int at = (TRANS ? e / ROWS : e % SB_S) * PITCH + (TRANS ? e % ROWS : e / SB_S);
+            sm.cs[buf][at] = NEED_AUX ? bwd_coefficient<T>(P.coef_mode, g[u], o[u], P.q) : g[u];
         }
         __syncthreads();
         if (s0 + SB_S < P.NS) fetch(s0 + SB_S);
         const int cnt = (int)(P.NS - s0 < SB_S ? P.NS - s0 : SB_S);
-        const T *sp = stream + s0 * P.D;
-        auto term = [&](int s, T y) {
-            T c[SB_R];
+        const T *cp = sm.cs[buf] + group * R;
+        auto term = [&](int s) {
+            const T y = sm.ys[buf][s][lane];
+            T c[R];
+            if constexpr (R == 4) {
+                load4<T>(c, cp + s * PITCH);
+            } else {
 #pragma unroll
-            for (int a = 0; a < SB_R; ++a) c[a] = cs[buf][s * PITCH + group * SB_R + a];
+                for (int a = 0; a < R; ++a) c[a] = cp[s * PITCH + a];
+            }
 #pragma unroll
-            for (int a = 0; a < SB_R; ++a) bwd_accumulate<PHI, T>(acc[a], x[a], y, c[a], T(0), q, P.pow_spec);
+            for (int a = 0; a < R; ++a) bwd_accumulate<PHI, T>(acc[a], x[a], y, c[a], T(0), q, P.pow_spec);
         };
-        int s = 0;
-        for (; s + 8 <= cnt; s += 8) {
-            T y[8];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) y[u] = sp[(s + u) * P.D];
-#pragma unroll
-            for (int u = 0; u < 8; ++u) term(s + u, y[u]);
+        if (cnt == SB_S) {
+#pragma unroll 8
+            for (int s = 0; s < SB_S; ++s) term(s);
+        } else {
+#pragma unroll 1
+            for (int s = 0; s < cnt; ++s) term(s);
         }
-        for (; s < cnt; ++s) term(s, sp[s * P.D]);
     }
     if (!k_ok) return;
 #pragma unroll
-    for (int a = 0; a < SB_R; ++a) {
+    for (int a = 0; a < R; ++a) {
         if (row + a >= P.NR) continue;
         T v = acc[a] * (T)P.post;
         if (P.w) v *= reinterpret_cast<const T *>(P.w)[b * P.D + k];
@@ -449,10 +464,18 @@ __global__ void __launch_bounds__(SB_THREADS) lp_backward_rows_kernel(const BwdP
     }
 }
 
+// CTAs [0, first) work on grad_x1 (P1), the others on grad_x2 (P2).
+template <typename T, int PHI, bool NEED_AUX, int R>
+__global__ void __launch_bounds__(SB_THREADS) lp_backward_rows_kernel(const BwdParams P1, const BwdParams P2, long long first) {
+    __shared__ RowsSmem<T, R> sm;
+    if (blockIdx.x < first) rows_walk<T, PHI, NEED_AUX, R, false>(P1, blockIdx.x, sm);
+    else rows_walk<T, PHI, NEED_AUX, R, true>(P2, blockIdx.x - first, sm);
+}
+
 // Where the rows kernel is faster than one thread per element.  Each of its walks is a chain of shared loads with a barrier every
 // 32 rows, at twice the elements per thread; it pays where forming a coefficient costs more than that (a division in float64, a power),
 // where the other kernel reads the gradient across its rows (some grad_x2 walks), or where one thread per element runs in more waves
-// than the GPU holds.  Times over one thread per element at 20 to 3000 rows, 9 to 500 features, 1000 streamed rows, for n = rows x
+// than the GPU holds.  Times over one thread per element (of the kernel as it was with the streamed rows read from L2) at 20 to 3000 rows, 9 to 500 features, 1000 streamed rows, for n = rows x
 // features (grad_x1 / grad_x2):
 //   float32  no coefficient  sign 1.3 / 0.4, d 1.5 / 0.7, d|d| 0.85 / 0.85 (n > 2^17.5: 1.0 / 0.8), power 2.1 / 1.4, product 1.1 / 1.2
 //            g / out         0.95 to 1.05 / 0.65, from n = 2^16.5 0.75 / 0.5;   g / out^2  1.3 / 1.4, from 2^17 0.75 / 0.65;
@@ -481,12 +504,25 @@ bool rows_pay(const BwdParams &P) {
     }
 }
 
+// The gradient block of a CTA of the tile kernel.
+template <typename T> struct BwdTile {
+    static constexpr int RR = 4, RK = sizeof(T) == 4 ? 8 : 4, NTHR = sizeof(T) == 4 ? 512 : 256;
+    typedef BwdSmem<T, RR, RK, NTHR> Smem;
+};
+
+// Fewer gradient blocks than a third of the SMs: one thread per gradient element, or several rows of a feature to a thread, instead
+// (TPW_DISABLE_SMALL_BWD=1 keeps the tile kernel); the walk per thread is bounded so that a launch stays in the millisecond range.
+template <typename T>
+bool is_small_backward(const BwdParams &P) {
+    typedef typename BwdTile<T>::Smem S;
+    const long long tiles = P.B * ((P.NR + S::TR - 1) / S::TR) * ((P.D + S::TK - 1) / S::TK);
+    return tiles * 3 < sm_count() && P.NS <= 65536 && P.B * P.NR * P.D < (1ll << 31) * 256 && !getenv("TPW_DISABLE_SMALL_BWD");
+}
+
 template <typename T, int PHI, bool NEED_AUX, bool TRANS>
 int launch_backward(BwdParams P, cudaStream_t stream) {
-    constexpr int RR = 4;
-    constexpr int RK = sizeof(T) == 4 ? 8 : 4;
-    constexpr int NTHR = sizeof(T) == 4 ? 512 : 256;
-    typedef BwdSmem<T, RR, RK, NTHR> S;
+    constexpr int RR = BwdTile<T>::RR, RK = BwdTile<T>::RK, NTHR = BwdTile<T>::NTHR;
+    typedef typename BwdTile<T>::Smem S;
     P.tiles_r = (P.NR + S::TR - 1) / S::TR;
     P.tiles_k = (P.D + S::TK - 1) / S::TK;
     const long long tiles = P.B * P.tiles_r * P.tiles_k;
@@ -496,20 +532,7 @@ int launch_backward(BwdParams P, cudaStream_t stream) {
                   "lp backward: a dimension exceeds 2^31-1");
     P.status = device_status_ptr();
 
-    // fewer gradient blocks than a third of the SMs: one thread per gradient element, or two rows of a feature to a thread, instead
-    // (TPW_DISABLE_SMALL_BWD=1 keeps the tile kernel); the walk per thread is bounded so that a launch stays in the millisecond range
-    if (tiles * 3 < sm_count() && P.NS <= 65536 && P.B * P.NR * P.D < (1ll << 31) * 256 && !getenv("TPW_DISABLE_SMALL_BWD")) {
-        if constexpr (rows_may_pay<T, PHI, NEED_AUX, TRANS>()) {
-            if (rows_pay<T, PHI, NEED_AUX, TRANS>(P)) {
-                P.tiles_k = (P.D + 31) / 32;
-                P.tiles_r = (P.NR + SB_ROWS - 1) / SB_ROWS;
-                const long long ctas = P.B * P.tiles_r * P.tiles_k;
-                TPW_CHECK_ARG(ctas < (1ll << 31), "lp backward: too many tiles (%lld)", ctas);
-                lp_backward_rows_kernel<T, PHI, NEED_AUX, TRANS><<<(unsigned)ctas, SB_THREADS, 0, stream>>>(P);
-                TPW_LAUNCH_OK("lp_backward_rows_kernel");
-                return TPW_OK;
-            }
-        }
+    if (is_small_backward<T>(P)) {
         const long long n = P.B * P.NR * P.D;
         lp_backward_small_kernel<T, PHI, NEED_AUX, TRANS><<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(P);
         TPW_LAUNCH_OK("lp_backward_small_kernel");
@@ -544,29 +567,49 @@ int launch_backward(BwdParams P, cudaStream_t stream) {
     return TPW_OK;
 }
 
-// One side (grad_x1 when trans == false, grad_x2 when true).
-template <typename T, int PHI, bool NEED_AUX>
-int launch_side(const BwdParams &base, bool trans, const void *x1, const void *x2, void *out, cudaStream_t stream) {
-    BwdParams P = base;
+// One side: grad_x1 when TRANS == false, grad_x2 when true.
+template <bool TRANS>
+BwdParams side_params(BwdParams P, const void *x1, const void *x2, void *out) {
     P.out = out;
-    if (!trans) {
-        P.rowop = x1; P.stream = x2; P.NR = base.N1; P.NS = base.N2;
-        return launch_backward<T, PHI, NEED_AUX, false>(P, stream);
+    P.rowop = TRANS ? x2 : x1; P.stream = TRANS ? x1 : x2;
+    P.NR = TRANS ? P.N2 : P.N1; P.NS = TRANS ? P.N1 : P.N2;
+    return P;
+}
+
+template <typename T, int PHI, bool NEED_AUX, int R>
+int launch_rows(BwdParams P1, BwdParams P2, bool rows1, bool rows2, cudaStream_t stream) {
+    long long ctas[2] = {0, 0};
+    for (int side = 0; side < 2; ++side) {
+        BwdParams &P = side == 0 ? P1 : P2;
+        P.tiles_k = (P.D + 31) / 32;
+        P.tiles_r = (P.NR + RowsSmem<T, R>::ROWS - 1) / RowsSmem<T, R>::ROWS;
+        if (side == 0 ? rows1 : rows2) ctas[side] = P.B * P.tiles_r * P.tiles_k;
     }
-    P.rowop = x2; P.stream = x1; P.NR = base.N2; P.NS = base.N1;
-    return launch_backward<T, PHI, NEED_AUX, true>(P, stream);
+    TPW_CHECK_ARG(ctas[0] + ctas[1] < (1ll << 31), "lp backward: too many tiles (%lld)", ctas[0] + ctas[1]);
+    lp_backward_rows_kernel<T, PHI, NEED_AUX, R><<<(unsigned)(ctas[0] + ctas[1]), SB_THREADS, 0, stream>>>(P1, P2, ctas[0]);
+    TPW_LAUNCH_OK("lp_backward_rows_kernel");
+    return TPW_OK;
 }
 
 template <typename T, int PHI, bool NEED_AUX>
 int launch_both(const BwdParams &base, const void *x1, const void *x2, void *g1, void *g2, cudaStream_t stream) {
-    if (g1) {
-        int st = launch_side<T, PHI, NEED_AUX>(base, false, x1, x2, g1, stream);
-        if (st != TPW_OK) return st;
+    const BwdParams P1 = side_params<false>(base, x1, x2, g1), P2 = side_params<true>(base, x1, x2, g2);
+    bool rows1 = false, rows2 = false;
+    int st;
+    if constexpr (rows_may_pay<T, PHI, NEED_AUX, false>() || rows_may_pay<T, PHI, NEED_AUX, true>()) {
+        rows1 = g1 && is_small_backward<T>(P1) && rows_pay<T, PHI, NEED_AUX, false>(P1);
+        rows2 = g2 && is_small_backward<T>(P2) && rows_pay<T, PHI, NEED_AUX, true>(P2);
+        if (rows1 || rows2) {
+            // four rows to a thread halve the reads of the streamed rows, where the GPU still gets a CTA per SM
+            const long long four = RowsSmem<T, 4>::ROWS, blocks = base.B * ((base.D + 31) / 32) *
+                                   ((rows1 ? (P1.NR + four - 1) / four : 0) + (rows2 ? (P2.NR + four - 1) / four : 0));
+            st = blocks >= sm_count() ? launch_rows<T, PHI, NEED_AUX, 4>(P1, P2, rows1, rows2, stream)
+                                      : launch_rows<T, PHI, NEED_AUX, 2>(P1, P2, rows1, rows2, stream);
+            if (st != TPW_OK) return st;
+        }
     }
-    if (g2) {
-        int st = launch_side<T, PHI, NEED_AUX>(base, true, x1, x2, g2, stream);
-        if (st != TPW_OK) return st;
-    }
+    if (g1 && !rows1 && (st = launch_backward<T, PHI, NEED_AUX, false>(P1, stream)) != TPW_OK) return st;
+    if (g2 && !rows2 && (st = launch_backward<T, PHI, NEED_AUX, true>(P2, stream)) != TPW_OK) return st;
     return TPW_OK;
 }
 
@@ -742,8 +785,8 @@ extern "C" int tpw_wminkowski_backward_w(int dtype, const void *grad, const void
     P.grad = grad; P.aux = aux; P.w = nullptr;
     P.B = B; P.N1 = N1; P.N2 = N2; P.D = D;
     P.post = 1.0; P.q = p; P.pow_spec = make_pow_spec(p); P.coef_mode = COEF_MUL;
-    int st = dtype == TPW_F32 ? launch_side<float, PHI_ABSPOW, true>(P, false, x1, x2, scratch, s)
-                              : launch_side<double, PHI_ABSPOW, true>(P, false, x1, x2, scratch, s);
+    int st = dtype == TPW_F32 ? launch_both<float, PHI_ABSPOW, true>(P, x1, x2, scratch, nullptr, s)
+                              : launch_both<double, PHI_ABSPOW, true>(P, x1, x2, scratch, nullptr, s);
     if (st != TPW_OK) return st;
     const long long n = B * D;
     const int threads = 128;
