@@ -7,55 +7,58 @@
 // is pinned at the POPC issue rate (C3, 65536 x 16384 x 1024 bits: 7.9 ms), the integer contraction leaves only
 // the operand stream from L2 and the 4-byte output write.
 //
-// Kernel: persistent, one CTA per SM, 576 threads -- warp 0 issues TMA (one lane), warp 1 owns tensor memory and
-// issues the MMAs (one lane), warps 2..17 drain the accumulators (TMEM lane quarter = warp % 4, column quarter =
-// (warp - 2) / 4).  Output tile 128 x 256; a k-step is 128 features = one 128-byte swizzled row per operand row,
-// consumed by four MMAs of K = 32; three stages of 16 KB (x1) + 32 KB (x2); two 256-column accumulators in tensor
-// memory, so the epilogue of tile t overlaps the MMAs of tile t + 1.  The operands are the caller's boolean
+// Kernel: persistent, one CTA per SM in pairs (clusters of two, cta_group::2), 576 threads -- warp 0 issues TMA (one lane),
+// warp 1 owns tensor memory and, in rank 0, issues the MMAs for both CTAs (one lane), warps 2..17 drain the accumulators (TMEM
+// lane quarter = warp % 4, 16 of every 64 columns).  A pair's output tile is 256 x 256, 128 rows to a CTA; a k-step is
+// 128 features = one 128-byte swizzled row per operand row, consumed by four MMAs of K = 32; stages of 16 KB (the CTA's x1
+// rows) + 16 KB (its half of the x2 rows); two 256-column accumulators in tensor memory, so the epilogue of tile t overlaps
+// the MMAs of tile t + 1.  Bound: operand reads and result writes share the way between L2 and the SMs (jaccard [32768, 16384,
+// 1024]: 440 us without the stores, 494 without the operand copies, 356 of MMAs and copies alone, 694 together; with 128 x 256
+// tiles per CTA, which read half as much again, and an epilogue of 23 instructions a distance, 720).  The operands are the caller's boolean
 // matrices as they lie in memory when their rows start on 16-byte boundaries, else copies with the rows padded by zeros
 // to a multiple of 16 bytes (bool_rows_kernel, which also counts the rows); the TMA unit zero-fills rows and features
 // past the edge, and zeros add nothing to a count.  Every CTA loads its own tiles with plain per-CTA TMA loads from
 // this GPU's memory.
 //
-// An epilogue warp stages its 32 x 32 block of results in shared memory (128-byte swizzle) and writes it out either
-// with its own 128-bit stores or, for the metrics whose arithmetic is long enough to hide it, by handing the block to
-// the copy engine (a TMA store on the output's tensor map, which also clips the rows past N1).  Where N2 is no multiple
-// of 4 the staged block is written one 128-byte row segment per instruction, lane l its word l.
+// Results leave through shared memory (tile_store.cuh).  [65536, 16384, 1024] jaccard 1447 -> 1315 us, [30011, 10007, 167] hamming
+// 564 -> 429 us.
 //
-// Every mbarrier wait is bounded; a role that gives up raises a CTA-wide abort flag, everybody falls through to the
-// final barrier, tensor memory is released and the device status word reports the site.  The one wait without a
-// bound of its own is cp.async.bulk.wait_group.read, which returns when the copy engine has read a block this warp
-// committed itself.
+// Every mbarrier wait is bounded; a role that gives up raises the pair's abort flag, everybody falls through to the
+// final barrier, tensor memory is released and the device status word reports the site.
 #include "bool_epilogue.cuh"
 #include "common.cuh"
+#include "tcgen05.cuh"
+#include "tile_store.cuh"
 
 #include <type_traits>
-#include "tcgen05.cuh"
 
 #include <stdlib.h>
 
 namespace tpw {
 namespace {
 
-constexpr int BM = 128;             // x1 rows per tile (TMEM lanes)
+constexpr int BM = 128;             // x1 rows per CTA (TMEM lanes); a pair's tile has twice as many
 constexpr int BN = 256;             // x2 rows per tile (TMEM columns per accumulator)
 constexpr int BKB = 128;            // features (bytes) per k-step
-constexpr int kStages = 3;
-constexpr int A_BYTES = BM * BKB;   // 16 KB
-constexpr int B_BYTES = BN * BKB;   // 32 KB
+constexpr int A_BYTES = BM * BKB;       // 16 KB
+constexpr int B_BYTES = BN / 2 * BKB;   // 16 KB: this CTA's half
 constexpr int STAGE_BYTES = A_BYTES + B_BYTES;
-constexpr int OFF_BAR = kStages * STAGE_BYTES;
-// barriers: full[3], empty[3], tmem_full[2], tmem_empty[2]; then the TMEM base address and the abort flag
-constexpr int OFF_TMEM_PTR = OFF_BAR + (2 * kStages + 4) * 8;
-constexpr int OFF_ABORT = OFF_TMEM_PTR + 4;
-constexpr int OFF_STAGE = (OFF_ABORT + 4 + 1023) / 1024 * 1024; // per epilogue warp a 32 x 32 float staging block (1024-byte aligned: it is also the source of a swizzled TMA store)
-constexpr int kEpilogueWarps = 16;            // four per TMEM lane quarter, each draining a quarter of the columns
-constexpr int OFF_POP = OFF_STAGE + kEpilogueWarps * 4096;      // per epilogue warp the 64 x2 row counts of its column quarter
-constexpr int SMEM_BYTES = OFF_POP + kEpilogueWarps * 256;
-constexpr int SMEM_ALLOC = SMEM_BYTES + 1024;
+constexpr int kEpilogueWarps = 16;            // four per TMEM lane quarter, each with 16 of every 64 columns
+// Shared memory.  RAGGED results need the whole tile's rows staged (tile_store.cuh), which leaves room for two operand stages
+// instead of four: their bound is the stores.
+template <bool RAGGED> struct Layout {
+    static constexpr int kStages = RAGGED ? 2 : 4;
+    static constexpr int OFF_BAR = kStages * STAGE_BYTES;
+    // barriers: full, empty [kStages], tmem_full[2], tmem_empty[2]; then the TMEM base address and the abort flag
+    static constexpr int OFF_TMEM_PTR = OFF_BAR + (2 * kStages + 4) * 8;
+    static constexpr int OFF_ABORT = OFF_TMEM_PTR + 4;
+    static constexpr int OFF_STAGE = (OFF_ABORT + 4 + 127) / 128 * 128;
+    static constexpr int OFF_POP = OFF_STAGE + (RAGGED ? BM * BN * 4 : kStoreBytes);   // per epilogue warp the x2 row counts of its 64 columns
+    static constexpr int SMEM_ALLOC = OFF_POP + kEpilogueWarps * 256 + 1024;
+    static_assert(SMEM_ALLOC <= 232448, "exceeds the dynamic shared memory of one CTA");
+};
 constexpr int kThreads = 64 + 32 * kEpilogueWarps;
 constexpr uint32_t kTmemCols = 512;
-static_assert(SMEM_ALLOC <= 232448, "exceeds the dynamic shared memory of one CTA");
 
 struct BoolTcParams {
     const int32_t *pop1, *pop2;
@@ -63,8 +66,6 @@ struct BoolTcParams {
     long long B, N1, N2, D;
     long long tiles_m, tiles_n, tiles;
     int metric;
-    int vec_store;   // N2 % 4 == 0, out and pop2 16-byte aligned
-    int tma_store;   // the staged 32 x 32 blocks leave through the output's tensor map
     float inv_d;     // 1/D when D is a power of two, else 0
     int *status;
 };
@@ -74,7 +75,7 @@ __device__ __forceinline__ void tc_mma_i8(uint32_t tmem_d, uint64_t adesc, uint6
     asm volatile(
         "{\n\t.reg .pred p;\n\t"
         "setp.ne.b32 p, %4, 0;\n\t"
-        "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}"
+        "tcgen05.mma.cta_group::2.kind::i8 [%0], %1, %2, %3, p;\n\t}"
         ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
@@ -121,76 +122,86 @@ bool_rows_kernel(const uint8_t *__restrict__ src, uint8_t *__restrict__ dst, int
 // One instantiation per metric: with the metric a compile-time constant the epilogue's switch folds to the one case,
 // which keeps the unrolled per-element code small enough for the instruction cache (with a run-time metric the 32
 // inlined copies of the whole switch made the epilogue, not the contraction, the bound).
-template <int METRIC>
-__global__ void __launch_bounds__(kThreads, 1)
-bool_count_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y,
-                          const __grid_constant__ CUtensorMap map_out, const BoolTcParams P) {
+template <int METRIC, bool RAGGED>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+bool_count_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __grid_constant__ CUtensorMap map_y, const BoolTcParams P) {
+    typedef Layout<RAGGED> L;
+    constexpr int kStages = L::kStages;
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem + OFF_BAR);
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + L::OFF_BAR);   // rank 0's: both CTAs' copies of a stage have landed
     uint64_t *empty = full + kStages;
     uint64_t *tmem_full = empty + kStages;
-    uint64_t *tmem_empty = tmem_full + 2;
-    uint32_t *tmem_ptr = reinterpret_cast<uint32_t *>(smem + OFF_TMEM_PTR);
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + OFF_ABORT);
+    uint64_t *tmem_empty = tmem_full + 2;                                // rank 0's: both CTAs have drained the accumulator
+    uint32_t *tmem_ptr = reinterpret_cast<uint32_t *>(smem + L::OFF_TMEM_PTR);
+    int *abort_flag = reinterpret_cast<int *>(smem + L::OFF_ABORT);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank();       // the pair's tile: rows of rank 0, then rows of rank 1
+    const int pair = blockIdx.x >> 1, pairs = gridDim.x >> 1, tiles = (int)P.tiles;   // 2^31 tiles would be a result of 2^49 bytes
+    auto place = [&](int tile, int &tn, int &tm, int &b) {
+        tn = tile % (int)P.tiles_n; tile /= (int)P.tiles_n;
+        tm = tile % (int)P.tiles_m;
+        b = tile / (int)P.tiles_m;
+    };
     const int nkb = (int)((P.D + BKB - 1) / BKB);
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int a = 0; a < 2; ++a) { mbar_init(&tmem_full[a], 1); mbar_init(&tmem_empty[a], kEpilogueWarps); }
+        for (int a = 0; a < 2; ++a) { mbar_init(&tmem_full[a], 1); mbar_init(&tmem_empty[a], 2 * kEpilogueWarps); }
         *abort_flag = 0;
         mbar_init_fence();
         tma_prefetch_descriptor(&map_x);
         tma_prefetch_descriptor(&map_y);
     }
-    if (warp == 1) {
-        tmem_alloc(tmem_ptr, kTmemCols);
-        tmem_relinquish();
-    }
+    if (warp == 1) tmem_alloc_pair(tmem_ptr, kTmemCols);
     tc_fence_before();
     __syncthreads();
+    cluster_sync();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr;
+    auto give_up = [&](int site) {
+        raise_abort_pair(abort_flag);
+        if (P.status) atomicCAS(P.status, 0, (10 << 16) | site);
+    };
 
     if (warp == 0) {
-        // ---------------- TMA producer ----------------
+        // ---------------- TMA producer: this CTA's rows of x1, its half of the x2 rows ----------------
         if (lane == 0) {
             uint32_t it = 0;
             bool ok = true;
-            for (long long tile = blockIdx.x; tile < P.tiles && ok; tile += gridDim.x) {
-                long long t = tile;
-                const long long tn = t % P.tiles_n; t /= P.tiles_n;
-                const long long tm = t % P.tiles_m;
-                const long long b = t / P.tiles_m;
+            for (int tile = pair; tile < tiles && ok; tile += pairs) {
+                int tn, tm, b;
+                place(tile, tn, tm, b);
                 for (int kb = 0; kb < nkb; ++kb, ++it) {
                     const int s = it % kStages;
                     const uint32_t use = it / kStages;
                     if (use > 0 && !wait_or_abort(&empty[s], (use - 1) & 1, abort_flag)) {
-                        *abort_flag = 1;
-                        if (P.status) atomicCAS(P.status, 0, (10 << 16) | 1);
+                        give_up(1);
                         ok = false;
                         break;
                     }
                     unsigned char *st = smem + s * STAGE_BYTES;
-                    mbar_expect_tx(&full[s], STAGE_BYTES);
-                    tma_load_3d(st, &map_x, &full[s], kb * BKB, (int)(tm * BM), (int)b);
-                    tma_load_3d(st + A_BYTES, &map_y, &full[s], kb * BKB, (int)(tn * BN), (int)b);
+                    const uint32_t bar = cluster_addr(&full[s], 0);
+                    if (rank == 0) mbar_expect_tx(&full[s], 2 * STAGE_BYTES);
+                    tma_load_3d_pair(st, &map_x, bar, kb * BKB, tm * 2 * BM + (int)rank * BM, b);
+                    tma_load_3d_pair(st + A_BYTES, &map_y, bar, kb * BKB, tn * BN + (int)rank * (BN / 2), b);
                 }
             }
+            // after a wait that gave up, stay (bounded) until the copies under way have landed in both CTAs
+            if (!ok && rank == 0)
+                for (uint32_t u = it > (uint32_t)kStages ? it - kStages : 0; u < it; ++u) mbar_wait_bounded(&full[u % kStages], (u / kStages) & 1);
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            const uint32_t idesc = make_idesc_i8(BM, BN);
+        // ---------------- MMA issuer: rank 0, for both ----------------
+        if (lane == 0 && rank == 0) {
+            const uint32_t idesc = make_idesc_i8(2 * BM, BN);
             uint32_t it = 0, acount = 0;
             bool ok = true;
-            for (long long tile = blockIdx.x; tile < P.tiles && ok; tile += gridDim.x, ++acount) {
+            for (int tile = pair; tile < tiles && ok; tile += pairs, ++acount) {
                 const uint32_t a = acount & 1, ause = acount >> 1;
-                if (ause > 0 && !wait_or_abort(&tmem_empty[a], (ause - 1) & 1, abort_flag)) {
-                    *abort_flag = 1;
-                    if (P.status) atomicCAS(P.status, 0, (10 << 16) | 2);
+                if (ause > 0 && !wait_or_abort<true>(&tmem_empty[a], (ause - 1) & 1, abort_flag)) {
+                    give_up(2);
                     ok = false;
                     break;
                 }
@@ -198,9 +209,8 @@ bool_count_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
                 const uint32_t d_tmem = tmem_base + a * BN;
                 for (int kb = 0; kb < nkb; ++kb, ++it) {
                     const int s = it % kStages;
-                    if (!wait_or_abort(&full[s], (it / kStages) & 1, abort_flag)) {
-                        *abort_flag = 1;
-                        if (P.status) atomicCAS(P.status, 0, (10 << 16) | 3);
+                    if (!wait_or_abort<true>(&full[s], (it / kStages) & 1, abort_flag)) {
+                        give_up(3);
                         ok = false;
                         break;
                     }
@@ -213,141 +223,118 @@ bool_count_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
 #pragma unroll
                     for (int k = 0; k < BKB / 32; ++k)
                         if (k < kmma) tc_mma_i8(d_tmem, dx + 2 * k, dy + 2 * k, idesc, (kb | k) != 0);
-                    tc_commit(&empty[s]);   // the stage may be refilled once these MMAs have read it
+                    tc_commit_pair(&empty[s]);   // the stage may be refilled, in both CTAs, once these MMAs have read it
                 }
-                if (ok) tc_commit(&tmem_full[a]);
+                if (ok) tc_commit_pair(&tmem_full[a]);
             }
         }
     } else {
         // ---------------- epilogue: warps 2..17 ----------------
         const int q = warp & 3;
-        const int cpart = (warp - 2) >> 2;           // which quarter of the tile's 256 columns
-        constexpr int NCB = BN / 32 / (kEpilogueWarps / 4);   // 32-column blocks per warp and tile
+        const int cq = (warp - 2) >> 2;              // which 16 of every 64 columns
+        constexpr int kPasses = BN / kStoreCols;
         uint32_t tcount = 0;
-        bool ok = true;
-        const int D = (int)P.D;
-        unsigned char *stg = smem + OFF_STAGE + (warp - 2) * 4096;
-        for (long long tile = blockIdx.x; tile < P.tiles && ok; tile += gridDim.x, ++tcount) {
-            long long t = tile;
-            const long long tn = t % P.tiles_n; t /= P.tiles_n;
-            const long long tm = t % P.tiles_m;
-            const long long b = t / P.tiles_m;
+        const int D = (int)P.D, N2 = (int)P.N2;
+        // metrics with a packed form, on counts small enough for it: the row counts are kept as floats
+        const bool packed = kPackedEpilogue<METRIC> && P.D < kQuotientMax;
+        float *stage = reinterpret_cast<float *>(smem + L::OFF_STAGE + q * (RAGGED ? 32 * BN * 4 : 2 * kStoreBuffer));
+        int32_t *popw = reinterpret_cast<int32_t *>(smem + L::OFF_POP + (warp - 2) * 256);
+        const uint32_t drained[2] = {cluster_addr(&tmem_empty[0], 0), cluster_addr(&tmem_empty[1], 0)};
+        for (int tile = pair; tile < tiles; tile += pairs, ++tcount) {
+            int tn, tm, b;
+            place(tile, tn, tm, b);
             const uint32_t a = tcount & 1;
             // What the epilogue needs besides the counts depends on the tile index alone: fetch it before waiting for the
             // accumulator, so that the L2 round trip hides behind the contraction instead of sitting in every column block.
-            const long long i = tm * BM + q * 32 + lane;
-            const bool row_ok = i < P.N1;
-            const int pa = row_ok ? __ldg(P.pop1 + b * P.N1 + i) : 0;
-            const int32_t *pb = P.pop2 + b * P.N2;
-            int32_t *popw = reinterpret_cast<int32_t *>(smem + OFF_POP + (warp - 2) * 256);
+            const int row_base = tm * 2 * BM + (int)rank * BM + q * 32;
+            const int rows = (int)P.N1 - row_base;      // of this quarter's block, if not all 32
+            const int pa = lane < rows ? __ldg(P.pop1 + b * P.N1 + row_base + lane) : 0;
             {
-                const long long jc = tn * BN + cpart * (NCB * 32) + lane * 2;   // 64 counts per warp: two per lane
+                // 64 counts per warp, two per lane: entry e is column 64 (e / 16) + 16 cq + e % 16
+                const int jc = tn * BN + (lane >> 3) * kStoreCols + cq * 16 + (lane & 7) * 2;
+                const int32_t *pb = P.pop2 + b * P.N2;
                 int2 v = make_int2(0, 0);
-                if (P.vec_store && jc + 2 <= P.N2) v = __ldg(reinterpret_cast<const int2 *>(pb + jc));
-                else {
-                    if (jc + 0 < P.N2) v.x = __ldg(pb + jc + 0);
-                    if (jc + 1 < P.N2) v.y = __ldg(pb + jc + 1);
-                }
+                if (jc < N2) v.x = __ldg(pb + jc);
+                if (jc + 1 < N2) v.y = __ldg(pb + jc + 1);
+                if (packed) v = make_int2(__float_as_int((float)v.x), __float_as_int((float)v.y));
                 __syncwarp();   // the previous tile's reads of this area are done
                 *reinterpret_cast<int2 *>(popw + lane * 2) = v;
-                __syncwarp();
             }
-            if (!wait_or_abort(&tmem_full[a], (tcount >> 1) & 1, abort_flag)) {
-                *abort_flag = 1;
-                if (lane == 0 && P.status) atomicCAS(P.status, 0, (10 << 16) | 4);
-                ok = false;
-                break;
-            }
+            const bool here = wait_or_abort(&tmem_full[a], (tcount >> 1) & 1, abort_flag);
+            if (!here && lane == 0) give_up(4);
+            if (!quarter_all(q, here)) break;            // all four warps of the quarter, or none: they meet at the stores' barriers
             tc_fence_after();
-            const long long row_base = tm * BM + q * 32;
+            float *out = P.out + (b * P.N1 + row_base) * P.N2 + tn * BN;
+            const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + a * BN + cq * 16;
+            const int cols = N2 - tn * BN, passes = cols < BN ? (cols + kStoreCols - 1) / kStoreCols : kPasses;
             // the mean metrics multiply by 1 / D where D is a power of two and divide otherwise: decided here, once per
             // tile, so that the per-element code holds one of the two
-            auto drain = [&](auto inv_tag, float inv_d) {
+            auto drain = [&](auto packed_tag, auto inv_tag, float inv_d) {
+                constexpr bool PACKED = decltype(packed_tag)::value;
                 constexpr int INV = decltype(inv_tag)::value;
 #pragma unroll 1
-            for (int c = cpart * NCB; c < (cpart + 1) * NCB; ++c) {
-                uint32_t r[32];
-                tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + a * BN + c * 32, r);
-                tmem_ld_wait();
-                const long long j0 = tn * BN + c * 32;
-                if (j0 >= P.N2) continue;
-                const bool whole = P.vec_store && j0 + 32 <= P.N2;
-                {
-                    // this thread's row (past N2 the counts are zero and nothing is stored) ...
-                    float4 o[8];
-#pragma unroll
-                    for (int v = 0; v < 8; ++v) {
-                        const int4 nb = *reinterpret_cast<const int4 *>(popw + (c - cpart * NCB) * 32 + 4 * v);
-                        o[v].x = bool_epilogue<true, INV>(METRIC, (int)r[4 * v + 0], pa, nb.x, D, inv_d);
-                        o[v].y = bool_epilogue<true, INV>(METRIC, (int)r[4 * v + 1], pa, nb.y, D, inv_d);
-                        o[v].z = bool_epilogue<true, INV>(METRIC, (int)r[4 * v + 2], pa, nb.z, D, inv_d);
-                        o[v].w = bool_epilogue<true, INV>(METRIC, (int)r[4 * v + 3], pa, nb.w, D, inv_d);
+                for (int p = 0; p < passes; ++p) {
+                    uint32_t r[16];
+                    tmem_ld16(acc + p * kStoreCols, r);
+                    tmem_ld_wait();
+                    if (p + 1 == passes) {
+                        // this warp has drained its part of accumulator `a`
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane == 0) mbar_arrive_cluster(drained[a]);
                     }
-                    if (P.tma_store) {
-                        // by now the copy engine has read the previous block out of the staging area
-                        if (lane == 0) tma_store_wait_read();
-                        __syncwarp();
+                    float o[16];
+#pragma unroll
+                    for (int v = 0; v < 4; ++v) {
+                        const int4 nb = *reinterpret_cast<const int4 *>(popw + p * 16 + 4 * v);
+                        if constexpr (PACKED) {
+                            const f32x2 a2 = pack2((float)pa, (float)pa);
+                            unpack2(bool_epilogue_packed<METRIC, INV>(r[4 * v], r[4 * v + 1], a2, pack2(__int_as_float(nb.x), __int_as_float(nb.y)),
+                                                                      (float)D, inv_d), o[4 * v], o[4 * v + 1]);
+                            unpack2(bool_epilogue_packed<METRIC, INV>(r[4 * v + 2], r[4 * v + 3], a2, pack2(__int_as_float(nb.z), __int_as_float(nb.w)),
+                                                                      (float)D, inv_d), o[4 * v + 2], o[4 * v + 3]);
+                        } else {
+                            o[4 * v + 0] = bool_epilogue<true, INV>(METRIC, (int)r[4 * v + 0], pa, nb.x, D, inv_d);
+                            o[4 * v + 1] = bool_epilogue<true, INV>(METRIC, (int)r[4 * v + 1], pa, nb.y, D, inv_d);
+                            o[4 * v + 2] = bool_epilogue<true, INV>(METRIC, (int)r[4 * v + 2], pa, nb.z, D, inv_d);
+                            o[4 * v + 3] = bool_epilogue<true, INV>(METRIC, (int)r[4 * v + 3], pa, nb.w, D, inv_d);
+                        }
                     }
-                    // ... staged with a 16-byte-chunk XOR swizzle ...
-#pragma unroll
-                    for (int v = 0; v < 8; ++v) *reinterpret_cast<float4 *>(stg + lane * 128 + ((v ^ (lane & 7)) << 4)) = o[v];
-                    if (whole && P.tma_store) {
-                        // ... which is the layout of a 128-byte swizzled 32 x 32 box: one lane hands the block to the copy
-                        // engine (rows past N1 are clipped by the tensor map) and the warp goes on to its next block
-                        fence_proxy_async_smem();
-                        __syncwarp();
-                        if (lane == 0) {
-                            tma_store_3d(&map_out, stg, (int)j0, (int)row_base, (int)b);
-                            tma_store_commit();
-                        }
-                    } else if (whole) {
-                        __syncwarp();
-                        // ... and written out four full 128-byte row segments per instruction
-#pragma unroll
-                        for (int itr = 0; itr < 8; ++itr) {
-                            const int rr = itr * 4 + (lane >> 3), cc = lane & 7;
-                            const float4 o = *reinterpret_cast<const float4 *>(stg + rr * 128 + ((cc ^ (rr & 7)) << 4));
-                            if (row_base + rr < P.N1)
-                                __stcs(reinterpret_cast<float4 *>(P.out + (b * P.N1 + row_base + rr) * P.N2 + j0) + cc, o);
-                        }
-                        __syncwarp();
+                    if constexpr (RAGGED) {
+                        stage_values<BN>(stage, o, p * kStoreCols + cq * 16, lane);
                     } else {
-                        __syncwarp();
-                        // ... and written out one row segment of up to 32 words per instruction
-                        const int rows = P.N1 - row_base < 32 ? (int)(P.N1 - row_base) : 32;
-                        float *op = P.out + (b * P.N1 + row_base) * P.N2 + j0 + lane;
-                        if (j0 + lane < P.N2) {
-#pragma unroll 8
-                            for (int rr = 0; rr < rows; ++rr)
-                                op[rr * P.N2] = *reinterpret_cast<const float *>(stg + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) + (lane & 3) * 4);
-                        }
-                        __syncwarp();
+                        // the vote ahead of the next tile keeps its first pass from a buffer that is still read
+                        float *buf = stage + (p & 1) * (32 * kStoreCols);
+                        stage_values<kStoreCols>(buf, o, cq * 16, lane);
+                        quarter_sync(q);
+                        store_rows<kStoreCols, true>(buf, out + p * kStoreCols, P.N2, rows, cols - p * kStoreCols, true, cq, lane);
                     }
                 }
-            }
+                if constexpr (RAGGED) {
+                    quarter_sync(q);
+                    store_rows<BN, true>(stage, out, P.N2, rows, cols, false, cq, lane);
+                }
             };
+            typedef std::integral_constant<bool, kPackedEpilogue<METRIC>> Packed;   // never taken where the metric has no such form
             if (METRIC == TPW_BOOL_EQ_MEAN || METRIC == TPW_BOOL_NE_MEAN) {
-                if (P.inv_d != 0.f) drain(std::integral_constant<int, 1>{}, P.inv_d);
-                else if (P.D < kQuotientMax) drain(std::integral_constant<int, 2>{}, approximate_reciprocal((float)P.D));
-                else drain(std::integral_constant<int, 0>{}, 0.f);
-            } else if (METRIC == TPW_BOOL_JACCARD && P.D < kQuotientMax) {
-                drain(std::integral_constant<int, 2>{}, 0.f);
+                if (packed && P.inv_d != 0.f) drain(Packed{}, std::integral_constant<int, 1>{}, P.inv_d);
+                else if (packed) drain(Packed{}, std::integral_constant<int, 2>{}, approximate_reciprocal((float)P.D));
+                else if (P.inv_d != 0.f) drain(std::false_type{}, std::integral_constant<int, 1>{}, P.inv_d);
+                else drain(std::false_type{}, std::integral_constant<int, 0>{}, 0.f);
+            } else if (packed) {
+                drain(Packed{}, std::integral_constant<int, 2>{}, 0.f);
             } else {
-                drain(std::integral_constant<int, -1>{}, P.inv_d);
+                drain(std::false_type{}, std::integral_constant<int, -1>{}, P.inv_d);
             }
-            // this warp has drained its part of accumulator `a`
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&tmem_empty[a]);
         }
     }
 
-    if (warp >= 2 && lane == 0 && P.tma_store) tma_store_wait_read();   // shared memory stays valid until the last block is read
     tc_fence_before();
     __syncthreads();
+    cluster_sync();   // neither CTA's shared memory goes while the other may still read it or arrive in it
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, kTmemCols);
+        tmem_dealloc_pair(tmem_base, kTmemCols);
     }
 }
 
@@ -420,37 +407,28 @@ extern "C" int tpw_bool_metric_forward_rows(int metric, const uint8_t *x1, const
     P.pop1 = x1_popcount; P.pop2 = x2_popcount; P.out = out;
     P.B = B; P.N1 = N1; P.N2 = N2; P.D = D;
     P.metric = metric;
-    P.vec_store = (N2 % 4 == 0 && aligned16(out) && aligned16(x2_popcount)) ? 1 : 0;
     P.inv_d = (D & (D - 1)) == 0 ? 1.0f / (float)D : 0.f;
-    P.tiles_m = (N1 + BM - 1) / BM;
+    P.tiles_m = (N1 + 2 * BM - 1) / (2 * BM);
     P.tiles_n = (N2 + BN - 1) / BN;
     P.tiles = B * P.tiles_m * P.tiles_n;
     P.status = device_status_ptr();
     CUtensorMap mx, my;
     int st = make_tensor_map_3d(&mx, x1, 1, pitch, N1, B, BKB, BM, true);
     if (st != TPW_OK) return st;
-    st = make_tensor_map_3d(&my, x2, 1, pitch, N2, B, BKB, BN, true);
+    st = make_tensor_map_3d(&my, x2, 1, pitch, N2, B, BKB, BN / 2, true);
     if (st != TPW_OK) return st;
-    CUtensorMap mo;
-    memset(&mo, 0, sizeof(mo));
-    // Metrics whose epilogue divides keep a warp busy long enough per block for the copy engine to drain the staging
-    // area behind it (jaccard at 65536 x 16384 x 1024: 2.06 -> 1.80 ms); for the sums and the power-of-two means the
-    // warp's own 128-bit stores are faster (hamming: 1.32 against 1.49 ms).  TPW_BOOL_TC_STORES=plain|tma overrides.
-    const bool cheap = metric == TPW_BOOL_AND_SUM || metric == TPW_BOOL_OR_SUM || metric == TPW_BOOL_XOR_SUM ||
-                       metric == TPW_BOOL_EQ_SUM || metric == TPW_BOOL_NE_SUM ||
-                       ((metric == TPW_BOOL_EQ_MEAN || metric == TPW_BOOL_NE_MEAN) && P.inv_d != 0.f);
-    const char *stores = getenv("TPW_BOOL_TC_STORES");
-    P.tma_store = P.vec_store && (stores ? stores[0] == 't' : !cheap) ? 1 : 0;
-    if (P.tma_store) {
-        st = make_tensor_map_3d(&mo, out, 4, N2, N1, B, 32, 32, true);
-        if (st != TPW_OK) return st;
-    }
     cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const long long grid = P.tiles < sm_count() ? P.tiles : sm_count();
+    const long long pairs = sm_count() / 2, grid = 2 * (P.tiles < pairs ? P.tiles : pairs);
+    const bool ragged = N2 % 4 != 0 || !aligned16(out);
+#define TPW_BOOL_TC_LAUNCH(M, RAGGED)                                                                                          \
+    do {                                                                                                                       \
+        auto kern = bool_count_tcgen05_kernel<M, RAGGED>;                                                                      \
+        TPW_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<RAGGED>::SMEM_ALLOC));      \
+        kern<<<(unsigned)grid, kThreads, Layout<RAGGED>::SMEM_ALLOC, s>>>(mx, my, P);                                          \
+    } while (0)
 #define TPW_BOOL_TC_CASE(M)                                                                                                    \
     case M:                                                                                                                    \
-        TPW_CUDA_OK(cudaFuncSetAttribute(bool_count_tcgen05_kernel<M>, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_ALLOC)); \
-        bool_count_tcgen05_kernel<M><<<(unsigned)grid, kThreads, SMEM_ALLOC, s>>>(mx, my, mo, P);                                  \
+        if (ragged) TPW_BOOL_TC_LAUNCH(M, true); else TPW_BOOL_TC_LAUNCH(M, false);                                            \
         break
     switch (metric) {
         TPW_BOOL_TC_CASE(TPW_BOOL_AND_SUM); TPW_BOOL_TC_CASE(TPW_BOOL_OR_SUM); TPW_BOOL_TC_CASE(TPW_BOOL_XOR_SUM);
@@ -462,6 +440,7 @@ extern "C" int tpw_bool_metric_forward_rows(int metric, const uint8_t *x1, const
         default: return fail(TPW_ERR_INVALID, "tpw_bool_metric_forward_tc: unknown metric %d", metric);
     }
 #undef TPW_BOOL_TC_CASE
+#undef TPW_BOOL_TC_LAUNCH
     TPW_LAUNCH_OK("bool_count_tcgen05_kernel");
     return TPW_OK;
 }

@@ -9,12 +9,17 @@
 // fp32 rounding of the sum).  Row norms are summed in fp32 from the unsplit values by the same
 // pre-pass.
 //
-// Kernel.  Persistent, one CTA per SM, 320 threads: warp 0 = TMA producer (one lane), warp 1 =
-// tensor-memory owner and MMA issuer (one lane), warps 2..9 = epilogue (each owns the 32 TMEM lanes
-// its warp id selects and one half of the columns).  Output tile 128 x 256; k-step 64 bf16 = one 128-byte swizzled row; a stage
-// holds xh, xl (2 x 16 KB) and yh, yl (2 x 32 KB); two stages.  The 512 TMEM columns hold two
-// 128 x 256 fp32 accumulators so the epilogue of tile t overlaps the MMAs of tile t + 1.
-// No cluster launch: every CTA fetches its own tiles, with plain per-CTA TMA loads, from this GPU's memory.
+// Kernel.  Persistent, one CTA per SM in pairs (clusters of two, cta_group::2), 576 threads: warp 0 = TMA producer (one lane),
+// warp 1 = tensor-memory owner and, in rank 0, MMA issuer for both CTAs (one lane), warps 2..17 = epilogue.  A pair's output
+// tile is 256 x 256, 128 rows to a CTA; k-step 64 bf16 = one 128-byte swizzled row.  The ring has five slots of 32 KB: the CTA's 128
+// rows of x and its half, 128 rows, of y, high and low parts in turn.  The 512 TMEM columns hold two 128 x 256 fp32
+// accumulators per CTA, so the epilogue of tile t overlaps the MMAs of tile t + 1.  Where the tile is stored all sixteen
+// epilogue warps drain it, four to a TMEM lane quarter, each 16 of every 64 columns; of the row-minimum and top-k epilogues
+// eight warps own each accumulator, two to a lane quarter, each half of the columns.
+// Why pairs: L2 -> SM traffic stands at 35 to 43 bytes a clock and SM whatever runs beside it.  A 128 x 256 tile per CTA takes 96 KB of
+// operands per 1536 tensor-core clocks; a pair takes 64 KB, which the tensor cores wait for no longer (sqeuclidean [16384, 16384,
+// 512] without its stores: 700 thousand clocks where the MMAs alone are 688), and less energy: under the power cap sqeuclidean [131072,
+// 16384, 512] 6.15 -> 5.55 ms.  Every CTA fetches its own rows, with plain TMA loads, from this GPU's memory.
 //
 // Three more instantiations share the pipeline: (1) kind::tf32 operands (high/low tf32 parts in fp32
 // containers, 32 elements per k-step) for the gradient products of the backward and for plain dot
@@ -29,6 +34,7 @@
 #include "common.cuh"
 #include "packed_f32x2.cuh"
 #include "tcgen05.cuh"
+#include "tile_store.cuh"
 
 #include <cuda_bf16.h>
 #include <math.h>
@@ -38,24 +44,27 @@
 namespace tpw {
 namespace {
 
-constexpr int BM = 128;           // rows of x1 per tile (TMEM lanes)
+constexpr int BM = 128;           // rows of x1 per CTA (TMEM lanes)
+constexpr int TM = 2 * BM;        // rows of x1 per tile of a pair
 constexpr int BN = 256;           // rows of x2 per tile (TMEM columns per accumulator)
+constexpr int HN = BN / 2;        // of which each CTA stages half
 constexpr int BK = 64;            // bf16 per k-step: 128 bytes
-constexpr int kStages = 2;
+constexpr int kSlots = 5;
 constexpr int kMmasPerStep = 4;    // a 128-byte operand row feeds four MMAs of 32 bytes (16 bf16 or 8 tf32) each
 constexpr int A_BYTES = BM * BK * 2;          // 16 KB
-constexpr int B_BYTES = BN * BK * 2;          // 32 KB
-constexpr int STAGE_BYTES = 2 * A_BYTES + 2 * B_BYTES; // xh | xl | yh | yl = 96 KB
-constexpr int OFF_BAR = kStages * STAGE_BYTES;
-// barriers: full_hi[2], full_lo[2], empty[2], tmem_full[2], tmem_empty[2]; then the TMEM base address and the abort flag
-constexpr int OFF_TMEM_PTR = OFF_BAR + 10 * 8;
+constexpr int B_BYTES = HN * BK * 2;          // 16 KB
+constexpr int SLOT_BYTES = A_BYTES + B_BYTES; // one part (high or low) of a k-step
+constexpr int OFF_BAR = kSlots * SLOT_BYTES;
+// barriers: full[5], empty[5], tmem_full[2], tmem_empty[2]; then the TMEM base address and the abort flag
+constexpr int OFF_TMEM_PTR = OFF_BAR + (2 * kSlots + 4) * 8;
 constexpr int OFF_ABORT = OFF_TMEM_PTR + 4;
-// per epilogue warp a 32 x 32 fp32 staging block (4 KB) used to turn "one row per thread" into
-// "eight lanes per 128-byte row segment" before the global stores
+// staging of the stored tiles (tile_store.cuh); the top-k epilogue keeps its keys there, 4 KB to a warp
 constexpr int OFF_STAGE = (OFF_ABORT + 4 + 127) / 128 * 128;
-constexpr int SMEM_BYTES = OFF_STAGE + 8 * 4096;
+constexpr int kEpilogueWarps = 16;
+constexpr int SMEM_BYTES = OFF_STAGE + kStoreBytes;
+static_assert(kStoreBytes >= kEpilogueWarps * 4096, "room for the top-k keys");
 constexpr int SMEM_ALLOC = SMEM_BYTES + 1024;
-constexpr int kEpilogueWarps = 8;             // two per TMEM lane quarter, each draining half of the columns
+static_assert(SMEM_ALLOC <= 232448, "exceeds the dynamic shared memory of one CTA");
 constexpr int kThreads = 64 + 32 * kEpilogueWarps;
 constexpr uint32_t kTmemCols = 512;
 
@@ -82,7 +91,7 @@ struct GemmParams {
     long long cols;
     const int *lo_any;        // [2] whether any low part of the x (y) operand is non-zero; NULL: treat both as non-zero
     int lo_always;            // bit 0 / 1: the x / y operand's low parts are used whatever lo_any says
-    float *partial;           // tf32: [grid][2][BM][BN] sums of the tiles that a CTA has only a part of (NULL: whole tiles only)
+    float *partial;           // tf32: [pair][2][TM][BN] sums of the tiles that a pair has only a part of (NULL: whole tiles only)
     int *status;
 };
 
@@ -94,14 +103,14 @@ __device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
+            "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
             ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
             : "memory");
     else
         asm volatile(
             "{\n\t.reg .pred p;\n\t"
             "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+            "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
             ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
             : "memory");
 }
@@ -119,11 +128,11 @@ __device__ __forceinline__ uint64_t make_smem_desc_mn(uint32_t smem_addr) {
     return d;
 }
 // Instruction descriptor: D = fp32 (bits [4,6) = 1); A and B formats in bits [7,10) and [10,13):
-// 1 = bf16 under kind::f16, 2 = tf32 under kind::tf32; bit 15 / bit 16 = 1 when A / B is MN-major
-// (0: K-major); N >> 3 in bits [17,23), M >> 4 in bits [24,29).
-__device__ __forceinline__ uint32_t make_idesc(int M, int N, bool tf32, bool a_mn = false, bool b_mn = false) {
+// 1 = bf16 under kind::f16, 2 = tf32 under kind::tf32; bit 15 = 1 when A is MN-major
+// (0: K-major; B is K-major, bit 16 = 0); N >> 3 in bits [17,23), M >> 4 in bits [24,29).
+__device__ __forceinline__ uint32_t make_idesc(int M, int N, bool tf32, bool a_mn) {
     const uint32_t fmt = tf32 ? 2u : 1u;
-    return (1u << 4) | (fmt << 7) | (fmt << 10) | ((a_mn ? 1u : 0u) << 15) | ((b_mn ? 1u : 0u) << 16) |
+    return (1u << 4) | (fmt << 7) | (fmt << 10) | ((a_mn ? 1u : 0u) << 15) |
            ((uint32_t)(N >> 3) << 17) | ((uint32_t)(M >> 4) << 24);
 }
 
@@ -139,6 +148,65 @@ __device__ __forceinline__ float dot_epilogue(float dot, float n1, float n2, boo
     const float dist = 1.f - s;
     if (EPI == TPW_DOT_COSINE_DIST) return fminf(fmaxf(dist, 0.f), 2.f);
     return dist;
+}
+
+// sqrt(x) for x >= 0, two at a time: one step of Newton's iteration for the square root from the approximate reciprocal square
+// root (relative error below 2^-22, so the step leaves only its own rounding: within one float32 of sqrtf).  The term added
+// under the root keeps it away from 1 / 0 and changes no x above 2^-100.  x has to be finite.
+__device__ __forceinline__ f32x2 newton_sqrt(f32x2 x) {
+    const f32x2 tiny = pack2(1.17549435e-38f, 1.17549435e-38f);
+    float a, b, ra, rb;
+    unpack2(add2(x, tiny), a, b);
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(ra) : "f"(a));
+    asm("rsqrt.approx.ftz.f32 %0, %1;" : "=f"(rb) : "f"(b));
+    const f32x2 r = pack2(ra, rb), root = mul2(x, r), half = mul2(r, pack2(0.5f, 0.5f));
+    return fma2(fma2(mul2(root, pack2(-1.f, -1.f)), root, x), half, root);
+}
+
+// dot_epilogue for 16 columns of one row, two lanes to an instruction (the same values, the root excepted as above).  With the
+// scalar form, 23 instructions per Euclidean distance, the epilogue and not the contraction was the bound: euclidean
+// [16, 4096, 4096, 256] forward 700 -> 445 us.
+template <int EPI>
+__device__ __forceinline__ void dot_epilogue16(const uint32_t (&dot)[16], float n1, const float (&n2)[16], float (&o)[16]) {
+    const f32x2 row = pack2(n1, n1);
+    f32x2 v[8];
+#pragma unroll
+    for (int u = 0; u < 8; ++u) {
+        const f32x2 d = pack2(__uint_as_float(dot[2 * u]), __uint_as_float(dot[2 * u + 1])), col = pack2(n2[2 * u], n2[2 * u + 1]);
+        if (EPI == TPW_DOT_LINEAR) v[u] = d;
+        else if (EPI == TPW_DOT_SQEUCLIDEAN || EPI == TPW_DOT_EUCLIDEAN) v[u] = fma2(d, pack2(-2.f, -2.f), add2(row, col));
+        else v[u] = mul2(d, mul2(row, col));
+        if (EPI == TPW_DOT_COSINE_DIST || EPI == TPW_DOT_ONE_MINUS_SIM) v[u] = sub2(pack2(1.f, 1.f), v[u]);
+        unpack2(v[u], o[2 * u], o[2 * u + 1]);
+    }
+    if (EPI == TPW_DOT_SQEUCLIDEAN || EPI == TPW_DOT_EUCLIDEAN) {
+#pragma unroll
+        for (int u = 0; u < 16; ++u) o[u] = fmaxf(o[u], 0.f);
+    }
+    if (EPI == TPW_DOT_COSINE_DIST) {
+#pragma unroll
+        for (int u = 0; u < 16; ++u) o[u] = fminf(fmaxf(o[u], 0.f), 2.f);
+    }
+    if (EPI == TPW_DOT_EUCLIDEAN) {
+        float m = 0.f;
+#pragma unroll
+        for (int u = 0; u < 8; ++u) m = max3_abs(m, o[2 * u], o[2 * u + 1]);
+        if (__any_sync(0xffffffffu, m > 3.402823466e+38f)) {   // an infinite distance somewhere in the warp
+#pragma unroll 1
+            for (int u = 0; u < 16; ++u) {
+                // one element per trip, picked by comparison: the registers have no index
+                float x = o[0];
+#pragma unroll
+                for (int w = 1; w < 16; ++w) x = w == u ? o[w] : x;
+                x = sqrtf(x);
+#pragma unroll
+                for (int w = 0; w < 16; ++w) o[w] = w == u ? x : o[w];
+            }
+        } else {
+#pragma unroll
+            for (int u = 0; u < 8; ++u) unpack2(newton_sqrt(pack2(o[2 * u], o[2 * u + 1])), o[2 * u], o[2 * u + 1]);
+        }
+    }
 }
 
 // dot_epilogue without the cosine distance's upper clamp, for the top-k epilogue: columns are ordered the same way as long as
@@ -184,55 +252,48 @@ __device__ __forceinline__ void sorted_insert(unsigned long long (&lst)[N], unsi
     lst[0] = key < lst[0] ? key : lst[0];
 }
 
-// A warp's staged 32 x 32 block (16-byte chunks XOR-swizzled by the row) to rows of `pitch` floats that need not be 16-byte
-// aligned: one row segment of up to 32 consecutive words per instruction.  (One row per thread, as it was before, touched
-// 32 rows with every store: cosine [5000, 4111, 768] in bfloat16, forward and backward, 803 -> 707 us.)
-__device__ __forceinline__ void store_block_ragged(const unsigned char *stg, float *dst, long long pitch, long long rows, long long cols,
-                                                   int lane) {
-    if (lane >= cols) return;
-    const int n = rows < 32 ? (int)rows : 32;
-#pragma unroll 8
-    for (int rr = 0; rr < n; ++rr)
-        dst[rr * pitch + lane] = *reinterpret_cast<const float *>(stg + rr * 128 + (((lane >> 2) ^ (rr & 7)) << 4) + (lane & 3) * 4);
-}
-
-// The largest of a lane's k keys (32 words apart) and its slot.  Not inlined: the top-k epilogue has four copies of its caller, and
-// few tile halves come here.
+// The k smallest of a lane's n >= k keys (32 words apart), moved to its first k places; returns the largest of them and its slot.
+// Not inlined: few tile halves come here.
 struct KeySlot {
     unsigned long long key;
     int slot;
 };
-__device__ __noinline__ KeySlot largest_key(const unsigned long long *buf, int k) {
+__device__ __noinline__ KeySlot keep_smallest(unsigned long long *buf, int n, int k) {
     KeySlot m{0, 0};
+    for (;; --n) {
+        m = {0, 0};
 #pragma unroll 1
-    for (int t = 0; t < k; t += 8) {   // eight loads under way together
-        unsigned long long held[8];
+        for (int t = 0; t < n; t += 8) {   // eight loads under way together
+            unsigned long long held[8];
 #pragma unroll
-        for (int u = 0; u < 8; ++u) held[u] = t + u < k ? buf[(t + u) * 32] : 0;
+            for (int u = 0; u < 8; ++u) held[u] = t + u < n ? buf[(t + u) * 32] : 0;
 #pragma unroll
-        for (int u = 0; u < 8; ++u)
-            if (t + u < k && held[u] >= m.key) m = {held[u], t + u};
+            for (int u = 0; u < 8; ++u)
+                if (t + u < n && held[u] >= m.key) m = {held[u], t + u};
+        }
+        if (n == k) return m;
+        buf[m.slot * 32] = buf[(n - 1) * 32];
     }
-    return m;
 }
 
-// The share of a product that falls to one CTA: whole tiles, every gridDim.x-th.  With a scratch for partial tiles (tf32) only
+// The share of a product that falls to one pair: whole tiles, every pairs-th.  With a scratch for partial tiles (tf32) only
 // the full waves go that way; the chunks of the tiles that are left over are dealt out evenly, and a tile cut by the end of
 // a share is finished by product_fixup_kernel.
 template <typename I>
 struct ProductShare {
     I tile_at, tile_last, base;   // whole tiles; first tile of those dealt out
     int stride, nch;
-    int at, last;                 // this CTA's chunks of the tiles dealt out
+    int at, last;                 // this pair's chunks of the tiles dealt out
     __device__ __forceinline__ ProductShare(const GemmParams &P, int nch_) {
         nch = nch_;
-        stride = (int)gridDim.x;
+        const int pair = (int)(blockIdx.x >> 1);
+        stride = (int)(gridDim.x >> 1);
         const long long left = P.partial ? P.tiles % stride : 0, all = left * nch;
         base = (I)(P.tiles - left);
-        tile_at = (I)blockIdx.x;
+        tile_at = (I)pair;
         tile_last = base;
-        at = (int)(all * blockIdx.x / stride);
-        last = (int)(all * (blockIdx.x + 1) / stride);
+        at = (int)(all * pair / stride);
+        last = (int)(all * (pair + 1) / stride);
     }
     // the next piece: chunks [c0, c1) of a tile
     __device__ __forceinline__ bool next(I &tile, int &c0, int &c1) {
@@ -252,34 +313,35 @@ struct ProductShare {
     }
 };
 
-// AMN / BMN (tf32 only): the operand is MN-major, i.e. its global rows run along k and each row holds
-// the tile's M (or N) values contiguously, so a matrix can be contracted over its row index without a
+// AMN (tf32 only): the x operand is MN-major, i.e. its global rows run along k and each row holds
+// the tile's M values contiguously, so a matrix can be contracted over its row index without a
 // transposed copy.  Such a tile is staged as blocks of {32 values, 32 k-rows} (one TMA box each, 4 KB,
 // 128-byte swizzle with 32-byte atoms): block m holds values 32m..32m+31, an MMA consumes 8 k-rows = 1024 bytes.
-template <int EPI, bool SELF, bool TF32, bool ROWMIN = false, bool AMN = false, bool BMN = false, int TOPK = 0>
-__global__ void __launch_bounds__(kThreads, 1)
+template <int EPI, bool SELF, bool TF32, bool ROWMIN = false, bool AMN = false, int TOPK = 0>
+__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
 gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_constant__ CUtensorMap map_xl,
                    const __grid_constant__ CUtensorMap map_yh, const __grid_constant__ CUtensorMap map_yl,
                    const GemmParams P) {
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    // a stage lands in two halves so that the xh.yh products can start while xl, yl are still in flight
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem + OFF_BAR);   // xh + yh of a stage
-    uint64_t *full_lo = full + kStages;                               // xl + yl of a stage
-    uint64_t *empty = full_lo + kStages;
-    uint64_t *tmem_full = empty + kStages;
-    uint64_t *tmem_empty = tmem_full + 2;
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + OFF_BAR);   // rank 0's: both CTAs' copies of a slot have landed
+    uint64_t *empty = full + kSlots;
+    uint64_t *tmem_full = empty + kSlots;
+    uint64_t *tmem_empty = tmem_full + 2;                             // rank 0's: both CTAs have drained the accumulator
     uint32_t *tmem_ptr = reinterpret_cast<uint32_t *>(smem + OFF_TMEM_PTR);
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(smem + OFF_ABORT);
+    int *abort_flag = reinterpret_cast<int *>(smem + OFF_ABORT);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+    const uint32_t rank = cluster_rank();
     constexpr int BKE = TF32 ? BK / 2 : BK; // operand elements per k-step
+    constexpr bool STORED = !ROWMIN && TOPK == 0;
+    constexpr int kDrains = STORED ? kEpilogueWarps : kEpilogueWarps / 2;   // warps of a CTA that drain one accumulator
     typedef std::conditional_t<TF32, int, long long> Index;   // a stored product has fewer than 2^31 tiles
     const int nkb = (int)((P.D + BKE - 1) / BKE);
 
     if (threadIdx.x == 0) {
-        for (int s = 0; s < kStages; ++s) { mbar_init(&full[s], 1); mbar_init(&full_lo[s], 1); mbar_init(&empty[s], 1); }
-        for (int a = 0; a < 2; ++a) { mbar_init(&tmem_full[a], 1); mbar_init(&tmem_empty[a], kEpilogueWarps); }
+        for (int s = 0; s < kSlots; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
+        for (int a = 0; a < 2; ++a) { mbar_init(&tmem_full[a], 1); mbar_init(&tmem_empty[a], 2 * kDrains); }
         *abort_flag = 0;
         mbar_init_fence();
         tma_prefetch_descriptor(&map_xh);
@@ -287,25 +349,27 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
         tma_prefetch_descriptor(&map_yh);
         tma_prefetch_descriptor(&map_yl);
     }
-    if (warp == 1) {
-        tmem_alloc(tmem_ptr, kTmemCols);
-        tmem_relinquish();
-    }
+    if (warp == 1) tmem_alloc_pair(tmem_ptr, kTmemCols);
     tc_fence_before();
     __syncthreads();
+    cluster_sync();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr;
+    auto give_up = [&](int site) {
+        raise_abort_pair(abort_flag);
+        if (P.status) atomicCAS(P.status, 0, (4 << 16) | site);
+    };
     // Operands that the high parts hold exactly (16-bit inputs, small integers) have no low parts: their tiles are neither
     // loaded nor multiplied.  The products left out are zeros added to a finished sum; an infinite or NaN input has a NaN low part.
     // cosine of bfloat16 [5000, 768] x [4111, 768], forward and backward: 707 -> 652 us.
     const bool need_xl = !P.lo_any || (P.lo_always & 1) || P.lo_any[0] != 0;
     const bool need_yl = !P.lo_any || (P.lo_always & 2) || P.lo_any[1] != 0;
-    const uint32_t lo_bytes = (need_xl ? A_BYTES : 0) + (need_yl ? B_BYTES : 0);
+    const int parts = need_xl || need_yl ? 2 : 1;   // slots per k-step
 
     if (warp == 0) {
-        // ---------------- TMA producer ----------------
+        // ---------------- TMA producer: this CTA's rows of x, its half of the rows of y ----------------
         if (lane == 0) {
-            uint32_t it = 0;
+            uint32_t s = 0, use = 0, issued = 0;     // slot, how often it has been filled before
             bool ok = true;
             const int kchunk = (P.kchunk > 0 && P.kchunk < nkb) ? P.kchunk : nkb;
             ProductShare<Index> share(P, (nkb + kchunk - 1) / kchunk);
@@ -313,109 +377,99 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
             for (int c0, c1; ok && share.next(tile, c0, c1);) {
                 long long tn, tm, b;
                 decode_tile<TOPK != 0>(tile, P, tn, tm, b);
+                const int row = (int)(tm * TM) + (int)rank * BM, col = (int)(tn * BN) + (int)rank * HN;
                 const int kend = c1 * kchunk < nkb ? c1 * kchunk : nkb;
-                for (int kb = c0 * kchunk; kb < kend; ++kb, ++it) {
-                    const int s = it % kStages;
-                    const uint32_t use = it / kStages;
-                    if (use > 0 && !wait_or_abort(&empty[s], (use - 1) & 1, abort_flag)) {
-                        *abort_flag = 1;
-                        if (P.status) atomicCAS(P.status, 0, (4 << 16) | 1);
-                        ok = false;
-                        break;
-                    }
-                    unsigned char *st = smem + s * STAGE_BYTES;
-                    static_assert(TF32 || !(AMN || BMN), "MN-major staging is laid out for 32-bit operands");
-                    mbar_expect_tx(&full[s], A_BYTES + B_BYTES);
-                    if constexpr (AMN) {
+                for (int kb = c0 * kchunk; kb < kend && ok; ++kb) {
+                    for (int part = 0; part < parts; ++part) {
+                        if (use > 0 && !wait_or_abort(&empty[s], (use - 1) & 1, abort_flag)) {
+                            give_up(1);
+                            ok = false;
+                            break;
+                        }
+                        unsigned char *st = smem + s * SLOT_BYTES;
+                        const uint32_t bar = cluster_addr(&full[s], 0);
+                        const bool load_x = part == 0 || need_xl, load_y = part == 0 || need_yl;
+                        if (rank == 0) mbar_expect_tx(&full[s], 2 * ((load_x ? A_BYTES : 0) + (load_y ? B_BYTES : 0)));
+                        static_assert(TF32 || !AMN, "MN-major staging is laid out for 32-bit operands");
+                        if (load_x) {
+                            const CUtensorMap *map = part == 0 ? &map_xh : &map_xl;
+                            if constexpr (AMN) {
 #pragma unroll
-                        for (int m = 0; m < BM / 32; ++m)
-                            tma_load_3d(st + m * 4096, &map_xh, &full[s], (int)(tm * BM) + 32 * m, kb * BKE, (int)b);
-                    } else {
-                        tma_load_3d(st, &map_xh, &full[s], kb * BKE, (int)(tm * BM), (int)b);
-                    }
-                    if constexpr (BMN) {
-#pragma unroll
-                        for (int m = 0; m < BN / 32; ++m)
-                            tma_load_3d(st + 2 * A_BYTES + m * 4096, &map_yh, &full[s], (int)(tn * BN) + 32 * m, kb * BKE, (int)b);
-                    } else {
-                        tma_load_3d(st + 2 * A_BYTES, &map_yh, &full[s], kb * BKE, (int)(tn * BN), (int)b);
-                    }
-                    if (lo_bytes == 0) continue;
-                    mbar_expect_tx(&full_lo[s], lo_bytes);
-                    if (!need_xl) {
-                    } else if constexpr (AMN) {
-#pragma unroll
-                        for (int m = 0; m < BM / 32; ++m)
-                            tma_load_3d(st + A_BYTES + m * 4096, &map_xl, &full_lo[s], (int)(tm * BM) + 32 * m, kb * BKE, (int)b);
-                    } else {
-                        tma_load_3d(st + A_BYTES, &map_xl, &full_lo[s], kb * BKE, (int)(tm * BM), (int)b);
-                    }
-                    if (!need_yl) {
-                    } else if constexpr (BMN) {
-#pragma unroll
-                        for (int m = 0; m < BN / 32; ++m)
-                            tma_load_3d(st + 2 * A_BYTES + B_BYTES + m * 4096, &map_yl, &full_lo[s], (int)(tn * BN) + 32 * m, kb * BKE, (int)b);
-                    } else {
-                        tma_load_3d(st + 2 * A_BYTES + B_BYTES, &map_yl, &full_lo[s], kb * BKE, (int)(tn * BN), (int)b);
+                                for (int m = 0; m < BM / 32; ++m) tma_load_3d_pair(st + m * 4096, map, bar, row + 32 * m, kb * BKE, (int)b);
+                            } else {
+                                tma_load_3d_pair(st, map, bar, kb * BKE, row, (int)b);
+                            }
+                        }
+                        if (load_y) tma_load_3d_pair(st + A_BYTES, part == 0 ? &map_yh : &map_yl, bar, kb * BKE, col, (int)b);
+                        ++issued;
+                        if (++s == kSlots) { s = 0; ++use; }
                     }
                 }
             }
+            // after a wait that gave up, stay (bounded) until the copies under way have landed in both CTAs
+            if (!ok && rank == 0)
+                for (uint32_t u = issued > (uint32_t)kSlots ? issued - kSlots : 0; u < issued; ++u) mbar_wait_bounded(&full[u % kSlots], (u / kSlots) & 1);
         }
     } else if (warp == 1) {
-        // ---------------- MMA issuer ----------------
-        if (lane == 0) {
-            const uint32_t idesc = make_idesc(BM, BN, TF32, AMN, BMN);
-            uint32_t it = 0, acount = 0;
+        // ---------------- MMA issuer: rank 0, for both CTAs ----------------
+        if (lane == 0 && rank == 0) {
+            const uint32_t idesc = make_idesc(TM, BN, TF32, AMN);
+            uint32_t s = 0, phase = 0, acount = 0;
             bool ok = true;
             const int kchunk = (P.kchunk > 0 && P.kchunk < nkb) ? P.kchunk : nkb;
             ProductShare<Index> share(P, (nkb + kchunk - 1) / kchunk);
             Index tile;
+            auto arrived = [&](int site) {
+                if (!wait_or_abort<true>(&full[s], phase, abort_flag)) {
+                    give_up(site);
+                    return false;
+                }
+                tc_fence_after();
+                return true;
+            };
+            auto x_desc = [&](uint32_t slot) {
+                const uint32_t at = smem_u32(smem + slot * SLOT_BYTES);
+                return AMN ? make_smem_desc_mn(at) : make_smem_desc(at);
+            };
+            auto y_desc = [&](uint32_t slot) { return make_smem_desc(smem_u32(smem + slot * SLOT_BYTES + A_BYTES)); };
             for (int c0, c1; ok && share.next(tile, c0, c1);) {
                 // one accumulator per chunk of k-steps: the tensor cores add into tensor memory with
                 // truncation, so long reductions are cut into chunks that the epilogue sums in registers
                 const int kend = c1 * kchunk < nkb ? c1 * kchunk : nkb;
                 for (int kb0 = c0 * kchunk; kb0 < kend && ok; kb0 += kchunk, ++acount) {
                     const uint32_t a = acount & 1, ause = acount >> 1;
-                    if (ause > 0 && !wait_or_abort(&tmem_empty[a], (ause - 1) & 1, abort_flag)) {
-                        *abort_flag = 1;
-                        if (P.status) atomicCAS(P.status, 0, (4 << 16) | 2);
+                    if (ause > 0 && !wait_or_abort<true>(&tmem_empty[a], (ause - 1) & 1, abort_flag)) {
+                        give_up(2);
                         ok = false;
                         break;
                     }
                     tc_fence_after();
                     const uint32_t d_tmem = tmem_base + a * BN;
                     const int kb1 = kb0 + kchunk < nkb ? kb0 + kchunk : nkb;
-                    for (int kb = kb0; kb < kb1; ++kb, ++it) {
-                        const int s = it % kStages;
-                        if (!wait_or_abort(&full[s], (it / kStages) & 1, abort_flag)) {
-                            *abort_flag = 1;
-                            if (P.status) atomicCAS(P.status, 0, (4 << 16) | 3);
+                    for (int kb = kb0; kb < kb1; ++kb) {
+                        if (!arrived(3)) {
                             ok = false;
                             break;
                         }
-                        tc_fence_after();
-                        const uint32_t sb = smem_u32(smem + s * STAGE_BYTES);
-                        const uint64_t dxh = AMN ? make_smem_desc_mn(sb) : make_smem_desc(sb);
-                        const uint64_t dxl = AMN ? make_smem_desc_mn(sb + A_BYTES) : make_smem_desc(sb + A_BYTES);
-                        const uint64_t dyh = BMN ? make_smem_desc_mn(sb + 2 * A_BYTES) : make_smem_desc(sb + 2 * A_BYTES);
-                        const uint64_t dyl = BMN ? make_smem_desc_mn(sb + 2 * A_BYTES + B_BYTES) : make_smem_desc(sb + 2 * A_BYTES + B_BYTES);
+                        const uint32_t hi = s;
+                        const uint64_t dxh = x_desc(hi), dyh = y_desc(hi);
                         // K-major: one MMA consumes 32 bytes of the swizzled row (16 bf16 or 8 tf32), so the start
                         // address advances by 2 units of 16 bytes; MN-major: 8 k-rows = 1024 bytes = 64 units
-                        constexpr uint64_t ka = AMN ? 64 : 2, kbn = BMN ? 64 : 2;
+                        constexpr uint64_t ka = AMN ? 64 : 2, kbn = 2;
 #pragma unroll
                         for (int k = 0; k < kMmasPerStep; ++k)
                             tc_mma<TF32>(d_tmem, dxh + ka * k, dyh + kbn * k, idesc, ((kb - kb0) | k) != 0);
-                        if (lo_bytes == 0) {
-                            tc_commit(&empty[s]);
+                        if (++s == kSlots) { s = 0; phase ^= 1; }
+                        if (parts == 1) {
+                            tc_commit_pair(&empty[hi]);
                             continue;
                         }
-                        if (!wait_or_abort(&full_lo[s], (it / kStages) & 1, abort_flag)) {
-                            *abort_flag = 1;
-                            if (P.status) atomicCAS(P.status, 0, (4 << 16) | 5);
+                        if (!arrived(5)) {
                             ok = false;
                             break;
                         }
-                        tc_fence_after();
+                        const uint32_t lo = s;
+                        const uint64_t dxl = x_desc(lo), dyl = y_desc(lo);
                         if (need_xl && need_yl) {
 #pragma unroll
                             for (int k = 0; k < kMmasPerStep; ++k) {
@@ -427,167 +481,299 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
 #pragma unroll
                             for (int k = 0; k < kMmasPerStep; ++k) tc_mma<TF32>(d_tmem, da + ka * k, db + kbn * k, idesc, 1);
                         }
-                        tc_commit(&empty[s]); // the stage may be refilled once these MMAs have read it
+                        tc_commit_pair(&empty[hi]); // both slots may be refilled, in both CTAs, once these MMAs have read them
+                        tc_commit_pair(&empty[lo]);
+                        if (++s == kSlots) { s = 0; phase ^= 1; }
                     }
-                    if (ok) tc_commit(&tmem_full[a]);
+                    if (ok) tc_commit_pair(&tmem_full[a]);
                 }
             }
         }
     } else {
-        // ---------------- epilogue: warps 2..9, TMEM lanes 32*(warp % 4) .. +31, column half (warp-2)/4 ----------------
+        // ---------------- epilogue: warps 2..17, TMEM lanes 32*(warp % 4) .. +31 ----------------
         const int q = warp & 3;
-        const int chalf = (warp - 2) >> 2;
+        const uint32_t drained[2] = {cluster_addr(&tmem_empty[0], 0), cluster_addr(&tmem_empty[1], 0)};
         uint32_t tcount = 0;
         bool ok = true;
-        if constexpr (TF32) {
-            // Chunked reduction (plain products only): every chunk's accumulator is added, rounded to
-            // nearest, into 128 register-resident sums per thread; the tile is stored after its last chunk.
-            static_assert(!TF32 || EPI == TPW_DOT_LINEAR, "the tf32 pipeline serves the plain products");
-            const int kchunk = (P.kchunk > 0 && P.kchunk < nkb) ? P.kchunk : nkb;
-            const int nchunks = (nkb + kchunk - 1) / kchunk;
-            uint32_t acount = 0;
-            ProductShare<Index> share(P, nchunks);
-            const int start = share.at;
-            Index tile;
-            for (int c0, c1; ok && share.next(tile, c0, c1);) {
-                long long t = tile;
-                const long long tn = t % P.tiles_n; t /= P.tiles_n;
-                const long long tm = t % P.tiles_m;
-                const long long b = t / P.tiles_m;
-                float sums[BN / 2];
+        auto release = [&](uint32_t a) {   // this warp has drained its part of accumulator a
+            tc_fence_before();
+            __syncwarp();
+            if (lane == 0) mbar_arrive_cluster(drained[a]);
+        };
+        auto ready = [&](uint32_t a, uint32_t parity, int site) {
+            const bool here = wait_or_abort(&tmem_full[a], parity, abort_flag);
+            if (!here && lane == 0) give_up(site);
+            tc_fence_after();
+            return here;
+        };
+        const long long pairs = gridDim.x >> 1;
+        if constexpr (STORED) {
+            const int cq = (warp - 2) >> 2;              // which 16 of every 64 columns
+            float *stage = reinterpret_cast<float *>(smem + OFF_STAGE + q * 2 * kStoreBuffer);
+            const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16);
+            if constexpr (TF32) {
+                // Chunked reduction (plain products only): every chunk's accumulator is added, rounded to
+                // nearest, into 64 register-resident sums per thread; the tile is stored after its last chunk.
+                static_assert(!TF32 || EPI == TPW_DOT_LINEAR, "the tf32 pipeline serves the plain products");
+                const int kchunk = (P.kchunk > 0 && P.kchunk < nkb) ? P.kchunk : nkb;
+                const int nchunks = (nkb + kchunk - 1) / kchunk;
+                uint32_t acount = 0;
+                ProductShare<Index> share(P, nchunks);
+                const int start = share.at;
+                Index tile;
+                for (int c0, c1; ok && share.next(tile, c0, c1);) {
+                    long long t = tile;
+                    const long long tn = t % P.tiles_n; t /= P.tiles_n;
+                    const long long tm = t % P.tiles_m;
+                    const long long b = t / P.tiles_m;
+                    float sums[BN / kStoreCols][16];
 #pragma unroll
-                for (int v = 0; v < BN / 2; ++v) sums[v] = 0.f;
-                for (int ch = c0; ch < c1 && ok; ++ch, ++acount) {
-                    const uint32_t a = acount & 1;
-                    if (!wait_or_abort(&tmem_full[a], (acount >> 1) & 1, abort_flag)) {
-                        *abort_flag = 1;
-                        if (lane == 0 && P.status) atomicCAS(P.status, 0, (4 << 16) | 6);
-                        ok = false;
-                        break;
+                    for (int p = 0; p < BN / kStoreCols; ++p)
+#pragma unroll
+                        for (int v = 0; v < 16; ++v) sums[p][v] = 0.f;
+                    for (int ch = c0; ch < c1; ++ch, ++acount) {
+                        const uint32_t a = acount & 1;
+                        ok = ready(a, (acount >> 1) & 1, 6);
+                        if (!ok) break;
+#pragma unroll
+                        for (int p = 0; p < BN / kStoreCols; p += 2) {   // two loads under way: 64 sums leave few registers
+                            uint32_t r0[16], r1[16];
+                            tmem_ld16(acc + a * BN + p * kStoreCols + cq * 16, r0);
+                            tmem_ld16(acc + a * BN + (p + 1) * kStoreCols + cq * 16, r1);
+                            tmem_ld_wait();
+#pragma unroll
+                            for (int v = 0; v < 16; ++v) sums[p][v] += __uint_as_float(r0[v]);
+#pragma unroll
+                            for (int v = 0; v < 16; ++v) sums[p + 1][v] += __uint_as_float(r1[v]);
+                        }
+                        release(a);
                     }
-                    tc_fence_after();
+                    // all four warps of the lane quarter go on, or none: they meet at the barriers of the stores
+                    ok = quarter_all(q, ok);
+                    if (!ok) break;
+                    const long long row_base = tm * TM + rank * BM + q * 32;
+                    const bool part = c1 - c0 < nchunks;
+                    // a share holds at most two parts of tiles, one at its start and one at its end
+                    const long long slot = (long long)(blockIdx.x >> 1) * 2 + ((tile - share.base) * nchunks + c0 == start ? 0 : 1);
+                    float *dst = part ? P.partial + (slot * TM + rank * BM + q * 32) * BN : P.out + (b * P.N1 + row_base) * P.N2 + tn * BN;
+                    const long long pitch = part ? BN : P.N2;
+                    const int rows = row_base < P.N1 ? (int)(P.N1 - row_base) : 0, cols = P.N2 - tn * BN < BN ? (int)(P.N2 - tn * BN) : BN;
 #pragma unroll
-                    for (int c = 0; c < BN / 32; ++c) {   // sixteen columns at a time: 128 sums leave few registers
-                        uint32_t r[16];
-                        tmem_ld16(tmem_base + ((uint32_t)(q * 32) << 16) + a * BN + chalf * (BN / 2) + c * 16, r);
-                        tmem_ld_wait();
-#pragma unroll
-                        for (int v = 0; v < 16; ++v) sums[c * 16 + v] += __uint_as_float(r[v]);
+                    for (int p = 0; p < BN / kStoreCols; ++p) {
+                        if (p * kStoreCols >= cols) continue;
+                        float *buf = stage + (p & 1) * (32 * kStoreCols);
+                        stage_values<kStoreCols>(buf, sums[p], cq * 16, lane);
+                        quarter_sync(q);
+                        // a part is stored in whole 64-column segments and finished by product_fixup_kernel
+                        store_rows<kStoreCols, false>(buf, dst + p * kStoreCols, pitch, part ? 32 : rows, part ? kStoreCols : cols - p * kStoreCols,
+                                                      part || P.vec_store, cq, lane);
                     }
-                    tc_fence_before();
-                    __syncwarp();
-                    if (lane == 0) mbar_arrive(&tmem_empty[a]);
                 }
-                if (!ok) break;
-                unsigned char *stg = smem + OFF_STAGE + (warp - 2) * 4096;
-                const long long row_base = tm * BM + q * 32;
-                const bool part = c1 - c0 < nchunks;
-                // a share holds at most two parts of tiles, one at its start and one at its end
-                float *pdst = P.partial + ((long long)blockIdx.x * 2 + ((tile - share.base) * nchunks + c0 == start ? 0 : 1)) * (BM * BN);
+            } else {
+                for (long long tile = blockIdx.x >> 1; tile < P.tiles; tile += pairs, ++tcount) {
+                    long long tn, tm, b;
+                    decode_tile<false>(tile, P, tn, tm, b);
+                    const uint32_t a = tcount & 1;
+                    // the row's norm depends on the tile index alone: fetched before the wait
+                    const long long row_base = tm * TM + rank * BM + q * 32, i = row_base + lane;
+                    const float n1 = (EPI != TPW_DOT_LINEAR && i < P.N1) ? P.n1sq[b * P.N1 + i] : 0.f;
+                    // all four warps of the lane quarter go on, or none: they meet at the barriers of the stores
+                    if (!quarter_all(q, ready(a, (tcount >> 1) & 1, 4))) break;
+                    const int rows = row_base < P.N1 ? (int)(P.N1 - row_base < 32 ? P.N1 - row_base : 32) : 0;
+                    const int cols = P.N2 - tn * BN < BN ? (int)(P.N2 - tn * BN) : BN, passes = (cols + kStoreCols - 1) / kStoreCols;
+                    const float *n2p = P.n2sq + b * P.N2 + tn * BN;
+                    float *out = P.out + (b * P.N1 + row_base) * P.N2 + tn * BN;
+                    // this thread's 16 columns from col (a multiple of 16) on
+                    auto columns = [&](int col, bool last, float (&o)[16]) {
+                        const int left = cols - col;
+                        float n2[16];
+                        if (EPI != TPW_DOT_LINEAR) {
+                            if (P.vec_store && left >= 16) {
 #pragma unroll
-                for (int c = 0; c < BN / 64; ++c) {
-                    const int col = (chalf * (BN / 64) + c) * 32;
-                    const long long j0 = tn * BN + col;
-                    if (j0 >= P.N2) continue;
+                                for (int v = 0; v < 4; ++v) {
+                                    const float4 t = __ldg(reinterpret_cast<const float4 *>(n2p + col) + v);
+                                    n2[4 * v] = t.x; n2[4 * v + 1] = t.y; n2[4 * v + 2] = t.z; n2[4 * v + 3] = t.w;
+                                }
+                            } else {
 #pragma unroll
-                    for (int v = 0; v < 8; ++v)
-                        *reinterpret_cast<float4 *>(stg + lane * 128 + ((v ^ (lane & 7)) << 4)) =
-                            make_float4(sums[c * 32 + 4 * v], sums[c * 32 + 4 * v + 1], sums[c * 32 + 4 * v + 2], sums[c * 32 + 4 * v + 3]);
-                    __syncwarp();
-                    if (part || (P.vec_store && j0 + 32 <= P.N2)) {
-                        float *dst = part ? pdst + q * 32 * BN + col : P.out + (b * P.N1 + row_base) * P.N2 + j0;
-                        const long long pitch = part ? BN : P.N2;
+                                for (int v = 0; v < 16; ++v) n2[v] = v < left ? __ldg(n2p + col + v) : 0.f;
+                            }
+                        }
+                        uint32_t r[16];
+                        tmem_ld16(acc + a * BN + col, r);
+                        tmem_ld_wait();
+                        if (last) release(a);
+                        dot_epilogue16<EPI>(r, n1, n2, o);
+                        if constexpr (SELF) {
+                            const long long j0 = tn * BN + col;
+                            if (row_base < j0 + 16 && j0 < row_base + 32) {
 #pragma unroll
-                        for (int it = 0; it < 8; ++it) {
-                            const int rr = it * 4 + (lane >> 3), cc = lane & 7;
-                            const float4 o = *reinterpret_cast<const float4 *>(stg + rr * 128 + ((cc ^ (rr & 7)) << 4));
-                            if (row_base + rr < P.N1) reinterpret_cast<float4 *>(dst + rr * pitch)[cc] = o;
+                                for (int v = 0; v < 16; ++v)
+                                    if (i == j0 + v) o[v] = 0.f;
+                            }
+                        }
+                    };
+                    if (P.vec_store) {
+#pragma unroll 1
+                        for (int p = 0; p < passes; ++p) {
+                            float o[16];
+                            columns(p * kStoreCols + cq * 16, p + 1 == passes, o);
+                            float *buf = stage + (p & 1) * (32 * kStoreCols);
+                            stage_values<kStoreCols>(buf, o, cq * 16, lane);
+                            quarter_sync(q);
+                            store_rows<kStoreCols, false>(buf, out + p * kStoreCols, P.N2, rows, cols - p * kStoreCols, true, cq, lane);
                         }
                     } else {
-                        store_block_ragged(stg, P.out + (b * P.N1 + row_base) * P.N2 + j0, P.N2, P.N1 - row_base, P.N2 - j0, lane);
+                        constexpr int kWide = 2 * kStoreCols;   // both buffers as one
+#pragma unroll 1
+                        for (int p = 0; p < passes; ++p) {
+                            float o[16];
+                            columns(p * kStoreCols + cq * 16, p + 1 == passes, o);
+                            stage_values<kWide>(stage, o, (p & 1) * kStoreCols + cq * 16, lane);
+                            if ((p & 1) == 0 && p + 1 < passes) continue;
+                            const int first = (p & ~1) * kStoreCols;
+                            quarter_sync(q);
+                            store_rows<kWide, false>(stage, out + first, P.N2, rows, cols - first, false, cq, lane);
+                            quarter_sync(q);
+                        }
                     }
-                    __syncwarp();
                 }
             }
-        } else
-        for (long long tile = blockIdx.x; tile < P.tiles && ok; tile += gridDim.x, ++tcount) {
-            long long tn, tm, b;
-            decode_tile<TOPK != 0>(tile, P, tn, tm, b);
-            const uint32_t a = tcount & 1;
-            if (!wait_or_abort(&tmem_full[a], (tcount >> 1) & 1, abort_flag)) {
-                *abort_flag = 1;
-                if (lane == 0 && P.status) atomicCAS(P.status, 0, (4 << 16) | 4);
-                ok = false;
-                break;
-            }
-            tc_fence_after();
-            const long long i = tm * BM + q * 32 + lane;
-            const bool row_ok = i < P.N1;
-            const float n1 = (EPI != TPW_DOT_LINEAR && row_ok) ? P.n1sq[b * P.N1 + i] : 0.f;
-            const float *n2p = P.n2sq + b * P.N2;
-            unsigned long long best = ~0ull;
-            // TOPK > 0: keys at or above the bound of the row's k-th smallest key cannot be among its k smallest
-            unsigned long long bound = 0;
-            if constexpr (TOPK > 0) {
-                // rows past N1: nothing passes; any value read while other tiles lower it is a bound
-                if (row_ok) bound = *reinterpret_cast<volatile unsigned long long *>(P.topk_thr + b * P.N1 + i);
-            }
-            if constexpr (TOPK != 0) {
-                // Columns past the last count as NaN, which no minimum takes and no comparison passes.  TOPK < 0 keeps the minimum
-                // of every group of columns.  TOPK > 0: the minimum of eight distances decides for all of them whether any lane of the
-                // warp has one within its limit; then every lane puts its next passing column into its own words of the
-                // staging area, until none has one left (most tile halves have none or one a lane), and once a lane
-                // holds k keys the largest gives way to a smaller one.
-                const int k = P.topk_k;
-                const long long cols = TOPK < 0 ? P.cols : P.N2;
-                unsigned long long *buf = reinterpret_cast<unsigned long long *>(smem + OFF_STAGE + (warp - 2) * 4096) + lane;   // [k][32 lanes]
-                int cnt = 0, worst = 0;                       // keys held, slot of the largest once there are k
-                unsigned long long limit = bound;             // keys have to stay below it
-                auto limit_value = [&]() {                    // every distance whose key is below the limit is at most this
-                    const uint32_t hi = (uint32_t)(limit >> 32);
-                    // a limit at or above the upper clamp lets every raw value through
-                    return hi >= 0x7f800000u || (EPI == TPW_DOT_COSINE_DIST && hi >= 0x40000000u) ? INFINITY : __uint_as_float(hi);
-                };
-                float lim = limit_value();
-                float gm[16];                                 // TOPK < 0: minima of the half's columns of every residue modulo 16
-#pragma unroll
-                for (int t = 0; t < 16; ++t) gm[t] = INFINITY;
+        } else {
+            // warps 2..9 own the even accumulators, warps 10..17 the odd ones; each drains half of the columns
+            const int chalf = ((warp - 2) >> 2) & 1;
+            const uint32_t a = (uint32_t)(warp - 2) >> 3;
+            const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16) + a * BN + chalf * (BN / 2);
+            constexpr int kLast = BN / 64 - 1;
+            for (long long tile = (long long)(blockIdx.x >> 1) + a * pairs; tile < P.tiles; tile += 2 * pairs, ++tcount) {
+                long long tn, tm, b;
+                decode_tile<TOPK != 0>(tile, P, tn, tm, b);
+                const long long i = tm * TM + rank * BM + q * 32 + lane;
+                const bool row_ok = i < P.N1;
+                const float n1 = row_ok ? P.n1sq[b * P.N1 + i] : 0.f;
+                const float *n2p = P.n2sq + b * P.N2;
+                const long long col0 = tn * BN + chalf * (BN / 2);
+                if (!ready(a, tcount & 1, 4)) break;
+                if constexpr (ROWMIN) {
+                    // streaming row minimum: this thread owns row i and folds its columns into one key
+                    // (the epilogue value is non-negative, so its bit pattern orders like an unsigned integer)
+                    unsigned long long best = ~0ull;
 #pragma unroll 1
-                for (int c = chalf * (BN / 64); c < (chalf + 1) * (BN / 64); ++c) {
-                    const long long j0 = tn * BN + c * 32;
-                    if (j0 < cols) {
+                    for (int c = 0; c <= kLast; ++c) {
+                        const long long j0 = col0 + c * 32;
                         uint32_t r[32];
-                        tmem_ld32(tmem_base + ((uint32_t)(q * 32) << 16) + a * BN + c * 32, r);
+                        tmem_ld32(acc + c * 32, r);
                         tmem_ld_wait();
+                        if (c == kLast) release(a);
+                        if (j0 >= P.N2) continue;
+#pragma unroll
+                        for (int v = 0; v < 32; ++v) {
+                            const long long j = j0 + v;
+                            const float nn = j < P.N2 ? __ldg(n2p + j) : 0.f;
+                            const float o = dot_epilogue<EPI>(__uint_as_float(r[v]), n1, nn, false);
+                            const unsigned long long key = ((unsigned long long)__float_as_uint(o) << 32) | (unsigned long long)(uint32_t)j;
+                            if (j < P.N2 && key < best) best = key;
+                        }
+                    }
+                    if (row_ok && best != ~0ull) atomicMin(P.rowmin_keys + b * P.N1 + i, best);
+                }
+                if constexpr (TOPK != 0) {
+                    // Columns past the last count as NaN, which no minimum takes and no comparison passes.  TOPK < 0 keeps the minimum
+                    // of every group of columns.  TOPK > 0: the minimum of eight distances decides for all of them whether any lane of the
+                    // warp has one within its limit; if so, every lane appends its passing columns to its own words of the
+                    // staging area, eight predicated stores without a loop.  Room for 16 keys a lane: a lane that holds more than 8
+                    // (a row whose bound is loose) sends the warp's next groups through the loop below, which keeps the k smallest.
+                    // (One passing column per trip of such a loop for every group: 10 nearest of [50000, 20000, 128], the pass over all
+                    // columns 1.07 -> 0.95 ms; without any candidates it takes 0.45.)
+                    const int k = P.topk_k;
+                    const long long cols = TOPK < 0 ? P.cols : P.N2;
+                    unsigned long long *buf = reinterpret_cast<unsigned long long *>(smem + OFF_STAGE + (warp - 2) * 4096) + lane;   // [16][32 lanes]
+                    float *norms = reinterpret_cast<float *>(smem + OFF_STAGE + (warp - 2) * 4096);                                  // TOPK < 0: [128]
+                    int cnt = 0;                                  // keys held
+                    // keys have to stay below the bound of the row's k-th smallest; any value read while other tiles lower it is one
+                    unsigned long long limit = 0;
+                    if constexpr (TOPK > 0) {
+                        if (row_ok) limit = *reinterpret_cast<volatile unsigned long long *>(P.topk_thr + b * P.N1 + i);
+                    }
+                    auto limit_value = [&]() {                    // every distance whose key is below the limit is at most this
+                        const uint32_t hi = (uint32_t)(limit >> 32);
+                        // a limit at or above the upper clamp lets every raw value through
+                        return hi >= 0x7f800000u || (EPI == TPW_DOT_COSINE_DIST && hi >= 0x40000000u) ? INFINITY : __uint_as_float(hi);
+                    };
+                    float lim = row_ok ? limit_value() : -1.f;    // rows past N1: nothing passes
+                    float gm[16];                                 // TOPK < 0: minima of the half's columns of every residue modulo 16
+#pragma unroll
+                    for (int t = 0; t < 16; ++t) gm[t] = INFINITY;
+                    if constexpr (TOPK < 0) {
+                        // the sampled rows' norms lie apart: fetched once per tile half (NaN past the last column)
+                        __syncwarp();
+#pragma unroll
+                        for (int t = 0; t < 4; ++t) {
+                            const long long j = col0 + t * 32 + lane;
+                            norms[t * 32 + lane] = j < cols ? __ldg(n2p + j * P.col_step) : NAN;
+                        }
+                        __syncwarp();
+                    }
+#pragma unroll 1
+                    for (int c = 0; c <= kLast; ++c) {
+                        const long long j0 = col0 + c * 32;
+                        uint32_t r[32];
+                        tmem_ld32(acc + c * 32, r);
+                        tmem_ld_wait();
+                        if (c == kLast) release(a);
+                        if (j0 >= cols) continue;
                         const bool whole = TOPK > 0 && P.vec_store && j0 + 32 <= cols;
 #pragma unroll
                         for (int g = 0; g < 4; ++g) {
                             float nn[8], o[8];
-                            if (whole) {
+                            if (whole || TOPK < 0) {
 #pragma unroll
                                 for (int u = 0; u < 2; ++u) {
-                                    const float4 v4 = __ldg(reinterpret_cast<const float4 *>(n2p + j0 + 8 * g) + u);
+                                    const float4 v4 = TOPK < 0 ? reinterpret_cast<const float4 *>(norms + c * 32 + 8 * g)[u]
+                                                               : __ldg(reinterpret_cast<const float4 *>(n2p + j0 + 8 * g) + u);
                                     nn[4 * u] = v4.x; nn[4 * u + 1] = v4.y; nn[4 * u + 2] = v4.z; nn[4 * u + 3] = v4.w;
                                 }
                             } else {
 #pragma unroll
-                                for (int v = 0; v < 8; ++v)
-                                    nn[v] = j0 + 8 * g + v < cols ? __ldg(n2p + (j0 + 8 * g + v) * (TOPK < 0 ? P.col_step : 1)) : 0.f;
+                                for (int v = 0; v < 8; ++v) nn[v] = j0 + 8 * g + v < cols ? __ldg(n2p + (j0 + 8 * g + v)) : 0.f;
                             }
 #pragma unroll
                             for (int v = 0; v < 8; ++v) {
                                 o[v] = raw_distance<EPI>(__uint_as_float(r[8 * g + v]), n1, nn[v]);
-                                if (!whole && j0 + 8 * g + v >= cols) o[v] = NAN;
+                                if (TOPK < 0 ? isnan(nn[v]) : !whole && j0 + 8 * g + v >= cols) o[v] = NAN;
                             }
-                            const float m = min3(min3(o[0], o[1], o[2]), min3(o[3], o[4], o[5]), fminf(o[6], o[7]));
                             if constexpr (TOPK < 0) {
 #pragma unroll
                                 for (int v = 0; v < 8; ++v) gm[(g & 1) * 8 + v] = fminf(gm[(g & 1) * 8 + v], o[v]);
-                            } else if (__any_sync(0xffffffffu, m <= lim)) {
+                            } else {
+                                const float m = min3(min3(o[0], o[1], o[2]), min3(o[3], o[4], o[5]), fminf(o[6], o[7]));
+                                if (!__any_sync(0xffffffffu, m <= lim)) continue;
+                                if (__all_sync(0xffffffffu, cnt <= 8)) {
+                                    uint32_t at = smem_u32(buf) + cnt * 256;
+#pragma unroll
+                                    for (int v = 0; v < 8; ++v)
+                                        if (o[v] <= lim) {
+                                            asm volatile("st.shared.v2.b32 [%0], {%1, %2};" ::"r"(at), "r"((uint32_t)(j0 + 8 * g + v)),
+                                                         "r"(__float_as_uint(clamp_distance<EPI>(o[v])))
+                                                         : "memory");
+                                            at += 256;
+                                        }
+                                    cnt = (at - smem_u32(buf)) >> 8;
+                                    continue;
+                                }
                                 uint32_t mask = 0;
 #pragma unroll
                                 for (int v = 0; v < 8; ++v)
                                     if (o[v] <= lim) mask |= 1u << v;
+                                int worst = 0;
+                                auto shrink = [&]() {
+                                    const KeySlot last = keep_smallest(buf, cnt, k);
+                                    cnt = k;
+                                    limit = last.key;
+                                    worst = last.slot;
+                                    lim = limit_value();
+                                };
+                                if (cnt >= k) shrink();
 #pragma unroll 1
                                 while (__any_sync(0xffffffffu, mask != 0)) {
                                     const int v = __ffs(mask) - 1;       // -1: nothing left in this lane
@@ -598,140 +784,69 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                                         if (v == u) ov = o[u];
                                     const unsigned long long key = ((unsigned long long)__float_as_uint(clamp_distance<EPI>(ov)) << 32) |
                                                                    (unsigned long long)(uint32_t)(j0 + 8 * g + v);
-                                    const bool take = v >= 0 && key < limit;
-                                    if (take) buf[(cnt < k ? cnt : worst) * 32] = key;
-                                    if (take && ++cnt >= k) {
-                                        cnt = k;
-                                        const KeySlot last = largest_key(buf, k);
-                                        limit = last.key;
-                                        worst = last.slot;
-                                        lim = limit_value();
-                                    }
+                                    if (v < 0 || key >= limit) continue;
+                                    buf[(cnt < k ? cnt : worst) * 32] = key;
+                                    if (cnt < k) ++cnt;
+                                    if (cnt == k) shrink();
                                 }
                             }
                         }
                     }
-                }
-                if constexpr (TOPK < 0) {
+                    if constexpr (TOPK < 0) {
 #pragma unroll
-                    for (int t = 0; t < 16; ++t) gm[t] = clamp_distance<EPI>(gm[t]);
-                    const long long at = ((b * P.N1 + i) * P.tiles_n + tn) * 2 + chalf;
-                    float4 *dst = reinterpret_cast<float4 *>(P.gmin) + (P.col_group == 8 ? at * 4 : at);
-                    if (!row_ok) {
-                    } else if (P.col_group == 8) {
+                        for (int t = 0; t < 16; ++t) gm[t] = clamp_distance<EPI>(gm[t]);
+                        const long long at = ((b * P.N1 + i) * P.tiles_n + tn) * 2 + chalf;
+                        float4 *dst = reinterpret_cast<float4 *>(P.gmin) + (P.col_group == 8 ? at * 4 : at);
+                        if (!row_ok) {
+                        } else if (P.col_group == 8) {
 #pragma unroll
-                        for (int t = 0; t < 4; ++t) dst[t] = make_float4(gm[4 * t], gm[4 * t + 1], gm[4 * t + 2], gm[4 * t + 3]);
-                    } else {
-                        auto least = [&](int t) { return fminf(min3(gm[t], gm[t + 4], gm[t + 8]), gm[t + 12]); };
-                        dst[0] = make_float4(least(0), least(1), least(2), least(3));
-                    }
-                }
-                if constexpr (TOPK > 0) {
-                    // behind the keys that other tile halves have written (their order does not matter: the keys are unique
-                    // and the merge looks at all of them)
-                    if (cnt == k) atomicMin(P.topk_thr + b * P.N1 + i, limit);   // k keys up to it, which are written here
-                    if (cnt > 0) {
-                        const int at = atomicAdd(P.topk_count + b * P.N1 + i, cnt);
-                        unsigned long long *dst = P.topk_lists + (b * P.N1 + i) * P.topk_L * k + at;
-#pragma unroll 1
-                        for (int t = 0; t < cnt; ++t) dst[t] = buf[t * 32];
-                    }
-                    __syncwarp();
-                }
-            } else
-#pragma unroll 1
-            for (int c = chalf * (BN / 64); c < (chalf + 1) * (BN / 64); ++c) {
-                uint32_t r[32];
-                const uint32_t taddr = tmem_base + ((uint32_t)(q * 32) << 16) + a * BN + c * 32;
-                tmem_ld32(taddr, r);
-                tmem_ld_wait();
-                const long long j0 = tn * BN + c * 32;
-                if (j0 >= P.N2) continue;
-                if constexpr (ROWMIN) {
-                    // streaming row minimum: this thread owns row i and folds its 32 columns into one key
-                    // (the epilogue value is non-negative, so its bit pattern orders like an unsigned integer)
-#pragma unroll
-                    for (int v = 0; v < 32; ++v) {
-                        const long long j = j0 + v;
-                        const float nn = j < P.N2 ? __ldg(n2p + j) : 0.f;
-                        const float o = dot_epilogue<EPI>(__uint_as_float(r[v]), n1, nn, false);
-                        const unsigned long long key = ((unsigned long long)__float_as_uint(o) << 32) | (unsigned long long)(uint32_t)j;
-                        if (j < P.N2 && key < best) best = key;
-                    }
-                    continue;
-                }
-                // epilogue math on this thread's row, staged with a 16-byte-chunk XOR swizzle ...
-                unsigned char *stg = smem + OFF_STAGE + (warp - 2) * 4096;
-                const long long row_base = tm * BM + q * 32;
-                const bool whole = P.vec_store && j0 + 32 <= P.N2;
-                auto stage = [&](auto whole_tag) {
-                    constexpr bool WHOLE = decltype(whole_tag)::value;
-#pragma unroll
-                    for (int v = 0; v < 8; ++v) {
-                        float4 nn = make_float4(0.f, 0.f, 0.f, 0.f);
-                        if (EPI != TPW_DOT_LINEAR) {
-                            if (WHOLE) {
-                                nn = __ldg(reinterpret_cast<const float4 *>(n2p + j0) + v);
-                            } else {
-                                if (j0 + 4 * v + 0 < P.N2) nn.x = __ldg(n2p + j0 + 4 * v + 0);
-                                if (j0 + 4 * v + 1 < P.N2) nn.y = __ldg(n2p + j0 + 4 * v + 1);
-                                if (j0 + 4 * v + 2 < P.N2) nn.z = __ldg(n2p + j0 + 4 * v + 2);
-                                if (j0 + 4 * v + 3 < P.N2) nn.w = __ldg(n2p + j0 + 4 * v + 3);
-                            }
+                            for (int t = 0; t < 4; ++t) dst[t] = make_float4(gm[4 * t], gm[4 * t + 1], gm[4 * t + 2], gm[4 * t + 3]);
+                        } else {
+                            auto least = [&](int t) { return fminf(min3(gm[t], gm[t + 4], gm[t + 8]), gm[t + 12]); };
+                            dst[0] = make_float4(least(0), least(1), least(2), least(3));
                         }
-                        float4 o;
-                        o.x = dot_epilogue<EPI>(__uint_as_float(r[4 * v + 0]), n1, nn.x, SELF && i == j0 + 4 * v + 0);
-                        o.y = dot_epilogue<EPI>(__uint_as_float(r[4 * v + 1]), n1, nn.y, SELF && i == j0 + 4 * v + 1);
-                        o.z = dot_epilogue<EPI>(__uint_as_float(r[4 * v + 2]), n1, nn.z, SELF && i == j0 + 4 * v + 2);
-                        o.w = dot_epilogue<EPI>(__uint_as_float(r[4 * v + 3]), n1, nn.w, SELF && i == j0 + 4 * v + 3);
-                        *reinterpret_cast<float4 *>(stg + lane * 128 + ((v ^ (lane & 7)) << 4)) = o;
                     }
-                };
-                if (whole) stage(std::true_type{}); else stage(std::false_type{});
-                __syncwarp();
-                if (whole) {
-                    // ... and written out four full 128-byte row segments per instruction
-#pragma unroll
-                    for (int it = 0; it < 8; ++it) {
-                        const int rr = it * 4 + (lane >> 3), cc = lane & 7;
-                        const float4 o = *reinterpret_cast<const float4 *>(stg + rr * 128 + ((cc ^ (rr & 7)) << 4));
-                        if (row_base + rr < P.N1)
-                            reinterpret_cast<float4 *>(P.out + (b * P.N1 + row_base + rr) * P.N2 + j0)[cc] = o;
+                    if constexpr (TOPK > 0) {
+                        if (cnt >= k) {
+                            limit = keep_smallest(buf, cnt, k).key;
+                            cnt = k;
+                            atomicMin(P.topk_thr + b * P.N1 + i, limit);   // k keys up to it, which are written here
+                        }
+                        // behind the keys that other tile halves have written (their order does not matter: the keys are unique
+                        // and the merge looks at all of them)
+                        if (cnt > 0) {
+                            const int at = atomicAdd(P.topk_count + b * P.N1 + i, cnt);
+                            unsigned long long *dst = P.topk_lists + (b * P.N1 + i) * P.topk_L * k + at;
+#pragma unroll 1
+                            for (int t = 0; t < cnt; ++t) dst[t] = buf[t * 32];
+                        }
+                        __syncwarp();
                     }
-                } else {
-                    store_block_ragged(stg, P.out + (b * P.N1 + row_base) * P.N2 + j0, P.N2, P.N1 - row_base, P.N2 - j0, lane);
                 }
-                __syncwarp();
             }
-            if constexpr (ROWMIN) {
-                if (row_ok && best != ~0ull) atomicMin(P.rowmin_keys + b * P.N1 + i, best);
-            }
-            // this warp has drained its quarter of accumulator `a`
-            tc_fence_before();
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&tmem_empty[a]);
         }
     }
 
     tc_fence_before();
     __syncthreads();
+    cluster_sync();   // neither CTA's shared memory goes while the other may still read it or arrive in it
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc(tmem_base, kTmemCols);
+        tmem_dealloc_pair(tmem_base, kTmemCols);
     }
 }
 
-// Tiles whose chunks several CTAs share: the parts' sums, added in the order of the chunks.  One CTA per 16 rows of a tile.
+// Tiles whose chunks several pairs share: the parts' sums, added in the order of the chunks.  One CTA per 16 rows of a tile.
 __global__ void __launch_bounds__(BN)
-product_fixup_kernel(const GemmParams P, int nch, long long ctas) {
-    const long long left = P.tiles % ctas, base = P.tiles - left, local = blockIdx.x / (BM / 16), tile = base + local;
-    const int row0 = (int)(blockIdx.x % (BM / 16)) * 16, col = threadIdx.x;
+product_fixup_kernel(const GemmParams P, int nch, long long pairs) {
+    const long long left = P.tiles % pairs, base = P.tiles - left, local = blockIdx.x / (TM / 16), tile = base + local;
+    const int row0 = (int)(blockIdx.x % (TM / 16)) * 16, col = threadIdx.x;
     const long long all = left * nch, u0 = local * nch, u1 = u0 + nch;
-    auto start_of = [&](long long c) { return all * c / ctas; };
-    long long c = u0 * ctas / all;                  // the share that holds chunk u0, up to rounding
+    auto start_of = [&](long long c) { return all * c / pairs; };
+    long long c = u0 * pairs / all;                 // the share that holds chunk u0, up to rounding
     while (c > 0 && start_of(c) > u0) --c;
     while (start_of(c + 1) <= u0) ++c;
-    if (start_of(c + 1) >= u1) return;              // one CTA had the whole tile
+    if (start_of(c + 1) >= u1) return;              // one pair had the whole tile
     long long t = tile;
     const long long tn = t % P.tiles_n; t /= P.tiles_n;
     const long long tm = t % P.tiles_m;
@@ -741,16 +856,16 @@ product_fixup_kernel(const GemmParams P, int nch, long long ctas) {
     float s[16];
 #pragma unroll
     for (int r = 0; r < 16; ++r) s[r] = 0.f;
-    for (; c < ctas && start_of(c) < u1; ++c) {
-        if (start_of(c + 1) == start_of(c)) continue;   // fewer chunks than CTAs: an empty share
-        const float *src = P.partial + (c * 2 + (start_of(c) >= u0 ? 0 : 1)) * (BM * BN) + row0 * BN + col;
+    for (; c < pairs && start_of(c) < u1; ++c) {
+        if (start_of(c + 1) == start_of(c)) continue;   // fewer chunks than pairs: an empty share
+        const float *src = P.partial + (c * 2 + (start_of(c) >= u0 ? 0 : 1)) * (TM * BN) + row0 * BN + col;
 #pragma unroll
         for (int r = 0; r < 16; ++r)
-            if (tm * BM + row0 + r < P.N1) s[r] += src[r * BN];
+            if (tm * TM + row0 + r < P.N1) s[r] += src[r * BN];
     }
 #pragma unroll
     for (int r = 0; r < 16; ++r) {
-        const long long i = tm * BM + row0 + r;
+        const long long i = tm * TM + row0 + r;
         if (i < P.N1) P.out[(b * P.N1 + i) * P.N2 + j] = s[r];
     }
 }
@@ -871,7 +986,6 @@ struct SplitParams {
     const float *a, *aux;       // [B,R,C]
     const float *n1, *n2;       // COEF_COSINE: row norms [B,R], [B,C]
     float *hi, *lo;             // [B,R,Cp]   (STRAIGHT)
-    int *lo_any;                // set to 1 where some low part is not zero; may be NULL
     int *clear;                 // four words to set to 0 for the launches that follow; may be NULL
     float *rowpart, *colpart;   // [B,TC,R], [B,TR,C]   (SUMS)
     long long R, C, Cp, TR, TC;
@@ -929,7 +1043,6 @@ split_tile_kernel(const SplitParams P) {
             if (col + e < P.C) nb[e] = P.n2[b * P.C + col + e];
     }
     float colp[4] = {0.f, 0.f, 0.f, 0.f};
-    uint32_t any = 0;
 #pragma unroll
     for (int r = 0; r < 4; ++r) {
         const long long row = r0 + ty + 16 * r;
@@ -969,7 +1082,6 @@ split_tile_kernel(const SplitParams P) {
             h.w = rn_tf32(v[3]); l.w = rn_tf32(v[3] - h.w);
             *reinterpret_cast<float4 *>(P.hi + (b * P.R + row) * P.Cp + col) = h;
             *reinterpret_cast<float4 *>(P.lo + (b * P.R + row) * P.Cp + col) = l;
-            if (!SUMS) any |= (__float_as_uint(l.x) | __float_as_uint(l.y) | __float_as_uint(l.z) | __float_as_uint(l.w)) & 0x7fffffffu;
         }
         if (SUMS) {
             float s = (rs[0] + rs[1]) + (rs[2] + rs[3]);
@@ -978,9 +1090,7 @@ split_tile_kernel(const SplitParams P) {
             if (tx == 0 && row < P.R) P.rowpart[(b * P.TC + blockIdx.x) * P.R + row] = s;
         }
     }
-    if constexpr (!SUMS) {
-        if (P.lo_any && __syncthreads_or(any != 0) && tid == 0) *P.lo_any = 1;
-    } else {
+    if constexpr (SUMS) {
 #pragma unroll
         for (int e = 0; e < 4; ++e) colacc[ty * PT + 4 * tx + e] = colp[e];
         __syncthreads();
@@ -991,6 +1101,53 @@ split_tile_kernel(const SplitParams P) {
             P.colpart[(b * P.TR + blockIdx.y) * P.C + c0 + tid] = s;
         }
     }
+}
+
+// tf32 high/low copies of a matrix's transpose, [B,C,Rp]: rows of the copy run along the source's row index, zero filled to Rp.
+// The product's other operand then lies K-major, staged by one copy of 128 rows instead of four of {32 values, 32 rows}: C^T x1 of
+// [16, 4096, 4096, 256] 620 -> 570 us.  (The products' bound is the copies' latency: with neither MMAs nor epilogue they take as long.)
+__global__ void __launch_bounds__(256)
+split_transposed_kernel(const float *__restrict__ src, float *__restrict__ hi, float *__restrict__ lo, int *lo_any,
+                        long long R, long long C, long long Rp, int vec_in) {
+    __shared__ float tile[PT][PT + 1];
+    const int tid = threadIdx.x;
+    const long long b = blockIdx.z, r0 = (long long)blockIdx.y * PT, c0 = (long long)blockIdx.x * PT;
+    const float *a = src + b * R * C;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int r = u * 16 + (tid >> 4), c = (tid & 15) * 4;
+        const long long row = r0 + r, col = c0 + c;
+        float v[4] = {0.f, 0.f, 0.f, 0.f};
+        if (row < R) {
+            if (vec_in && col + 3 < C) {
+                const float4 t = *reinterpret_cast<const float4 *>(a + row * C + col);
+                v[0] = t.x; v[1] = t.y; v[2] = t.z; v[3] = t.w;
+            } else {
+#pragma unroll
+                for (int e = 0; e < 4; ++e)
+                    if (col + e < C) v[e] = a[row * C + col + e];
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < 4; ++e) tile[c + e][r] = v[e];
+    }
+    __syncthreads();
+    uint32_t any = 0;
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+        const int c = u * 16 + (tid >> 4), r = (tid & 15) * 4;
+        const long long col = c0 + c, row = r0 + r;
+        if (col >= C || row >= Rp) continue;
+        float4 h, l;
+        h.x = rn_tf32(tile[c][r]); l.x = rn_tf32(tile[c][r] - h.x);
+        h.y = rn_tf32(tile[c][r + 1]); l.y = rn_tf32(tile[c][r + 1] - h.y);
+        h.z = rn_tf32(tile[c][r + 2]); l.z = rn_tf32(tile[c][r + 2] - h.z);
+        h.w = rn_tf32(tile[c][r + 3]); l.w = rn_tf32(tile[c][r + 3] - h.w);
+        *reinterpret_cast<float4 *>(hi + (b * C + col) * Rp + row) = h;
+        *reinterpret_cast<float4 *>(lo + (b * C + col) * Rp + row) = l;
+        any |= (__float_as_uint(l.x) | __float_as_uint(l.y) | __float_as_uint(l.z) | __float_as_uint(l.w)) & 0x7fffffffu;
+    }
+    if (__syncthreads_or(any != 0) && tid == 0) *lo_any = 1;
 }
 
 // sums[b,n] = part[b,0,n] + part[b,1,n] + ... in that order (deterministic)
@@ -1019,23 +1176,24 @@ __global__ void grad_finish_kernel(float *__restrict__ g, const float *__restric
 // tiles scatters the CTAs over batches whose operands do not fit L2 together: 660 -> 880 us a product of euclidean
 // [16, 4096, 4096, 256].)  cosine bfloat16 [5000, 4111, 768], both products: 302 -> 277 us; euclidean [2, 1500, 1100, 192]: 100 -> 50 us.
 constexpr int kProductChunk = 2;               // k-steps of 32
-constexpr long long kPartialBytes = 2ll * BM * BN * 4;
+constexpr long long kPartialBytes = 2ll * TM * BN * 4;   // per pair
+inline long long pair_count() { return sm_count() / 2; }
 inline long long product_chunks(long long K) { return ((K + BK / 2 - 1) / (BK / 2) + kProductChunk - 1) / kProductChunk; }
-inline long long product_tiles(long long B, long long M, long long N) { return B * ((M + BM - 1) / BM) * ((N + BN - 1) / BN); }
+inline long long product_tiles(long long B, long long M, long long N) { return B * ((M + TM - 1) / TM) * ((N + BN - 1) / BN); }
 inline bool deals_chunks(long long B, long long M, long long N, long long K) {
-    const long long tiles = product_tiles(B, M, N), nsm = sm_count(), left = tiles % nsm;
+    const long long tiles = product_tiles(B, M, N), pairs = pair_count(), left = tiles % pairs;
     // one wave more or less in a long queue, or a tile of a few chunks, is not worth the second kernel
-    return tiles <= 8 * nsm && product_chunks(K) >= 16 && product_chunks(K) < (1 << 20) && left > 0 && left * 100 < nsm * 92;
+    return tiles <= 8 * pairs && product_chunks(K) >= 16 && product_chunks(K) < (1 << 20) && left > 0 && left * 100 < pairs * 92;
 }
-inline long long product_ctas(long long B, long long M, long long N, long long K, bool room) {
-    const long long tiles = product_tiles(B, M, N), nsm = sm_count();
-    if (tiles >= nsm) return nsm;
+inline long long product_pairs(long long B, long long M, long long N, long long K, bool room) {
+    const long long tiles = product_tiles(B, M, N), pairs = pair_count();
+    if (tiles >= pairs) return pairs;
     const long long most = room && deals_chunks(B, M, N, K) ? tiles * product_chunks(K) / 4 : tiles;
-    return most < nsm ? (most > tiles ? most : tiles) : nsm;
+    return most < pairs ? (most > tiles ? most : tiles) : pairs;
 }
 
 struct BwdScratch {
-    long long N2p, Dp, TR, TC;
+    long long N1p, N2p, TR, TC;
     long long off_chi, off_clo, off_x1hi, off_x1lo, off_x2hi, off_x2lo;
     long long off_rowpart, off_colpart, off_rowsum, off_colsum, off_lo, total;
     long long off_part, with_part;   // partial tiles of the products, where they are worth it (with_part == total: not)
@@ -1044,17 +1202,17 @@ struct BwdScratch {
 inline BwdScratch bwd_scratch_layout(long long B, long long N1, long long N2, long long D) {
     BwdScratch L;
     L.N2p = align_up(N2, 4);
-    L.Dp = align_up(D, 4);
+    L.N1p = align_up(N1, 4);
     L.TR = (N1 + PT - 1) / PT;
     L.TC = (N2 + PT - 1) / PT;
     long long off = 0;
     auto take = [&](long long bytes) { const long long o = off; off += align_up(bytes, 1024); return o; };
     L.off_chi = take(B * N1 * L.N2p * 4);
     L.off_clo = take(B * N1 * L.N2p * 4);
-    L.off_x1hi = take(B * N1 * L.Dp * 4);
-    L.off_x1lo = take(B * N1 * L.Dp * 4);
-    L.off_x2hi = take(B * N2 * L.Dp * 4);
-    L.off_x2lo = take(B * N2 * L.Dp * 4);
+    L.off_x1hi = take(B * D * L.N1p * 4);
+    L.off_x1lo = take(B * D * L.N1p * 4);
+    L.off_x2hi = take(B * D * L.N2p * 4);
+    L.off_x2lo = take(B * D * L.N2p * 4);
     L.off_rowpart = take(B * L.TC * N1 * 4);
     L.off_colpart = take(B * L.TR * N2 * 4);
     L.off_rowsum = take(B * N1 * 4);
@@ -1062,7 +1220,7 @@ inline BwdScratch bwd_scratch_layout(long long B, long long N1, long long N2, lo
     L.off_lo = take(4 * sizeof(int));
     L.total = off;
     L.off_part = off;
-    L.with_part = deals_chunks(B, N1, D, N2) || deals_chunks(B, N2, D, N1) ? off + sm_count() * kPartialBytes : off;
+    L.with_part = deals_chunks(B, N1, D, N2) || deals_chunks(B, N2, D, N1) ? off + pair_count() * kPartialBytes : off;
     return L;
 }
 
@@ -1089,10 +1247,10 @@ struct Tf32Operand {
     bool mn;
 };
 
-// out[b,m,n] = sum_k A[b](m,k) * Bm[b](n,k); K = length of the reduction.  A K-major operand holds
+// out[b,m,n] = sum_k A[b](m,k) * Bm[b](n,k), Bm K-major; K = length of the reduction.  A K-major operand holds
 // `pitch` >= K elements per row (zero beyond K), an MN-major operand has exactly K rows per batch.
 // lo_any (may be NULL): lo_any[1] says whether Bm has any low part; A's are always used.
-// partial (may be NULL): kPartialBytes per SM, for products that deal out chunks instead of whole tiles.
+// partial (may be NULL): kPartialBytes per pair of SMs, for products that deal out chunks instead of whole tiles.
 int launch_tf32_product(const Tf32Operand &A, const Tf32Operand &Bm, float *out, const int *lo_any, float *partial,
                         long long B, long long M, long long N, long long K, cudaStream_t s) {
     CUtensorMap mah, mal, mbh, mbl;
@@ -1103,13 +1261,13 @@ int launch_tf32_product(const Tf32Operand &A, const Tf32Operand &Bm, float *out,
     };
     if ((st = encode(&mah, A.hi, A, M, BM)) != TPW_OK) return st;
     if ((st = encode(&mal, A.lo, A, M, BM)) != TPW_OK) return st;
-    if ((st = encode(&mbh, Bm.hi, Bm, N, BN)) != TPW_OK) return st;
-    if ((st = encode(&mbl, Bm.lo, Bm, N, BN)) != TPW_OK) return st;
+    if ((st = encode(&mbh, Bm.hi, Bm, N, HN)) != TPW_OK) return st;
+    if ((st = encode(&mbl, Bm.lo, Bm, N, HN)) != TPW_OK) return st;
     GemmParams P;
     memset(&P, 0, sizeof(P));
     P.out = out;
     P.B = B; P.N1 = M; P.N2 = N; P.D = K; // K-major tails beyond K are zero padding or zero fill
-    P.tiles_m = (M + BM - 1) / BM;
+    P.tiles_m = (M + TM - 1) / TM;
     P.tiles_n = (N + BN - 1) / BN;
     P.tiles = B * P.tiles_m * P.tiles_n;
     P.epilogue = TPW_DOT_LINEAR;
@@ -1120,23 +1278,21 @@ int launch_tf32_product(const Tf32Operand &A, const Tf32Operand &Bm, float *out,
     P.kchunk = kProductChunk;
     P.vec_store = (N % 4 == 0 && aligned16(out)) ? 1 : 0;
     P.status = device_status_ptr();
-    const long long ctas = product_ctas(B, M, N, K, partial != nullptr);
+    const long long pairs = product_pairs(B, M, N, K, partial != nullptr);
     P.partial = partial != nullptr && deals_chunks(B, M, N, K) ? partial : nullptr;
-    const unsigned grid = (unsigned)ctas;
-#define TPW_TF32_LAUNCH(AMN, BMN)                                                                                         \
+    const unsigned grid = 2 * (unsigned)pairs;
+#define TPW_TF32_LAUNCH(AMN)                                                                                              \
     do {                                                                                                                  \
-        auto kern = gemm_metric_kernel<TPW_DOT_LINEAR, false, true, false, AMN, BMN>;                                     \
+        auto kern = gemm_metric_kernel<TPW_DOT_LINEAR, false, true, false, AMN>;                                          \
         TPW_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_ALLOC));                 \
         kern<<<grid, kThreads, SMEM_ALLOC, s>>>(mah, mal, mbh, mbl, P);                                                   \
     } while (0)
-    if (!A.mn && !Bm.mn) TPW_TF32_LAUNCH(false, false);
-    else if (!A.mn && Bm.mn) TPW_TF32_LAUNCH(false, true);
-    else if (A.mn && Bm.mn) TPW_TF32_LAUNCH(true, true);
-    else return fail(TPW_ERR_UNSUPPORTED, "tf32 product: MN-major A with K-major B is not instantiated");
+    if (A.mn) TPW_TF32_LAUNCH(true);
+    else TPW_TF32_LAUNCH(false);
 #undef TPW_TF32_LAUNCH
     TPW_LAUNCH_OK("gemm_metric_kernel (tf32)");
-    if (P.partial && P.tiles % ctas != 0) {
-        product_fixup_kernel<<<(unsigned)(P.tiles % ctas * (BM / 16)), BN, 0, s>>>(P, (int)product_chunks(K), ctas);
+    if (P.partial && P.tiles % pairs != 0) {
+        product_fixup_kernel<<<(unsigned)(P.tiles % pairs * (TM / 16)), BN, 0, s>>>(P, (int)product_chunks(K), pairs);
         TPW_LAUNCH_OK("product_fixup_kernel");
     }
     return TPW_OK;
@@ -1308,13 +1464,13 @@ int prepare_bf16_operands(const void *x1, const void *x2, void *scratch, bool re
     int st;
     if ((st = make_tensor_map_3d(&M.mxh, xh, 2, L.Dp, N1, B, BK, BM, true)) != TPW_OK) return st;
     if ((st = make_tensor_map_3d(&M.mxl, xl, 2, L.Dp, N1, B, BK, BM, true)) != TPW_OK) return st;
-    if ((st = make_tensor_map_3d(&M.myh, yh, 2, L.Dp, N2, B, BK, BN, true)) != TPW_OK) return st;
-    if ((st = make_tensor_map_3d(&M.myl, yl, 2, L.Dp, N2, B, BK, BN, true)) != TPW_OK) return st;
+    if ((st = make_tensor_map_3d(&M.myh, yh, 2, L.Dp, N2, B, BK, HN, true)) != TPW_OK) return st;
+    if ((st = make_tensor_map_3d(&M.myl, yl, 2, L.Dp, N2, B, BK, HN, true)) != TPW_OK) return st;
     memset(&P, 0, sizeof(P));
     P.n1sq = n1; P.n2sq = n2;
     P.lo_any = lo_any;
     P.B = B; P.N1 = N1; P.N2 = N2; P.D = L.Dp;
-    P.tiles_m = (N1 + BM - 1) / BM;
+    P.tiles_m = (N1 + TM - 1) / TM;
     P.tiles_n = (N2 + BN - 1) / BN;
     P.tiles = B * P.tiles_m * P.tiles_n;
     P.status = device_status_ptr();
@@ -1358,7 +1514,7 @@ extern "C" int tpw_dot_topk_forward_ws(int epilogue, int k, const void *x1, cons
     P.epilogue = cosine ? TPW_DOT_COSINE_DIST : TPW_DOT_SQEUCLIDEAN;
     P.topk_lists = lists; P.topk_thr = thr; P.topk_count = counts; P.topk_k = k; P.topk_L = (int)T.L;
     P.vec_store = N2 % 4 == 0 ? 1 : 0;   // the squared x2 norms of a batch start on 16-byte boundaries
-    const long long nsm = sm_count();
+    const long long pairs = pair_count();
     const long long tiles_n_all = (N2 + BN - 1) / BN;
     const long long rows = B * N1;
     const unsigned mblocks = (unsigned)((rows * 32 + 255) / 256);
@@ -1366,7 +1522,7 @@ extern "C" int tpw_dot_topk_forward_ws(int epilogue, int k, const void *x1, cons
     const int take_sqrt = epilogue == TPW_DOT_EUCLIDEAN ? 1 : 0;
 #define TPW_TOPK_LAUNCH(EPI, CAP)                                                                                         \
     do {                                                                                                                  \
-        auto kern = gemm_metric_kernel<EPI, false, false, false, false, false, CAP>;                                      \
+        auto kern = gemm_metric_kernel<EPI, false, false, false, false, CAP>;                                             \
         TPW_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_ALLOC));                 \
         kern<<<grid, kThreads, SMEM_ALLOC, s>>>(M.mxh, M.mxl, M.myh, M.myl, P);                                           \
         TPW_LAUNCH_OK("gemm_metric_kernel (top-k)");                                                                      \
@@ -1390,13 +1546,13 @@ extern "C" int tpw_dot_topk_forward_ws(int epilogue, int k, const void *x1, cons
     if ((tiles_n_all >= 8 || k > 2) && (groups < 32 ? groups : 32) >= k) {
         const CUtensorMap all_h = M.myh, all_l = M.myl;
         const unsigned char *yh = base + L.off_yh, *yl = base + L.off_yl;
-        if ((st = make_tensor_map_3d_pitched(&M.myh, yh, 2, L.Dp, cols, B, step * L.Dp * 2, N2 * L.Dp * 2, BK, BN)) != TPW_OK) return st;
-        if ((st = make_tensor_map_3d_pitched(&M.myl, yl, 2, L.Dp, cols, B, step * L.Dp * 2, N2 * L.Dp * 2, BK, BN)) != TPW_OK) return st;
+        if ((st = make_tensor_map_3d_pitched(&M.myh, yh, 2, L.Dp, cols, B, step * L.Dp * 2, N2 * L.Dp * 2, BK, HN)) != TPW_OK) return st;
+        if ((st = make_tensor_map_3d_pitched(&M.myl, yl, 2, L.Dp, cols, B, step * L.Dp * 2, N2 * L.Dp * 2, BK, HN)) != TPW_OK) return st;
         P.tiles_n = sample;
         P.tiles = B * P.tiles_m * P.tiles_n;
         P.cols = cols; P.col_step = (int)step; P.col_group = group;
         P.gmin = reinterpret_cast<float *>(lists);
-        const unsigned grid = (unsigned)(P.tiles < nsm ? P.tiles : nsm);
+        const unsigned grid = 2 * (unsigned)(P.tiles < pairs ? P.tiles : pairs);
         if (cosine) TPW_TOPK_LAUNCH(TPW_DOT_COSINE_DIST, -1); else TPW_TOPK_LAUNCH(TPW_DOT_SQEUCLIDEAN, -1);
         topk_bound_kernel<<<mblocks, 256, 0, s>>>(P.gmin, thr, counts, rows, (int)(BN / group * sample), k);
         TPW_LAUNCH_OK("topk_bound_kernel");
@@ -1407,7 +1563,7 @@ extern "C" int tpw_dot_topk_forward_ws(int epilogue, int k, const void *x1, cons
     }
     P.tiles_n = tiles_n_all;
     P.tiles = B * P.tiles_m * P.tiles_n;
-    const unsigned grid = (unsigned)(P.tiles < nsm ? P.tiles : nsm);
+    const unsigned grid = 2 * (unsigned)(P.tiles < pairs ? P.tiles : pairs);
     if (cosine) TPW_TOPK_LAUNCH(TPW_DOT_COSINE_DIST, 1); else TPW_TOPK_LAUNCH(TPW_DOT_SQEUCLIDEAN, 1);
     if (k <= 8) topk_merge_kernel<8><<<mblocks, 256, 0, s>>>(lists, counts, val_out, idx64, rows, T.L * k, k, take_sqrt);
     else topk_merge_kernel<16><<<mblocks, 256, 0, s>>>(lists, counts, val_out, idx64, rows, T.L * k, k, take_sqrt);
@@ -1445,8 +1601,8 @@ extern "C" int tpw_dot_rowmin_forward_ws(int epilogue, const void *x1, const voi
     if ((st = prepare_bf16_operands(x1, x2, scratch, cosine, B, N1, N2, D, s, M, P)) != TPW_OK) return st;
     P.epilogue = cosine ? TPW_DOT_COSINE_DIST : TPW_DOT_SQEUCLIDEAN;
     P.rowmin_keys = keys;
-    const long long nsm = sm_count();
-    const unsigned grid = (unsigned)(P.tiles < nsm ? P.tiles : nsm);
+    const long long pairs = pair_count();
+    const unsigned grid = 2 * (unsigned)(P.tiles < pairs ? P.tiles : pairs);
     if (cosine) {
         auto kern = gemm_metric_kernel<TPW_DOT_COSINE_DIST, false, false, true>;
         TPW_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_ALLOC));
@@ -1537,8 +1693,8 @@ extern "C" int tpw_dot_metric_forward_ws(int dtype, int epilogue, int engine,
     P.self = self ? 1 : 0;
     P.vec_store = (N2 % 4 == 0 && aligned16(out)) ? 1 : 0;
     TPW_CHECK_ARG(P.tiles < (1ll << 40), "tpw_dot_metric_forward_ws: too many tiles");
-    const long long nsm = sm_count();
-    const unsigned grid = (unsigned)(P.tiles < nsm ? P.tiles : nsm);
+    const long long pairs = pair_count();
+    const unsigned grid = 2 * (unsigned)(P.tiles < pairs ? P.tiles : pairs);
 #define TPW_GEMM_LAUNCH(EPI, SELF)                                                                                        \
     do {                                                                                                                  \
         auto kern = gemm_metric_kernel<EPI, SELF, false>;                                                                        \
@@ -1618,22 +1774,19 @@ static int dense_backward_tensor(int coef, int epilogue, bool sums, float s_mm, 
     for (int side = 0; side < 2; ++side) {
         void *gout = side == 0 ? grad_x1 : grad_x2;
         if (!gout) continue;
-        // side 0: grad_x1[N1,D] = C . X2, X2 [N2,D] contracted over its rows; side 1: grad_x2[N2,D] = C^T . X1
-        const void *xk = side == 0 ? x2 : x1;   // operand contracted against (MN-major: its rows are k)
+        // side 0: grad_x1[N1,D] = C . X2; side 1: grad_x2[N2,D] = C^T . X1
+        const void *xk = side == 0 ? x2 : x1;   // operand contracted against: its transpose is the K-major one
         const void *xo = side == 0 ? x1 : x2;   // rows that receive the gradient
-        const long long Nk = side == 0 ? N2 : N1, No = side == 0 ? N1 : N2;
+        const long long Nk = side == 0 ? N2 : N1, No = side == 0 ? N1 : N2, Np = side == 0 ? L.N2p : L.N1p;
         float *xhi = F(side == 0 ? L.off_x2hi : L.off_x1hi), *xlo = F(side == 0 ? L.off_x2lo : L.off_x1lo);
-        SplitParams X;
-        memset(&X, 0, sizeof(X));
-        X.a = static_cast<const float *>(xk);
-        X.hi = xhi; X.lo = xlo;
-        X.R = Nk; X.C = D; X.Cp = L.Dp;
-        X.vec_in = (D % 4 == 0 && aligned16(xk)) ? 1 : 0;
-        X.lo_any = lo_any + 2 * side + 1;
-        if ((st = launch_split<COEF_ID, false>(X, B, s)) != TPW_OK) return st;
-        const Tf32Operand Xmn{xhi, xlo, L.Dp, true};
-        if (side == 0) st = launch_tf32_product(Ck, Xmn, static_cast<float *>(gout), lo_any, partial, B, N1, D, N2, s);
-        else st = launch_tf32_product(Cmn, Xmn, static_cast<float *>(gout), lo_any + 2, partial, B, N2, D, N1, s);
+        const long long gx = (D + PT - 1) / PT, gy = (Nk + PT - 1) / PT;
+        TPW_CHECK_ARG(gy <= 65535 && B <= 65535, "dense backward: more than 65535 row tiles or batches");
+        split_transposed_kernel<<<dim3((unsigned)gx, (unsigned)gy, (unsigned)B), 256, 0, s>>>(
+            static_cast<const float *>(xk), xhi, xlo, lo_any + 2 * side + 1, Nk, D, Np, D % 4 == 0 && aligned16(xk) ? 1 : 0);
+        TPW_LAUNCH_OK("split_transposed_kernel");
+        const Tf32Operand Xk{xhi, xlo, Np, false};
+        if (side == 0) st = launch_tf32_product(Ck, Xk, static_cast<float *>(gout), lo_any, partial, B, N1, D, N2, s);
+        else st = launch_tf32_product(Cmn, Xk, static_cast<float *>(gout), lo_any + 2, partial, B, N2, D, N1, s);
         if (st != TPW_OK) return st;
         const float *sumv = F(side == 0 ? L.off_rowsum : L.off_colsum);
         if (coef == COEF_COSINE) {
