@@ -576,6 +576,12 @@ TPW_API int tpw_prf_div_forward(int dtype, int mode, const void *x, const void *
 TPW_API int tpw_prf_div_backward(int dtype, int mode, const void *grad, const void *x, const void *y,
                          void *grad_x, void *grad_y, int64_t n, tpw_stream_t stream);
 
+/* ---- 16-bit floats ------------------------------------------------------------------------------ */
+
+/* dst[i] = src[i] as float32, exactly; src: bfloat16 (bf16 != 0) or IEEE half.  Both 16-byte aligned.  The reference's own kernels
+   compute in the narrow type; the host layer widens on entry instead. */
+TPW_API int tpw_widen(int bf16, const void *src, float *dst, int64_t n, tpw_stream_t stream);
+
 /* ---- measured issue peaks (roofline denominators for the CUDA-core kernels) -------------------- */
 
 /*

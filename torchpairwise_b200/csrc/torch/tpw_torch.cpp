@@ -98,6 +98,19 @@ struct Prepared {
     Tensor s1, s2;   // a and b without the leading dimension that an unbatched call lacks
 };
 
+// x in the type that the kernels compute in, contiguous.  Contiguous 16-bit floats go through the library's own kernel, which takes
+// half the time of the general converting copy; everything else (views, other types) through that copy.
+Tensor in_type(const Tensor &x, at::ScalarType dt) {
+    const auto from = x.scalar_type();
+    if (dt != at::kFloat || (from != at::kBFloat16 && from != at::kHalf) || !x.is_cuda() || !x.is_contiguous() || x.is_neg() || x.numel() == 0 ||
+        reinterpret_cast<uintptr_t>(x.const_data_ptr()) % 16 != 0)
+        return x.to(dt).contiguous();
+    c10::cuda::CUDAGuard dg(x.device());
+    Tensor out = at::empty(x.sizes(), x.options().dtype(dt));
+    TPW_CALL(tpw_widen(from == at::kBFloat16, x.const_data_ptr(), out.mutable_data_ptr<float>(), x.numel(), stream_of(x)));
+    return out;
+}
+
 // contiguous() + leading batch dimension (e.g. OPS/cuda/ppminkowski_kernel.cu:70-90)
 Prepared prepare(const Tensor &x1, const Tensor &x2, at::ScalarType dt) {
     require_cuda(x1);
@@ -109,8 +122,8 @@ Prepared prepare(const Tensor &x1, const Tensor &x2, at::ScalarType dt) {
     TORCH_CHECK(unbatched || x1.size(0) == x2.size(0), "batch_size of x1 and x2 do not match.");
     TORCH_CHECK(x1.size(-1) == x2.size(-1), "feature dimension of x1 and x2 do not match.");
     Prepared p;
-    p.a = x1.to(dt).contiguous();
-    p.b = x2.is_same(x1) ? p.a : x2.to(dt).contiguous();
+    p.a = in_type(x1, dt);
+    p.b = x2.is_same(x1) ? p.a : in_type(x2, dt);
     p.unbatched = unbatched;
     p.s1 = p.a;
     p.s2 = p.b;
@@ -308,7 +321,7 @@ struct CdistFn : torch::autograd::Function<CdistFn> {
             a = pad_features(a);
             b = pad_features(b);
         }
-        Tensor g = go[0].to(a.scalar_type()).contiguous();
+        Tensor g = in_type(go[0], a.scalar_type());
         if (ub) g = g.unsqueeze(0);
         Tensor g1, g2;
         if (ctx->needs_input_grad(0)) g1 = p == 0 ? at::zeros_like(a) : at::empty_like(a);
@@ -351,7 +364,7 @@ struct PPMinkowskiFn : torch::autograd::Function<PPMinkowskiFn> {
     }
     static std::pair<Tensor, Tensor> raw_backward(const Tensor &grad, const Tensor &a, const Tensor &b, double p, bool ub) {
         c10::cuda::CUDAGuard dg(a.device());
-        Tensor g = grad.to(a.scalar_type()).contiguous();
+        Tensor g = in_type(grad, a.scalar_type());
         if (ub) g = g.unsqueeze(0);
         Tensor g1 = at::zeros_like(a), g2 = at::zeros_like(b);
         const int64_t B = a.size(0), N1 = a.size(1), N2 = b.size(1), D = a.size(2);
@@ -401,7 +414,7 @@ struct JensenShannonFn : torch::autograd::Function<JensenShannonFn> {
     static std::pair<Tensor, Tensor> raw_backward(const Tensor &grad, const Tensor &a, const Tensor &b, const Tensor &out,
                                                   double scale, bool ub) {
         c10::cuda::CUDAGuard dg(a.device());
-        Tensor g = grad.to(a.scalar_type()).contiguous();
+        Tensor g = in_type(grad, a.scalar_type());
         if (ub) g = g.unsqueeze(0);
         Tensor g1 = at::empty_like(a), g2 = at::empty_like(b);
         TPW_CALL(tpw_jensenshannon_backward(code_of(a), g.data_ptr(), out.defined() ? out.data_ptr() : nullptr, a.data_ptr(), b.data_ptr(),
@@ -439,7 +452,7 @@ struct PairSumFn : torch::autograd::Function<PairSumFn> {
     }
     static std::pair<Tensor, Tensor> raw_backward(const Tensor &grad, const Tensor &a, const Tensor &b, int metric, bool ub) {
         c10::cuda::CUDAGuard dg(a.device());
-        Tensor g = grad.to(a.scalar_type()).contiguous();
+        Tensor g = in_type(grad, a.scalar_type());
         if (ub) g = g.unsqueeze(0);
         Tensor g1 = at::empty_like(a), g2 = at::empty_like(b);
         TPW_CALL(tpw_pair_sum_backward(code_of(a), metric, g.data_ptr(), a.data_ptr(), b.data_ptr(), g1.data_ptr(), g2.data_ptr(),
@@ -473,7 +486,7 @@ struct HaversineFn : torch::autograd::Function<HaversineFn> {
     }
     static std::pair<Tensor, Tensor> raw_backward(const Tensor &grad, const Tensor &a, const Tensor &b, bool ub) {
         c10::cuda::CUDAGuard dg(a.device());
-        Tensor g = grad.to(a.scalar_type()).contiguous();
+        Tensor g = in_type(grad, a.scalar_type());
         if (ub) g = g.unsqueeze(0);
         Tensor g1 = at::empty_like(a), g2 = at::empty_like(b);
         TPW_CALL(tpw_haversine_backward(code_of(a), g.data_ptr(), a.data_ptr(), b.data_ptr(), g1.data_ptr(), g2.data_ptr(),
@@ -518,7 +531,7 @@ struct WMinkowskiFn : torch::autograd::Function<WMinkowskiFn> {
     static std::tuple<Tensor, Tensor, Tensor> raw_backward(const Tensor &grad, const Tensor &a, const Tensor &b, const Tensor &w,
                                                            double p, bool ub, bool need_w = true) {
         c10::cuda::CUDAGuard dg(a.device());
-        Tensor g = grad.to(a.scalar_type()).contiguous();
+        Tensor g = in_type(grad, a.scalar_type());
         if (ub) g = g.unsqueeze(0);
         const int64_t B = a.size(0), N1 = a.size(1), N2 = b.size(1), D = a.size(2);
         // the finite-p kernels write every element, the p = inf kernel adds into zeros
@@ -577,7 +590,7 @@ struct CosineFn : torch::autograd::Function<CosineFn> {
         const auto dt = static_cast<at::ScalarType>(ctx->saved_data["dt"].toInt());
         const int epilogue = static_cast<int>(ctx->saved_data["epilogue"].toInt());
         c10::cuda::CUDAGuard dg(a.device());
-        Tensor g = go[0].to(a.scalar_type()).contiguous();
+        Tensor g = in_type(go[0], a.scalar_type());
         if (ub) g = g.unsqueeze(0);
         const int64_t B = a.size(0), N1 = a.size(1), N2 = b.size(1), D = a.size(2);
         const int code = code_of(a);
@@ -698,7 +711,7 @@ struct HausdorffFn : torch::autograd::Function<HausdorffFn> {
         const bool ub = ctx->saved_data["unbatched"].toBool();
         const Tensor a = batched(s[0], ub, 4), b = batched(s[1], ub, 4), out = batched(s[2], ub), i1 = batched(s[3], ub), i2 = batched(s[4], ub);
         const auto dt = static_cast<at::ScalarType>(ctx->saved_data["dt"].toInt());
-        Tensor g = go[0].to(a.scalar_type()).contiguous();
+        Tensor g = in_type(go[0], a.scalar_type());
         if (ub) g = g.unsqueeze(0);
         auto gg = hausdorff_grads(g, a, b, out, i1, i2);
         const Tensor &g1 = gg.first, &g2 = gg.second;
@@ -1161,7 +1174,7 @@ struct LinearKernelFn : torch::autograd::Function<LinearKernelFn> {
         const Tensor a = batched(s[0], ub), b = batched(s[1], ub);
         const auto dt = static_cast<at::ScalarType>(ctx->saved_data["dt"].toInt());
         c10::cuda::CUDAGuard dg(a.device());
-        Tensor g = go[0].to(a.scalar_type()).contiguous();
+        Tensor g = in_type(go[0], a.scalar_type());
         if (ub) g = g.unsqueeze(0);
         Tensor g1 = at::zeros_like(a), g2 = at::zeros_like(b);
         if (a.numel() > 0 && b.numel() > 0) dense_backward(TPW_LP_BWD_MATMUL, g, nullptr, a, b, g1, g2);
