@@ -1106,13 +1106,24 @@ split_tile_kernel(const SplitParams P) {
 // tf32 high/low copies of a matrix's transpose, [B,C,Rp]: rows of the copy run along the source's row index, zero filled to Rp.
 // The product's other operand then lies K-major, staged by one copy of 128 rows instead of four of {32 values, 32 rows}: C^T x1 of
 // [16, 4096, 4096, 256] 620 -> 570 us.  (The products' bound is the copies' latency: with neither MMAs nor epilogue they take as long.)
+struct Transposed {
+    const float *src;
+    float *hi, *lo;
+    int *lo_any;
+    long long R, Rp;
+    int vec_in;
+};
 __global__ void __launch_bounds__(256)
-split_transposed_kernel(const float *__restrict__ src, float *__restrict__ hi, float *__restrict__ lo, int *lo_any,
-                        long long R, long long C, long long Rp, int vec_in) {
+split_transposed_kernel(const Transposed first, const Transposed second, long long C, int operands) {
     __shared__ float tile[PT][PT + 1];
-    const int tid = threadIdx.x;
-    const long long b = blockIdx.z, r0 = (long long)blockIdx.y * PT, c0 = (long long)blockIdx.x * PT;
-    const float *a = src + b * R * C;
+    const Transposed &P = blockIdx.z % operands == 0 ? first : second;   // both in one launch
+    const long long R = P.R, Rp = P.Rp;
+    float *__restrict__ hi = P.hi, *__restrict__ lo = P.lo;
+    int *lo_any = P.lo_any;
+    const int vec_in = P.vec_in, tid = threadIdx.x;
+    const long long b = blockIdx.z / operands, r0 = (long long)blockIdx.y * PT, c0 = (long long)blockIdx.x * PT;
+    if (r0 >= Rp) return;
+    const float *__restrict__ a = P.src + b * R * C;
 #pragma unroll
     for (int u = 0; u < 4; ++u) {
         const int r = u * 16 + (tid >> 4), c = (tid & 15) * 4;
@@ -1150,23 +1161,42 @@ split_transposed_kernel(const float *__restrict__ src, float *__restrict__ hi, f
     if (__syncthreads_or(any != 0) && tid == 0) *lo_any = 1;
 }
 
-// sums[b,n] = part[b,0,n] + part[b,1,n] + ... in that order (deterministic)
-__global__ void reduce_partials_kernel(const float *__restrict__ part, float *__restrict__ sums, long long B, long long T, long long N) {
+// sums[b,n] = part[b,0,n] + part[b,1,n] + ... in that order (deterministic); the row sums and, in the second row of CTAs, the
+// column sums
+struct Partials {
+    const float *part;
+    float *sums;
+    long long T, N;
+};
+__global__ void reduce_partials_kernel(const Partials first, const Partials second, long long B) {
+    const Partials &P = blockIdx.y == 0 ? first : second;
     const long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x;
-    if (t >= B * N) return;
-    const long long b = t / N, n = t % N;
+    if (t >= B * P.N) return;
+    const long long b = t / P.N, n = t % P.N;
     float s = 0.f;
-    for (long long k = 0; k < T; ++k) s += part[(b * T + k) * N + n];
-    sums[t] = s;
+    for (long long k = 0; k < P.T; ++k) s += P.part[(b * P.T + k) * P.N + n];
+    P.sums[t] = s;
 }
 
-// g[r,k] = s_mm * g[r,k] + s_row * x[r,k] * sums[r]
-__global__ void grad_finish_kernel(float *__restrict__ g, const float *__restrict__ x, const float *__restrict__ sums,
-                                   long long rows, long long D, float s_mm, float s_row) {
-    const long long n = rows * D;
+// g[r,k] = s_mm * g[r,k] + s_row * x[r,k] * sums[r] for one gradient or, in the second row of CTAs, the other; VEC elements of a
+// row to a thread
+struct Finish {
+    float *g;
+    const float *x, *sums;
+    long long rows;
+};
+template <int VEC>
+__global__ void grad_finish_kernel(const Finish first, const Finish second, long long D, float s_mm, float s_row) {
+    struct alignas(VEC * 4) Pack { float v[VEC]; };
+    const Finish &P = blockIdx.y == 0 ? first : second;
+    const long long per = D / VEC, n = P.rows * per;
     for (long long t = blockIdx.x * (long long)blockDim.x + threadIdx.x; t < n; t += (long long)gridDim.x * blockDim.x) {
-        const float base = s_mm * g[t];
-        g[t] = sums ? fmaf(s_row * x[t], sums[t / D], base) : base;
+        const float sum = P.sums[t / per];
+        Pack g = reinterpret_cast<Pack *>(P.g)[t];
+        const Pack x = reinterpret_cast<const Pack *>(P.x)[t];
+#pragma unroll
+        for (int u = 0; u < VEC; ++u) g.v[u] = fmaf(s_row * x.v[u], sum, s_mm * g.v[u]);
+        reinterpret_cast<Pack *>(P.g)[t] = g;
     }
 }
 
@@ -1765,39 +1795,59 @@ static int dense_backward_tensor(int coef, int epilogue, bool sums, float s_mm, 
     else st = launch_split<COEF_ID, false>(C, B, s);
     if (st != TPW_OK) return st;
     if (sums) {
-        reduce_partials_kernel<<<(unsigned)((B * N1 + 255) / 256), 256, 0, s>>>(F(L.off_rowpart), F(L.off_rowsum), B, L.TC, N1);
-        reduce_partials_kernel<<<(unsigned)((B * N2 + 255) / 256), 256, 0, s>>>(F(L.off_colpart), F(L.off_colsum), B, L.TR, N2);
+        const long long most = B * (N1 > N2 ? N1 : N2);
+        reduce_partials_kernel<<<dim3((unsigned)((most + 255) / 256), 2), 256, 0, s>>>(
+            Partials{F(L.off_rowpart), F(L.off_rowsum), L.TC, N1}, Partials{F(L.off_colpart), F(L.off_colsum), L.TR, N2}, B);
         TPW_LAUNCH_OK("reduce_partials_kernel");
     }
-    const long long cap = (long long)sm_count() * 8;
     const Tf32Operand Ck{F(L.off_chi), F(L.off_clo), L.N2p, false}, Cmn{F(L.off_chi), F(L.off_clo), L.N2p, true};
+    // side 0: grad_x1[N1,D] = C . X2; side 1: grad_x2[N2,D] = C^T . X1.  xk: operand contracted against (its transpose is the K-major
+    // one); xo: rows that receive the gradient
+    Transposed T[2];
+    Finish fin[2];
+    int sides = 0;
+    bool vec = D % 4 == 0;
+    long long most = 0;
     for (int side = 0; side < 2; ++side) {
         void *gout = side == 0 ? grad_x1 : grad_x2;
         if (!gout) continue;
-        // side 0: grad_x1[N1,D] = C . X2; side 1: grad_x2[N2,D] = C^T . X1
-        const void *xk = side == 0 ? x2 : x1;   // operand contracted against: its transpose is the K-major one
-        const void *xo = side == 0 ? x1 : x2;   // rows that receive the gradient
-        const long long Nk = side == 0 ? N2 : N1, No = side == 0 ? N1 : N2, Np = side == 0 ? L.N2p : L.N1p;
-        float *xhi = F(side == 0 ? L.off_x2hi : L.off_x1hi), *xlo = F(side == 0 ? L.off_x2lo : L.off_x1lo);
-        const long long gx = (D + PT - 1) / PT, gy = (Nk + PT - 1) / PT;
-        TPW_CHECK_ARG(gy <= 65535 && B <= 65535, "dense backward: more than 65535 row tiles or batches");
-        split_transposed_kernel<<<dim3((unsigned)gx, (unsigned)gy, (unsigned)B), 256, 0, s>>>(
-            static_cast<const float *>(xk), xhi, xlo, lo_any + 2 * side + 1, Nk, D, Np, D % 4 == 0 && aligned16(xk) ? 1 : 0);
-        TPW_LAUNCH_OK("split_transposed_kernel");
-        const Tf32Operand Xk{xhi, xlo, Np, false};
+        const void *xk = side == 0 ? x2 : x1, *xo = side == 0 ? x1 : x2;
+        T[sides] = Transposed{static_cast<const float *>(xk), F(side == 0 ? L.off_x2hi : L.off_x1hi), F(side == 0 ? L.off_x2lo : L.off_x1lo),
+                              lo_any + 2 * side + 1, side == 0 ? N2 : N1, side == 0 ? L.N2p : L.N1p, D % 4 == 0 && aligned16(xk) ? 1 : 0};
+        fin[sides] = Finish{static_cast<float *>(gout), static_cast<const float *>(xo), F(side == 0 ? L.off_rowsum : L.off_colsum), B * (side == 0 ? N1 : N2)};
+        vec = vec && aligned16(gout) && aligned16(xo);
+        if (T[sides].Rp > most) most = T[sides].Rp;
+        ++sides;
+    }
+    const long long gx = (D + PT - 1) / PT, gy = (most + PT - 1) / PT;
+    TPW_CHECK_ARG(gy <= 65535 && B <= 65535, "dense backward: more than 65535 row tiles or batches");
+    if (B * sides <= 65535) {
+        split_transposed_kernel<<<dim3((unsigned)gx, (unsigned)gy, (unsigned)(B * sides)), 256, 0, s>>>(T[0], T[sides - 1], D, sides);
+    } else {
+        for (int at = 0; at < sides; ++at)
+            split_transposed_kernel<<<dim3((unsigned)gx, (unsigned)gy, (unsigned)B), 256, 0, s>>>(T[at], T[at], D, 1);
+    }
+    TPW_LAUNCH_OK("split_transposed_kernel");
+    for (int side = 0, at = 0; side < 2; ++side) {
+        void *gout = side == 0 ? grad_x1 : grad_x2;
+        if (!gout) continue;
+        const Tf32Operand Xk{T[at].hi, T[at].lo, T[at].Rp, false};
         if (side == 0) st = launch_tf32_product(Ck, Xk, static_cast<float *>(gout), lo_any, partial, B, N1, D, N2, s);
         else st = launch_tf32_product(Cmn, Xk, static_cast<float *>(gout), lo_any + 2, partial, B, N2, D, N1, s);
         if (st != TPW_OK) return st;
-        const float *sumv = F(side == 0 ? L.off_rowsum : L.off_colsum);
         if (coef == COEF_COSINE) {
             // the norm part of the chain: g[r,:] += term[r] * x[r,:] / norm[r]
-            if ((st = tpw_cosine_backward_finish(TPW_F32, gout, xo, side == 0 ? norm1 : norm2, sumv, B * No, D, s)) != TPW_OK) return st;
-        } else if (sums) {
-            const long long n = B * No * D, blocks = (n + 255) / 256;
-            grad_finish_kernel<<<(unsigned)(blocks < cap ? blocks : cap), 256, 0, s>>>(
-                static_cast<float *>(gout), static_cast<const float *>(xo), sumv, B * No, D, s_mm, s_row);
-            TPW_LAUNCH_OK("grad_finish_kernel");
+            if ((st = tpw_cosine_backward_finish(TPW_F32, gout, fin[at].x, side == 0 ? norm1 : norm2, fin[at].sums, fin[at].rows, D, s)) != TPW_OK) return st;
         }
+        ++at;
+    }
+    if (sums && coef != COEF_COSINE) {
+        const long long rows = fin[0].rows > fin[sides - 1].rows ? fin[0].rows : fin[sides - 1].rows, cap = (long long)sm_count() * 8;
+        const long long blocks = (rows * (vec ? D / 4 : D) + 255) / 256;
+        const dim3 grid((unsigned)(blocks < cap ? blocks : cap), (unsigned)sides);
+        if (vec) grad_finish_kernel<4><<<grid, 256, 0, s>>>(fin[0], fin[sides - 1], D, s_mm, s_row);
+        else grad_finish_kernel<1><<<grid, 256, 0, s>>>(fin[0], fin[sides - 1], D, s_mm, s_row);
+        TPW_LAUNCH_OK("grad_finish_kernel");
     }
     return TPW_OK;
 }
