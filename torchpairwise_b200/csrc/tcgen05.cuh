@@ -112,16 +112,11 @@ __device__ __forceinline__ void raise_abort_pair(int *abort_flag) {
 template <bool PAIR = false>
 __device__ __forceinline__ bool wait_or_abort(uint64_t *bar, uint32_t parity, volatile int *abort_flag) {
     auto done = [&]() { return PAIR ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity); };
-    // the clock is read after 64 polls: most waits are shorter than that
-    uint64_t t0 = 0;
+    if (done()) return true;
+    const uint64_t t0 = globaltimer_ns();
     for (uint32_t it = 0; it < kSpinLimit; ++it) {
         if (done()) return true;
-        if ((it & 63u) == 63u) {
-            if (*abort_flag) return false;
-            const uint64_t t = globaltimer_ns();
-            if (t0 == 0) t0 = t;
-            else if (t - t0 > kWaitBudgetNs) return false;
-        }
+        if ((it & 63u) == 63u && (*abort_flag || globaltimer_ns() - t0 > kWaitBudgetNs)) return false;
     }
     return false;
 }
