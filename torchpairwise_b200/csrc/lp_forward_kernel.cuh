@@ -33,7 +33,7 @@ struct FwdParams {
     double p;            // exponent of K_PGEN
     int pow_spec;        // make_pow_spec(p): how the float kernel evaluates |d|^p
     double out_exponent; // finite kinds: out = sum ^ out_exponent
-    int root_mode;       // 0 none, 1 sqrt, 2 cbrt, 3 pow(out_exponent), 4 1 / sqrt
+    int root_mode;       // 0 none, 1 sqrt, 2 cbrt, 3 pow(out_exponent), 4 1 / sqrt (p = 2)
     double scale;        // K_JS: factor applied to the finished sum (before the optional square root)
     int epilogue;        // K_DOT: tpw_dot_epilogue; K_NE*: bit0 = report equal count, bit1 = mean
     int vec_store;       // 4-byte outputs, N2 % 4 == 0, 16-byte aligned base: staged 128-bit stores
@@ -182,7 +182,7 @@ __device__ __forceinline__ void apply_root(T (&acc)[R][R], const FwdParams &P) {
         for (int a = 0; a < R; ++a)
 #pragma unroll
             for (int c = 0; c < R; ++c) acc[a][c] = t_cbrt(acc[a][c]);
-    } else if (P.root_mode == 4) {
+    } else if (KIND == K_P2 && P.root_mode == 4) {
 #pragma unroll
         for (int a = 0; a < R; ++a)
 #pragma unroll
@@ -708,7 +708,7 @@ int lp_forward_typed(FwdParams P, double p, double out_exponent, cudaStream_t st
     if (out_exponent == 1.0) P.root_mode = 0;
     else if (out_exponent == 0.5) P.root_mode = 1;
     else if (p == 3.0 && out_exponent == 1.0 / 3.0) P.root_mode = 2;
-    else if (out_exponent == -0.5) P.root_mode = 4;   // the weighted p = 2 backward's coefficient: float64 [1500, 1301, 75] 80 us with pow, 63 so
+    else if (p == 2.0 && out_exponent == -0.5) P.root_mode = 4;   // the weighted p = 2 backward's coefficient: float64 [1500, 1301, 75] 80 us with pow, 63 so
     else P.root_mode = 3;
     if (p == 1.0) return launch_forward_w<T, K_L1, EPI>(P, stream);
     if (p == 2.0) return launch_forward_w<T, K_P2, EPI>(P, stream);
