@@ -24,7 +24,7 @@
 // 564 -> 429 us.
 //
 // Every mbarrier wait is bounded; a role that gives up raises the pair's abort flag, everybody falls through to the
-// final barrier, tensor memory is released and the device status word reports the site.
+// final barrier, what is under way arrives (pair_exit.cuh), tensor memory is released and the device status word reports the site.
 #include "bool_epilogue.cuh"
 #include "common.cuh"
 #include "tcgen05.cuh"
@@ -49,10 +49,11 @@ constexpr int kEpilogueWarps = 16;            // four per TMEM lane quarter, eac
 template <bool RAGGED> struct Layout {
     static constexpr int kStages = RAGGED ? 2 : 4;
     static constexpr int OFF_BAR = kStages * STAGE_BYTES;
-    // barriers: full, empty [kStages], tmem_full[2], tmem_empty[2]; then the TMEM base address and the abort flag
+    // barriers: full, empty [kStages], tmem_full[2], tmem_empty[2]; then the TMEM base address, the abort flag and the pair's counts
     static constexpr int OFF_TMEM_PTR = OFF_BAR + (2 * kStages + 4) * 8;
     static constexpr int OFF_ABORT = OFF_TMEM_PTR + 4;
-    static constexpr int OFF_STAGE = (OFF_ABORT + 4 + 127) / 128 * 128;
+    static constexpr int OFF_COUNTS = OFF_ABORT + 4;
+    static constexpr int OFF_STAGE = (OFF_COUNTS + (int)sizeof(PairCounts) + 127) / 128 * 128;
     static constexpr int OFF_POP = OFF_STAGE + (RAGGED ? BM * BN * 4 : kStoreBytes);   // per epilogue warp the x2 row counts of its 64 columns
     static constexpr int SMEM_ALLOC = OFF_POP + kEpilogueWarps * 256 + 1024;
     static_assert(SMEM_ALLOC <= 232448, "exceeds the dynamic shared memory of one CTA");
@@ -135,6 +136,7 @@ bool_count_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
     uint64_t *tmem_empty = tmem_full + 2;                                // rank 0's: both CTAs have drained the accumulator
     uint32_t *tmem_ptr = reinterpret_cast<uint32_t *>(smem + L::OFF_TMEM_PTR);
     int *abort_flag = reinterpret_cast<int *>(smem + L::OFF_ABORT);
+    PairCounts *counts = reinterpret_cast<PairCounts *>(smem + L::OFF_COUNTS);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();       // the pair's tile: rows of rank 0, then rows of rank 1
@@ -188,9 +190,8 @@ bool_count_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
                     tma_load_3d_pair(st + A_BYTES, &map_y, bar, kb * BKB, tn * BN + (int)rank * (BN / 2), b);
                 }
             }
-            // after a wait that gave up, stay (bounded) until the copies under way have landed in both CTAs
-            if (!ok && rank == 0)
-                for (uint32_t u = it > (uint32_t)kStages ? it - kStages : 0; u < it; ++u) mbar_wait_bounded(&full[u % kStages], (u / kStages) & 1);
+            if (ok && !wait_for_releases(empty, it, kStages, abort_flag)) give_up(5);
+            publish_pair(&counts->issued[rank], it);
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer: rank 0, for both ----------------
@@ -225,8 +226,11 @@ bool_count_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
                         if (k < kmma) tc_mma_i8(d_tmem, dx + 2 * k, dy + 2 * k, idesc, (kb | k) != 0);
                     tc_commit_pair(&empty[s]);   // the stage may be refilled, in both CTAs, once these MMAs have read it
                 }
-                if (ok) tc_commit_pair(&tmem_full[a]);
+                if (!ok) break;      // acount: accumulators handed over
+                tc_commit_pair(&tmem_full[a]);
             }
+            publish_pair(&counts->used, it);
+            publish_pair(&counts->filled, acount);
         }
     } else {
         // ---------------- epilogue: warps 2..17 ----------------
@@ -332,6 +336,11 @@ bool_count_tcgen05_kernel(const __grid_constant__ CUtensorMap map_x, const __gri
     tc_fence_before();
     __syncthreads();
     cluster_sync();   // neither CTA's shared memory goes while the other may still read it or arrive in it
+    if (*reinterpret_cast<volatile int *>(abort_flag)) {   // raised in both CTAs or in neither
+        if (threadIdx.x == 0) drain_pair(full, empty, tmem_full, kStages, counts, rank, [](uint32_t) { return (uint32_t)STAGE_BYTES; });
+        __syncthreads();
+        cluster_sync();
+    }
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc_pair(tmem_base, kTmemCols);

@@ -28,9 +28,9 @@
 // truncation; see dense_backward_tensor below); (2) a row-minimum epilogue that folds each thread's
 // accumulator row into one 64-bit key and stores no tile; (3) SELF, which zeroes the diagonal.
 //
-// Every wait (mbarrier) is bounded; a warp that gives up raises a CTA-wide abort flag that the other
-// roles poll, everybody falls through to the final barrier, tensor memory is released, and the
-// device status word reports the site.
+// Every wait (mbarrier) is bounded; a warp that gives up raises the pair's abort flag that the other
+// roles poll, everybody falls through to the final barrier, what is under way arrives (pair_exit.cuh),
+// tensor memory is released, and the device status word reports the site.
 #include "common.cuh"
 #include "packed_f32x2.cuh"
 #include "tcgen05.cuh"
@@ -55,11 +55,12 @@ constexpr int A_BYTES = BM * BK * 2;          // 16 KB
 constexpr int B_BYTES = HN * BK * 2;          // 16 KB
 constexpr int SLOT_BYTES = A_BYTES + B_BYTES; // one part (high or low) of a k-step
 constexpr int OFF_BAR = kSlots * SLOT_BYTES;
-// barriers: full[5], empty[5], tmem_full[2], tmem_empty[2]; then the TMEM base address and the abort flag
+// barriers: full[5], empty[5], tmem_full[2], tmem_empty[2]; then the TMEM base address, the abort flag and the pair's counts
 constexpr int OFF_TMEM_PTR = OFF_BAR + (2 * kSlots + 4) * 8;
 constexpr int OFF_ABORT = OFF_TMEM_PTR + 4;
+constexpr int OFF_COUNTS = OFF_ABORT + 4;
 // staging of the stored tiles (tile_store.cuh); the top-k epilogue keeps its keys there, 4 KB to a warp
-constexpr int OFF_STAGE = (OFF_ABORT + 4 + 127) / 128 * 128;
+constexpr int OFF_STAGE = (OFF_COUNTS + (int)sizeof(PairCounts) + 127) / 128 * 128;
 constexpr int kEpilogueWarps = 16;
 constexpr int SMEM_BYTES = OFF_STAGE + kStoreBytes;
 static_assert(kStoreBytes >= kEpilogueWarps * 4096, "room for the top-k keys");
@@ -330,6 +331,7 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
     uint64_t *tmem_empty = tmem_full + 2;                             // rank 0's: both CTAs have drained the accumulator
     uint32_t *tmem_ptr = reinterpret_cast<uint32_t *>(smem + OFF_TMEM_PTR);
     int *abort_flag = reinterpret_cast<int *>(smem + OFF_ABORT);
+    PairCounts *counts = reinterpret_cast<PairCounts *>(smem + OFF_COUNTS);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const uint32_t rank = cluster_rank();
@@ -406,15 +408,14 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                     }
                 }
             }
-            // after a wait that gave up, stay (bounded) until the copies under way have landed in both CTAs
-            if (!ok && rank == 0)
-                for (uint32_t u = issued > (uint32_t)kSlots ? issued - kSlots : 0; u < issued; ++u) mbar_wait_bounded(&full[u % kSlots], (u / kSlots) & 1);
+            if (ok && !wait_for_releases(empty, issued, kSlots, abort_flag)) give_up(7);
+            publish_pair(&counts->issued[rank], issued);
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer: rank 0, for both CTAs ----------------
         if (lane == 0 && rank == 0) {
             const uint32_t idesc = make_idesc(TM, BN, TF32, AMN);
-            uint32_t s = 0, phase = 0, acount = 0;
+            uint32_t s = 0, phase = 0, acount = 0, used = 0;
             bool ok = true;
             const int kchunk = (P.kchunk > 0 && P.kchunk < nkb) ? P.kchunk : nkb;
             ProductShare<Index> share(P, (nkb + kchunk - 1) / kchunk);
@@ -462,9 +463,12 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                         if (++s == kSlots) { s = 0; phase ^= 1; }
                         if (parts == 1) {
                             tc_commit_pair(&empty[hi]);
+                            ++used;
                             continue;
                         }
                         if (!arrived(5)) {
+                            tc_commit_pair(&empty[hi]);   // for drain_pair: the MMAs above are under way
+                            ++used;
                             ok = false;
                             break;
                         }
@@ -483,11 +487,15 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                         }
                         tc_commit_pair(&empty[hi]); // both slots may be refilled, in both CTAs, once these MMAs have read them
                         tc_commit_pair(&empty[lo]);
+                        used += 2;
                         if (++s == kSlots) { s = 0; phase ^= 1; }
                     }
-                    if (ok) tc_commit_pair(&tmem_full[a]);
+                    if (!ok) break;      // acount: accumulators handed over
+                    tc_commit_pair(&tmem_full[a]);
                 }
             }
+            publish_pair(&counts->used, used);
+            publish_pair(&counts->filled, acount);
         }
     } else {
         // ---------------- epilogue: warps 2..17, TMEM lanes 32*(warp % 4) .. +31 ----------------
@@ -830,6 +838,15 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
     tc_fence_before();
     __syncthreads();
     cluster_sync();   // neither CTA's shared memory goes while the other may still read it or arrive in it
+    if (*reinterpret_cast<volatile int *>(abort_flag)) {   // raised in both CTAs or in neither
+        if (threadIdx.x == 0)
+            drain_pair(full, empty, tmem_full, kSlots, counts, rank, [&](uint32_t u) {
+                const bool high = u % parts == 0;
+                return (uint32_t)((high || need_xl ? A_BYTES : 0) + (high || need_yl ? B_BYTES : 0));
+            });
+        __syncthreads();
+        cluster_sync();
+    }
     if (warp == 1) {
         tc_fence_after();
         tmem_dealloc_pair(tmem_base, kTmemCols);

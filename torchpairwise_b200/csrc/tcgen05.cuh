@@ -2,6 +2,7 @@
 // (gemm_tcgen05.cu: bf16 and tf32 contractions; bool_tcgen05.cu: 8-bit integer counts).
 #pragma once
 #include "common.cuh"
+#include "pair_exit.cuh"
 
 namespace tpw {
 namespace {
@@ -119,6 +120,43 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t *bar, uint32_t parity, vo
         if ((it & 63u) == 63u && (*abort_flag || globaltimer_ns() - t0 > kWaitBudgetNs)) return false;
     }
     return false;
+}
+
+// How far the roles of a pair came, at the same offset of both CTAs' shared memory: operand uses issued by either producer, uses
+// read (their slots' empty barriers committed), accumulators handed to the epilogue.  Written once by each role when it stops.
+struct PairCounts {
+    uint32_t issued[2], used, filled;
+};
+__device__ __forceinline__ void publish_pair(uint32_t *word, uint32_t value) {
+    for (uint32_t r = 0; r < 2; ++r)
+        asm volatile("st.volatile.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr(word, r)), "r"(value) : "memory");
+}
+// bytes of a copy that was never issued, counted as arrived
+__device__ __forceinline__ void mbar_complete_tx(uint64_t *bar, uint32_t bytes) {
+    asm volatile("mbarrier.complete_tx.relaxed.cluster.shared::cluster.b64 [%0], %1;" ::"r"(cluster_addr(bar, 0)), "r"(bytes) : "memory");
+}
+// The producer's last step in a run without errors: the commits that release the slots have arrived in this CTA (pair_exit.cuh).
+__device__ __forceinline__ bool wait_for_releases(uint64_t *empty, uint32_t issued, uint32_t slots, volatile int *abort_flag) {
+    for (uint32_t u = first_of_last_uses(issued, slots); u < issued; ++u)
+        if (!wait_or_abort(&empty[u % slots], parity_of_use(u, slots), abort_flag)) return false;
+    return true;
+}
+// The same after a wait that gave up, by one thread of each CTA when all roles of both have stopped: copies and commits that are still
+// under way arrive, each waited for with the usual bound.  bytes(u): what one CTA copies for use u.
+template <typename F>
+__device__ __noinline__ void drain_pair(uint64_t *full, uint64_t *empty, uint64_t *tmem_full, uint32_t slots, volatile PairCounts *c,
+                                        uint32_t rank, F bytes) {
+    const uint32_t i0 = c->issued[0], i1 = c->issued[1], used = c->used, filled = c->filled;
+    if (rank == 0) {
+        for (uint32_t u = used; u < (i0 > i1 ? i0 : i1); ++u) {
+            const PairDebt debt = debt_of_use(u, i0, i1);
+            if (debt == PairDebt::arm_other) mbar_expect_tx(&full[u % slots], bytes(u));
+            if (debt == PairDebt::forgive) mbar_complete_tx(&full[u % slots], bytes(u));
+        }
+        for (uint32_t u = used; u < (i0 > i1 ? i0 : i1); ++u) mbar_wait_bounded(&full[u % slots], parity_of_use(u, slots));
+    }
+    for (uint32_t u = first_of_last_uses(used, slots); u < used; ++u) mbar_wait_bounded(&empty[u % slots], parity_of_use(u, slots));
+    for (uint32_t u = first_of_last_uses(filled, 2); u < filled; ++u) mbar_wait_bounded(&tmem_full[u % 2], parity_of_use(u, 2));
 }
 
 } // namespace
