@@ -151,9 +151,9 @@ __device__ __forceinline__ float dot_epilogue(float dot, float n1, float n2, boo
     return dist;
 }
 
-// sqrt(x) for x >= 0, two at a time: one step of Newton's iteration for the square root from the approximate reciprocal square
-// root (relative error below 2^-22, so the step leaves only its own rounding: within one float32 of sqrtf).  The term added
-// under the root keeps it away from 1 / 0 and changes no x above 2^-100.  x has to be finite.
+// sqrt(x) for x = 0 or 2^-100 <= x < infinity, two at a time: one step of Newton's iteration for the square root from the
+// approximate reciprocal square root (relative error below 2^-22, so the step leaves only its own rounding: within one float32 of
+// sqrtf).  The term added under the root keeps it away from 1 / 0 and, 2^-126, changes no x of that range.
 __device__ __forceinline__ f32x2 newton_sqrt(f32x2 x) {
     const f32x2 tiny = pack2(1.17549435e-38f, 1.17549435e-38f);
     float a, b, ra, rb;
@@ -163,6 +163,7 @@ __device__ __forceinline__ f32x2 newton_sqrt(f32x2 x) {
     const f32x2 r = pack2(ra, rb), root = mul2(x, r), half = mul2(r, pack2(0.5f, 0.5f));
     return fma2(fma2(mul2(root, pack2(-1.f, -1.f)), root, x), half, root);
 }
+constexpr float kRootLow = 7.88860905e-31f;   // 2^-100
 
 // dot_epilogue for 16 columns of one row, two lanes to an instruction (the same values, the root excepted as above).  With the
 // scalar form, 23 instructions per Euclidean distance, the epilogue and not the contraction was the bound: euclidean
@@ -189,19 +190,25 @@ __device__ __forceinline__ void dot_epilogue16(const uint32_t (&dot)[16], float 
         for (int u = 0; u < 16; ++u) o[u] = fminf(fmaxf(o[u], 0.f), 2.f);
     }
     if (EPI == TPW_DOT_EUCLIDEAN) {
-        float m = 0.f;
+        float most = 0.f, least = INFINITY;
 #pragma unroll
-        for (int u = 0; u < 8; ++u) m = max3_abs(m, o[2 * u], o[2 * u + 1]);
-        if (__any_sync(0xffffffffu, m > 3.402823466e+38f)) {   // an infinite distance somewhere in the warp
-#pragma unroll 1
-            for (int u = 0; u < 16; ++u) {
-                // one element per trip, picked by comparison: the registers have no index
-                float x = o[0];
+        for (int u = 0; u < 8; ++u) {
+            most = max3_abs(most, o[2 * u], o[2 * u + 1]);
+            least = min3(least, o[2 * u], o[2 * u + 1]);
+        }
+        if (__any_sync(0xffffffffu, most > 3.402823466e+38f || least < kRootLow)) {
+            // A distance somewhere in the warp that newton_sqrt does not take.  Small ones are rooted 2^80 times as large, where the
+            // term under the root changes none of them (the smallest subnormal is 2^-149) and multiplying by either power of two is
+            // exact; infinity is its own root.
 #pragma unroll
-                for (int w = 1; w < 16; ++w) x = w == u ? o[w] : x;
-                x = sqrtf(x);
-#pragma unroll
-                for (int w = 0; w < 16; ++w) o[w] = w == u ? x : o[w];
+            for (int u = 0; u < 16; u += 2) {
+                const bool small0 = o[u] < kRootLow, small1 = o[u + 1] < kRootLow;
+                const f32x2 up = pack2(small0 ? 1.2089258196146292e24f : 1.f, small1 ? 1.2089258196146292e24f : 1.f);
+                const f32x2 down = pack2(small0 ? 9.0949470177292824e-13f : 1.f, small1 ? 9.0949470177292824e-13f : 1.f);   // 2^-40
+                float a, b;
+                unpack2(mul2(newton_sqrt(mul2(pack2(o[u], o[u + 1]), up)), down), a, b);
+                o[u] = o[u] > 3.402823466e+38f ? o[u] : a;
+                o[u + 1] = o[u + 1] > 3.402823466e+38f ? o[u + 1] : b;
             }
         } else {
 #pragma unroll
