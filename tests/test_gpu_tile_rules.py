@@ -45,3 +45,22 @@ def test_euclidean_root_of_small_distances(tensor_cores, scale, n2):
     root = sq.double().sqrt()
     root[3], out[3] = 0, 0
     assert bool(((out.double() - root).abs() <= 2 ** -23 * root).all())
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("b,n1,n2", [(1, 1, 5), (2, 7, 300), (1, 8, 257), (2, 9, 31), (1, 17, 64), (1, 500, 3)])
+def test_cosine_backward_column_sums(tpw, dtype, b, n1, n2):
+    """colterm[j] = sum_i d(denominator) n1[i], n1 terms of up to five roundings added one after the other; pairs with a zero norm add nothing."""
+    from torchpairwise_b200 import _abi
+    g = torch.Generator().manual_seed(n1 + n2)
+    up, out = torch.randn(b, n1, n2, generator=g).to(dtype).cuda(), (torch.rand(b, n1, n2, generator=g) * 2).to(dtype).cuda()
+    a, c = (torch.rand(b, n, generator=g).to(dtype).cuda() + 0.5 for n in (n1, n2))
+    a[:, n1 // 2] = 0
+    dm, row, col = torch.empty_like(up), torch.empty_like(a), torch.empty_like(c)
+    _abi.check(_abi.lib.tpw_cosine_backward_prepare(_abi.F32 if dtype == torch.float32 else _abi.F64, _abi.DOT_COSINE_DIST, up.data_ptr(), out.data_ptr(),
+                                                    a.data_ptr(), c.data_ptr(), dm.data_ptr(), row.data_ptr(), col.data_ptr(), b, n1, n2,
+                                                    torch.cuda.current_stream().cuda_stream))
+    den = a.double()[:, :, None] * c.double()[:, None]
+    term = torch.where(den == 0, 0.0, up.double() / den * (1 - out.double())) * a.double()[:, :, None]
+    bound = (n1 + 8) * torch.finfo(dtype).eps * torch.where(den == 0, 0.0, (up.double() / den).abs() * (1 + out.double())).mul(a.double()[:, :, None]).sum(1)
+    assert bool(((col.double() - term.sum(1)).abs() <= bound).all())

@@ -108,12 +108,26 @@ __global__ void cosine_prepare_cols_kernel(const T *g, const T *out, const T *n1
     const long long b = idx / N2, j = idx % N2;
     const T nb = n2[idx];
     T acc = T(0);
-    for (long long i = 0; i < N1; ++i) {
-        const long long e = (b * N1 + i) * N2 + j;
+    const T *na = n1 + b * N1;
+    auto term = [&](T gv, T ov, T n) {
         T dm, dd;
-        cosine_terms(g[e], out[e], n1[b * N1 + i], nb, epilogue, dm, dd);
-        acc += dd * n1[b * N1 + i];
+        cosine_terms(gv, ov, n, nb, epilogue, dm, dd);
+        acc += dd * n;
+    };
+    // Bound: latency, a column's rows one after the other.  The divisions' slow path keeps the compiler from loading ahead of them, so
+    // eight rows are fetched together: [512, 512] float32 149 -> 59 us.
+    long long i = 0;
+    for (; i + 8 <= N1; i += 8) {
+        T gv[8], ov[8], nv[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u) {
+            const long long e = (b * N1 + i + u) * N2 + j;
+            gv[u] = g[e]; ov[u] = out[e]; nv[u] = na[i + u];
+        }
+#pragma unroll
+        for (int u = 0; u < 8; ++u) term(gv[u], ov[u], nv[u]);
     }
+    for (; i < N1; ++i) term(g[(b * N1 + i) * N2 + j], out[(b * N1 + i) * N2 + j], na[i]);
     colterm[idx] = acc;
 }
 
