@@ -64,3 +64,20 @@ def test_cosine_backward_column_sums(tpw, dtype, b, n1, n2):
     term = torch.where(den == 0, 0.0, up.double() / den * (1 - out.double())) * a.double()[:, :, None]
     bound = (n1 + 8) * torch.finfo(dtype).eps * torch.where(den == 0, 0.0, (up.double() / den).abs() * (1 + out.double())).mul(a.double()[:, :, None]).sum(1)
     assert bool(((col.double() - term.sum(1)).abs() <= bound).all())
+
+
+# Gradient products whose tiles are no multiple of the 74 pairs: 1, 28 and 73 left over, in parts of one chunk, of several, and nearly whole.
+@pytest.mark.parametrize("b,n1,n2,d", [(15, 1131, 1393, 192), (1, 7000, 1030, 100), (1, 200, 9000, 130), (7, 900, 1200, 250), (1, 18600, 1100, 64)])
+def test_gradients_of_tiles_that_several_pairs_share(tpw, b, n1, n2, d):
+    """From the distances as they were returned: the coefficients' and the operands' splits and float32 sums of n2 (n1) terms in chunks are
+    within 2^-18 of the terms' magnitudes."""
+    g = torch.Generator().manual_seed(n1)
+    x1, x2 = torch.randn(b, n1, d, generator=g).cuda().requires_grad_(), torch.randn(b, n2, d, generator=g).cuda().requires_grad_()
+    up = torch.randn(b, n1, n2, generator=g).cuda()
+    out = tpw.euclidean_distances(x1, x2)
+    g1, g2 = torch.autograd.grad(out, (x1, x2), up)
+    c = up.double() / out.detach().double()
+    for got, x, y, m in ((g1, x1.detach().double(), x2.detach().double(), c), (g2, x2.detach().double(), x1.detach().double(), c.transpose(1, 2))):
+        want = m.sum(2, keepdim=True) * x - m @ y
+        size = m.abs().sum(2, keepdim=True) * x.abs() + m.abs() @ y.abs()
+        assert bool(((got - want).abs() <= 2 ** -18 * size).all())

@@ -860,38 +860,58 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
     }
 }
 
-// Tiles whose chunks several pairs share: the parts' sums, added in the order of the chunks.  One CTA per 16 rows of a tile.
+// Tiles whose chunks several pairs share: the parts' sums, added in the order of the chunks; ROWS rows of a tile to a CTA.  What it takes is
+// the parts' latency.  A tile or two left over lie in many parts (one for every chunk or two) and make few CTAs: four rows and eight parts in
+// flight; many tiles lie in two or three each: sixteen rows.  [15, 1131, 1393, 192], 1 and 16 tiles left over: 47 us for both launches when
+// parts were read one at a time, each behind three 64-bit divisions for its place; 14 now.
+template <int ROWS>
 __global__ void __launch_bounds__(BN)
 product_fixup_kernel(const GemmParams P, int nch, long long pairs) {
-    const long long left = P.tiles % pairs, base = P.tiles - left, local = blockIdx.x / (TM / 16), tile = base + local;
-    const int row0 = (int)(blockIdx.x % (TM / 16)) * 16, col = threadIdx.x;
+    constexpr int PARTS = 32 / ROWS;
+    __shared__ int parts[BN], before[BN / 32];      // deals_chunks: no more pairs than threads
+    const long long left = P.tiles % pairs, base = P.tiles - left, local = blockIdx.x / (TM / ROWS), tile = base + local;
+    const int row0 = (int)(blockIdx.x % (TM / ROWS)) * ROWS, col = threadIdx.x, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     const long long all = left * nch, u0 = local * nch, u1 = u0 + nch;
-    auto start_of = [&](long long c) { return all * c / pairs; };
-    long long c = u0 * pairs / all;                 // the share that holds chunk u0, up to rounding
-    while (c > 0 && start_of(c) > u0) --c;
-    while (start_of(c + 1) <= u0) ++c;
-    if (start_of(c + 1) >= u1) return;              // one pair had the whole tile
+    // the shares that hold chunks of this tile, shares without chunks (fewer chunks than pairs) left out: one thread looks at each
+    const int c = threadIdx.x;
+    const bool narrow = all * BN < (1ll << 31);     // 32-bit divisions do
+    const long long begin = narrow ? (int)all * c / (int)pairs : all * c / pairs, end = narrow ? (int)all * (c + 1) / (int)pairs : all * (c + 1) / pairs;
+    const bool holds = c < pairs && begin < end && begin < u1 && end > u0;
+    const uint32_t vote = __ballot_sync(0xffffffffu, holds);
+    if (lane == 0) before[warp] = __popc(vote);
+    __syncthreads();
+    int n = 0, at = __popc(vote & ((1u << lane) - 1));
+#pragma unroll
+    for (int w = 0; w < BN / 32; ++w) {
+        if (w < warp) at += before[w];
+        n += before[w];
+    }
+    if (holds) parts[at] = c * 2 + (begin >= u0 ? 0 : 1);
+    __syncthreads();
+    if (n == 1) return;                             // one pair had the whole tile
     long long t = tile;
     const long long tn = t % P.tiles_n; t /= P.tiles_n;
     const long long tm = t % P.tiles_m;
     const long long b = t / P.tiles_m;
     const long long j = tn * BN + col;
-    if (j >= P.N2) return;
-    float s[16];
+    const int rows = P.N1 - tm * TM - row0 < ROWS ? (int)(P.N1 - tm * TM - row0) : ROWS;
+    if (j >= P.N2 || rows <= 0) return;
+    const float *src = P.partial + row0 * BN + col;
+    float s[ROWS] = {};
+    for (int k = 0; k < n; k += PARTS) {
+        float v[PARTS][ROWS];
 #pragma unroll
-    for (int r = 0; r < 16; ++r) s[r] = 0.f;
-    for (; c < pairs && start_of(c) < u1; ++c) {
-        if (start_of(c + 1) == start_of(c)) continue;   // fewer chunks than pairs: an empty share
-        const float *src = P.partial + (c * 2 + (start_of(c) >= u0 ? 0 : 1)) * (TM * BN) + row0 * BN + col;
+        for (int u = 0; u < PARTS; ++u)
 #pragma unroll
-        for (int r = 0; r < 16; ++r)
-            if (tm * TM + row0 + r < P.N1) s[r] += src[r * BN];
+            for (int r = 0; r < ROWS; ++r) v[u][r] = k + u < n && r < rows ? src[(long long)parts[k + u] * (TM * BN) + r * BN] : 0.f;
+#pragma unroll
+        for (int u = 0; u < PARTS; ++u)
+#pragma unroll
+            for (int r = 0; r < ROWS; ++r) s[r] += v[u][r];
     }
 #pragma unroll
-    for (int r = 0; r < 16; ++r) {
-        const long long i = tm * TM + row0 + r;
-        if (i < P.N1) P.out[(b * P.N1 + i) * P.N2 + j] = s[r];
-    }
+    for (int r = 0; r < ROWS; ++r)
+        if (r < rows) P.out[(b * P.N1 + tm * TM + row0 + r) * P.N2 + j] = s[r];
 }
 
 // fp32 rows -> bf16 high/low parts (row pitch Dp, zero padded) and a per-row fp32 scalar: the
@@ -1237,7 +1257,7 @@ inline long long product_tiles(long long B, long long M, long long N) { return B
 inline bool deals_chunks(long long B, long long M, long long N, long long K) {
     const long long tiles = product_tiles(B, M, N), pairs = pair_count(), left = tiles % pairs;
     // one wave more or less in a long queue, or a tile of a few chunks, is not worth the second kernel
-    return tiles <= 8 * pairs && product_chunks(K) >= 16 && product_chunks(K) < (1 << 20) && left > 0 && left * 100 < pairs * 92;
+    return pairs <= BN && tiles <= 8 * pairs && product_chunks(K) >= 16 && product_chunks(K) < (1 << 20) && left > 0 && left * 100 < pairs * 92;
 }
 inline long long product_pairs(long long B, long long M, long long N, long long K, bool room) {
     const long long tiles = product_tiles(B, M, N), pairs = pair_count();
@@ -1346,7 +1366,9 @@ int launch_tf32_product(const Tf32Operand &A, const Tf32Operand &Bm, float *out,
 #undef TPW_TF32_LAUNCH
     TPW_LAUNCH_OK("gemm_metric_kernel (tf32)");
     if (P.partial && P.tiles % pairs != 0) {
-        product_fixup_kernel<<<(unsigned)(P.tiles % pairs * (TM / 16)), BN, 0, s>>>(P, (int)product_chunks(K), pairs);
+        const long long left = P.tiles % pairs;
+        if (left * (TM / 16) < 2 * sm_count()) product_fixup_kernel<4><<<(unsigned)(left * (TM / 4)), BN, 0, s>>>(P, (int)product_chunks(K), pairs);
+        else product_fixup_kernel<16><<<(unsigned)(left * (TM / 16)), BN, 0, s>>>(P, (int)product_chunks(K), pairs);
         TPW_LAUNCH_OK("product_fixup_kernel");
     }
     return TPW_OK;
