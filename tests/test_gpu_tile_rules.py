@@ -81,3 +81,15 @@ def test_gradients_of_tiles_that_several_pairs_share(tpw, b, n1, n2, d):
         want = m.sum(2, keepdim=True) * x - m @ y
         size = m.abs().sum(2, keepdim=True) * x.abs() + m.abs() @ y.abs()
         assert bool(((got - want).abs() <= 2 ** -18 * size).all())
+
+
+@pytest.mark.parametrize("lead,n1", [((), 128), ((), 129), ((), 256), ((), 257), ((), 300), ((), 385), ((3,), 300), ((2,), 640)])
+@pytest.mark.parametrize("n2", [300, 2049, 30011])
+def test_nearest_row_where_the_last_tile_is_half_empty(tensor_cores, lead, n1, n2):
+    """The smallest of the row of distances that the same engine stores, and a column that holds it."""
+    g = torch.Generator().manual_seed(n1 + n2)
+    x1, x2 = torch.randn(*lead, n1, 72, generator=g).cuda(), torch.randn(*lead, n2, 72, generator=g).cuda()
+    x1[..., -1, :] = x2[..., n2 - 1, :]
+    at, nearest = tensor_cores.pairwise_argmin_min(x1, x2, "sqeuclidean")
+    sq = tensor_cores.sqeuclidean_distances(x1, x2)
+    assert torch.equal(nearest, sq.amin(-1)) and torch.equal(sq.gather(-1, at.unsqueeze(-1)).squeeze(-1), nearest)
