@@ -93,3 +93,45 @@ def test_nearest_row_where_the_last_tile_is_half_empty(tensor_cores, lead, n1, n
     at, nearest = tensor_cores.pairwise_argmin_min(x1, x2, "sqeuclidean")
     sq = tensor_cores.sqeuclidean_distances(x1, x2)
     assert torch.equal(nearest, sq.amin(-1)) and torch.equal(sq.gather(-1, at.unsqueeze(-1)).squeeze(-1), nearest)
+
+
+@pytest.mark.parametrize("lead,n1,n2,d", [((), 5003, 4111, 167), ((), 6001, 6003, 167), ((3,), 6001, 2003, 1024), ((), 2300, 9999, 1024), ((5,), 2100, 1031, 1100), ((), 385, 259, 4096)])
+def test_ragged_boolean_counts_in_steady_state(tpw, lead, n1, n2, d):
+    from torchpairwise_b200 import _abi
+    assert _abi.lib.tpw_bool_rows_pitch(lead[0] if lead else 1, n1, n2, d) > 0          # the tensor cores' problem
+    g = torch.Generator().manual_seed(d)
+    x1, x2 = (torch.rand(*lead, n1, d, generator=g) < 0.2).cuda(), (torch.rand(*lead, n2, d, generator=g) < 0.2).cuda()
+    both = x1.float() @ x2.float().transpose(-1, -2)          # below 2^24: exact
+    a, b = x1.float().sum(-1)[..., :, None], x2.float().sum(-1)[..., None, :]
+    union, differ = a + b - both, a + b - 2 * both
+    zero = torch.zeros((), device="cuda")
+    assert torch.equal(tpw.jaccard_distances(x1, x2), torch.where(union == 0, zero, differ / union))
+    assert torch.equal(tpw.hamming_distances(x1, x2), differ / torch.tensor(float(d), device="cuda"))
+
+
+@pytest.mark.parametrize("b,n1,n2", [(1, 3000, 4112), (3, 700, 1024), (1, 4400, 2308), (2, 300, 260), (1, 6000, 6004)])
+@pytest.mark.parametrize("d", [256, 720, 1040, 2064])
+def test_boolean_results_on_and_off_the_16_byte_grid_agree(tpw, b, n1, n2, d):
+    """Whichever form of the kernel runs -- it depends on the metric, on the features, on the result's size and on whether its rows start on
+    16-byte boundaries -- writes the same bits, the popcount kernel's, and nothing beside them."""
+    from torchpairwise_b200 import _abi
+    g = torch.Generator().manual_seed(n1)
+    x1, x2 = (torch.rand(b, n1, d, generator=g) < 0.3).cuda(), (torch.rand(b, n2, d, generator=g) < 0.3).cuda()
+    pop1, pop2 = x1.sum(-1, dtype=torch.int32), x2.sum(-1, dtype=torch.int32)
+    if b * n1 * n2 * d < 1 << 28:
+        pytest.skip("too small for the tensor cores")
+    words = (d + 127) // 128 * 4
+    w1, w2 = (torch.empty(b, n, words, dtype=torch.int32, device="cuda") for n in (n1, n2))
+    for x, w, pop, n in ((x1, w1, pop1, n1), (x2, w2, pop2, n2)):
+        _abi.check(_abi.lib.tpw_bitpack(x.data_ptr(), w.data_ptr(), pop.data_ptr(), b * n, d, words, torch.cuda.current_stream().cuda_stream))
+    for metric in (_abi.BOOL_METRICS[name] for name in ("jaccard", "eq_mean", "and_sum", "yule", "dice")):
+        res = [torch.empty(b * n1 * n2, device="cuda")]
+        _abi.check(_abi.lib.tpw_bool_metric_forward(metric, w1.data_ptr(), w2.data_ptr(), pop1.data_ptr(), pop2.data_ptr(), res[0].data_ptr(), b, n1, n2, d, words,
+                                                    torch.cuda.current_stream().cuda_stream))
+        for off in (0, 1):
+            buf = torch.full((b * n1 * n2 + 8,), -7.0, device="cuda")
+            _abi.check(_abi.lib.tpw_bool_metric_forward_tc(metric, x1.data_ptr(), x2.data_ptr(), pop1.data_ptr(), pop2.data_ptr(),
+                                                           buf.data_ptr() + 4 * off, b, n1, n2, d, torch.cuda.current_stream().cuda_stream))
+            assert bool((buf[:off] == -7).all()) and bool((buf[off + b * n1 * n2:] == -7).all())
+            res.append(buf[off:off + b * n1 * n2].clone())
+        assert torch.equal(res[0].view(torch.int32), res[1].view(torch.int32)) and torch.equal(res[0].view(torch.int32), res[2].view(torch.int32)), metric

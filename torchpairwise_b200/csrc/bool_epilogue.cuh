@@ -91,10 +91,12 @@ __device__ __forceinline__ float bool_epilogue(int metric, int n11, int a, int b
 // the quotient is quotient_of_counts, so the results are bool_epilogue's bit for bit; 6.5 arithmetic instructions per jaccard
 // distance where the integer form takes 14, and 4 for a mean where D is no power of two.
 // n0, n1: the two counts as integers; a2: |x| in both lanes; b2: |y| of the two columns.
+constexpr bool has_packed_epilogue(int metric) {
+    return metric == TPW_BOOL_AND_SUM || metric == TPW_BOOL_OR_SUM || metric == TPW_BOOL_XOR_SUM || metric == TPW_BOOL_NE_SUM ||
+           metric == TPW_BOOL_EQ_SUM || metric == TPW_BOOL_EQ_MEAN || metric == TPW_BOOL_NE_MEAN || metric == TPW_BOOL_JACCARD;
+}
 template <int METRIC>
-constexpr bool kPackedEpilogue = METRIC == TPW_BOOL_AND_SUM || METRIC == TPW_BOOL_OR_SUM || METRIC == TPW_BOOL_XOR_SUM ||
-                                 METRIC == TPW_BOOL_NE_SUM || METRIC == TPW_BOOL_EQ_SUM || METRIC == TPW_BOOL_EQ_MEAN ||
-                                 METRIC == TPW_BOOL_NE_MEAN || METRIC == TPW_BOOL_JACCARD;
+constexpr bool kPackedEpilogue = has_packed_epilogue(METRIC);
 template <int METRIC, int INV>
 __device__ __forceinline__ f32x2 bool_epilogue_packed(uint32_t n0, uint32_t n1, f32x2 a2, f32x2 b2, float D, float inv_d) {
     const float kMagic = 8388608.f;   // 2^23: its mantissa takes a count as it is

@@ -369,7 +369,7 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
     tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr;
     auto give_up = [&](int site) {
-        raise_abort_pair(abort_flag);
+        raise_abort(abort_flag, 2);
         if (P.status) atomicCAS(P.status, 0, (4 << 16) | site);
     };
     // Operands that the high parts hold exactly (16-bit inputs, small integers) have no low parts: their tiles are neither
@@ -420,7 +420,7 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                 }
             }
             if (ok && !wait_for_releases(empty, issued, kSlots, abort_flag)) give_up(7);
-            publish_pair(&counts->issued[rank], issued);
+            publish(&counts->issued[rank], issued, 2);
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer: rank 0, for both CTAs ----------------
@@ -505,8 +505,8 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                     tc_commit_pair(&tmem_full[a]);
                 }
             }
-            publish_pair(&counts->used, used);
-            publish_pair(&counts->filled, acount);
+            publish(&counts->used, used, 2);
+            publish(&counts->filled, acount, 2);
         }
     } else {
         // ---------------- epilogue: warps 2..17, TMEM lanes 32*(warp % 4) .. +31 ----------------

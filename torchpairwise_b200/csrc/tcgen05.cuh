@@ -44,6 +44,23 @@ __device__ __forceinline__ void tc_commit_pair(uint64_t *bar) {   // arrives at 
         "h"((uint16_t)3)
         : "memory");
 }
+// the same for a CTA by itself
+__device__ __forceinline__ void tmem_alloc(uint32_t *smem_dst, uint32_t ncols) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(smem_dst)), "r"(ncols)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void tmem_dealloc(uint32_t taddr, uint32_t ncols) {
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
+}
+template <bool PAIR>
+__device__ __forceinline__ void tc_commit(uint64_t *bar) {
+    if (PAIR)
+        tc_commit_pair(bar);
+    else
+        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar))
+                     : "memory");
+}
 // copy into this CTA's shared memory that completes on a barrier of the pair (shared::cluster address)
 __device__ __forceinline__ void tma_load_3d_pair(void *dst, const CUtensorMap *map, uint32_t cluster_bar, int c0, int c1, int c2) {
     asm volatile(
@@ -52,6 +69,18 @@ __device__ __forceinline__ void tma_load_3d_pair(void *dst, const CUtensorMap *m
         "l"(reinterpret_cast<uint64_t>(map)), "r"(c0), "r"(c1), "r"(c2), "r"(cluster_bar)
         : "memory");
 }
+// Shared memory written by threads and then read by the copy engine; 3-D tiled store shared -> global as a bulk async-group (the tensor
+// map clips what lies outside the tensor; c0 must keep c0 * element size a multiple of 16 bytes and no coordinate may be negative),
+// its commit, and the wait until every committed store has read its shared-memory source.
+__device__ __forceinline__ void fence_proxy_async_smem() { asm volatile("fence.proxy.async.shared::cta;" ::: "memory"); }
+__device__ __forceinline__ void tma_store_3d(const CUtensorMap *map, const void *src, int c0, int c1, int c2) {
+    asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%1, %2, %3}], [%4];" ::"l"(
+                     reinterpret_cast<uint64_t>(map)),
+                 "r"(c0), "r"(c1), "r"(c2), "r"(smem_u32(src))
+                 : "memory");
+}
+__device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+__device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
 // try_wait on a barrier at which threads of the other CTA arrive
 __device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t *bar, uint32_t parity) {
     uint32_t ok;
@@ -104,9 +133,9 @@ __device__ __forceinline__ uint64_t make_smem_desc(uint32_t smem_addr) {
     d |= (uint64_t)2 << 61;
     return d;
 }
-// Raises the abort flag of both CTAs of a pair (the flag lies at the same offset in both).
-__device__ __forceinline__ void raise_abort_pair(int *abort_flag) {
-    for (uint32_t r = 0; r < 2; ++r)
+// Raises the abort flag of both CTAs of a pair (the flag lies at the same offset in both), or of the one CTA.
+__device__ __forceinline__ void raise_abort(int *abort_flag, uint32_t ctas) {
+    for (uint32_t r = 0; r < ctas; ++r)
         asm volatile("st.volatile.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr(abort_flag, r)), "r"(1) : "memory");
 }
 // Bounded mbarrier wait that also gives up when another role raised the abort flag.  PAIR: threads of the other CTA arrive too.
@@ -127,8 +156,8 @@ __device__ __forceinline__ bool wait_or_abort(uint64_t *bar, uint32_t parity, vo
 struct PairCounts {
     uint32_t issued[2], used, filled;
 };
-__device__ __forceinline__ void publish_pair(uint32_t *word, uint32_t value) {
-    for (uint32_t r = 0; r < 2; ++r)
+__device__ __forceinline__ void publish(uint32_t *word, uint32_t value, uint32_t ctas) {
+    for (uint32_t r = 0; r < ctas; ++r)
         asm volatile("st.volatile.shared::cluster.u32 [%0], %1;" ::"r"(cluster_addr(word, r)), "r"(value) : "memory");
 }
 // bytes of a copy that was never issued, counted as arrived
