@@ -135,3 +135,31 @@ def test_boolean_results_on_and_off_the_16_byte_grid_agree(tpw, b, n1, n2, d):
             assert bool((buf[:off] == -7).all()) and bool((buf[off + b * n1 * n2:] == -7).all())
             res.append(buf[off:off + b * n1 * n2].clone())
         assert torch.equal(res[0].view(torch.int32), res[1].view(torch.int32)) and torch.equal(res[0].view(torch.int32), res[2].view(torch.int32)), metric
+
+
+# More tiles than two for each of the 74 pairs of SMs, or each of the 148 SMs, so that accumulators, slots and staging areas are used
+# again, with last column tiles of one 64-column pass among them: rows of the result off the 16-byte grid and on it, few and many
+# features, results within L2 and larger, which take a CTA by itself or a pair to a tile.
+STEADY = [((), 5003, 4111, 72), ((), 2300, 9999, 65), ((5,), 2100, 1031, 64), ((), 6200, 6001, 64), ((), 5003, 4111, 264), ((), 5003, 4112, 72),
+          ((3,), 2100, 2052, 100), ((), 5003, 4112, 200), ((3,), 2100, 2052, 200)]
+EDGES = [((), n1, n2, d) for n1, n2 in [(128, 256), (129, 257), (256, 259), (257, 511), (385, 300), (700, 1026), (700, 1028)] for d in (64, 136, 320)]
+
+
+@pytest.mark.parametrize("lead,n1,n2,d", STEADY + EDGES)
+def test_contractions_of_one_cta_and_of_pairs(tensor_cores, lead, n1, n2, d):
+    """The three-product split of the distances drops at most 2^-15 |x| |y| of a dot product, float32 sums of d terms and the epilogue add
+    (d + 8) 2^-24 of |x|^2 + |y|^2; the plain product's split drops 2^-20 |x| |y|."""
+    g = torch.Generator().manual_seed(n1 + d)
+    x1, x2 = torch.randn(*lead, n1, d, generator=g).cuda(), torch.randn(*lead, n2, d, generator=g).cuda()
+    a, b = x1.double(), x2.double()
+    na, nb = a.norm(dim=-1)[..., :, None], b.norm(dim=-1)[..., None, :]
+    bound = 2 ** -14 * na * nb + (d + 8) * 2 ** -24 * (na ** 2 + nb ** 2)
+    dot = a @ b.transpose(-1, -2)
+    sq = na ** 2 + nb ** 2 - 2 * dot
+    assert bool(((tensor_cores.sqeuclidean_distances(x1, x2) - sq).abs() <= bound).all())
+    assert bool(((tensor_cores.euclidean_distances(x1, x2).double() ** 2 - sq).abs() <= 1.01 * bound + 2 ** -22 * sq).all())
+    assert bool(((tensor_cores.cosine_distances(x1, x2) - (1 - dot / (na * nb))).abs() <= bound / (na * nb)).all())
+    assert bool(((tensor_cores.linear_kernel(x1, x2) - dot).abs() <= ((d + 8) * 2 ** -24 + 2 ** -20) * na * nb).all())
+    if not lead:
+        own = tensor_cores.sqeuclidean_distances(x1, x1)
+        assert bool((own.diagonal() == 0).all()) and bool(((own - (na ** 2 + na.T ** 2 - 2 * a @ a.T)).abs() <= 2 ** -14 * na * na.T + (d + 8) * 2 ** -24 * (na ** 2 + na.T ** 2)).all())

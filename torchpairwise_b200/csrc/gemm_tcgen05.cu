@@ -9,17 +9,19 @@
 // fp32 rounding of the sum).  Row norms are summed in fp32 from the unsplit values by the same
 // pre-pass.
 //
-// Kernel.  Persistent, one CTA per SM in pairs (clusters of two, cta_group::2), 576 threads: warp 0 = TMA producer (one lane),
-// warp 1 = tensor-memory owner and, in rank 0, MMA issuer for both CTAs (one lane), warps 2..17 = epilogue.  A pair's output
+// Kernel.  Persistent, one CTA per SM, in pairs (clusters of two, cta_group::2) or by itself (single_pays), 576 threads: warp 0 = TMA producer
+// (one lane), warp 1 = tensor-memory owner and, in rank 0, MMA issuer for both CTAs (one lane), warps 2..17 = epilogue.  A pair's output
 // tile is 256 x 256, 128 rows to a CTA; k-step 64 bf16 = one 128-byte swizzled row.  The ring has five slots of 32 KB: the CTA's 128
 // rows of x and its half, 128 rows, of y, high and low parts in turn.  The 512 TMEM columns hold two 128 x 256 fp32
-// accumulators per CTA, so the epilogue of tile t overlaps the MMAs of tile t + 1.  Where the tile is stored all sixteen
+// accumulators per CTA, so the epilogue of tile t overlaps the MMAs of tile t + 1.  Where a pair's tile is stored all sixteen
 // epilogue warps drain it, four to a TMEM lane quarter, each 16 of every 64 columns; of the row-minimum and top-k epilogues
 // eight warps own each accumulator, two to a lane quarter, each half of the columns.
 // Why pairs: L2 -> SM traffic stands at 35 to 43 bytes a clock and SM whatever runs beside it.  A 128 x 256 tile per CTA takes 96 KB of
 // operands per 1536 tensor-core clocks; a pair takes 64 KB, which the tensor cores wait for no longer (sqeuclidean [16384, 16384,
 // 512] without its stores: 700 thousand clocks where the MMAs alone are 688), and less energy: under the power cap sqeuclidean [131072,
 // 16384, 512] 6.15 -> 5.55 ms.  Every CTA fetches its own rows, with plain TMA loads, from this GPU's memory.
+// A CTA by itself has a tile of 128 x 256 and three slots of 48 KB; each of its warps drains 64 columns (of the plain products of
+// tf32 parts, eight warps, 128 columns and four slots) and stores them in blocks of 32 x 32 without meeting another.
 //
 // Three more instantiations share the pipeline: (1) kind::tf32 operands (high/low tf32 parts in fp32
 // containers, 32 elements per k-step) for the gradient products of the backward and for plain dot
@@ -49,24 +51,26 @@ constexpr int TM = 2 * BM;        // rows of x1 per tile of a pair
 constexpr int BN = 256;           // rows of x2 per tile (TMEM columns per accumulator)
 constexpr int HN = BN / 2;        // of which each CTA stages half
 constexpr int BK = 64;            // bf16 per k-step: 128 bytes
-constexpr int kSlots = 5;
 constexpr int kMmasPerStep = 4;    // a 128-byte operand row feeds four MMAs of 32 bytes (16 bf16 or 8 tf32) each
 constexpr int A_BYTES = BM * BK * 2;          // 16 KB
-constexpr int B_BYTES = HN * BK * 2;          // 16 KB
-constexpr int SLOT_BYTES = A_BYTES + B_BYTES; // one part (high or low) of a k-step
-constexpr int OFF_BAR = kSlots * SLOT_BYTES;
-// barriers: full[5], empty[5], tmem_full[2], tmem_empty[2]; then the TMEM base address, the abort flag and the pair's counts
-constexpr int OFF_TMEM_PTR = OFF_BAR + (2 * kSlots + 4) * 8;
-constexpr int OFF_ABORT = OFF_TMEM_PTR + 4;
-constexpr int OFF_COUNTS = OFF_ABORT + 4;
-// staging of the stored tiles (tile_store.cuh); the top-k epilogue keeps its keys there, 4 KB to a warp
-constexpr int OFF_STAGE = (OFF_COUNTS + (int)sizeof(PairCounts) + 127) / 128 * 128;
-constexpr int kEpilogueWarps = 16;
-constexpr int SMEM_BYTES = OFF_STAGE + kStoreBytes;
-static_assert(kStoreBytes >= kEpilogueWarps * 4096, "room for the top-k keys");
-constexpr int SMEM_ALLOC = SMEM_BYTES + 1024;
-static_assert(SMEM_ALLOC <= 232448, "exceeds the dynamic shared memory of one CTA");
-constexpr int kThreads = 64 + 32 * kEpilogueWarps;
+// Shared memory of a pair's CTA and of a CTA by itself (single_pays): the ring of operand slots, one part (high or low) of a k-step each,
+// barriers full, empty [kSlots], tmem_full[2], tmem_empty[2], the TMEM base address, the abort flag and the pair's counts; staging
+// of the stored tiles (tile_store.cuh; 4 KB to a warp of a CTA by itself), where the top-k epilogue keeps its keys, 4 KB to a warp.
+template <bool PAIR, bool TF32 = false> struct Ring {
+    // a tf32 product by itself has eight epilogue warps, half of the staging, and with it a fourth slot: a tile of 64 features
+    static constexpr int kSlots = PAIR ? 5 : TF32 ? 4 : 3, kWarps = PAIR || !TF32 ? 16 : 8, kThreads = 64 + 32 * kWarps;
+    static constexpr int B_BYTES = (PAIR ? HN : BN) * BK * 2;
+    static constexpr int SLOT_BYTES = A_BYTES + B_BYTES;
+    static constexpr int OFF_BAR = kSlots * SLOT_BYTES;
+    static constexpr int OFF_TMEM_PTR = OFF_BAR + (2 * kSlots + 4) * 8;
+    static constexpr int OFF_ABORT = OFF_TMEM_PTR + 4;
+    static constexpr int OFF_COUNTS = OFF_ABORT + 4;
+    static constexpr int OFF_STAGE = (OFF_COUNTS + (int)sizeof(PairCounts) + 127) / 128 * 128;
+    static constexpr int SMEM_ALLOC = OFF_STAGE + (PAIR ? kStoreBytes : kWarps * 4096) + 1024;
+    static_assert(SMEM_ALLOC <= 232448, "exceeds the dynamic shared memory of one CTA");
+};
+static_assert(kStoreBytes >= Ring<true>::kWarps * 4096, "room for the top-k keys");
+constexpr int SMEM_ALLOC = Ring<true>::SMEM_ALLOC, kThreads = Ring<true>::kThreads;
 constexpr uint32_t kTmemCols = 512;
 
 struct GemmParams {
@@ -98,22 +102,20 @@ struct GemmParams {
 
 // D[tmem] (+)= A[smem] * B[smem]^T, fp32 accumulate; TF32 = false: bf16 operands (K = 16 per
 // instruction), true: tf32 operands in 32-bit containers (K = 8 per instruction)
-template <bool TF32>
+template <bool TF32, bool PAIR>
 __device__ __forceinline__ void tc_mma(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-    if (TF32)
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::2.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-            ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-            : "memory");
-    else
-        asm volatile(
-            "{\n\t.reg .pred p;\n\t"
-            "setp.ne.b32 p, %4, 0;\n\t"
-            "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-            ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-            : "memory");
+#define TPW_MMA(GROUP, KIND)                                                                                              \
+    asm volatile(                                                                                                         \
+        "{\n\t.reg .pred p;\n\t"                                                                                          \
+        "setp.ne.b32 p, %4, 0;\n\t"                                                                                       \
+        "tcgen05.mma.cta_group::" GROUP ".kind::" KIND " [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem_d),                        \
+        "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)                                                               \
+        : "memory")
+    if (TF32 && PAIR) TPW_MMA("2", "tf32");
+    else if (TF32) TPW_MMA("1", "tf32");
+    else if (PAIR) TPW_MMA("2", "f16");
+    else TPW_MMA("1", "f16");
+#undef TPW_MMA
 }
 // MN-major 32-bit tile: the only layout tcgen05 takes for it is the 128-byte swizzle with 32-byte
 // atoms (layout type 1): rows of 128 bytes are k, four rows form one 512-byte atom (stride between
@@ -292,10 +294,10 @@ struct ProductShare {
     I tile_at, tile_last, base;   // whole tiles; first tile of those dealt out
     int stride, nch;
     int at, last;                 // this pair's chunks of the tiles dealt out
-    __device__ __forceinline__ ProductShare(const GemmParams &P, int nch_) {
+    __device__ __forceinline__ ProductShare(const GemmParams &P, int nch_, int ctas) {   // ctas: 2, or 1 where a CTA works by itself
         nch = nch_;
-        const int pair = (int)(blockIdx.x >> 1);
-        stride = (int)(gridDim.x >> 1);
+        const int pair = (int)blockIdx.x / ctas;
+        stride = (int)gridDim.x / ctas;
         const long long left = P.partial ? P.tiles % stride : 0, all = left * nch;
         base = (I)(P.tiles - left);
         tile_at = (I)pair;
@@ -329,32 +331,35 @@ __device__ __forceinline__ bool rank_1_is_idle(long long tm, const GemmParams &P
 // the tile's M values contiguously, so a matrix can be contracted over its row index without a
 // transposed copy.  Such a tile is staged as blocks of {32 values, 32 k-rows} (one TMA box each, 4 KB,
 // 128-byte swizzle with 32-byte atoms): block m holds values 32m..32m+31, an MMA consumes 8 k-rows = 1024 bytes.
-template <int EPI, bool SELF, bool TF32, bool ROWMIN = false, bool AMN = false, int TOPK = 0>
-__global__ void __cluster_dims__(2, 1, 1) __launch_bounds__(kThreads, 1)
+template <int EPI, bool SELF, bool TF32, bool ROWMIN = false, bool AMN = false, int TOPK = 0, bool PAIR = true>
+__global__ void __cluster_dims__(PAIR ? 2 : 1, 1, 1) __launch_bounds__(Ring<PAIR, TF32>::kThreads, 1)
 gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_constant__ CUtensorMap map_xl,
                    const __grid_constant__ CUtensorMap map_yh, const __grid_constant__ CUtensorMap map_yl,
                    const GemmParams P) {
+    typedef Ring<PAIR, TF32> L;
+    constexpr int kSlots = L::kSlots, B_BYTES = L::B_BYTES, SLOT_BYTES = L::SLOT_BYTES, kCtas = PAIR ? 2 : 1, kTileRows = kCtas * BM;
     extern __shared__ unsigned char smem_raw[];
     unsigned char *smem = reinterpret_cast<unsigned char *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
-    uint64_t *full = reinterpret_cast<uint64_t *>(smem + OFF_BAR);   // rank 0's: both CTAs' copies of a slot have landed
+    uint64_t *full = reinterpret_cast<uint64_t *>(smem + L::OFF_BAR);   // rank 0's: both CTAs' copies of a slot have landed
     uint64_t *empty = full + kSlots;
     uint64_t *tmem_full = empty + kSlots;
     uint64_t *tmem_empty = tmem_full + 2;                             // rank 0's: both CTAs have drained the accumulator
-    uint32_t *tmem_ptr = reinterpret_cast<uint32_t *>(smem + OFF_TMEM_PTR);
-    int *abort_flag = reinterpret_cast<int *>(smem + OFF_ABORT);
-    PairCounts *counts = reinterpret_cast<PairCounts *>(smem + OFF_COUNTS);
+    uint32_t *tmem_ptr = reinterpret_cast<uint32_t *>(smem + L::OFF_TMEM_PTR);
+    int *abort_flag = reinterpret_cast<int *>(smem + L::OFF_ABORT);
+    PairCounts *counts = reinterpret_cast<PairCounts *>(smem + L::OFF_COUNTS);
 
     const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-    const uint32_t rank = cluster_rank();
+    const uint32_t rank = PAIR ? cluster_rank() : 0;
     constexpr int BKE = TF32 ? BK / 2 : BK; // operand elements per k-step
     constexpr bool STORED = !ROWMIN && TOPK == 0;
-    constexpr int kDrains = STORED ? kEpilogueWarps : kEpilogueWarps / 2;   // warps of a CTA that drain one accumulator
+    static_assert(PAIR || (STORED && !AMN), "a CTA by itself stores plain tiles");
+    constexpr int kDrains = STORED ? L::kWarps : L::kWarps / 2;   // warps of a CTA that drain one accumulator
     typedef std::conditional_t<TF32, int, long long> Index;   // a stored product has fewer than 2^31 tiles
     const int nkb = (int)((P.D + BKE - 1) / BKE);
 
     if (threadIdx.x == 0) {
         for (int s = 0; s < kSlots; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], 1); }
-        for (int a = 0; a < 2; ++a) { mbar_init(&tmem_full[a], 1); mbar_init(&tmem_empty[a], 2 * kDrains); }
+        for (int a = 0; a < 2; ++a) { mbar_init(&tmem_full[a], 1); mbar_init(&tmem_empty[a], kCtas * kDrains); }
         *abort_flag = 0;
         mbar_init_fence();
         tma_prefetch_descriptor(&map_xh);
@@ -362,14 +367,16 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
         tma_prefetch_descriptor(&map_yh);
         tma_prefetch_descriptor(&map_yl);
     }
-    if (warp == 1) tmem_alloc_pair(tmem_ptr, kTmemCols);
+    if (warp == 1) {
+        if (PAIR) tmem_alloc_pair(tmem_ptr, kTmemCols); else tmem_alloc(tmem_ptr, kTmemCols);
+    }
     tc_fence_before();
     __syncthreads();
-    cluster_sync();
+    if (PAIR) cluster_sync();
     tc_fence_after();
     const uint32_t tmem_base = *tmem_ptr;
     auto give_up = [&](int site) {
-        raise_abort(abort_flag, 2);
+        raise_abort(abort_flag, kCtas);
         if (P.status) atomicCAS(P.status, 0, (4 << 16) | site);
     };
     // Operands that the high parts hold exactly (16-bit inputs, small integers) have no low parts: their tiles are neither
@@ -385,12 +392,12 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
             uint32_t s = 0, use = 0, issued = 0;     // slot, how often it has been filled before
             bool ok = true;
             const int kchunk = (P.kchunk > 0 && P.kchunk < nkb) ? P.kchunk : nkb;
-            ProductShare<Index> share(P, (nkb + kchunk - 1) / kchunk);
+            ProductShare<Index> share(P, (nkb + kchunk - 1) / kchunk, kCtas);
             Index tile;
             for (int c0, c1; ok && share.next(tile, c0, c1);) {
                 long long tn, tm, b;
                 decode_tile<TOPK != 0>(tile, P, tn, tm, b);
-                const int row = (int)(tm * TM) + (ROWMIN && rank_1_is_idle(tm, P) ? 0 : (int)rank * BM), col = (int)(tn * BN) + (int)rank * HN;
+                const int row = (int)(tm * kTileRows) + (ROWMIN && rank_1_is_idle(tm, P) ? 0 : (int)rank * BM), col = (int)(tn * BN) + (int)rank * HN;
                 const int kend = c1 * kchunk < nkb ? c1 * kchunk : nkb;
                 for (int kb = c0 * kchunk; kb < kend && ok; ++kb) {
                     for (int part = 0; part < parts; ++part) {
@@ -400,9 +407,9 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                             break;
                         }
                         unsigned char *st = smem + s * SLOT_BYTES;
-                        const uint32_t bar = cluster_addr(&full[s], 0);
+                        const uint32_t bar = PAIR ? cluster_addr(&full[s], 0) : 0;
                         const bool load_x = part == 0 || need_xl, load_y = part == 0 || need_yl;
-                        if (rank == 0) mbar_expect_tx(&full[s], 2 * ((load_x ? A_BYTES : 0) + (load_y ? B_BYTES : 0)));
+                        if (rank == 0) mbar_expect_tx(&full[s], kCtas * ((load_x ? A_BYTES : 0) + (load_y ? B_BYTES : 0)));
                         static_assert(TF32 || !AMN, "MN-major staging is laid out for 32-bit operands");
                         if (load_x) {
                             const CUtensorMap *map = part == 0 ? &map_xh : &map_xl;
@@ -410,29 +417,35 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
 #pragma unroll
                                 for (int m = 0; m < BM / 32; ++m) tma_load_3d_pair(st + m * 4096, map, bar, row + 32 * m, kb * BKE, (int)b);
                             } else {
-                                tma_load_3d_pair(st, map, bar, kb * BKE, row, (int)b);
+                                if constexpr (PAIR) tma_load_3d_pair(st, map, bar, kb * BKE, row, (int)b);
+                                else tma_load_3d(st, map, &full[s], kb * BKE, row, (int)b);
                             }
                         }
-                        if (load_y) tma_load_3d_pair(st + A_BYTES, part == 0 ? &map_yh : &map_yl, bar, kb * BKE, col, (int)b);
+                        if (load_y) {
+                            const CUtensorMap *map = part == 0 ? &map_yh : &map_yl;
+                            if constexpr (PAIR) tma_load_3d_pair(st + A_BYTES, map, bar, kb * BKE, col, (int)b);
+                            else tma_load_3d(st + A_BYTES, map, &full[s], kb * BKE, col, (int)b);
+                        }
                         ++issued;
                         if (++s == kSlots) { s = 0; ++use; }
                     }
                 }
             }
             if (ok && !wait_for_releases(empty, issued, kSlots, abort_flag)) give_up(7);
-            publish(&counts->issued[rank], issued, 2);
+            publish(&counts->issued[rank], issued, kCtas);
+            if (!PAIR) publish(&counts->issued[1], issued, 1);
         }
     } else if (warp == 1) {
         // ---------------- MMA issuer: rank 0, for both CTAs ----------------
         if (lane == 0 && rank == 0) {
-            const uint32_t idesc = make_idesc(TM, BN, TF32, AMN);
+            const uint32_t idesc = make_idesc(kTileRows, BN, TF32, AMN);
             uint32_t s = 0, phase = 0, acount = 0, used = 0;
             bool ok = true;
             const int kchunk = (P.kchunk > 0 && P.kchunk < nkb) ? P.kchunk : nkb;
-            ProductShare<Index> share(P, (nkb + kchunk - 1) / kchunk);
+            ProductShare<Index> share(P, (nkb + kchunk - 1) / kchunk, kCtas);
             Index tile;
             auto arrived = [&](int site) {
-                if (!wait_or_abort<true>(&full[s], phase, abort_flag)) {
+                if (!wait_or_abort<PAIR>(&full[s], phase, abort_flag)) {
                     give_up(site);
                     return false;
                 }
@@ -450,7 +463,7 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                 const int kend = c1 * kchunk < nkb ? c1 * kchunk : nkb;
                 for (int kb0 = c0 * kchunk; kb0 < kend && ok; kb0 += kchunk, ++acount) {
                     const uint32_t a = acount & 1, ause = acount >> 1;
-                    if (ause > 0 && !wait_or_abort<true>(&tmem_empty[a], (ause - 1) & 1, abort_flag)) {
+                    if (ause > 0 && !wait_or_abort<PAIR>(&tmem_empty[a], (ause - 1) & 1, abort_flag)) {
                         give_up(2);
                         ok = false;
                         break;
@@ -470,15 +483,15 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                         constexpr uint64_t ka = AMN ? 64 : 2, kbn = 2;
 #pragma unroll
                         for (int k = 0; k < kMmasPerStep; ++k)
-                            tc_mma<TF32>(d_tmem, dxh + ka * k, dyh + kbn * k, idesc, ((kb - kb0) | k) != 0);
+                            tc_mma<TF32, PAIR>(d_tmem, dxh + ka * k, dyh + kbn * k, idesc, ((kb - kb0) | k) != 0);
                         if (++s == kSlots) { s = 0; phase ^= 1; }
                         if (parts == 1) {
-                            tc_commit_pair(&empty[hi]);
+                            tc_commit<PAIR>(&empty[hi]);
                             ++used;
                             continue;
                         }
                         if (!arrived(5)) {
-                            tc_commit_pair(&empty[hi]);   // for drain_pair: the MMAs above are under way
+                            tc_commit<PAIR>(&empty[hi]);   // for drain_pair: the MMAs above are under way
                             ++used;
                             ok = false;
                             break;
@@ -488,36 +501,38 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                         if (need_xl && need_yl) {
 #pragma unroll
                             for (int k = 0; k < kMmasPerStep; ++k) {
-                                tc_mma<TF32>(d_tmem, dxh + ka * k, dyl + kbn * k, idesc, 1);
-                                tc_mma<TF32>(d_tmem, dxl + ka * k, dyh + kbn * k, idesc, 1);
+                                tc_mma<TF32, PAIR>(d_tmem, dxh + ka * k, dyl + kbn * k, idesc, 1);
+                                tc_mma<TF32, PAIR>(d_tmem, dxl + ka * k, dyh + kbn * k, idesc, 1);
                             }
                         } else {
                             const uint64_t da = need_xl ? dxl : dxh, db = need_xl ? dyh : dyl;
 #pragma unroll
-                            for (int k = 0; k < kMmasPerStep; ++k) tc_mma<TF32>(d_tmem, da + ka * k, db + kbn * k, idesc, 1);
+                            for (int k = 0; k < kMmasPerStep; ++k) tc_mma<TF32, PAIR>(d_tmem, da + ka * k, db + kbn * k, idesc, 1);
                         }
-                        tc_commit_pair(&empty[hi]); // both slots may be refilled, in both CTAs, once these MMAs have read them
-                        tc_commit_pair(&empty[lo]);
+                        tc_commit<PAIR>(&empty[hi]); // both slots may be refilled, in both CTAs, once these MMAs have read them
+                        tc_commit<PAIR>(&empty[lo]);
                         used += 2;
                         if (++s == kSlots) { s = 0; phase ^= 1; }
                     }
                     if (!ok) break;      // acount: accumulators handed over
-                    tc_commit_pair(&tmem_full[a]);
+                    tc_commit<PAIR>(&tmem_full[a]);
                 }
             }
-            publish(&counts->used, used, 2);
-            publish(&counts->filled, acount, 2);
+            publish(&counts->used, used, kCtas);
+            publish(&counts->filled, acount, kCtas);
         }
     } else {
         // ---------------- epilogue: warps 2..17, TMEM lanes 32*(warp % 4) .. +31 ----------------
         const int q = warp & 3;
-        const uint32_t drained[2] = {cluster_addr(&tmem_empty[0], 0), cluster_addr(&tmem_empty[1], 0)};
+        const uint32_t drained[2] = {PAIR ? cluster_addr(&tmem_empty[0], 0) : 0, PAIR ? cluster_addr(&tmem_empty[1], 0) : 0};
         uint32_t tcount = 0;
         bool ok = true;
         auto release = [&](uint32_t a) {   // this warp has drained its part of accumulator a
             tc_fence_before();
             __syncwarp();
-            if (lane == 0) mbar_arrive_cluster(drained[a]);
+            if (lane == 0) {
+                if (PAIR) mbar_arrive_cluster(drained[a]); else mbar_arrive(&tmem_empty[a]);
+            }
         };
         auto ready = [&](uint32_t a, uint32_t parity, int site) {
             const bool here = wait_or_abort(&tmem_full[a], parity, abort_flag);
@@ -525,10 +540,33 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
             tc_fence_after();
             return here;
         };
-        const long long pairs = gridDim.x >> 1;
+        const long long pairs = gridDim.x / kCtas;
+        // A pair's warps meet at the barriers of the stores: all four of a lane quarter go on, or none.  A CTA's own: the warp by itself.
+        auto together = [&](bool here) { return PAIR ? quarter_all(q, here) : __all_sync(0xffffffffu, here) != 0; };
+        // a CTA by itself: 32 staged columns of this warp, from column `first` of the tile on, to the result
+        auto store_block = [&](const float *block, float *dst, long long pitch, int first, int rows, int cols) {
+            __syncwarp();
+            if (P.vec_store && first + 32 <= cols) {
+                const int cc = lane & 7;
+#pragma unroll
+                for (int it = 0; it < 8; ++it) {
+                    const int row = it * 4 + (lane >> 3);
+                    const float4 v = *reinterpret_cast<const float4 *>(block + row * 32 + ((cc ^ (row & 7)) << 2));
+                    if (row < rows) reinterpret_cast<float4 *>(dst + row * pitch + first)[cc] = v;
+                }
+            } else if (first + lane < cols) {
+                const int n = rows < 32 ? rows : 32;
+                float *p = dst + first + lane;
+#pragma unroll 8
+                for (int row = 0; row < n; ++row) p[row * pitch] = block[row * 32 + (((lane >> 2) ^ (row & 7)) << 2) + (lane & 3)];
+            }
+            __syncwarp();
+        };
         if constexpr (STORED) {
-            const int cq = (warp - 2) >> 2;              // which 16 of every 64 columns
-            float *stage = reinterpret_cast<float *>(smem + OFF_STAGE + q * 2 * kStoreBuffer);
+            // which 16 of every 64 columns; a CTA by itself: which kCols
+            const int cq = (warp - 2) >> 2;
+            constexpr int kCols = 4 * BN / L::kWarps, kFirst = PAIR ? 16 : kCols, kStep = PAIR ? kStoreCols : 16;
+            float *stage = reinterpret_cast<float *>(smem + L::OFF_STAGE + (PAIR ? q * 2 * kStoreBuffer : (warp - 2) * 4096));
             const uint32_t acc = tmem_base + ((uint32_t)(q * 32) << 16);
             if constexpr (TF32) {
                 // Chunked reduction (plain products only): every chunk's accumulator is added, rounded to
@@ -537,7 +575,7 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                 const int kchunk = (P.kchunk > 0 && P.kchunk < nkb) ? P.kchunk : nkb;
                 const int nchunks = (nkb + kchunk - 1) / kchunk;
                 uint32_t acount = 0;
-                ProductShare<Index> share(P, nchunks);
+                ProductShare<Index> share(P, nchunks, kCtas);
                 const int start = share.at;
                 Index tile;
                 for (int c0, c1; ok && share.next(tile, c0, c1);) {
@@ -545,9 +583,9 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                     const long long tn = t % P.tiles_n; t /= P.tiles_n;
                     const long long tm = t % P.tiles_m;
                     const long long b = t / P.tiles_m;
-                    float sums[BN / kStoreCols][16];
+                    float sums[kCols / 16][16];
 #pragma unroll
-                    for (int p = 0; p < BN / kStoreCols; ++p)
+                    for (int p = 0; p < kCols / 16; ++p)
 #pragma unroll
                         for (int v = 0; v < 16; ++v) sums[p][v] = 0.f;
                     for (int ch = c0; ch < c1; ++ch, ++acount) {
@@ -555,10 +593,10 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                         ok = ready(a, (acount >> 1) & 1, 6);
                         if (!ok) break;
 #pragma unroll
-                        for (int p = 0; p < BN / kStoreCols; p += 2) {   // two loads under way: 64 sums leave few registers
+                        for (int p = 0; p < kCols / 16; p += 2) {   // two loads under way: the sums leave few registers
                             uint32_t r0[16], r1[16];
-                            tmem_ld16(acc + a * BN + p * kStoreCols + cq * 16, r0);
-                            tmem_ld16(acc + a * BN + (p + 1) * kStoreCols + cq * 16, r1);
+                            tmem_ld16(acc + a * BN + p * kStep + cq * kFirst, r0);
+                            tmem_ld16(acc + a * BN + (p + 1) * kStep + cq * kFirst, r1);
                             tmem_ld_wait();
 #pragma unroll
                             for (int v = 0; v < 16; ++v) sums[p][v] += __uint_as_float(r0[v]);
@@ -567,10 +605,20 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                         }
                         release(a);
                     }
-                    // all four warps of the lane quarter go on, or none: they meet at the barriers of the stores
-                    ok = quarter_all(q, ok);
+                    ok = together(ok);
                     if (!ok) break;
-                    const long long row_base = tm * TM + rank * BM + q * 32;
+                    const long long row_base = tm * kTileRows + rank * BM + q * 32;
+                    if constexpr (!PAIR) {
+                        const int rows = row_base < P.N1 ? (int)(P.N1 - row_base < 32 ? P.N1 - row_base : 32) : 0;
+                        const int cols = P.N2 - tn * BN < BN ? (int)(P.N2 - tn * BN) : BN;
+#pragma unroll
+                        for (int p = 0; p < kCols / 16; p += 2) {
+                            stage_values<32>(stage, sums[p], 0, lane);
+                            stage_values<32>(stage, sums[p + 1], 16, lane);
+                            store_block(stage, P.out + (b * P.N1 + row_base) * P.N2 + tn * BN, P.N2, cq * kCols + p * 16, rows, cols);
+                        }
+                        continue;
+                    }
                     const bool part = c1 - c0 < nchunks;
                     // a share holds at most two parts of tiles, one at its start and one at its end
                     const long long slot = (long long)(blockIdx.x >> 1) * 2 + ((tile - share.base) * nchunks + c0 == start ? 0 : 1);
@@ -589,15 +637,14 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                     }
                 }
             } else {
-                for (long long tile = blockIdx.x >> 1; tile < P.tiles; tile += pairs, ++tcount) {
+                for (long long tile = blockIdx.x / kCtas; tile < P.tiles; tile += pairs, ++tcount) {
                     long long tn, tm, b;
                     decode_tile<false>(tile, P, tn, tm, b);
                     const uint32_t a = tcount & 1;
                     // the row's norm depends on the tile index alone: fetched before the wait
-                    const long long row_base = tm * TM + rank * BM + q * 32, i = row_base + lane;
+                    const long long row_base = tm * kTileRows + rank * BM + q * 32, i = row_base + lane;
                     const float n1 = (EPI != TPW_DOT_LINEAR && i < P.N1) ? P.n1sq[b * P.N1 + i] : 0.f;
-                    // all four warps of the lane quarter go on, or none: they meet at the barriers of the stores
-                    if (!quarter_all(q, ready(a, (tcount >> 1) & 1, 4))) break;
+                    if (!together(ready(a, (tcount >> 1) & 1, 4))) break;
                     const int rows = row_base < P.N1 ? (int)(P.N1 - row_base < 32 ? P.N1 - row_base : 32) : 0;
                     const int cols = P.N2 - tn * BN < BN ? (int)(P.N2 - tn * BN) : BN, passes = (cols + kStoreCols - 1) / kStoreCols;
                     const float *n2p = P.n2sq + b * P.N2 + tn * BN;
@@ -632,7 +679,15 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                             }
                         }
                     };
-                    if (P.vec_store) {
+                    if constexpr (!PAIR) {
+#pragma unroll 1
+                        for (int c = 0; c < kCols / 16; ++c) {
+                            float o[16];
+                            columns(cq * kCols + c * 16, c + 1 == kCols / 16, o);
+                            stage_values<32>(stage, o, (c & 1) * 16, lane);
+                            if (c & 1) store_block(stage, out, P.N2, cq * kCols + (c - 1) * 16, rows, cols);
+                        }
+                    } else if (P.vec_store) {
 #pragma unroll 1
                         for (int p = 0; p < passes; ++p) {
                             float o[16];
@@ -708,8 +763,8 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                     // columns 1.07 -> 0.95 ms; without any candidates it takes 0.45.)
                     const int k = P.topk_k;
                     const long long cols = TOPK < 0 ? P.cols : P.N2;
-                    unsigned long long *buf = reinterpret_cast<unsigned long long *>(smem + OFF_STAGE + (warp - 2) * 4096) + lane;   // [16][32 lanes]
-                    float *norms = reinterpret_cast<float *>(smem + OFF_STAGE + (warp - 2) * 4096);                                  // TOPK < 0: [128]
+                    unsigned long long *buf = reinterpret_cast<unsigned long long *>(smem + L::OFF_STAGE + (warp - 2) * 4096) + lane;   // [16][32 lanes]
+                    float *norms = reinterpret_cast<float *>(smem + L::OFF_STAGE + (warp - 2) * 4096);                                  // TOPK < 0: [128]
                     int cnt = 0;                                  // keys held
                     // keys have to stay below the bound of the row's k-th smallest; any value read while other tiles lower it is one
                     unsigned long long limit = 0;
@@ -850,7 +905,7 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
 
     tc_fence_before();
     __syncthreads();
-    cluster_sync();   // neither CTA's shared memory goes while the other may still read it or arrive in it
+    if (PAIR) cluster_sync();   // neither CTA's shared memory goes while the other may still read it or arrive in it
     if (*reinterpret_cast<volatile int *>(abort_flag)) {   // raised in both CTAs or in neither
         if (threadIdx.x == 0)
             drain_pair(full, empty, tmem_full, kSlots, counts, rank, [&](uint32_t u) {
@@ -858,11 +913,11 @@ gemm_metric_kernel(const __grid_constant__ CUtensorMap map_xh, const __grid_cons
                 return (uint32_t)((high || need_xl ? A_BYTES : 0) + (high || need_yl ? B_BYTES : 0));
             });
         __syncthreads();
-        cluster_sync();
+        if (PAIR) cluster_sync();
     }
     if (warp == 1) {
         tc_fence_after();
-        tmem_dealloc_pair(tmem_base, kTmemCols);
+        if (PAIR) tmem_dealloc_pair(tmem_base, kTmemCols); else tmem_dealloc(tmem_base, kTmemCols);
     }
 }
 
@@ -993,6 +1048,20 @@ inline long long align_up(long long v, long long a) { return (v + a - 1) / a * a
 // large fp32 problems; everything else stays on the exact fp32/fp64 CUDA-core tile.
 inline bool auto_picks_tensor_cores(int dtype, long long B, long long N1, long long N2, long long D) {
     return dtype == TPW_F32 && D >= 64 && N1 >= 128 && N2 >= 256 && (double)B * N1 * N2 * D >= (double)(1ll << 28);
+}
+
+// Stored bf16 tiles: whether a CTA works by itself, on 128 x 256, instead of in a pair.  A pair saves operand copies but couples its 32 epilogue
+// warps, at the stores' barriers and at the accumulators; with few features the results are the bound.  Times of pairs and of single
+// CTAs over tiles of 128 x 256 with eight epilogue warps and word-wise ragged stores, sqeuclidean (euclidean) of [131072, 16384, D],
+// [30011, 10008, D] and [8000, 4000, D]:
+//   64 features   1.0 to 1.16 (0.6 to 0.7) and 0.71 to 0.81 (0.45 to 0.51);   128  0.92 to 1.05 (0.61 to 0.66) and 0.79 to 0.87 (0.51 to 0.54)
+//   160           1.02 (0.67 to 0.72) and 0.98 to 1.0 (0.63 to 0.67);   256  0.93 to 0.99 (0.7 to 0.78) and 1.01 to 1.1 (0.7 to 0.83)
+// and where rows of the result start on no 16-byte boundary, [30011, 10007, D] and [8000, 4001, D]:
+//   64            1.05 to 1.06 (0.75 to 0.78) and 1.11 to 1.22 (0.71 to 0.73), results within L2 0.96 (0.61): of larger ones two warps' stores
+//                 complete a sector only after it has left L2, the more the faster they follow each other;   96  1.03 and 1.03
+//   128 to 256    0.98 to 1.04 (0.75 to 0.79) and 0.88 to 0.97 (0.6 to 0.67);   500  0.86 and 1.14
+inline bool single_pays(bool aligned, double bytes, long long D) {
+    return aligned ? D <= 160 : D <= 256 && (D >= 96 || bytes <= 134217728.0);
 }
 
 struct ScratchLayout {
@@ -1331,7 +1400,8 @@ struct Tf32Operand {
 // `pitch` >= K elements per row (zero beyond K), an MN-major operand has exactly K rows per batch.
 // lo_any (may be NULL): lo_any[1] says whether Bm has any low part; A's are always used.
 // partial (may be NULL): kPartialBytes per pair of SMs, for products that deal out chunks instead of whole tiles.
-int launch_tf32_product(const Tf32Operand &A, const Tf32Operand &Bm, float *out, const int *lo_any, float *partial,
+// single: tiles of a CTA by itself instead of pairs' (A K-major, no partial tiles).
+int launch_tf32_product(const Tf32Operand &A, const Tf32Operand &Bm, float *out, const int *lo_any, float *partial, bool single,
                         long long B, long long M, long long N, long long K, cudaStream_t s) {
     CUtensorMap mah, mal, mbh, mbl;
     int st;
@@ -1341,13 +1411,13 @@ int launch_tf32_product(const Tf32Operand &A, const Tf32Operand &Bm, float *out,
     };
     if ((st = encode(&mah, A.hi, A, M, BM)) != TPW_OK) return st;
     if ((st = encode(&mal, A.lo, A, M, BM)) != TPW_OK) return st;
-    if ((st = encode(&mbh, Bm.hi, Bm, N, HN)) != TPW_OK) return st;
-    if ((st = encode(&mbl, Bm.lo, Bm, N, HN)) != TPW_OK) return st;
+    if ((st = encode(&mbh, Bm.hi, Bm, N, single ? BN : HN)) != TPW_OK) return st;
+    if ((st = encode(&mbl, Bm.lo, Bm, N, single ? BN : HN)) != TPW_OK) return st;
     GemmParams P;
     memset(&P, 0, sizeof(P));
     P.out = out;
     P.B = B; P.N1 = M; P.N2 = N; P.D = K; // K-major tails beyond K are zero padding or zero fill
-    P.tiles_m = (M + TM - 1) / TM;
+    P.tiles_m = single ? (M + BM - 1) / BM : (M + TM - 1) / TM;
     P.tiles_n = (N + BN - 1) / BN;
     P.tiles = B * P.tiles_m * P.tiles_n;
     P.epilogue = TPW_DOT_LINEAR;
@@ -1359,16 +1429,18 @@ int launch_tf32_product(const Tf32Operand &A, const Tf32Operand &Bm, float *out,
     P.vec_store = (N % 4 == 0 && aligned16(out)) ? 1 : 0;
     P.status = device_status_ptr();
     const long long pairs = product_pairs(B, M, N, K, partial != nullptr);
-    P.partial = partial != nullptr && deals_chunks(B, M, N, K) ? partial : nullptr;
-    const unsigned grid = 2 * (unsigned)pairs;
-#define TPW_TF32_LAUNCH(AMN)                                                                                              \
+    P.partial = !single && partial != nullptr && deals_chunks(B, M, N, K) ? partial : nullptr;
+    const unsigned grid = single ? (unsigned)(P.tiles < sm_count() ? P.tiles : sm_count()) : 2 * (unsigned)pairs;
+#define TPW_TF32_LAUNCH(AMN, PAIR)                                                                                        \
     do {                                                                                                                  \
-        auto kern = gemm_metric_kernel<TPW_DOT_LINEAR, false, true, false, AMN>;                                          \
-        TPW_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_ALLOC));                 \
-        kern<<<grid, kThreads, SMEM_ALLOC, s>>>(mah, mal, mbh, mbl, P);                                                   \
+        auto kern = gemm_metric_kernel<TPW_DOT_LINEAR, false, true, false, AMN, 0, PAIR>;                                 \
+        typedef Ring<PAIR, true> L;                                                                                       \
+        TPW_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, L::SMEM_ALLOC));              \
+        kern<<<grid, L::kThreads, L::SMEM_ALLOC, s>>>(mah, mal, mbh, mbl, P);                                             \
     } while (0)
-    if (A.mn) TPW_TF32_LAUNCH(true);
-    else TPW_TF32_LAUNCH(false);
+    if (single) TPW_TF32_LAUNCH(false, false);
+    else if (A.mn) TPW_TF32_LAUNCH(true, true);
+    else TPW_TF32_LAUNCH(false, true);
 #undef TPW_TF32_LAUNCH
     TPW_LAUNCH_OK("gemm_metric_kernel (tf32)");
     if (P.partial && P.tiles % pairs != 0) {
@@ -1529,7 +1601,7 @@ struct Bf16Operands {
 };
 int prepare_bf16_operands(const void *x1, const void *x2, void *scratch, bool reciprocal_norms,
                           long long B, long long N1, long long N2, long long D, cudaStream_t s,
-                          Bf16Operands &M, GemmParams &P) {
+                          Bf16Operands &M, GemmParams &P, bool pairs = true) {
     const ScratchLayout L = scratch_layout(B, N1, N2, D, false);
     unsigned char *base = static_cast<unsigned char *>(scratch);
     __nv_bfloat16 *xh = reinterpret_cast<__nv_bfloat16 *>(base + L.off_xh), *xl = reinterpret_cast<__nv_bfloat16 *>(base + L.off_xl);
@@ -1546,13 +1618,13 @@ int prepare_bf16_operands(const void *x1, const void *x2, void *scratch, bool re
     int st;
     if ((st = make_tensor_map_3d(&M.mxh, xh, 2, L.Dp, N1, B, BK, BM, true)) != TPW_OK) return st;
     if ((st = make_tensor_map_3d(&M.mxl, xl, 2, L.Dp, N1, B, BK, BM, true)) != TPW_OK) return st;
-    if ((st = make_tensor_map_3d(&M.myh, yh, 2, L.Dp, N2, B, BK, HN, true)) != TPW_OK) return st;
-    if ((st = make_tensor_map_3d(&M.myl, yl, 2, L.Dp, N2, B, BK, HN, true)) != TPW_OK) return st;
+    if ((st = make_tensor_map_3d(&M.myh, yh, 2, L.Dp, N2, B, BK, pairs ? HN : BN, true)) != TPW_OK) return st;
+    if ((st = make_tensor_map_3d(&M.myl, yl, 2, L.Dp, N2, B, BK, pairs ? HN : BN, true)) != TPW_OK) return st;
     memset(&P, 0, sizeof(P));
     P.n1sq = n1; P.n2sq = n2;
     P.lo_any = lo_any;
     P.B = B; P.N1 = N1; P.N2 = N2; P.D = L.Dp;
-    P.tiles_m = (N1 + TM - 1) / TM;
+    P.tiles_m = pairs ? (N1 + TM - 1) / TM : (N1 + BM - 1) / BM;
     P.tiles_n = (N2 + BN - 1) / BN;
     P.tiles = B * P.tiles_m * P.tiles_n;
     P.status = device_status_ptr();
@@ -1741,7 +1813,10 @@ extern "C" int tpw_dot_metric_forward_ws(int dtype, int epilogue, int engine,
             X.vec_in = (D % 4 == 0 && aligned16(X.a)) ? 1 : 0;
             if ((st = launch_split<COEF_ID, false>(X, B, s)) != TPW_OK) return st;
         }
-        return launch_tf32_product(Tf32Operand{xhi, xlo, Dp, false}, Tf32Operand{yhi, ylo, Dp, false}, static_cast<float *>(out), nullptr, nullptr, B, N1, N2, Dp, s);
+        // Over pairs', plain products of [131072, 16384, D], [30011, 10007 or 10008, D] and [8000, 4000 or 4001, D]: 64 to 128 features 0.64 to
+        // 0.98, 256 0.76 to 0.98, 384 0.83 to 1.01, 500 0.98 to 1.13 as the operands become the bound.
+        const bool single = D <= 384;
+        return launch_tf32_product(Tf32Operand{xhi, xlo, Dp, false}, Tf32Operand{yhi, ylo, Dp, false}, static_cast<float *>(out), nullptr, nullptr, single, B, N1, N2, Dp, s);
     }
     if (engine == TPW_ENGINE_AUTO && auto_picks_tensor_cores(dtype, B, N1, N2, D) && scratch != nullptr &&
         scratch_bytes >= scratch_layout(B, N1, N2, D, false).total)
@@ -1769,19 +1844,24 @@ extern "C" int tpw_dot_metric_forward_ws(int dtype, int epilogue, int engine,
     Bf16Operands M;
     GemmParams P;
     int st;
-    if ((st = prepare_bf16_operands(x1, x2, scratch, recip, B, N1, N2, D, s, M, P)) != TPW_OK) return st;
+    const bool single = single_pays(N2 % 4 == 0 && aligned16(out), 4.0 * B * N1 * N2, D);
+    if ((st = prepare_bf16_operands(x1, x2, scratch, recip, B, N1, N2, D, s, M, P, !single)) != TPW_OK) return st;
     P.out = static_cast<float *>(out);
     P.epilogue = epilogue;
     P.self = self ? 1 : 0;
     P.vec_store = (N2 % 4 == 0 && aligned16(out)) ? 1 : 0;
     TPW_CHECK_ARG(P.tiles < (1ll << 40), "tpw_dot_metric_forward_ws: too many tiles");
-    const long long pairs = pair_count();
-    const unsigned grid = 2 * (unsigned)(P.tiles < pairs ? P.tiles : pairs);
+    const long long ctas = single ? 1 : 2, most = sm_count() / ctas;
+    const unsigned grid = (unsigned)(ctas * (P.tiles < most ? P.tiles : most));
+#define TPW_GEMM_LAUNCH_FORM(EPI, SELF, PAIR)                                                                             \
+    do {                                                                                                                  \
+        auto kern = gemm_metric_kernel<EPI, SELF, false, false, false, 0, PAIR>;                                          \
+        TPW_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, Ring<PAIR>::SMEM_ALLOC));     \
+        kern<<<grid, Ring<PAIR>::kThreads, Ring<PAIR>::SMEM_ALLOC, s>>>(M.mxh, M.mxl, M.myh, M.myl, P);                     \
+    } while (0)
 #define TPW_GEMM_LAUNCH(EPI, SELF)                                                                                        \
     do {                                                                                                                  \
-        auto kern = gemm_metric_kernel<EPI, SELF, false>;                                                                        \
-        TPW_CUDA_OK(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_ALLOC));                 \
-        kern<<<grid, kThreads, SMEM_ALLOC, s>>>(M.mxh, M.mxl, M.myh, M.myl, P);                                           \
+        if (single) TPW_GEMM_LAUNCH_FORM(EPI, SELF, false); else TPW_GEMM_LAUNCH_FORM(EPI, SELF, true);                   \
     } while (0)
     switch (epilogue) {
         case TPW_DOT_LINEAR: TPW_GEMM_LAUNCH(TPW_DOT_LINEAR, false); break;
@@ -1796,6 +1876,7 @@ extern "C" int tpw_dot_metric_forward_ws(int dtype, int epilogue, int engine,
             break;
     }
 #undef TPW_GEMM_LAUNCH
+#undef TPW_GEMM_LAUNCH_FORM
     TPW_LAUNCH_OK("gemm_metric_kernel");
     return TPW_OK;
 }
@@ -1884,8 +1965,8 @@ static int dense_backward_tensor(int coef, int epilogue, bool sums, float s_mm, 
         void *gout = side == 0 ? grad_x1 : grad_x2;
         if (!gout) continue;
         const Tf32Operand Xk{T[at].hi, T[at].lo, T[at].Rp, false};
-        if (side == 0) st = launch_tf32_product(Ck, Xk, static_cast<float *>(gout), lo_any, partial, B, N1, D, N2, s);
-        else st = launch_tf32_product(Cmn, Xk, static_cast<float *>(gout), lo_any + 2, partial, B, N2, D, N1, s);
+        if (side == 0) st = launch_tf32_product(Ck, Xk, static_cast<float *>(gout), lo_any, partial, false, B, N1, D, N2, s);
+        else st = launch_tf32_product(Cmn, Xk, static_cast<float *>(gout), lo_any + 2, partial, false, B, N2, D, N1, s);
         if (st != TPW_OK) return st;
         if (coef == COEF_COSINE) {
             // the norm part of the chain: g[r,:] += term[r] * x[r,:] / norm[r]
