@@ -163,3 +163,32 @@ def test_contractions_of_one_cta_and_of_pairs(tensor_cores, lead, n1, n2, d):
     if not lead:
         own = tensor_cores.sqeuclidean_distances(x1, x1)
         assert bool((own.diagonal() == 0).all()) and bool(((own - (na ** 2 + na.T ** 2 - 2 * a @ a.T)).abs() <= 2 ** -14 * na * na.T + (d + 8) * 2 ** -24 * (na ** 2 + na.T ** 2)).all())
+
+
+# At least 148 blocks of 32 rows by 32 features, one to each SM, but fewer than 49 gradient blocks of 64 x 64 (float64) or 128 x 128.
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("shape", [(1, 1500, 1480, 128), (3, 480, 500, 100), (1, 3000, 70, 60), (2, 33, 750, 128)])
+def test_walk_of_four_rows_to_a_thread_equals_the_tile_kernel(tpw, monkeypatch, dtype, shape):
+    """Both gradients of a call, and either alone, are the tile kernel's bit for bit."""
+    from torchpairwise_b200 import _abi
+    lib, (b, n1, n2, d) = _abi.lib, shape
+    g = torch.Generator().manual_seed(n1 + n2)
+    x1, x2 = torch.randn(b, n1, d, generator=g).to(dtype).cuda(), torch.randn(b, n2, d, generator=g).to(dtype).cuda()
+    up, aux = torch.randn(b, n1, n2, generator=g).to(dtype).cuda(), (torch.rand(b, n1, n2, generator=g) + 0.5).to(dtype).cuda()
+    w = torch.rand(b, d, generator=g).to(dtype).cuda()
+    aux[:, 3, 5] = 0
+    code = _abi.F32 if dtype == torch.float32 else _abi.F64
+    modes = [(_abi.LP_BWD_CDIST, p) for p in (1.0, 2.0, 3.0, 2.5)] + [(m, p) for m in (_abi.LP_BWD_PPMINKOWSKI, _abi.LP_BWD_WMINKOWSKI) for p in (1.0, 2.0, 3.0, 1.5)]
+    for mode, p in modes + [(_abi.LP_BWD_MATMUL, 2.0)]:
+        def gradients(first, second):
+            g1, g2 = torch.full_like(x1, math.nan), torch.full_like(x2, math.nan)
+            _abi.check(lib.tpw_lp_backward(code, mode, up.data_ptr(), aux.data_ptr(), x1.data_ptr(), x2.data_ptr(),
+                                           w.data_ptr() if mode == _abi.LP_BWD_WMINKOWSKI else None, g1.data_ptr() if first else None,
+                                           g2.data_ptr() if second else None, b, n1, n2, d, p, torch.cuda.current_stream().cuda_stream))
+            return g1, g2
+        got, one, two = gradients(True, True), gradients(True, False)[0], gradients(False, True)[1]
+        monkeypatch.setenv("TPW_DISABLE_SMALL_BWD", "1")
+        want = gradients(True, True)
+        monkeypatch.delenv("TPW_DISABLE_SMALL_BWD")
+        assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]), (mode, p)
+        assert torch.equal(one, want[0]) and torch.equal(two, want[1]), (mode, p)

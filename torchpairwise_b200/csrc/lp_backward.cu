@@ -472,36 +472,31 @@ __global__ void __launch_bounds__(SB_THREADS) lp_backward_rows_kernel(const BwdP
     else rows_walk<T, PHI, NEED_AUX, R, true>(P2, blockIdx.x - first, sm);
 }
 
-// Where the rows kernel is faster than one thread per element.  Each of its walks is a chain of shared loads with a barrier every
-// 32 rows, at twice the elements per thread; it pays where forming a coefficient costs more than that (a division in float64, a power),
-// where the other kernel reads the gradient across its rows (some grad_x2 walks), or where one thread per element runs in more waves
-// than the GPU holds.  Times over one thread per element (of the kernel as it was with the streamed rows read from L2) at 20 to 3000 rows, 9 to 500 features, 1000 streamed rows, for n = rows x
-// features (grad_x1 / grad_x2):
-//   float32  no coefficient  sign 1.3 / 0.4, d 1.5 / 0.7, d|d| 0.85 / 0.85 (n > 2^17.5: 1.0 / 0.8), power 2.1 / 1.4, product 1.1 / 1.2
-//            g / out         0.95 to 1.05 / 0.65, from n = 2^16.5 0.75 / 0.5;   g / out^2  1.3 / 1.4, from 2^17 0.75 / 0.65;
-//            power of out    0.2 to 0.4;   weights  1.2 to 3, d from 2^17 0.85 / 0.7
-//   float64  no coefficient  sign 1.0, d 0.5 / 0.9, d|d| 1.25, power 1.4 to 1.9, product 0.4 / 1.05
-//            any of out      0.3 to 0.95;   weights  1.1 to 1.9, from 2^16.5 0.6 to 0.8 (power never below 1.1)
-//   the maximum's gradient (it compares with the auxiliary value in every term) 1.5 to 3 in both types
-template <typename T, int PHI, bool NEED_AUX, bool TRANS>
+// Where the rows kernel is faster than one thread per element: nearly everywhere.  Times of the rows kernel over those of one thread
+// per element at 20 to 6000 rows, 9 to 1500 features and 300 to 1500 streamed rows, for n = rows x features (grad_x1 / grad_x2):
+//   float32  no coefficient  sign 0.63 to 0.92 (700 x 200: 1.1) / 0.17 to 0.6, d 0.6 to 0.9 / 0.4 to 0.75, d|d| 0.4 to 0.8, product 0.4 to 0.85
+//            g / out         0.4 to 0.75 / 0.25 to 0.5;   g / out^2  0.4 to 0.8 / 0.3 to 0.6;   power of out  0.2 to 0.45
+//            weights         sign, d, d|d| 0.5 to 1.0 / 0.35 to 0.8;   power 0.8 to 1.8 / 0.6 to 1.6, power without coefficient 0.9 to 2.1 / 0.7 to 1.5
+//   float64  no coefficient  sign 0.8, from n = 2^16 1.0 to 1.2 / 0.3 to 0.65, d 0.2 to 0.5 / 0.4 to 0.8, d|d| 0.5 to 0.9, product 0.2 to 0.85
+//            any of out      0.15 to 0.45, power 0.55 to 0.95
+//            weights         d, d|d| 0.4 to 1.0 (n = 2^8: 1.08), sign 1.0 to 1.35, from n = 2^16 0.4 to 0.9;   power 1.05 to 1.9, without coefficient too
+//   below 16 features, where more than half of a warp's lanes have none: float32 1.0 to 1.4 for grad_x1 unless the coefficients cost
+//   much, or with weights; float64 as above
+// (the maximum's gradient compares with the auxiliary value in every term and stays with one thread per element).
+template <int PHI> constexpr bool phi_is_power = PHI == PHI_SGNPOW || PHI == PHI_ABSPOW;
+template <int PHI, bool NEED_AUX>
 constexpr bool rows_may_pay() {
-    if (PHI == PHI_SGN_EQ) return false;
-    if (NEED_AUX) return true;
-    if (sizeof(T) == 4) return PHI == PHI_DABS || (TRANS && (PHI == PHI_SGN || PHI == PHI_D));
-    return PHI == PHI_D || (PHI == PHI_Y && !TRANS);
+    return PHI != PHI_SGN_EQ && (NEED_AUX || !phi_is_power<PHI>);
 }
 template <typename T, int PHI, bool NEED_AUX, bool TRANS>
 bool rows_pay(const BwdParams &P) {
-    if (!rows_may_pay<T, PHI, NEED_AUX, TRANS>() || P.D <= 8) return false;
-    const long long n = P.B * P.NR * P.D, more = 90000, many = 131072;
-    if (!NEED_AUX) return sizeof(T) == 8 || TRANS || n < many;
-    switch (P.coef_mode) {
-        case COEF_DIV_POW: return true;
-        case COEF_DIV_O: return sizeof(T) == 8 || TRANS || n >= more;
-        case COEF_DIV_O2: return sizeof(T) == 8 || n >= many;
-        case COEF_MUL: return sizeof(T) == 8 ? PHI != PHI_SGNPOW && n >= more : PHI == PHI_D && n >= many;
-        default: return false;
-    }
+    if (!rows_may_pay<PHI, NEED_AUX>() || P.D <= 8) return false;
+    const long long n = P.B * P.NR * P.D;
+    const bool weights = NEED_AUX && P.coef_mode == COEF_MUL;
+    if (phi_is_power<PHI>) return !weights;
+    if (sizeof(T) == 4 && P.D < 16) return NEED_AUX ? !weights && TRANS : PHI == PHI_DABS || PHI == PHI_Y || TRANS;
+    if (weights) return sizeof(T) == 4 || n >= (PHI == PHI_SGN ? 65536 : 4096);
+    return !(sizeof(T) == 8 && PHI == PHI_SGN && !TRANS) || n < 65536;
 }
 
 // The gradient block of a CTA of the tile kernel.
@@ -516,11 +511,11 @@ template <typename T>
 bool is_small_backward(const BwdParams &P) {
     typedef typename BwdTile<T>::Smem S;
     const long long tiles = P.B * ((P.NR + S::TR - 1) / S::TR) * ((P.D + S::TK - 1) / S::TK);
-    return tiles * 3 < sm_count() && P.NS <= 65536 && P.B * P.NR * P.D < (1ll << 31) * 256 && !getenv("TPW_DISABLE_SMALL_BWD");
+    return tiles * 3 < sm_count() && P.NS <= 65536 && P.B * P.NR * P.D < (1ll << 31) * 256;
 }
 
 template <typename T, int PHI, bool NEED_AUX, bool TRANS>
-int launch_backward(BwdParams P, cudaStream_t stream) {
+int launch_backward(BwdParams P, bool small, cudaStream_t stream) {
     constexpr int RR = BwdTile<T>::RR, RK = BwdTile<T>::RK, NTHR = BwdTile<T>::NTHR;
     typedef typename BwdTile<T>::Smem S;
     P.tiles_r = (P.NR + S::TR - 1) / S::TR;
@@ -532,7 +527,7 @@ int launch_backward(BwdParams P, cudaStream_t stream) {
                   "lp backward: a dimension exceeds 2^31-1");
     P.status = device_status_ptr();
 
-    if (is_small_backward<T>(P)) {
+    if (small) {
         const long long n = P.B * P.NR * P.D;
         lp_backward_small_kernel<T, PHI, NEED_AUX, TRANS><<<(unsigned)((n + 255) / 256), 256, 0, stream>>>(P);
         TPW_LAUNCH_OK("lp_backward_small_kernel");
@@ -594,22 +589,26 @@ int launch_rows(BwdParams P1, BwdParams P2, bool rows1, bool rows2, cudaStream_t
 template <typename T, int PHI, bool NEED_AUX>
 int launch_both(const BwdParams &base, const void *x1, const void *x2, void *g1, void *g2, cudaStream_t stream) {
     const BwdParams P1 = side_params<false>(base, x1, x2, g1), P2 = side_params<true>(base, x1, x2, g2);
-    bool rows1 = false, rows2 = false;
+    bool small1 = g1 && is_small_backward<T>(P1), small2 = g2 && is_small_backward<T>(P2), rows1 = false, rows2 = false;
+    if ((small1 || small2) && getenv("TPW_DISABLE_SMALL_BWD")) small1 = small2 = false;
     int st;
-    if constexpr (rows_may_pay<T, PHI, NEED_AUX, false>() || rows_may_pay<T, PHI, NEED_AUX, true>()) {
-        rows1 = g1 && is_small_backward<T>(P1) && rows_pay<T, PHI, NEED_AUX, false>(P1);
-        rows2 = g2 && is_small_backward<T>(P2) && rows_pay<T, PHI, NEED_AUX, true>(P2);
+    if constexpr (rows_may_pay<PHI, NEED_AUX>()) {
+        rows1 = small1 && rows_pay<T, PHI, NEED_AUX, false>(P1);
+        rows2 = small2 && rows_pay<T, PHI, NEED_AUX, true>(P2);
         if (rows1 || rows2) {
-            // four rows to a thread halve the reads of the streamed rows, where the GPU still gets a CTA per SM
+            // Four rows to a thread halve the reads of the streamed rows but also the warps: two are faster (1.0 to 1.4 times, 1.98
+            // where a float64 power keeps the arithmetic busy) until there are blocks of four for one and a half times the SMs, then
+            // slower (0.7 to 0.97; float64 power still 1.06).  A plain product, with the least arithmetic per read: from 90 blocks on.
             const long long four = RowsSmem<T, 4>::ROWS, blocks = base.B * ((base.D + 31) / 32) *
                                    ((rows1 ? (P1.NR + four - 1) / four : 0) + (rows2 ? (P2.NR + four - 1) / four : 0));
-            st = blocks >= sm_count() ? launch_rows<T, PHI, NEED_AUX, 4>(P1, P2, rows1, rows2, stream)
-                                      : launch_rows<T, PHI, NEED_AUX, 2>(P1, P2, rows1, rows2, stream);
+            const bool use_four = !(sizeof(T) == 8 && phi_is_power<PHI>) && blocks * 2 >= sm_count() * (PHI == PHI_Y ? 1 : 3);
+            st = use_four ? launch_rows<T, PHI, NEED_AUX, 4>(P1, P2, rows1, rows2, stream)
+                          : launch_rows<T, PHI, NEED_AUX, 2>(P1, P2, rows1, rows2, stream);
             if (st != TPW_OK) return st;
         }
     }
-    if (g1 && !rows1 && (st = launch_backward<T, PHI, NEED_AUX, false>(P1, stream)) != TPW_OK) return st;
-    if (g2 && !rows2 && (st = launch_backward<T, PHI, NEED_AUX, true>(P2, stream)) != TPW_OK) return st;
+    if (g1 && !rows1 && (st = launch_backward<T, PHI, NEED_AUX, false>(P1, small1, stream)) != TPW_OK) return st;
+    if (g2 && !rows2 && (st = launch_backward<T, PHI, NEED_AUX, true>(P2, small2, stream)) != TPW_OK) return st;
     return TPW_OK;
 }
 
