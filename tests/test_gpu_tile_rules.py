@@ -192,3 +192,14 @@ def test_walk_of_four_rows_to_a_thread_equals_the_tile_kernel(tpw, monkeypatch, 
         monkeypatch.delenv("TPW_DISABLE_SMALL_BWD")
         assert torch.equal(got[0], want[0]) and torch.equal(got[1], want[1]), (mode, p)
         assert torch.equal(one, want[0]) and torch.equal(two, want[1]), (mode, p)
+
+
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+def test_widen_takes_more_than_one_turn(tpw, dtype):
+    """More elements than the largest grid has in one turn (16 blocks of 256 threads of 8 to an SM), no multiple of eight."""
+    from torchpairwise_b200 import _abi
+    n = torch.cuda.get_device_properties(0).multi_processor_count * 16 * 2048 + 3 * 2048 + 5
+    x = torch.randn(n, generator=torch.Generator().manual_seed(n)).to(dtype).cuda()
+    out = torch.full((n + 4,), 7.0, device="cuda")
+    _abi.check(_abi.lib.tpw_widen(int(dtype == torch.bfloat16), x.data_ptr(), out.data_ptr(), n, torch.cuda.current_stream().cuda_stream))
+    assert torch.equal(out[:n], x.float()) and bool((out[n:] == 7).all())
