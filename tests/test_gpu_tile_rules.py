@@ -194,6 +194,26 @@ def test_walk_of_four_rows_to_a_thread_equals_the_tile_kernel(tpw, monkeypatch, 
         assert torch.equal(one, want[0]) and torch.equal(two, want[1]), (mode, p)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.float64])
+@pytest.mark.parametrize("shape", [(1, 75, 5, 64), (2, 300, 200, 40), (1, 1500, 1480, 100), (1, 40, 70, 12)])
+def test_jensenshannon_gradients_by_rows_equal_the_tile_kernel(tpw, monkeypatch, dtype, shape):
+    from torchpairwise_b200 import _abi
+    b, n1, n2, d = shape
+    g = torch.Generator().manual_seed(n1)
+    x1, x2 = (torch.rand(b, n, d, generator=g).to(dtype).cuda() for n in (n1, n2))
+    x1[:, 2, 3:7], x2[:, 1, 5] = 0, 0
+    up, out = torch.randn(b, n1, n2, generator=g).to(dtype).cuda(), (torch.rand(b, n1, n2, generator=g) + 0.5).to(dtype).cuda()
+    code, res = _abi.F32 if dtype == torch.float32 else _abi.F64, []
+    for tile in (False, True):
+        if tile:
+            monkeypatch.setenv("TPW_DISABLE_SMALL_BWD", "1")
+        g1, g2 = torch.full_like(x1, math.nan), torch.full_like(x2, math.nan)
+        _abi.check(_abi.lib.tpw_jensenshannon_backward(code, up.data_ptr(), out.data_ptr(), x1.data_ptr(), x2.data_ptr(), g1.data_ptr(), g2.data_ptr(),
+                                                       b, n1, n2, d, 0.5, torch.cuda.current_stream().cuda_stream))
+        res.append((g1, g2))
+    assert torch.equal(res[0][0], res[1][0]) and torch.equal(res[0][1], res[1][1])
+
+
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
 def test_widen_takes_more_than_one_turn(tpw, dtype):
     """More elements than the largest grid has in one turn (16 blocks of 256 threads of 8 to an SM), no multiple of eight."""

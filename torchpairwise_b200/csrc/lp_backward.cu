@@ -482,11 +482,13 @@ __global__ void __launch_bounds__(SB_THREADS) lp_backward_rows_kernel(const BwdP
 //            weights         d, d|d| 0.4 to 1.0 (n = 2^8: 1.08), sign 1.0 to 1.35, from n = 2^16 0.4 to 0.9;   power 1.05 to 1.9, without coefficient too
 //   below 16 features, where more than half of a warp's lanes have none: float32 1.0 to 1.4 for grad_x1 unless the coefficients cost
 //   much, or with weights; float64 as above
-// (the maximum's gradient compares with the auxiliary value in every term and stays with one thread per element).
+//   rooted Jensen-Shannon terms: float32 0.6 to 0.9, float64 0.6 to 1.0
+// The maximum's gradient compares with the auxiliary value in every term and stays with one thread per element; so do the canberra, chi2 and
+// unrooted Jensen-Shannon terms, which form no coefficient (canberra float64 [1500, 1301, 75] 660 us, 782 by rows).
 template <int PHI> constexpr bool phi_is_power = PHI == PHI_SGNPOW || PHI == PHI_ABSPOW;
 template <int PHI, bool NEED_AUX>
 constexpr bool rows_may_pay() {
-    return PHI != PHI_SGN_EQ && (NEED_AUX || !phi_is_power<PHI>);
+    return (PHI <= PHI_Y || PHI == PHI_JS) && (NEED_AUX || !(phi_is_power<PHI> || PHI == PHI_JS));
 }
 template <typename T, int PHI, bool NEED_AUX, bool TRANS>
 bool rows_pay(const BwdParams &P) {
@@ -597,11 +599,11 @@ int launch_both(const BwdParams &base, const void *x1, const void *x2, void *g1,
         rows2 = small2 && rows_pay<T, PHI, NEED_AUX, true>(P2);
         if (rows1 || rows2) {
             // Four rows to a thread halve the reads of the streamed rows but also the warps: two are faster (1.0 to 1.4 times, 1.98
-            // where a float64 power keeps the arithmetic busy) until there are blocks of four for one and a half times the SMs, then
-            // slower (0.7 to 0.97; float64 power still 1.06).  A plain product, with the least arithmetic per read: from 90 blocks on.
+            // where a float64 power or logarithm keeps the arithmetic busy) until there are blocks of four for one and a half times the SMs, then
+            // slower (0.7 to 0.97; float64 power still 1.06).  A plain product, with the least arithmetic per read: from half the SMs on.
             const long long four = RowsSmem<T, 4>::ROWS, blocks = base.B * ((base.D + 31) / 32) *
                                    ((rows1 ? (P1.NR + four - 1) / four : 0) + (rows2 ? (P2.NR + four - 1) / four : 0));
-            const bool use_four = !(sizeof(T) == 8 && phi_is_power<PHI>) && blocks * 2 >= sm_count() * (PHI == PHI_Y ? 1 : 3);
+            const bool use_four = !(sizeof(T) == 8 && (phi_is_power<PHI> || PHI == PHI_JS)) && blocks * 2 >= sm_count() * (PHI == PHI_Y ? 1 : 3);
             st = use_four ? launch_rows<T, PHI, NEED_AUX, 4>(P1, P2, rows1, rows2, stream)
                           : launch_rows<T, PHI, NEED_AUX, 2>(P1, P2, rows1, rows2, stream);
             if (st != TPW_OK) return st;
